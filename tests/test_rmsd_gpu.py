@@ -132,3 +132,44 @@ def test_small_and_degenerate_chains(built, dtype):
     assert np.isfinite(g).all()
     for b in range(10):
         assert np.all(g[b, 3 * na[b]:] == 0.0)
+
+
+def _at_offset(v, off, dtype):
+    """A contiguous CUDA tensor of v whose storage starts `off` elements into an allocation."""
+    t = torch.empty(v.size + off, dtype=dtype, device="cuda")[off:].view(v.shape)
+    t.copy_(torch.tensor(v, dtype=dtype))
+    return t
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float64])
+@pytest.mark.parametrize("B,N,offs", [(40, 41, (0, 0)), (40, 42, (1, 1)), (40, 43, (3, 3)), (40, 41, (0, 1)),
+                                      (320, 61, (0, 0)), (620, 70, (2, 2)), (4, 4099, (0, 0))])
+def test_atom_groups_at_every_alignment_and_block_size(built, dtype, B, N, offs):
+    """Rows that start at every place of a 16-byte block (odd strides, offset storage, the
+    two sets alike or not), counts from 1 atom up around the groups of four, and batches on
+    both sides of each block size of the forward; rmsd, rotation-invariant gradient."""
+    from torchproteinlibrary_gb300.RMSD import Coords2RMSD
+    rng = np.random.default_rng(B + N)
+    na = np.where(np.arange(B) < 24, np.arange(B) + 1, rng.integers(25, N + 1, B)).astype(np.int32)
+    na[-1] = N
+    src = rng.standard_normal((B, 3 * N)) * 10 + 30
+    dst = rng.standard_normal((B, 3 * N)) * 10 - 20
+    x = _at_offset(src, offs[0], dtype).requires_grad_()
+    y = _at_offset(dst, offs[1], dtype)
+    w = torch.rand(B, dtype=dtype, device="cuda", generator=torch.Generator("cuda").manual_seed(1)) + 0.5
+    r = Coords2RMSD()(x, y, torch.tensor(na))
+    g, = torch.autograd.grad(r, x, w)
+    xs, ys = x.detach().double().cpu().numpy(), y.double().cpu().numpy()
+    ref, _, grads = oracle.rmsd(xs, ys, na)
+    # one or two atoms superpose exactly: there rmsd is 0 up to the rounding of the sums
+    tol = 1e-4 if dtype == torch.float32 else 1e-9
+    assert np.abs(r.detach().double().cpu().numpy() - ref)[na > 2].max() <= tol * ref.max()
+    g = g.double().cpu().numpy()
+    for b in range(B):
+        assert not g[b, 3 * na[b]:].any()
+        if na[b] < 8:  # nearly planar sets: the rotation is ill-conditioned
+            continue
+        n = int(na[b])
+        want = float(w[b]) * grads[b, :3 * n]
+        scale = np.abs(want).max()
+        assert np.abs(g[b, :3 * n] - want).max() <= (1e-3 if dtype == torch.float32 else 1e-8) * scale

@@ -7,19 +7,25 @@
 //
 // Here one CTA per chain does everything in one launch: optional centring, the
 // correlation R_ab = sum x_a y_b and R2 = sum |x|^2 + |y|^2 (sums in the coordinate
-// type per thread and per warp, in FP64 across the warps: GB300's FP64 rate is a
-// small fraction of its FP32 rate), the 4x4 matrix T (same layout as the
-// reference), its largest eigenpair by the characteristic-polynomial method on one
-// warp (key_eigen_warp: lane-parallel coefficients, FP32 Newton polished in FP64;
-// for float32 inputs the eigenvector, U and rmsd then in FP32: GB300, 256 chains of
-// about 2300 atoms, 18.6 -> 15.8 us per forward), U from the unit quaternion, UT = U^T and
+// type per thread and per warp, in FP64 across the warps), the 4x4 matrix T (same
+// layout as the reference), its largest eigenpair by the characteristic-polynomial
+// method on one warp (key_eigen_warp), U from the unit quaternion, UT = U^T and
 // rmsd = sqrt((R2 - 2 |lambda_max| + 1e-10) / N).  The backward is one launch with
-// one thread per atom (chains on x, blocks of atoms on y):
+// one thread per group of atoms (chains on x, blocks of groups on y):
 // dL/dx_i = g (x_i - UT y_i) / (rmsd N) on the centred coordinates.
+//
+// What bounds the float32 forward is the FP64 pipe: GB300 issues two FP64 lanes per
+// cycle and SM, conversions included, so an FP64 instruction of any warp holds the pipe
+// for 16 cycles whether one lane or 32 take part.  A form with every warp's partial sums
+// converted and the solve written for one lane spent about 280 of them per chain (ncu:
+// FP64 pipe 73 % busy; 4096 chains of 400..2303 atoms, 20 us of HBM traffic: 90 us per
+// layer call); this one about 100, and reads the coordinates once: 45 us.
 #include <cmath>
+#include <cstring>
 
 #include "tpl_common.cuh"
 #include "tpl_internal.h"
+#include "tpl_rows.cuh"
 
 namespace tpl {
 
@@ -72,12 +78,6 @@ __device__ __forceinline__ double det3(double a, double b, double c, double d, d
     return a * (e * k - f * h) - b * (d * k - f * g) + c * (d * h - e * g);
 }
 
-__device__ __forceinline__ double warp_sum_d(double v) {
-#pragma unroll
-    for (int off = 16; off > 0; off >>= 1) v += __shfl_xor_sync(0xffffffffu, v, off);
-    return v;
-}
-
 // Largest eigenpair of the symmetric 4x4 K by cyclic Jacobi rotations in FP64, on one
 // thread: the fallback of key_eigen_warp for a near-multiple largest root (collinear
 // or otherwise degenerate structures, two-atom chains), where Newton on the quartic
@@ -127,29 +127,24 @@ __device__ __forceinline__ void jacobi_top_eigenpair(const double *K, double *a,
     for (int i = 1; i < 4; i++)
         if (a[5 * i] > a[5 * best]) best = i;
     lam = a[5 * best];
+#pragma unroll
     for (int k = 0; k < 4; k++) q[k] = v[4 * k + best];
 }
 
-// The eigenvector for lam of key_eigen_warp<true>, in FP32: the largest row of the
-// cofactor matrix of K / e0 - (lam / e0) I (entries of order one), one cofactor per
+// The eigenvector of key_eigen_warp<true>, in FP32: the largest row of the cofactor
+// matrix of M = K - l I (entries of order one, in shared memory), one cofactor per
 // lane.  The root itself stays FP64: when the top two eigenvalues nearly meet it is
 // ill-conditioned, and an all-FP32 solve moved it by up to 3e-5 relative (a 2.4e-4
 // gradient error on one of 256 training-step chains), where this form matches the
 // FP64 solve to 1e-5 of the largest gradient.
-__device__ void eigvec_f32(const double *sK, double e0, double l, double (&q)[4]) {
+__device__ void eigvec_f32(const float *sM, double (&q)[4]) {
     const int lane = threadIdx.x & 31;
-    const float ief = e0 > 0.0 ? 1.f / (float)e0 : 0.f, sf = (float)l * ief;
     float cf = 0.f;
     if (lane < 16) {
         const int i = lane >> 2, j = lane & 3;
-        float m[9];
-        int t = 0;
+        float m[9];  // rows but i, columns but j
 #pragma unroll
-        for (int r = 0; r < 4; r++)
-            if (r != i)
-#pragma unroll
-                for (int c = 0; c < 4; c++)
-                    if (c != j) m[t++] = (float)sK[4 * r + c] * ief - (r == c ? sf : 0.f);
+        for (int t = 0; t < 9; t++) m[t] = sM[4 * (t / 3 + (t / 3 >= i)) + t % 3 + (t % 3 >= j)];
         cf = fmaf(m[0], fmaf(m[4], m[8], -m[5] * m[7]),
                   fmaf(-m[1], fmaf(m[3], m[8], -m[5] * m[6]), m[2] * fmaf(m[3], m[7], -m[4] * m[6])));
         if ((i + j) & 1) cf = -cf;
@@ -168,6 +163,7 @@ __device__ void eigvec_f32(const double *sK, double e0, double l, double (&q)[4]
     }
     const bool ok = bn > 1e-30f;
     const float inv = ok ? rsqrtf(bn) : 0.f;
+#pragma unroll
     for (int k = 0; k < 4; k++) q[k] = (double)(__shfl_sync(0xffffffffu, cf, 4 * best + k) * inv);
     if (!ok) {
         q[0] = 1.0;
@@ -175,65 +171,91 @@ __device__ void eigvec_f32(const double *sK, double e0, double l, double (&q)[4]
     }
 }
 
-// Largest eigenpair of the 4x4 key matrix K (symmetric and traceless, row-major in
-// shared memory) by its characteristic polynomial, as in Theobald's
+// Power of two that scales e0 into [0.5, 1), and its inverse (1 for e0 = 0, clamped well
+// inside the exponent range): the key matrix of a scaled correlation has coefficients
+// and eigenvalues of order one, and scaling back is exact.
+__device__ __forceinline__ void unit_scale(double e0, double &scale, double &inv) {
+    int e = ((__double2hiint(e0) >> 20) & 0x7ff) - 1022;
+    e = e0 != 0.0 ? max(-900, min(900, e)) : 0;
+    scale = __hiloint2double((1023 - e) << 20, 0);
+    inv = __hiloint2double((1023 + e) << 20, 0);
+}
+
+// The key matrix entry by entry (row-major, reference layout,
+// coords2rmsd_interface.cpp:146-149): K_e = +-R[a] +- R[b], and +- R[8] on the diagonal.
+constexpr int kKeyA[16] = {0, 5, 6, 1, 5, 0, 1, 2, 6, 1, 0, 5, 1, 2, 5, 0};
+constexpr int kKeyB[16] = {4, 7, 2, 3, 7, 4, 3, 6, 2, 3, 4, 7, 3, 6, 7, 4};
+constexpr unsigned kKeyNegA = 0x8400u, kKeyNegB = 0x913eu, kKeyNegC = 0x0420u;  // entries with a minus sign
+constexpr uint64_t pack_nibbles(const int (&v)[16]) {
+    uint64_t w = 0;
+    for (int i = 0; i < 16; i++) w |= (uint64_t)v[i] << (4 * i);
+    return w;
+}
+__device__ __forceinline__ double negate_if(double v, bool neg) {  // on the sign bit: no FP64 instruction
+    return __hiloint2double(__double2hiint(v) ^ (neg ? 0x80000000 : 0), __double2loint(v));
+}
+
+// Largest eigenpair of the 4x4 key matrix K (symmetric and traceless) of the
+// correlation R by its characteristic polynomial, as in Theobald's
 // quaternion-characteristic-polynomial method (Acta Cryst. A61, 478, 2005):
-// det(K - l I) = l^4 + c2 l^2 + c1 l + c0 with, by Newton's identities for a
-// traceless matrix, c2 = -tr(K^2)/2, c1 = -tr(K^3)/3, c0 = det K.
-//   * tr(K^2), tr(K^3) and det K are spread over the lanes: entry (i, j) of K^2 on
-//     lane 4 i + j, the cofactor expansion of det K along row 0 on lanes 16-19.
-//   * Newton's method from e0 >= l_max (e0 = (sum |x|^2 + |y|^2) / 2) descends
-//     monotonically to the largest root.  It runs in FP32 on s = l / e0, whose
-//     coefficients are of order one, and is then polished by three FP64 Newton
-//     steps whose quotient uses an FP32 reciprocal (each step gains about seven
-//     digits), so that only a handful of FP64 operations remain.
-//   * The eigenvector is the largest row of the cofactor matrix of K - l_max I
-//     (rank one for a simple root), one cofactor per lane.
+// det(K - l I) = l^4 + c2 l^2 + c1 l + c0, c2 = -2 |R|^2, c1 = -8 det R, c0 = det K.
+//   * R (nine doubles, shared memory) and e0 = (sum |x|^2 + |y|^2) / 2 >= l_max come
+//     scaled by unit_scale(), so nothing is divided to bring them to order one.
+//   * FP64 instructions are few: one entry of K per lane (two additions), |R|^2 as a
+//     shuffle sum, the cofactor expansion of det K along row 0 on four lanes.
+//   * Newton's method from e0 descends monotonically to the largest root.  It runs in
+//     FP32 and is then polished by three FP64 Newton steps whose quotient uses an FP32
+//     reciprocal (each step gains about seven digits).
+//   * The eigenvector is the largest row of the cofactor matrix of K - l I (rank one
+//     for a simple root), one cofactor per lane.
 //   * F32_VEC (float32 inputs): the eigenvector in FP32 instead (eigvec_f32).
-// Executed by a full warp; every lane returns lam and the unit q (q = 1, 0, 0, 0
-// when every cofactor vanishes).
+// sK: 16 doubles of scratch, sM: 16 floats, s_jac: 32 doubles.  Executed by a full
+// warp; every lane returns l (scaled) and the unit q (q = 1, 0, 0, 0 when every
+// cofactor vanishes).
 template <bool F32_VEC>
-__device__ void key_eigen_warp(const double *sK, double e0, double &lam, double (&q)[4], double *s_jac) {
-    const int lane = threadIdx.x & 31;
-    double t2 = 0.0, t3 = 0.0, c0 = 0.0;
-    if (lane < 16) {
-        const int i = lane >> 2, j = lane & 3;
-        double k2 = 0.0;  // (K^2)_ij
+__device__ void key_eigen_warp(const double *sR, double e0, double *sK, float *sM, double *s_jac, double &l,
+                               double (&q)[4]) {
+    const int lane = threadIdx.x & 31, e = lane & 15;
+    constexpr uint64_t kA = pack_nibbles(kKeyA), kB = pack_nibbles(kKeyB);
+    const bool diag = (e >> 2) == (e & 3);
+    double k = negate_if(sR[(kA >> (4 * e)) & 15], (kKeyNegA >> e) & 1u) +
+               negate_if(sR[(kB >> (4 * e)) & 15], (kKeyNegB >> e) & 1u);
+    if (diag) k += negate_if(sR[8], (kKeyNegC >> e) & 1u);
+    if (lane < 16) sK[e] = k;
+    double t2 = e < 9 ? sR[e] : 0.0;
+    t2 *= t2;
 #pragma unroll
-        for (int m = 0; m < 4; m++) k2 = fma(sK[4 * i + m], sK[4 * m + j], k2);
-        const double kij = sK[4 * i + j];
-        t2 = kij * kij;
-        t3 = k2 * sK[4 * j + i];
-    } else if (lane < 20) {
-        const int j = lane - 16;
+    for (int off = 8; off > 0; off >>= 1) t2 += __shfl_xor_sync(0xffffffffu, t2, off);
+    const double c2 = -2.0 * t2;
+    const double c1 = -8.0 * det3(sR[0], sR[1], sR[2], sR[3], sR[4], sR[5], sR[6], sR[7], sR[8]);
+    __syncwarp();
+    double c0;
+    {
+        const int j = lane & 3;
         const int ca = j == 0 ? 1 : 0, cb = j <= 1 ? 2 : 1, cc = j <= 2 ? 3 : 2;
-        c0 = sK[j] * det3(sK[4 + ca], sK[4 + cb], sK[4 + cc], sK[8 + ca], sK[8 + cb], sK[8 + cc], sK[12 + ca],
-                          sK[12 + cb], sK[12 + cc]);
-        if (j & 1) c0 = -c0;
+        c0 = negate_if(sK[j], j & 1) * det3(sK[4 + ca], sK[4 + cb], sK[4 + cc], sK[8 + ca], sK[8 + cb], sK[8 + cc],
+                                            sK[12 + ca], sK[12 + cb], sK[12 + cc]);
+        c0 += __shfl_xor_sync(0xffffffffu, c0, 1);
+        c0 += __shfl_xor_sync(0xffffffffu, c0, 2);
     }
-    t2 = warp_sum_d(t2);
-    t3 = warp_sum_d(t3);
-    c0 = warp_sum_d(c0);
-    const double c2 = -0.5 * t2, c1 = t3 * (-1.0 / 3.0);
-    double l = 0.0;
+    l = 0.0;
     if (e0 > 0.0) {
-        const double ie = 1.0 / e0, ie2 = ie * ie;
-        const float ief = (float)ie;
-        const float a2 = (float)(c2 * ie2), a1 = (float)(c1 * ie2 * ie), a0 = (float)(c0 * ie2 * ie2);
-        float s = 1.f;
+        const float e0f = (float)e0, a2 = (float)c2, a1 = (float)c1, a0 = (float)c0;
+        float s = e0f * 1.0000002f;  // not below e0
         for (int it = 0; it < 64; it++) {
             const float P = fmaf(fmaf(fmaf(s, s, a2), s, a1), s, a0);
             const float dP = fmaf(fmaf(4.f * s, s, 2.f * a2), s, a1);
             if (!(dP != 0.f)) break;
             const float d = P / dP;
             s -= d;
-            if (fabsf(d) <= 1e-6f) break;
+            if (fabsf(d) <= 1e-6f * e0f) break;
         }
-        l = (double)s * e0;
-        float corr = INFINITY;  // the last polish step, relative to e0
+        l = (double)s;
+        float corr = INFINITY;  // the last polish step
         for (int it = 0; it < 3; it++) {
-            const double P = fma(fma(fma(l, l, c2), l, c1), l, c0);
-            const double dP = fma(fma(4.0 * l, l, 2.0 * c2), l, c1);
+            const double l2 = l * l;
+            const double P = fma(fma(l2 + c2, l, c1), l, c0);
+            const double dP = fma(fma(4.0, l2, 2.0 * c2), l, c1);
             const float dPf = (float)dP;
             if (!(dPf != 0.f) || !isfinite(dPf)) {
                 corr = INFINITY;
@@ -241,37 +263,38 @@ __device__ void key_eigen_warp(const double *sK, double e0, double &lam, double 
             }
             const double d = P * (double)(1.f / dPf);
             l -= d;
-            corr = (float)d * ief;
+            corr = (float)d;
         }
         // a simple root has converged by the third polish step (each gains about
         // seven digits); a near-multiple one (the top eigenvalues of K nearly or
         // exactly equal) converges only linearly: a last step above 1e-10 of e0 sends
         // the chain to the Jacobi solve (the same decision on every lane)
-        if (!(fabsf(corr) <= 1e-10f)) {
+        if (!(fabsf(corr) <= 1e-10f * e0f)) {
             double lj = 0.0, qj[4] = {1.0, 0.0, 0.0, 0.0};
             if (lane == 0) jacobi_top_eigenpair(sK, s_jac, s_jac + 16, lj, qj);
-            lam = __shfl_sync(0xffffffffu, lj, 0);
-            for (int k = 0; k < 4; k++) q[k] = __shfl_sync(0xffffffffu, qj[k], 0);
+            l = __shfl_sync(0xffffffffu, lj, 0);
+#pragma unroll
+            for (int i = 0; i < 4; i++) q[i] = __shfl_sync(0xffffffffu, qj[i], 0);
             return;
         }
     }
-    lam = l;
     if (F32_VEC) {
-        eigvec_f32(sK, e0, l, q);
+        if (diag) k -= l;
+        if (lane < 16) sM[e] = (float)k;
+        __syncwarp();
+        eigvec_f32(sM, q);
         return;
     }
     // cofactor (i, j) of M = K - l I on lane 4 i + j
     double cof = 0.0;
     if (lane < 16) {
         const int i = lane >> 2, j = lane & 3;
-        double m[9];
-        int t = 0;
+        double m[9];  // rows but i, columns but j
 #pragma unroll
-        for (int r = 0; r < 4; r++)
-            if (r != i)
-#pragma unroll
-                for (int c = 0; c < 4; c++)
-                    if (c != j) m[t++] = sK[4 * r + c] - (r == c ? l : 0.0);
+        for (int t = 0; t < 9; t++) {
+            const int r = t / 3 + (t / 3 >= i), c = t % 3 + (t % 3 >= j);
+            m[t] = sK[4 * r + c] - (r == c ? l : 0.0);
+        }
         cof = det3(m[0], m[1], m[2], m[3], m[4], m[5], m[6], m[7], m[8]);
         if ((i + j) & 1) cof = -cof;
     }
@@ -289,93 +312,202 @@ __device__ void key_eigen_warp(const double *sK, double e0, double &lam, double 
         }
     }
     const double inv = bn > 1e-300 ? 1.0 / sqrt(bn) : 0.0;
-    for (int k = 0; k < 4; k++) q[k] = __shfl_sync(0xffffffffu, cof, 4 * best + k) * inv;
+#pragma unroll
+    for (int i = 0; i < 4; i++) q[i] = __shfl_sync(0xffffffffu, cof, 4 * best + i) * inv;
     if (!(bn > 1e-300)) {
         q[0] = 1.0;
         q[1] = q[2] = q[3] = 0.0;
     }
 }
 
-// The end of the float32 forward on warp 0: the FP64 key-matrix eigen solve (its
-// largest root is ill-conditioned in FP32 when the top two eigenvalues nearly meet),
-// then UT and rmsd in FP32.
-__device__ void rmsd_finish_f32(const RmsdArgs<float> &a, int b, int n, const double *s_out, double *s_K,
-                                const double *s_c, double *s_jac) {
-    const int tid = threadIdx.x;
-    if (tid == 0) {
-        const double *R = s_out;
-        const double F[16] = {R[0] + R[4] + R[8], R[5] - R[7], R[6] - R[2], R[1] - R[3],
-                              R[5] - R[7], R[0] - R[4] - R[8], R[1] + R[3], R[2] + R[6],
-                              R[6] - R[2], R[1] + R[3], -R[0] + R[4] - R[8], R[5] + R[7],
-                              R[1] - R[3], R[2] + R[6], R[5] + R[7], -R[0] - R[4] + R[8]};
-        for (int k = 0; k < 16; k++) s_K[k] = F[k];
-    }
-    __syncwarp();
-    const double r2 = s_out[9];
-    double lam, qd[4];
-    key_eigen_warp<true>(s_K, 0.5 * r2, lam, qd, s_jac);
-    if (tid != 0) return;
-    const float q[4] = {(float)qd[0], (float)qd[1], (float)qd[2], (float)qd[3]};
-    float U[9];
-    U[0] = q[0] * q[0] + q[1] * q[1] - q[2] * q[2] - q[3] * q[3];
-    U[1] = 2.f * (q[1] * q[2] - q[0] * q[3]);
-    U[2] = 2.f * (q[1] * q[3] + q[0] * q[2]);
-    U[3] = 2.f * (q[1] * q[2] + q[0] * q[3]);
-    U[4] = q[0] * q[0] - q[1] * q[1] + q[2] * q[2] - q[3] * q[3];
-    U[5] = 2.f * (q[2] * q[3] - q[0] * q[1]);
-    U[6] = 2.f * (q[1] * q[3] - q[0] * q[2]);
-    U[7] = 2.f * (q[2] * q[3] + q[0] * q[1]);
-    U[8] = q[0] * q[0] - q[1] * q[1] - q[2] * q[2] + q[3] * q[3];
-    float *ut = a.ut + (size_t)9 * b;
-    for (int j = 0; j < 3; j++)
-        for (int k = 0; k < 3; k++) ut[3 * j + k] = U[3 * k + j];
-    const float msd = n > 0 ? (float)(r2 - 2.0 * fabs(lam) + 1e-10) * (1.f / (float)n) : 0.f;
-    a.rmsd[b] = sqrtf(msd > 0.f ? msd : 0.f);
-    if (a.centroids)
-        for (int k = 0; k < 6; k++) a.centroids[6 * b + k] = s_c[k];
+// Rotation of the unit quaternion q, transposed (coords2rmsd_interface.cpp:36-46).
+template <typename T>
+__device__ __forceinline__ void store_ut(T *ut, T q0, T q1, T q2, T q3) {
+    ut[0] = q0 * q0 + q1 * q1 - q2 * q2 - q3 * q3;
+    ut[3] = T(2) * (q1 * q2 - q0 * q3);
+    ut[6] = T(2) * (q1 * q3 + q0 * q2);
+    ut[1] = T(2) * (q1 * q2 + q0 * q3);
+    ut[4] = q0 * q0 - q1 * q1 + q2 * q2 - q3 * q3;
+    ut[7] = T(2) * (q2 * q3 - q0 * q1);
+    ut[2] = T(2) * (q1 * q3 - q0 * q2);
+    ut[5] = T(2) * (q2 * q3 + q0 * q1);
+    ut[8] = q0 * q0 - q1 * q1 - q2 * q2 + q3 * q3;
 }
 
 template <typename T>
-__global__ void __launch_bounds__(kRmsdThreads) rmsd_fwd_kernel(RmsdArgs<T> a) {
+__device__ __forceinline__ int checked_atoms(const RmsdArgs<T> &a, int b) {
+    const int n = a.num_atoms[b];
+    if (n >= 0 && n <= a.atoms_stride) return n;
+    if (threadIdx.x == 0 && a.hdr) atomicCAS(&a.hdr->status, 0u, (unsigned)TPL_ERR_ATOMS);
+    return max(0, min(n, a.atoms_stride));
+}
+
+// One value of x0 / x1 / x2 by index, in registers.
+__device__ __forceinline__ float pick3(int i, float x0, float x1, float x2) { return i == 0 ? x0 : (i == 1 ? x1 : x2); }
+
+constexpr int kRmsdSums = 16;  // R (row-major), R2, sum x, sum y
+
+// float32 forward: one pass over the chain.  Both sets are taken relative to a
+// provisional centre, the mean of 16 atoms spread over the chain, and the sums are
+// moved to the true centroids afterwards in FP64 (R - n cx cy^T and so on): the
+// provisional centre is off by about a quarter of the radius of gyration, so the
+// sums keep the size, and the rounding, of centred ones, and the second read of every
+// coordinate goes.  Atoms are read as float4 groups (tpl_rows.cuh) where both rows
+// have the same alignment.
+template <int NT>
+__global__ void __launch_bounds__(NT) rmsd_fwd_f32_kernel(RmsdArgs<float> a) {
+    constexpr int NW = NT / 32;
+    __shared__ __align__(8) float s_red[4 * NW][kRmsdSums];
+    __shared__ double s_R[9], s_K[16], s_jac[32];
+    __shared__ float s_M[16];
+    const int b = blockIdx.x, tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+    const int n = checked_atoms(a, b);
+    const float *x = a.src + (size_t)b * 3 * a.atoms_stride;
+    const float *y = a.dst + (size_t)b * 3 * a.atoms_stride;
+    float c[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};  // provisional centres, the same on every thread
+    if (a.center && n > 0) {
+        const size_t i = (size_t)n * (2 * (lane & 15) + 1) / 32;
+#pragma unroll
+        for (int k = 0; k < 3; k++) {
+            c[k] = x[3 * i + k];
+            c[3 + k] = y[3 * i + k];
+        }
+#pragma unroll
+        for (int off = 8; off > 0; off >>= 1)
+#pragma unroll
+            for (int k = 0; k < 6; k++) c[k] += __shfl_xor_sync(0xffffffffu, c[k], off);
+#pragma unroll
+        for (int k = 0; k < 6; k++) c[k] *= 1.f / 16.f;
+    }
+    float v[kRmsdSums];
+#pragma unroll
+    for (int k = 0; k < kRmsdSums; k++) v[k] = 0.f;
+    auto add = [&](float (&s)[kRmsdSums], const float *xa, const float *ya) {
+        const float xi[3] = {xa[0] - c[0], xa[1] - c[1], xa[2] - c[2]}, yi[3] = {ya[0] - c[3], ya[1] - c[4], ya[2] - c[5]};
+#pragma unroll
+        for (int p = 0; p < 3; p++) {
+#pragma unroll
+            for (int r = 0; r < 3; r++) s[3 * p + r] = fmaf(xi[p], yi[r], s[3 * p + r]);
+            s[10 + p] += xi[p];
+            s[13 + p] += yi[p];
+        }
+        s[9] += xi[0] * xi[0] + xi[1] * xi[1] + xi[2] * xi[2] + yi[0] * yi[0] + yi[1] * yi[1] + yi[2] * yi[2];
+    };
+    int i0 = 0;  // first atom of the scalar loop; the atoms before the groups come last
+    const int head = row_head(x);
+    int nhead = 0;
+    if (head == row_head(y) && n > head) {
+        const int ng = (n - head) >> 2;
+        const float *xg = x + 3 * head, *yg = y + 3 * head;
+#pragma unroll 2
+        for (int g = tid; g < ng; g += NT) {
+            float xv[12], yv[12];
+            load_group(xg + 12 * g, xv);
+            load_group(yg + 12 * g, yv);
+            float s[kRmsdSums];  // the group's own sums first: fewer roundings at the size of the running sums
+#pragma unroll
+            for (int k = 0; k < kRmsdSums; k++) s[k] = 0.f;
+#pragma unroll
+            for (int q = 0; q < 4; q++) add(s, xv + 3 * q, yv + 3 * q);
+#pragma unroll
+            for (int k = 0; k < kRmsdSums; k++) v[k] += s[k];
+        }
+        i0 = head + 4 * ng;
+        nhead = head;
+    }
+    for (int i = i0 + tid - nhead; i < n; i += NT) {
+        const int at = i < i0 ? i - i0 + nhead : i;  // the nhead atoms before the groups, then the rest
+        add(v, x + 3 * at, y + 3 * at);
+    }
+    // Sums over eight lanes: a lane hands half of its values to its partner and keeps the
+    // sums of the other half, so that 16 values take 14 shuffles.  The four sums of a
+    // warp and the warps are then added in FP64: FP32 additions of ever larger sums up to
+    // the whole warp were most of the rounding error (rmsd against FP64, 4096 chains of
+    // 400..2303 atoms: 1.4e-6 with all five levels in FP32).
+#pragma unroll
+    for (int off = 16, h = kRmsdSums / 2; h > 1; off >>= 1, h >>= 1) {
+        const bool up = (lane & off) != 0;
+#pragma unroll
+        for (int k = 0; k < h; k++) {
+            const float give = up ? v[k] : v[k + h], keep = up ? v[k + h] : v[k];
+            v[k] = keep + __shfl_xor_sync(0xffffffffu, give, off);
+        }
+    }
+    // values 2 (lane >> 2) and the next, summed over the lanes with this lane's low bits
+    *reinterpret_cast<float2 *>(&s_red[4 * w + (lane & 3)][2 * (lane >> 2)]) = make_float2(v[0], v[1]);
+    __syncthreads();
+    if (w != 0) return;
+
+    // warp 0, in FP64: value lane & 15 over the warps, then moved to the true centroids
+    const int k = lane & 15;
+    double d = 0.0;
+#pragma unroll
+    for (int i = 0; i < 2 * NW; i++) d += (double)s_red[2 * NW * (lane >> 4) + i][k];
+    d += __shfl_xor_sync(0xffffffffu, d, 16);
+    if (a.center) {
+        double rn = 0.0;  // 1 / n: an FP32 reciprocal and one Newton step
+        if (n > 0) {
+            rn = (double)(1.f / (float)n);
+            rn = fma(rn, fma(-(double)n, rn, 1.0), rn);
+        }
+        const double m = d * rn;  // lanes 10 .. 15: the centroids from the provisional centres
+        if (lane >= 10 && lane < 16 && a.centroids) {
+            const float c_k = k < 13 ? pick3(k - 10, c[0], c[1], c[2]) : pick3(k - 13, c[3], c[4], c[5]);
+            a.centroids[6 * b + k - 10] = (double)c_k + m;
+        }
+        const double sx = __shfl_sync(0xffffffffu, d, 10 + (k < 9 ? k / 3 : 0));
+        const double my = __shfl_sync(0xffffffffu, m, 13 + (k < 9 ? k % 3 : 0));
+        double sq = k >= 10 ? d * m : 0.0;
+#pragma unroll
+        for (int off = 8; off > 0; off >>= 1) sq += __shfl_xor_sync(0xffffffffu, sq, off);
+        d -= k < 9 ? sx * my : sq;
+    } else if (lane < 6 && a.centroids) {
+        a.centroids[6 * b + lane] = 0.0;
+    }
+    const double r2 = __shfl_sync(0xffffffffu, d, 9);
+    double scale, inv;
+    unit_scale(0.5 * r2, scale, inv);
+    if (lane < 9) s_R[lane] = d * scale;
+    __syncwarp();
+    double l, q[4];
+    key_eigen_warp<true>(s_R, 0.5 * r2 * scale, s_K, s_M, s_jac, l, q);
+    if (lane != 0) return;
+    store_ut(a.ut + (size_t)9 * b, (float)q[0], (float)q[1], (float)q[2], (float)q[3]);
+    const float msd = n > 0 ? (float)(r2 - 2.0 * fabs(l * inv) + 1e-10) * (1.f / (float)n) : 0.f;
+    a.rmsd[b] = sqrtf(msd > 0.f ? msd : 0.f);
+}
+
+// float64 forward: two passes (centroids, then the correlation), everything in FP64.
+__global__ void __launch_bounds__(kRmsdThreads) rmsd_fwd_f64_kernel(RmsdArgs<double> a) {
     __shared__ double s_red[kRmsdWarps * 10];
     __shared__ double s_out[10];
-    __shared__ double s_K[16];
+    __shared__ double s_R[9], s_K[16];
     __shared__ double s_jac[32];  // scratch of the Jacobi fallback
-    __shared__ double s_c[6];  // centroids (src, dst)
-    __shared__ T s_ct[6];
+    __shared__ double s_c[6];     // centroids (src, dst)
     const int b = blockIdx.x, tid = threadIdx.x;
-    int n = a.num_atoms[b];
-    if (n < 0 || n > a.atoms_stride) {
-        if (tid == 0 && a.hdr) atomicCAS(&a.hdr->status, 0u, (unsigned)TPL_ERR_ATOMS);
-        n = max(0, min(n, a.atoms_stride));
-    }
-    const T *x = a.src + (size_t)b * 3 * a.atoms_stride;
-    const T *y = a.dst + (size_t)b * 3 * a.atoms_stride;
+    const int n = checked_atoms(a, b);
+    const double *x = a.src + (size_t)b * 3 * a.atoms_stride;
+    const double *y = a.dst + (size_t)b * 3 * a.atoms_stride;
     if (a.center) {
-        T sx[6] = {0, 0, 0, 0, 0, 0};
+        double sx[6] = {0, 0, 0, 0, 0, 0};
 #pragma unroll 4
         for (int i = tid; i < n; i += kRmsdThreads)
             for (int k = 0; k < 3; k++) {
                 sx[k] += x[3 * i + k];
                 sx[3 + k] += y[3 * i + k];
             }
-        block_sums<T, 6>(sx, s_red, s_out);
-        if (tid < 6) {  // one division per value, on six lanes (FP64 is slow on GB300)
-            const double v = n > 0 ? (sizeof(T) == 4 ? s_out[tid] * (double)(1.f / (float)n) : s_out[tid] / n) : 0.0;
-            s_c[tid] = v;
-            s_ct[tid] = (T)v;
-        }
+        block_sums<double, 6>(sx, s_red, s_out);
+        if (tid < 6) s_c[tid] = n > 0 ? s_out[tid] / n : 0.0;
     } else if (tid < 6) {
         s_c[tid] = 0.0;
-        s_ct[tid] = T(0);
     }
     __syncthreads();
-    T ct[6];
-    for (int k = 0; k < 6; k++) ct[k] = s_ct[k];
-    T acc[10] = {0, 0, 0, 0, 0, 0, 0, 0, 0, 0};  // R (row-major) and R2
+    double ct[6];
+    for (int k = 0; k < 6; k++) ct[k] = s_c[k];
+    double acc[10] = {0, 0, 0, 0, 0, 0, 0, 0, 0, 0};  // R (row-major) and R2
 #pragma unroll 4
     for (int i = tid; i < n; i += kRmsdThreads) {
-        T xi[3], yi[3];
+        double xi[3], yi[3];
         for (int k = 0; k < 3; k++) {
             xi[k] = x[3 * i + k] - ct[k];
             yi[k] = y[3 * i + k] - ct[3 + k];
@@ -384,46 +516,21 @@ __global__ void __launch_bounds__(kRmsdThreads) rmsd_fwd_kernel(RmsdArgs<T> a) {
             for (int q = 0; q < 3; q++) acc[3 * p + q] = fma(xi[p], yi[q], acc[3 * p + q]);
         acc[9] += xi[0] * xi[0] + xi[1] * xi[1] + xi[2] * xi[2] + yi[0] * yi[0] + yi[1] * yi[1] + yi[2] * yi[2];
     }
-    block_sums<T, 10>(acc, s_red, s_out);
-    if constexpr (sizeof(T) == 4) {
-        if (tid < 32) rmsd_finish_f32(a, b, n, s_out, s_K, s_c, s_jac);
-        return;
-    }
-    if (tid < 32) {
-        const double *R = s_out;
-        double tot[10];
-        for (int k = 0; k < 10; k++) tot[k] = s_out[k];
-        if (tid == 0) {
-            // quaternion matrix, same layout as the reference (coords2rmsd_interface.cpp:146-149)
-            const double F[16] = {R[0] + R[4] + R[8], R[5] - R[7], R[6] - R[2], R[1] - R[3],
-                                  R[5] - R[7], R[0] - R[4] - R[8], R[1] + R[3], R[2] + R[6],
-                                  R[6] - R[2], R[1] + R[3], -R[0] + R[4] - R[8], R[5] + R[7],
-                                  R[1] - R[3], R[2] + R[6], R[5] + R[7], -R[0] - R[4] + R[8]};
-            for (int k = 0; k < 16; k++) s_K[k] = F[k];
-        }
-        __syncwarp();
-        double lam, q[4];
-        key_eigen_warp<false>(s_K, 0.5 * tot[9], lam, q, s_jac);
-        if (tid != 0) return;
-        // rotation from the unit quaternion (coords2rmsd_interface.cpp:36-46)
-        double U[9];
-        U[0] = q[0] * q[0] + q[1] * q[1] - q[2] * q[2] - q[3] * q[3];
-        U[1] = 2.0 * (q[1] * q[2] - q[0] * q[3]);
-        U[2] = 2.0 * (q[1] * q[3] + q[0] * q[2]);
-        U[3] = 2.0 * (q[1] * q[2] + q[0] * q[3]);
-        U[4] = q[0] * q[0] - q[1] * q[1] + q[2] * q[2] - q[3] * q[3];
-        U[5] = 2.0 * (q[2] * q[3] - q[0] * q[1]);
-        U[6] = 2.0 * (q[1] * q[3] - q[0] * q[2]);
-        U[7] = 2.0 * (q[2] * q[3] + q[0] * q[1]);
-        U[8] = q[0] * q[0] - q[1] * q[1] - q[2] * q[2] + q[3] * q[3];
-        T *ut = a.ut + (size_t)9 * b;
-        for (int j = 0; j < 3; j++)
-            for (int k = 0; k < 3; k++) ut[3 * j + k] = (T)U[3 * k + j];
-        const double msd = n > 0 ? (tot[9] - 2.0 * fabs(lam) + 1e-10) / (double)n : 0.0;
-        a.rmsd[b] = (T)sqrt(msd > 0.0 ? msd : 0.0);
-        if (a.centroids)
-            for (int k = 0; k < 6; k++) a.centroids[6 * b + k] = s_c[k];
-    }
+    block_sums<double, 10>(acc, s_red, s_out);
+    if (tid >= 32) return;
+    const double r2 = s_out[9];
+    double scale, inv;
+    unit_scale(0.5 * r2, scale, inv);
+    if (tid < 9) s_R[tid] = s_out[tid] * scale;
+    __syncwarp();
+    double l, q[4];
+    key_eigen_warp<false>(s_R, 0.5 * r2 * scale, s_K, nullptr, s_jac, l, q);
+    if (tid != 0) return;
+    store_ut(a.ut + (size_t)9 * b, q[0], q[1], q[2], q[3]);
+    const double msd = n > 0 ? (r2 - 2.0 * fabs(l * inv) + 1e-10) / (double)n : 0.0;
+    a.rmsd[b] = sqrt(msd > 0.0 ? msd : 0.0);
+    if (a.centroids)
+        for (int k = 0; k < 6; k++) a.centroids[6 * b + k] = s_c[k];
 }
 
 template <typename T>
@@ -447,20 +554,38 @@ __global__ void __launch_bounds__(kRmsdThreads) rmsd_bwd_kernel(RmsdArgs<T> a) {
     for (int k = 0; k < 6; k++) c[k] = s_c[k];
     for (int k = 0; k < 9; k++) U[k] = s_U[k];
     const T scale = s_scale;
-    // one atom per thread: chains on x, blocks of atoms on y
-    const int i = blockIdx.y * kRmsdThreads + tid;
-    if (i < a.atoms_stride) {
-        if (i < n) {
-            T xi[3], yi[3];
-            for (int k = 0; k < 3; k++) {
-                xi[k] = x[3 * i + k] - c[k];
-                yi[k] = y[3 * i + k] - c[3 + k];
-            }
-            for (int k = 0; k < 3; k++)
-                gx[3 * i + k] = scale * (xi[k] - (U[3 * k] * yi[0] + U[3 * k + 1] * yi[1] + U[3 * k + 2] * yi[2]));
-        } else {
-            gx[3 * i] = gx[3 * i + 1] = gx[3 * i + 2] = T(0);
+    // one group of N atoms per thread: chains on x, blocks of groups on y; group 0 is the
+    // row's unaligned head, and whole groups move as 16-byte vectors (tpl_rows.cuh)
+    constexpr int N = Vec16<T>::n;
+    const int head = row_head(x);
+    const bool vec = head == row_head(y) && head == row_head(gx);
+    const int i0 = head + N * ((int)(blockIdx.y * kRmsdThreads + tid) - 1);
+    auto atom = [&](const T *xa, const T *ya, T *g) {
+        const T xi[3] = {xa[0] - c[0], xa[1] - c[1], xa[2] - c[2]}, yi[3] = {ya[0] - c[3], ya[1] - c[4], ya[2] - c[5]};
+#pragma unroll
+        for (int k = 0; k < 3; k++)
+            g[k] = scale * (xi[k] - (U[3 * k] * yi[0] + U[3 * k + 1] * yi[1] + U[3 * k + 2] * yi[2]));
+    };
+    if (vec && i0 >= 0 && i0 + N <= a.atoms_stride) {
+        T g[3 * N];
+#pragma unroll
+        for (int k = 0; k < 3 * N; k++) g[k] = T(0);
+        if (i0 < n) {
+            T xv[3 * N], yv[3 * N];
+            load_group(x + 3 * i0, xv);
+            load_group(y + 3 * i0, yv);
+#pragma unroll
+            for (int q = 0; q < N; q++)
+                if (i0 + q < n) atom(xv + 3 * q, yv + 3 * q, g + 3 * q);
         }
+        store_group(gx + 3 * i0, g);
+        return;
+    }
+    for (int i = max(i0, 0); i < min(i0 + N, a.atoms_stride); i++) {
+        T g[3] = {T(0), T(0), T(0)};
+        if (i < n) atom(x + 3 * i, y + 3 * i, g);
+#pragma unroll
+        for (int k = 0; k < 3; k++) gx[3 * i + k] = g[k];
     }
 }
 
@@ -469,7 +594,19 @@ static int rmsd_fwd_launch(const T *src, const T *dst, const int *num_atoms, int
                            T *ut, double *centroids, void *ws, cudaStream_t st) {
     if (B == 0) return TPL_OK;
     RmsdArgs<T> a{src, dst, num_atoms, stride, center, rmsd, ut, centroids, nullptr, nullptr, (WsHeader *)ws};
-    rmsd_fwd_kernel<T><<<B, kRmsdThreads, 0, st>>>(a);
+    if constexpr (sizeof(T) == 4) {
+        // Threads per chain: with few chains per SM the longest chain's loads bound the
+        // launch (256 chains of 50..500 residues, training step as a graph: 65.7 / 66.6 /
+        // 68.9 us at 512 / 256 / 128 threads); with many, a CTA holds its registers while
+        // its first warp solves, so small CTAs keep more chains' loads in flight (4096
+        // chains of 400..2303 atoms: 116 / 60 / 42 us; 64 threads: 46 us).
+        const int sms = device_sm_count();
+        if (B <= 2 * sms) rmsd_fwd_f32_kernel<512><<<B, 512, 0, st>>>(a);
+        else if (B <= 4 * sms) rmsd_fwd_f32_kernel<256><<<B, 256, 0, st>>>(a);
+        else rmsd_fwd_f32_kernel<128><<<B, 128, 0, st>>>(a);
+    } else {
+        rmsd_fwd_f64_kernel<<<B, kRmsdThreads, 0, st>>>(a);
+    }
     return cudaGetLastError() == cudaSuccess ? TPL_OK : TPL_ERR_LAUNCH;
 }
 
@@ -480,8 +617,10 @@ static int rmsd_bwd_launch(const T *grad_rmsd, const T *src, const T *dst, const
     if (B == 0) return TPL_OK;
     RmsdArgs<T> a{src, dst, num_atoms, stride, center, const_cast<T *>(rmsd), const_cast<T *>(ut),
                   const_cast<double *>(centroids), grad_rmsd, grad_src, nullptr};
-    const int ablocks = (max(stride, 1) + kRmsdThreads - 1) / kRmsdThreads;
-    if (ablocks > 65535) return TPL_ERR_UNSUPPORTED;
+    if ((max(stride, 1) + kRmsdThreads - 1) / kRmsdThreads > 65535) return TPL_ERR_UNSUPPORTED;
+    constexpr int N = Vec16<T>::n;
+    const int groups = (max(stride, 1) + N - 1) / N + 1;  // the head and the aligned groups
+    const int ablocks = (groups + kRmsdThreads - 1) / kRmsdThreads;
     rmsd_bwd_kernel<T><<<dim3((unsigned)B, (unsigned)ablocks), kRmsdThreads, 0, st>>>(a);
     return cudaGetLastError() == cudaSuccess ? TPL_OK : TPL_ERR_LAUNCH;
 }
