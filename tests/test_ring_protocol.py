@@ -74,3 +74,36 @@ def test_ring_handoffs_never_deadlock_or_mix(forward, warps):
         for seed in range(200):
             result, info = replay(progs, random.Random(seed), warps)
             assert result == "ok", (nchunk, seed, result, info)
+
+
+@pytest.mark.parametrize("warps", [4, 8])
+def test_chunk_stream_over_chains(warps):
+    """The Angles2Coords kernels run the chunks of a CTA's chains as one stream: each warp
+    steps its own (chain, chunk) by W and moves on to the next chain when the number runs
+    past the chain's chunks (at least one per chain).  Together the warps visit every chunk
+    of every chain once, warp w exactly the stream positions w, w + W, ..., and whether a
+    chunk waits for a handoff (not the stream's first) and signals one (not its last) follows
+    from the chain and chunk alone; the handoffs are then those of one chain that long."""
+    rng = random.Random(warps)
+    for _ in range(300):
+        chains = [max(1, rng.choice([0, 1, 2, 3, 4, 5, 9, 16, 40])) for _ in range(rng.randint(1, 12))]
+        stream = [(b, k) for b, n in enumerate(chains) for k in range(n)]
+        where = {}
+        for w in range(warps):
+            b, k = 0, w
+            while True:
+                while b < len(chains) and k >= chains[b]:
+                    k -= chains[b]
+                    b += 1
+                if b >= len(chains):
+                    break
+                where[(b, k)] = w
+                waits = not (b == 0 and k == 0)
+                signals = k + 1 < chains[b] or b + 1 < len(chains)
+                g = stream.index((b, k))
+                assert waits == (g > 0) and signals == (g + 1 < len(stream))
+                k += warps
+        assert [where.get(c) for c in stream] == [g % warps for g in range(len(stream))]
+        assert len(where) == len(stream)
+        result, info = replay(warp_programs(len(stream), True, warps), rng, warps)
+        assert result == "ok", (chains, result, info)

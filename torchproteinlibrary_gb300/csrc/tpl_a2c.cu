@@ -274,63 +274,118 @@ __device__ __forceinline__ void pair_point(const PairFrame &P, float x, float y,
     out[2] = fmaf(P.r2[0], x, fmaf(P.r2[1], y, fmaf(P.r2[2], z, P.p2)));
 }
 
+// The topology as the chunked float32 kernels read it: one 16-byte shared-memory load
+// per side-chain joint and per atom position, one word per residue letter.
+struct alignas(16) RingJoint {
+    float cb, sb, d;
+    int bits;  // atoms of the joint's group | index of its first side-chain atom << 8 | alpha fixed at 0 << 16
+};
+struct alignas(16) RingPoint {
+    float x, y, z, pad;
+};
+struct RingTopology {
+    RingJoint joint[kResTypes][kMaxScJoints];
+    RingPoint point[kResTypes][kMaxScAtoms];
+    uint32_t res_name[kResTypes];
+    uint32_t atom_name[kResTypes][16];
+    uint32_t letter[256];  // type | atoms << 8 | side-chain joints << 16 | Pro << 24; 0 for what is no residue letter
+};
+constexpr Topology<float> kTopoF32 = make_topology<float>();
+
+constexpr RingTopology make_ring_topology() {
+    const Topology<float> tp = make_topology<float>();
+    RingTopology r{};
+    for (int t = 0; t < kResTypes; t++) {
+        for (int k = 0; k < kMaxScJoints; k++)
+            r.joint[t][k] = {tp.jcb[t][k], tp.jsb[t][k], tp.jd[t][k],
+                             tp.jna[t][k] | tp.jfirst[t][k] << 8 | (tp.jchi[t][k] < 0 ? 1 << 16 : 0)};
+        for (int q = 0; q < kMaxScAtoms; q++) r.point[t][q] = {tp.sc[t][q][0], tp.sc[t][q][1], tp.sc[t][q][2], 0.f};
+        r.res_name[t] = tp.res_name[t];
+        for (int q = 0; q < kMaxResAtoms; q++) r.atom_name[t][q] = tp.atom_name[t][q];
+        r.letter[(unsigned char)kResLetters[t]] =
+            (uint32_t)(t | tp.natoms[t] << 8 | tp.njoints[t] << 16 | tp.pro[t] << 24);  // never 0: natoms >= 4
+    }
+    return r;
+}
+__device__ const RingTopology g_ring_topo = make_ring_topology();
+
+template <int NT>
+__device__ __forceinline__ void load_ring_topology(RingTopology &dst) {
+    const uint4 *src = reinterpret_cast<const uint4 *>(&g_ring_topo);
+    static_assert(sizeof(RingTopology) % 16 == 0, "topology size");
+    for (int i = threadIdx.x; i < (int)(sizeof(RingTopology) / 16); i += NT) reinterpret_cast<uint4 *>(&dst)[i] = src[i];
+}
+
+// The three backbone joints' constants as literals.
+template <int K>
+__device__ __forceinline__ void apply_backbone(PairFrame &f, float c, float s) {
+    constexpr float cb = kTopoF32.bb_cb[K], sb = kTopoF32.bb_sb[K], d = kTopoF32.bb_d[K];
+    apply_joint_pair(f, cb, sb, d, c, s);
+}
+
 // residue_atoms for float32 on paired frames, with the chi angles' cos and sin
 // computed beforehand (chi_c[q], chi_s[q] for chi_(q+1)): the same atoms in the
 // same slots, without the frame at the next N.
 template <typename Emit>
-__device__ __forceinline__ void residue_atoms_pair(const Topology<float> &tp, int ty, const PairFrame &P,
+__device__ __forceinline__ void residue_atoms_pair(const RingTopology &tp, uint32_t info, const PairFrame &P,
                                                    const float cs[2], const float sn[2], const float chi_c[5],
                                                    const float chi_s[5], Emit emit) {
+    const int ty = info & 0xff, na = (info >> 8) & 0xff, nj = (info >> 16) & 0xff;
     {
         const float x[3] = {P.p.x, P.p.y, P.p2};
         emit(0, x);
     }
     PairFrame F = P;
-    apply_joint_pair(F, tp.bb_cb[0], tp.bb_sb[0], tp.bb_d[0], cs[0], sn[0]);
+    apply_backbone<0>(F, cs[0], sn[0]);
     {
         const float x[3] = {F.p.x, F.p.y, F.p2};
         emit(1, x);
     }
-    const int na = tp.natoms[ty];
-    if (tp.pro[ty]) {
+    if (info >> 24) {  // Pro
+        constexpr float p[9] = {kTopoF32.pro_local[0][0], kTopoF32.pro_local[0][1], kTopoF32.pro_local[0][2],
+                                kTopoF32.pro_local[1][0], kTopoF32.pro_local[1][1], kTopoF32.pro_local[1][2],
+                                kTopoF32.pro_local[2][0], kTopoF32.pro_local[2][1], kTopoF32.pro_local[2][2]};
+#pragma unroll
         for (int a = 0; a < 3; a++) {
             float x[3];
-            pair_point(F, tp.pro_local[a][0], tp.pro_local[a][1], tp.pro_local[a][2], x);
+            pair_point(F, p[3 * a], p[3 * a + 1], p[3 * a + 2], x);
             emit(2 + a, x);
         }
     }
-    const int nj = tp.njoints[ty];
     if (nj > 0) {
         PairFrame S = F;
-        apply_rx_pair(S, tp.dummy_c, tp.dummy_s);
+        constexpr float dc = kTopoF32.dummy_c, ds = kTopoF32.dummy_s;
+        apply_rx_pair(S, dc, ds);
         // unrolled over the joints: joint k reads chi angle k or none (Ala's fixed
         // alpha; topology_layout_ok), so the angle is a register, not a select
 #pragma unroll
         for (int k = 0; k < kMaxScJoints; k++) {
             if (k >= nj) break;
-            const bool fixed = tp.jchi[ty][k] < 0;
-            apply_joint_pair(S, tp.jcb[ty][k], tp.jsb[ty][k], tp.jd[ty][k], fixed ? 1.f : chi_c[k],
-                             fixed ? 0.f : chi_s[k]);
-            const int f0 = tp.jfirst[ty][k];
+            const RingJoint j = tp.joint[ty][k];
+            const bool fixed = (j.bits >> 16) != 0;
+            apply_joint_pair(S, j.cb, j.sb, j.d, k == 0 && fixed ? 1.f : chi_c[k], k == 0 && fixed ? 0.f : chi_s[k]);
+            const int f0 = (j.bits >> 8) & 0xff, n = j.bits & 0xff;
             {  // the group's first atom sits at the joint's origin
                 const float x[3] = {S.p.x, S.p.y, S.p2};
                 emit(2 + f0, x);
             }
-            for (int a = 1; a < tp.jna[ty][k]; a++) {
+            for (int a = 1; a < n; a++) {
+                const RingPoint v = tp.point[ty][f0 + a];
                 float x[3];
-                pair_point(S, tp.sc[ty][f0 + a][0], tp.sc[ty][f0 + a][1], tp.sc[ty][f0 + a][2], x);
+                pair_point(S, v.x, v.y, v.z, x);
                 emit(2 + f0 + a, x);
             }
         }
     }
     PairFrame C = F;
-    apply_joint_pair(C, tp.bb_cb[1], tp.bb_sb[1], tp.bb_d[1], cs[1], sn[1]);
+    apply_backbone<1>(C, cs[1], sn[1]);
     {
         const float x[3] = {C.p.x, C.p.y, C.p2};
         emit(na - 2, x);
     }
+    constexpr float ox = kTopoF32.o_local[0], oy = kTopoF32.o_local[1], oz = kTopoF32.o_local[2];
     float x[3];
-    pair_point(C, tp.o_local[0], tp.o_local[1], tp.o_local[2], x);
+    pair_point(C, ox, oy, oz, x);
     emit(na - 1, x);
 }
 
@@ -449,195 +504,281 @@ __global__ void __launch_bounds__(NT) a2c_fwd_kernel(A2cArgs<T> a, int renorm) {
 }
 
 // ------------------------------------------ forward, four or eight warps per chain
-// One CTA of NW = 4 or 8 warps per chain and chunks of 32 residues, one per lane;
-// chunk k belongs to warp k % NW.  Per chunk a warp loads its residues' angles,
-// composes each residue's three backbone joints (N -> CA -> C -> next N), scans the
-// lane transforms and the atom counts over the warp, and places every atom of its
-// residue from the lane's frame at N into a per-warp staging buffer, from which the
-// chunk's contiguous atom range leaves with coalesced stores.  Only the chain frame
-// at the chunk start and the chunk's first atom index pass between warps, through
-// the named-barrier handoff of tpl_pair.cuh, so the chunk loop has no CTA-wide
-// barrier.  Positions are built relative to the chunk's first N atom and moved to
-// it as they are staged.
+// Chunks of 32 residues, one per lane, dealt round the NW = 4 or 8 warps of a CTA.  A
+// CTA takes chains b, b + grid, ... (persistent: the topology loads once) and their
+// chunks form one stream: chunk g of the stream is on warp g % NW, chain after chain,
+// with no CTA barrier anywhere, so that a short chain or a chain's last chunk leaves no
+// warp waiting.  Per chunk a warp composes each residue's three backbone joints
+// (N -> CA -> C -> next N), scans the lane transforms and the atom counts over the warp,
+// receives the chain frame and first atom index of its chunk from the warp of the chunk
+// before (the named-barrier handoff of tpl_pair.cuh; at a chain's first chunk the
+// handoff only keeps the order of the stream), and places every atom of its residue in a
+// per-warp buffer.  Positions are built relative to the chunk's first N atom and moved
+// to it as they are staged.
+//
+// Instruction issue and latency bound it (4096 x 500 random residues: issue active 46 %
+// with the CTA-synchronised form).  What is out of the way of the arithmetic:
+//   * the next chunk's angles come by cp.async while this one is worked on (a lane copies
+//     and reads only its own), and its letters one chunk ahead;
+//   * the coordinates leave as one bulk copy of the chunk's whole 16-byte blocks, issued
+//     by one lane; the values are staged at their global 16-byte phase;
+//   * names are staged as one 16-bit code per atom (type, slot) and looked up as they are
+//     stored, 0.9 instead of 3.6 KB per warp, which keeps six CTAs of four warps per SM.
 constexpr int kA2cChunk = 32;
 constexpr int kA2cStageAtoms = kA2cChunk * kMaxResAtoms;
 
-// The coordinate staging rows carry 4 words of slack: a chunk's values start at the
-// word offset of their global destination inside its 16-byte block (0..3), so that
-// whole blocks move as aligned 16-byte loads and stores (copy_span).
-template <int NW>
+// Per warp: the chunk's coordinates (4 words of slack for the 16-byte phase of their
+// destination), the next chunk's angles, the name codes (when names are written).
+struct alignas(16) A2cRingWarp {
+    float xyz[kA2cStageAtoms * 3 + 4];
+    float ang[8 * kA2cChunk];
+};
+template <int NW, bool NAMES>
 struct A2cRingSmem {
-    Topology<float> topo;
-    signed char lut[256];
-    alignas(16) float xyz[NW][kA2cStageAtoms * 3 + 4];
-    uint32_t res_name[NW][kA2cStageAtoms];  // present when names are written
-    uint32_t atom_name[NW][kA2cStageAtoms];
+    RingTopology topo;
+    A2cRingWarp warp[NW];
+    uint16_t code[NAMES ? NW : 1][NAMES ? kA2cStageAtoms : 8];
 };
 
 // Word offset of p inside its 16-byte block.
 __device__ __forceinline__ int block_offset(const void *p) { return (int)((reinterpret_cast<uintptr_t>(p) >> 2) & 3u); }
 
-// Copy n 4-byte words from the 16-byte-aligned staging row src (the values start at
-// src + block_offset(dst)) to dst, by the warp: every 16-byte block of dst that lies
-// whole inside [dst, dst + n) as one vector load and store, the ragged ends word by word.
-template <typename W, typename W4>
-__device__ __forceinline__ void copy_span(W *dst, const W *src, int n, int lane) {
-    const int sh = block_offset(dst);
-    W *base = dst - sh;  // 16-byte aligned; only words inside [dst, dst + n) are written
-    const int nb = (n + sh + 3) >> 2;
-    for (int b = lane; b < nb; b += 32) {
-        const int lo = 4 * b - sh;
-        if (lo >= 0 && lo + 4 <= n) {
-            *reinterpret_cast<W4 *>(base + 4 * b) = *reinterpret_cast<const W4 *>(src + 4 * b);
-        } else {
+__device__ __forceinline__ void cp_async4(float *dst_smem, const float *src) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"((unsigned)__cvta_generic_to_shared(dst_smem)),
+                 "l"(src)
+                 : "memory");
+}
+__device__ __forceinline__ void cp_async_wait_all() {
+    asm volatile("cp.async.commit_group;\ncp.async.wait_group 0;" ::: "memory");
+}
+
+// Store n words to dst from stg = stage + block_offset(dst), stage 16-byte aligned shared
+// memory written by the whole warp before a __syncwarp: the whole 16-byte blocks as one
+// bulk copy by lane 0, the words outside them by the first lanes.  The caller waits for
+// the copy's reads (bulk_reads_done) before it rewrites the buffer.
+__device__ __forceinline__ void bulk_store_span(float *dst, const float *stg, int n, int lane) {
+    const int head = min((4 - block_offset(dst)) & 3, n), body = (n - head) & ~3, tail = n - head - body;
+    if (lane < head) dst[lane] = stg[lane];
+    if (lane < tail) dst[head + body + lane] = stg[head + body + lane];
+    if (lane == 0 && body > 0)
+        asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;\n"
+                     "cp.async.bulk.commit_group;" ::"l"(dst + head),
+                     "r"((unsigned)__cvta_generic_to_shared(stg + head)), "r"(4 * body)
+                     : "memory");
+}
+__device__ __forceinline__ void bulk_reads_done() { asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory"); }
+__device__ __forceinline__ void async_proxy_fence() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
+
+// Zeros to n words from dst, by the warp.
+__device__ __forceinline__ void zero_span(uint32_t *dst, int n, int lane) {
+    const int head = min((4 - block_offset(dst)) & 3, max(n, 0)), nb = (max(n, 0) - head) >> 2;
+    if (lane < head) dst[lane] = 0u;
+    for (int i = lane; i < nb; i += 32) reinterpret_cast<uint4 *>(dst + head)[i] = make_uint4(0u, 0u, 0u, 0u);
+    if (lane < n - head - 4 * nb) dst[head + 4 * nb + lane] = 0u;
+}
+
+// Length of chain b for the chunked kernels, found by each warp for itself: the index of
+// the row's first NUL (at most the row stride), or 0, with the error recorded, when a
+// letter before it is no residue or the chain is longer than L.  atoms(chunk, n) is
+// called by the whole warp for every chunk of 32 letters in order, with the atom count of
+// this lane's residue.  table: letter -> word with the atom count in bits 8..15, 0 for
+// what is no residue.
+template <typename Table, typename Atoms>
+__device__ __forceinline__ int ring_chain_length(const A2cArgs<float> &a, int b, const Table *table, int lane,
+                                                 Atoms atoms) {
+    const unsigned char *row = a.seq + (size_t)b * a.seq_stride;
+    int len = a.seq_stride;
+    bool bad = false;
+    for (int j0 = 0; j0 < len; j0 += 128) {
+        unsigned char c[4];
 #pragma unroll
-            for (int e = 0; e < 4; e++)
-                if (lo + e >= 0 && lo + e < n) dst[lo + e] = src[sh + lo + e];
+        for (int u = 0; u < 4; u++) {
+            const int j = j0 + 32 * u + lane;
+            c[u] = j < a.seq_stride ? row[j] : (unsigned char)0;
+        }
+#pragma unroll
+        for (int u = 0; u < 4; u++) {
+            const int j1 = j0 + 32 * u;
+            if (j1 >= len) break;
+            const unsigned nul = __ballot_sync(0xffffffffu, c[u] == 0);
+            if (nul != 0u) len = min(len, j1 + __ffs(nul) - 1);
+            const unsigned info = table[c[u]];
+            const bool in = j1 + lane < len;
+            bad |= __any_sync(0xffffffffu, in && info == 0u);
+            if (j1 < len) atoms(j1 >> 5, in ? (int)((info >> 8) & 0xffu) : 0);
         }
     }
+    if (bad || len > a.L) {
+        if (lane == 0) a2c_error(a.hdr, bad ? TPL_ERR_SEQUENCE : TPL_ERR_LENGTH);
+        return 0;
+    }
+    return len;
 }
-template <int NW>
-constexpr size_t a2c_ring_smem_no_names() { return offsetof(A2cRingSmem<NW>, res_name); }
 
 template <int NW, bool NAMES>
 __global__ void __launch_bounds__(32 * NW, NW == 4 ? 6 : 3) a2c_fwd_ring_kernel(A2cArgs<float> a, int renorm, int nb) {
     constexpr int NT = 32 * NW;
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    A2cRingSmem<NW> &sm = *reinterpret_cast<A2cRingSmem<NW> *>(smem_raw);
+    A2cRingSmem<NW, NAMES> &sm = *reinterpret_cast<A2cRingSmem<NW, NAMES> *>(smem_raw);
     __shared__ __align__(16) float s_ring[NW][16];  // chain frame (12) and first atom index
-    __shared__ int s_len, s_bad, s_total;
 
-    const int tid = threadIdx.x, w = tid >> 5, lane = tid & 31;
-    load_topology<float, NT>(sm.topo, sm.lut);
-    const Topology<float> &tp = sm.topo;
-    // persistent: the grid fills the SMs once and each CTA takes chains b, b + grid, ...,
-    // so the topology loads once per CTA and no partial last wave of chains is left
-    // (GB300, 4096 x 500 random residues: forward 0.155 -> 0.152 ms, with names
-    // 0.203 -> 0.197 ms).  The barrier at the end of a chain orders its last reads of
-    // the shared state before the next chain's writes.
-    for (int b = blockIdx.x; b < nb; b += gridDim.x) {
-        if (tid == 0) s_total = 0;  // ordered before every chunk by the barriers of chain_length
-        const unsigned char *row = a.seq + (size_t)b * a.seq_stride;
-        const int len = chain_length<NT>(row, a.seq_stride, sm.lut, &s_len, &s_bad);
-        const bool ok = !s_bad && len <= a.L;
-        if (tid == 0) {
-            if (s_bad) a2c_error(a.hdr, TPL_ERR_SEQUENCE);
-            if (len > a.L) a2c_error(a.hdr, TPL_ERR_LENGTH);
+    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    load_ring_topology<NT>(sm.topo);
+    __syncthreads();
+    const RingTopology &tp = sm.topo;
+    float *stage = sm.warp[w].xyz, *abuf = sm.warp[w].ang + lane;
+
+    // the warp's next chunk: chunk k of chain b (length len, nch chunks; an empty or
+    // refused chain has one, which writes its zeros)
+    int b = blockIdx.x, k = w, len = 0, nch = 0;
+    unsigned char letter = 0;
+    auto enter = [&]() {
+        len = ring_chain_length(a, b, tp.letter, lane, [](int, int) {});
+        nch = max(1, (len + kA2cChunk - 1) / kA2cChunk);
+    };
+    auto settle = [&]() {  // chunk numbers past the chain's belong to the chains after it
+        while (k >= nch) {
+            k -= nch;
+            b += gridDim.x;
+            if (b >= nb) break;
+            enter();
         }
-        float *out = a.coords + (size_t)b * 3 * a.maxA;
-        uint32_t *rn = NAMES ? a.res_names + (size_t)b * a.maxA : nullptr;
-        uint32_t *an = NAMES ? a.atom_names + (size_t)b * a.maxA : nullptr;
-        const float *ang = a.angles + (size_t)b * 8 * a.L;
-        float *stage = sm.xyz[w];
-        const int nchunk = ok ? (len + kA2cChunk - 1) / kA2cChunk : 0;
-
-#pragma unroll 1
-        for (int k = w; k < nchunk; k += NW) {
-            const int j = k * kA2cChunk + lane;
-            const bool live = j < len;
-            const int ty = live ? sm.lut[row[j]] : 0;
-            const int na = live ? tp.natoms[ty] : 0;
-            // backbone angles; omega of the chain's last residue moves no atom
-            // cos and sin of the eight angles, in pairs and for every lane at once (the chi
-            // angles' outside the divergent side-chain walk); omega of the chain's last
-            // residue moves no atom
-            float cs[3] = {1.f, 1.f, 1.f}, sn[3] = {0.f, 0.f, 0.f};
-            float chc[5] = {1.f, 1.f, 1.f, 1.f, 1.f}, chs[5] = {0.f, 0.f, 0.f, 0.f, 0.f};
-            PairFrame t = pair_identity();
-            if (live) {
-                const float phi = ang[j], psi = ang[a.L + j];
-                const float om = j + 1 < len ? ang[2 * a.L + j] : 0.f;
-                float chi[5];
+    };
+    auto fetch = [&]() {
+        const int j = k * kA2cChunk + lane;
+        if (b < nb && j < len) {
+            letter = a.seq[(size_t)b * a.seq_stride + j];
+            const float *src = a.angles + (size_t)b * 8 * a.L + j;
 #pragma unroll
-                for (int q = 0; q < 5; q++) chi[q] = ang[(size_t)(3 + q) * a.L + j];
-                float m = fmaxf(fabsf(phi), fmaxf(fabsf(psi), fabsf(om)));
-#pragma unroll
-                for (int q = 0; q < 5; q++) m = fmaxf(m, fabsf(chi[q]));
-                if (m <= 1.0e4f) {  // NaN passes: sincos_fast2 returns NaN for it
-                    sincos_fast2(phi, psi, &sn[0], &cs[0], &sn[1], &cs[1]);
-                    sincos_fast2(om, chi[0], &sn[2], &cs[2], &chs[0], &chc[0]);
-                    sincos_fast2(chi[1], chi[2], &chs[1], &chc[1], &chs[2], &chc[2]);
-                    sincos_fast2(chi[3], chi[4], &chs[3], &chc[3], &chs[4], &chc[4]);
-                } else {
-                    sincos_poly(phi, &sn[0], &cs[0]);
-                    sincos_poly(psi, &sn[1], &cs[1]);
-                    sincos_poly(om, &sn[2], &cs[2]);
-#pragma unroll
-                    for (int q = 0; q < 5; q++) sincos_poly(chi[q], &chs[q], &chc[q]);
-                }
-#pragma unroll
-                for (int q = 0; q < 3; q++) apply_joint_pair(t, tp.bb_cb[q], tp.bb_sb[q], tp.bb_d[q], cs[q], sn[q]);
-            }
-            PairFrame tot;
-            const PairFrame E = warp_exclusive_total_pair(t, lane, renorm != 0, tot);
-            int ci = na;  // atoms of the lanes up to this one
-#pragma unroll
-            for (int off = 1; off < 32; off <<= 1) {
-                const int o = __shfl_up_sync(0xffffffffu, ci, off);
-                if (lane >= off) ci += o;
-            }
-            const int cnt = __shfl_sync(0xffffffffu, ci, 31), aoff = ci - na;
-
-            PairFrame F = pair_identity();  // chain frame at the chunk start
-            int abase = 0;                  // first atom of the chunk
-            if (k > 0) {
-                ring_wait<NW>(k);
-                F = pair_load(s_ring[k % NW]);
-                abase = __float_as_int(s_ring[k % NW][12]);
-            }
-            if (k + 1 < nchunk) {
-                PairFrame Fn = compose_pair(F, tot);
-                if (renorm) renormalize_pair(Fn);
-                if (lane == 0) {
-                    pair_store(s_ring[(k + 1) % NW], Fn);
-                    s_ring[(k + 1) % NW][12] = __int_as_float(abase + cnt);
-                }
-                ring_signal<NW>(k + 1);
-            } else if (lane == 0) {
-                s_total = abase + cnt;
-            }
-
-            const float org[3] = {F.p.x, F.p.y, F.p2};
-            PairFrame Fr = F;  // rotation only: positions relative to the chunk origin
-            Fr.p = make_float2(0.f, 0.f);
-            Fr.p2 = 0.f;
-            float *gdst = out + (size_t)3 * abase;
-            float *stg = stage + block_offset(gdst);  // the chunk's values keep their global 16-byte phase
-            if (live) {
-                const PairFrame P = compose_pair(Fr, E);
-                float *dst = stg + 3 * aoff;
-                residue_atoms_pair(tp, ty, P, cs, sn, chc, chs, [&](int slot, const float *x) {
-                    dst[3 * slot] = x[0] + org[0];
-                    dst[3 * slot + 1] = x[1] + org[1];
-                    dst[3 * slot + 2] = x[2] + org[2];
-                });
-                if (NAMES)
-                    for (int q = 0; q < na; q++) {
-                        sm.res_name[w][aoff + q] = tp.res_name[ty];
-                        sm.atom_name[w][aoff + q] = tp.atom_name[ty][q];
-                    }
-            }
-            __syncwarp();
-            const int nstore = max(0, min(cnt, a.maxA - abase));
-            copy_span<float, float4>(gdst, stage, 3 * nstore, lane);
-            if (NAMES)  // word stores: the names' own block phase would hold two more pointers through the walk
-                for (int i = lane; i < nstore; i += 32) {
-                    rn[abase + i] = sm.res_name[w][i];
-                    an[abase + i] = sm.atom_name[w][i];
-                }
-            __syncwarp();  // the warp's next chunk rewrites the staging buffers
+            for (int q = 0; q < 8; q++) cp_async4(abuf + q * kA2cChunk, src + (size_t)q * a.L);
         }
-        __syncthreads();
-        int total = s_total;
-        if (total > a.maxA) {
-            if (tid == 0) a2c_error(a.hdr, TPL_ERR_ATOMS);
-            total = a.maxA;
-        }
-        for (int i = 3 * total + tid; i < 3 * a.maxA; i += NT) out[i] = 0.f;
-        if (NAMES)
-            for (int i = total + tid; i < a.maxA; i += NT) rn[i] = an[i] = 0u;
-        __syncthreads();
+    };
+    if (b < nb) {
+        enter();
+        settle();
+        fetch();
     }
+#pragma unroll 1
+    while (b < nb) {
+        const int cb = b, ck = k, cnch = nch;
+        const int j = ck * kA2cChunk + lane;
+        const bool live = j < len, last = j + 1 >= len;
+        const uint32_t info = live ? tp.letter[letter] : 0u;
+        const int na = (info >> 8) & 0xff;
+        float ang[8];
+        cp_async_wait_all();
+#pragma unroll
+        for (int q = 0; q < 8; q++) ang[q] = live ? abuf[q * kA2cChunk] : 0.f;
+        if (last) ang[2] = 0.f;  // omega of the chain's last residue moves no atom
+        k += NW;
+        settle();
+        fetch();
+
+        // cos and sin of the eight angles, in pairs and for every lane at once (the chi
+        // angles' outside the divergent side-chain walk)
+        float cs[3], sn[3], chc[5], chs[5];
+        float m = 0.f;
+#pragma unroll
+        for (int q = 0; q < 8; q++) m = fmaxf(m, fabsf(ang[q]));
+        if (m <= 1.0e4f) {  // NaN passes: sincos_fast2 returns NaN for it
+            sincos_fast2(ang[0], ang[1], &sn[0], &cs[0], &sn[1], &cs[1]);
+            sincos_fast2(ang[2], ang[3], &sn[2], &cs[2], &chs[0], &chc[0]);
+            sincos_fast2(ang[4], ang[5], &chs[1], &chc[1], &chs[2], &chc[2]);
+            sincos_fast2(ang[6], ang[7], &chs[3], &chc[3], &chs[4], &chc[4]);
+        } else {
+#pragma unroll
+            for (int q = 0; q < 3; q++) sincos_poly(ang[q], &sn[q], &cs[q]);
+#pragma unroll
+            for (int q = 0; q < 5; q++) sincos_poly(ang[3 + q], &chs[q], &chc[q]);
+        }
+        PairFrame t = pair_identity();
+        if (live) {
+            apply_backbone<0>(t, cs[0], sn[0]);
+            apply_backbone<1>(t, cs[1], sn[1]);
+            apply_backbone<2>(t, cs[2], sn[2]);
+        }
+        PairFrame tot;
+        const PairFrame E = warp_exclusive_total_pair(t, lane, renorm != 0, tot);
+        int ci = na;  // atoms of the lanes up to this one
+#pragma unroll
+        for (int off = 1; off < 32; off <<= 1) {
+            const int o = __shfl_up_sync(0xffffffffu, ci, off);
+            if (lane >= off) ci += o;
+        }
+        const int cnt = __shfl_sync(0xffffffffu, ci, 31), aoff = ci - na;
+
+        PairFrame F = pair_identity();  // chain frame at the chunk start
+        int abase = 0;                  // first atom of the chunk
+        if (cb != (int)blockIdx.x || ck > 0) ring_wait<NW>(w);
+        if (ck > 0) {
+            F = pair_load(s_ring[w]);
+            abase = __float_as_int(s_ring[w][12]);
+        }
+        if (ck + 1 < cnch) {
+            PairFrame Fn = compose_pair(F, tot);
+            if (renorm) renormalize_pair(Fn);
+            if (lane == 0) {
+                pair_store(s_ring[(w + 1) % NW], Fn);
+                s_ring[(w + 1) % NW][12] = __int_as_float(abase + cnt);
+            }
+        }
+        if (ck + 1 < cnch || cb + (int)gridDim.x < nb) ring_signal<NW>((w + 1) % NW);
+
+        const float org[3] = {F.p.x, F.p.y, F.p2};
+        PairFrame Fr = F;  // rotation only: positions relative to the chunk origin
+        Fr.p = make_float2(0.f, 0.f);
+        Fr.p2 = 0.f;
+        float *out = a.coords + (size_t)cb * 3 * a.maxA;
+        float *gdst = out + (size_t)3 * abase;
+        float *stg = stage + block_offset(gdst);  // the chunk's values keep their global 16-byte phase
+        if (lane == 0) bulk_reads_done();
+        __syncwarp();  // the previous chunk has left the staging buffers
+        if (live) {
+            const PairFrame P = compose_pair(Fr, E);
+            float *dst = stg + 3 * aoff;
+            residue_atoms_pair(tp, info, P, cs, sn, chc, chs, [&](int slot, const float *x) {
+                dst[3 * slot] = x[0] + org[0];
+                dst[3 * slot + 1] = x[1] + org[1];
+                dst[3 * slot + 2] = x[2] + org[2];
+            });
+            if (NAMES) {
+                uint16_t *code = sm.code[NAMES ? w : 0] + aoff;
+                const int c0 = (int)(info & 0xff) << 4;
+#pragma unroll
+                for (int q = 0; q < kMaxResAtoms; q++)
+                    if (q < na) code[q] = (uint16_t)(c0 + q);
+            }
+        }
+        async_proxy_fence();
+        __syncwarp();
+        const int nstore = max(0, min(cnt, a.maxA - abase));
+        bulk_store_span(gdst, stg, 3 * nstore, lane);
+        uint32_t *rn = NAMES ? a.res_names + (size_t)cb * a.maxA : nullptr;
+        uint32_t *an = NAMES ? a.atom_names + (size_t)cb * a.maxA : nullptr;
+        if (NAMES) {
+            const uint16_t *code = sm.code[NAMES ? w : 0];
+            const uint32_t *atom_name = tp.atom_name[0];
+#pragma unroll 2
+            for (int i = lane; i < nstore; i += 32) {
+                const int c = code[i];
+                rn[abase + i] = tp.res_name[c >> 4];
+                an[abase + i] = atom_name[c];
+            }
+        }
+        if (ck + 1 == cnch) {  // the chain's last chunk also writes the zeros past its atoms
+            int total = abase + cnt;
+            if (total > a.maxA) {
+                if (lane == 0) a2c_error(a.hdr, TPL_ERR_ATOMS);
+                total = a.maxA;
+            }
+            zero_span(reinterpret_cast<uint32_t *>(out) + (size_t)3 * total, 3 * (a.maxA - total), lane);
+            if (NAMES) {
+                zero_span(rn + total, a.maxA - total, lane);
+                zero_span(an + total, a.maxA - total, lane);
+            }
+        }
+    }
+    if (lane == 0) bulk_reads_done();  // shared memory outlives the copies' reads
 }
 
 // ------------------------------------------------------------------ backward
@@ -949,239 +1090,304 @@ __device__ __forceinline__ void add_atom(const float *xs, const float *gs, const
     }
 }
 
-// The kernel: NW = 4 or 8 warps per chain on chunks of 32 residues (one per lane),
-// chunk k on warp (nchunk - 1 - k) % NW, last chunk first.  The chunks' first atom indices come from
-// one pass over the sequence at the start; per chunk a warp stages the chunk's atom
-// range of coordinates and dL/dx with coalesced loads, sums G and S over each
-// lane's residue about the chunk's first N atom, suffix-scans them over the warp
-// and takes the sums over later chunks from the warp of chunk k + 1 (G, S and that
-// chunk's first N atom, through the named-barrier handoff of tpl_pair.cuh).
-__device__ __forceinline__ void cp_async4(float *dst_smem, const float *src) {
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"((unsigned)__cvta_generic_to_shared(dst_smem)),
-                 "l"(src)
-                 : "memory");
+// The kernel: chunks of 32 residues, one per lane, last chunk first, dealt round NW = 4 or
+// 8 warps as one stream over the CTA's chains, as in a2c_fwd_ring_kernel (chains last to
+// first: the first CTAs read the rows the forward wrote last, which may still be in L2).
+// A warp finds the first atom of every chunk itself as it reads a chain's sequence.  Per
+// chunk it receives the atom range of coordinates and dL/dx in shared memory (one bulk
+// copy each of their whole 16-byte blocks, word copies of the ragged ends), walks each
+// lane's residue, suffix-scans the sums over the warp and takes the sums over later chunks
+// from the warp of chunk k + 1 (G, S and that chunk's first N atom, through the
+// named-barrier handoff of tpl_pair.cuh).  The buffers are free after the walk, so the
+// next chunk's copies run under the scan, the handoff and the stores.
+struct RingBwdJoint {
+    float inv_d;
+    int bits;  // atoms of the joint's group | index of its first side-chain atom << 8 | turned by a chi angle << 16
+};
+struct RingBwdTopology {
+    RingBwdJoint joint[kResTypes][kMaxScJoints];
+    uint16_t letter[256];  // type | atoms << 8; 0 for what is no residue letter
+};
+constexpr RingBwdTopology make_ring_bwd_topology() {
+    const Topology<float> tp = make_topology<float>();
+    RingBwdTopology r{};
+    for (int t = 0; t < kResTypes; t++) {
+        for (int k = 0; k < tp.njoints[t]; k++)
+            r.joint[t][k] = {1.f / tp.jd[t][k],
+                             tp.jna[t][k] | tp.jfirst[t][k] << 8 | (tp.jchi[t][k] < 0 ? 0 : 1 << 16)};
+        r.letter[(unsigned char)kResLetters[t]] = (uint16_t)(t | tp.natoms[t] << 8);
+    }
+    return r;
 }
-__device__ __forceinline__ void cp_async_wait_all() {
-    asm volatile("cp.async.commit_group;\ncp.async.wait_group 0;" ::: "memory");
-}
+__device__ const RingBwdTopology g_ring_bwd_topo = make_ring_bwd_topology();
 
 template <int NW>
 struct A2cBwdRingSmem {
-    Topology<float> topo;
-    signed char lut[256];
-    alignas(16) float x[NW][kA2cStageAtoms * 3 + 4];  // 4 floats of slack, as in A2cRingSmem
+    alignas(16) float x[NW][kA2cStageAtoms * 3 + 4];  // 4 words of slack for the 16-byte phase of the source
     alignas(16) float g[NW][kA2cStageAtoms * 3 + 4];
-    int base[1];  // first atom of each chunk, nchunk + 1 entries (dynamic)
+    RingBwdTopology topo;
+    int base[1];  // per warp: first atom of each chunk, max_chunks + 1 entries (dynamic)
 };
 
-__device__ __forceinline__ void cp_async16(float *dst_smem, const float *src) {
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((unsigned)__cvta_generic_to_shared(dst_smem)),
-                 "l"(src)
-                 : "memory");
+constexpr unsigned kA2cWaitPolls = 1u << 22;  // bounded mbarrier wait (about 0.5 s with the back-off)
+
+__device__ __forceinline__ unsigned smem_u32(const void *p) { return (unsigned)__cvta_generic_to_shared(p); }
+
+// Wait for the mbarrier phase of the given parity; false after kA2cWaitPolls polls.
+__device__ __forceinline__ bool a2c_mbar_wait(uint64_t *bar, unsigned parity) {
+    for (unsigned i = 0; i < kA2cWaitPolls; i++) {
+        unsigned done;
+        asm volatile(
+            "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}"
+            : "=r"(done)
+            : "r"(smem_u32(bar)), "r"(parity)
+            : "memory");
+        if (done) return true;
+        if (i >= 8) __nanosleep(100);
+    }
+    return false;
 }
 
-// Stage n floats of src into the 16-byte-aligned row dst, starting at
-// dst + block_offset(src), by the warp: 16-byte asynchronous copies for every block
-// of src that lies whole inside the span, 4-byte ones for the ragged ends.  Returns
-// where the values start.
-__device__ __forceinline__ float *stage_span_async(float *dst, const float *src, int n, int lane) {
-    const int sh = block_offset(src);
-    const float *base = src - sh;  // 16-byte aligned; only [src, src + n) is read
-    const int nb = (n + sh + 3) >> 2;
-    for (int b = lane; b < nb; b += 32) {
-        const int lo = 4 * b - sh;
-        if (lo >= 0 && lo + 4 <= n) {
-            cp_async16(dst + 4 * b, base + 4 * b);
-        } else {
-#pragma unroll
-            for (int e = 0; e < 4; e++)
-                if (lo + e >= 0 && lo + e < n) cp_async4(dst + sh + lo + e, src + lo + e);
-        }
+// The span [src, src + n) and its staging place dst + block_offset(src), dst 16-byte
+// aligned: `head` words before its whole 16-byte blocks, `body` words in them.
+struct StageSpan {
+    const float *src;
+    float *dst;
+    int head, body, tail;
+    __device__ __forceinline__ StageSpan(const float *s, float *row, int n) : src(s), dst(row + block_offset(s)) {
+        head = min((4 - block_offset(s)) & 3, n);
+        body = (n - head) & ~3;
+        tail = n - head - body;
     }
-    return dst + sh;
-}
+    __device__ __forceinline__ void ends(int lane) const {  // word copies outside the blocks (cp.async)
+        if (lane < head) cp_async4(dst + lane, src + lane);
+        if (lane < tail) cp_async4(dst + head + body + lane, src + head + body + lane);
+    }
+    __device__ __forceinline__ void blocks(uint64_t *bar) const {  // the blocks, by one lane
+        if (body > 0)
+            asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
+                             smem_u32(dst + head)),
+                         "l"(src + head), "r"(4 * body), "r"(smem_u32(bar))
+                         : "memory");
+    }
+};
 
 template <int NW>
-__global__ void __launch_bounds__(32 * NW) a2c_bwd_coords_ring_kernel(A2cArgs<float> a, int nb) {
+__global__ void __launch_bounds__(32 * NW) a2c_bwd_coords_ring_kernel(A2cArgs<float> a, int nb, int max_chunks) {
     constexpr int NT = 32 * NW;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     A2cBwdRingSmem<NW> &sm = *reinterpret_cast<A2cBwdRingSmem<NW> *>(smem_raw);
     __shared__ __align__(16) float s_ring[NW][12];
-    __shared__ int s_len, s_bad;
+    __shared__ __align__(8) uint64_t s_bar[NW];
 
-    // chains last to first: the first CTAs read the rows the forward wrote last, which may still be in L2
-    const int tid = threadIdx.x, w = tid >> 5, lane = tid & 31;
-    load_topology<float, NT>(sm.topo, sm.lut);
-    const Topology<float> &tp = sm.topo;
-    // persistent, as a2c_fwd_ring_kernel, counting down from the last chain (GB300,
-    // 4096 x 500: 0.199 -> 0.189 ms)
-    for (int b = nb - 1 - (int)blockIdx.x; b >= 0; b -= (int)gridDim.x) {
-        const unsigned char *row = a.seq + (size_t)b * a.seq_stride;
-        const int len = chain_length<NT>(row, a.seq_stride, sm.lut, &s_len, &s_bad);
-        float *gout = a.grad_angles + (size_t)b * 8 * a.L;
-        const float *xin = a.coords + (size_t)b * 3 * a.maxA;
-        const float *gin = a.grad_coords + (size_t)b * 3 * a.maxA;
-        bool ok = !s_bad && len <= a.L;
-        const int nchunk = ok ? (len + kA2cChunk - 1) / kA2cChunk : 0;
+    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    {
+        const uint32_t *src = reinterpret_cast<const uint32_t *>(&g_ring_bwd_topo);
+        for (int i = threadIdx.x; i < (int)(sizeof(RingBwdTopology) / 4); i += NT)
+            reinterpret_cast<uint32_t *>(&sm.topo)[i] = src[i];
+    }
+    if (lane == 0) {
+        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(&s_bar[w])) : "memory");
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    __syncthreads();
+    int *base = sm.base + w * (max_chunks + 1);
+    constexpr float inv_dphi = 1.f / kTopoF32.bb_d[0], inv_dpsi = 1.f / kTopoF32.bb_d[1],
+                    inv_dom = 1.f / kTopoF32.bb_d[2];
 
-        // atoms per chunk (warp w counts chunks w, w + 4, ...), then their exclusive prefix
-        for (int c = w; c < nchunk; c += NW) {
-            const int j = c * kA2cChunk + lane;
-            int n = j < len ? tp.natoms[sm.lut[row[j]]] : 0;
-#pragma unroll
-            for (int off = 16; off > 0; off >>= 1) n += __shfl_xor_sync(0xffffffffu, n, off);
-            if (lane == 0) sm.base[c + 1] = n;
+    // the warp's next chunk: the i-th of chain b counted from its last (length len, nch
+    // chunks; an empty or refused chain has one, which writes its zeros)
+    const int b_first = nb - 1 - (int)blockIdx.x;
+    int b = b_first, i = w, len = 0, nch = 0;
+    unsigned char letter = 0;
+    auto enter = [&]() {
+        int run = 0;
+        __syncwarp();  // every lane has read the bases of the chain before
+        len = ring_chain_length(a, b, sm.topo.letter, lane, [&](int c, int n) {
+            if (lane == 0 && c <= max_chunks) base[c] = run;
+            run += __reduce_add_sync(0xffffffffu, n);
+        });
+        if (len > 0 && run > a.maxA) {  // a chain whose atoms overflow the rows gets zeros
+            if (lane == 0) a2c_error(a.hdr, TPL_ERR_ATOMS);
+            len = 0;
         }
-        __syncthreads();
-        if (w == 0) {
-            int run = 0;
-            for (int c0 = 0; c0 < nchunk; c0 += 32) {
-                const int c = c0 + lane;
-                int v = c < nchunk ? sm.base[c + 1] : 0;
-#pragma unroll
-                for (int off = 1; off < 32; off <<= 1) {
-                    const int o = __shfl_up_sync(0xffffffffu, v, off);
-                    if (lane >= off) v += o;
-                }
-                if (c < nchunk) sm.base[c + 1] = run + v;
-                run += __shfl_sync(0xffffffffu, v, 31);
-            }
-            if (lane == 0) sm.base[0] = 0;
+        nch = max(1, (len + kA2cChunk - 1) / kA2cChunk);
+        if (lane == 0) {
+            if (len == 0) base[0] = run = 0;
+            base[nch] = run;
         }
-        __syncthreads();
-        const int total = nchunk > 0 ? sm.base[nchunk] : 0;
-        if (tid == 0) {
-            if (s_bad) a2c_error(a.hdr, TPL_ERR_SEQUENCE);
-            if (len > a.L) a2c_error(a.hdr, TPL_ERR_LENGTH);
-            if (ok && total > a.maxA) a2c_error(a.hdr, TPL_ERR_ATOMS);
+        __syncwarp();
+    };
+    auto settle = [&]() {
+        while (i >= nch) {
+            i -= nch;
+            b -= (int)gridDim.x;
+            if (b < 0) break;
+            enter();
         }
-        const int nrun = total > a.maxA ? 0 : nchunk;  // a chain whose atoms overflow the rows gets zeros
-        const float inv_dphi = 1.f / tp.bb_d[0], inv_dpsi = 1.f / tp.bb_d[1], inv_dom = 1.f / tp.bb_d[2];
-
+    };
+    bool failed = false;  // a bulk copy timed out: the remaining chunks only pass the carry on
+    auto fetch = [&]() {  // start the next chunk's copies
+        if (b < 0 || failed) return;
+        const int k = nch - 1 - i, j = k * kA2cChunk + lane, a0 = base[k], n3 = 3 * (base[k + 1] - a0);
+        if (j < len) letter = a.seq[(size_t)b * a.seq_stride + j];
+        const size_t at = (size_t)b * 3 * a.maxA + (size_t)3 * a0;
+        const StageSpan sx(a.coords + at, sm.x[w], n3), sg(a.grad_coords + at, sm.g[w], n3);
+        sx.ends(lane);
+        sg.ends(lane);
+        if (lane == 0) {
+            async_proxy_fence();  // the buffers were last read through the generic proxy
+            asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(&s_bar[w])),
+                         "r"(4 * (sx.body + sg.body))
+                         : "memory");
+            sx.blocks(&s_bar[w]);
+            sg.blocks(&s_bar[w]);
+        }
+    };
+    if (b >= 0) {
+        enter();
+        settle();
+        fetch();
+    }
+    unsigned parity = 0;
 #pragma unroll 1
-        for (int k = nrun - 1 - w; k >= 0; k -= NW) {
-            const int j = k * kA2cChunk + lane;
-            const bool live = j < len;
-            const int ty = live ? sm.lut[row[j]] : 0;
-            const int na = live ? tp.natoms[ty] : 0;
-            int inc = na;  // the residue's first atom inside the chunk: warp exclusive scan
+    while (b >= 0) {
+        const int cb = b, clen = len, k = nch - 1 - i, j = k * kA2cChunk + lane;
+        const bool live = j < clen;
+        const unsigned info = live ? sm.topo.letter[letter] : 0u;
+        const int ty = info & 0xff, na = info >> 8;
+        int inc = na;  // the residue's first atom inside the chunk: warp exclusive scan
 #pragma unroll
-            for (int off = 1; off < 32; off <<= 1) {
-                const int v = __shfl_up_sync(0xffffffffu, inc, off);
-                if (lane >= off) inc += v;
-            }
-            const int aoff = inc - na;
-            const int abase = sm.base[k], n3 = 3 * (sm.base[k + 1] - abase);
-            __syncwarp();  // the previous chunk's reads of the staging buffers are done
-            // asynchronous copies: every copy of the chunk is in flight before the one wait
-            const float *sx = stage_span_async(sm.x[w], xin + (size_t)3 * abase, n3, lane);
-            const float *sg = stage_span_async(sm.g[w], gin + (size_t)3 * abase, n3, lane);
+        for (int off = 1; off < 32; off <<= 1) {
+            const int v = __shfl_up_sync(0xffffffffu, inc, off);
+            if (lane >= off) inc += v;
+        }
+        const int aoff = inc - na;
+        const size_t at = (size_t)cb * 3 * a.maxA + (size_t)3 * base[k];
+        const float *sx = sm.x[w] + block_offset(a.coords + at), *sg = sm.g[w] + block_offset(a.grad_coords + at);
+        if (!failed) {
             cp_async_wait_all();
-            __syncwarp();
-            const float o[3] = {sx[0], sx[1], sx[2]};  // chunk origin: its first N atom
-            // One walk over the residue's atoms, last to first, from G = S = 0.  Every
-            // joint gradient u . (S - o x G) is linear in (G, S), so each joint's share of
-            // its own residue is taken here and the share of the later residues is added
-            // after the scan: complete for the chi joints (side-chain atoms only), and
-            // the own parts of psi and phi.  The walk ends with the residue's totals.
-            float v[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-            float gr[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-            float xN[3] = {0.f, 0.f, 0.f}, xA[3] = {0.f, 0.f, 0.f}, xC[3] = {0.f, 0.f, 0.f};
-            if (live) {
-                const float *X = sx + 3 * aoff, *Gg = sg + 3 * aoff;
-#pragma unroll
-                for (int c = 0; c < 3; c++) {
-                    xN[c] = X[c] - o[c];
-                    xA[c] = X[3 + c] - o[c];
-                    xC[c] = X[3 * (na - 2) + c] - o[c];
-                }
-                float *G = v, *S = v + 3;
-                add_atom(X + 3 * (na - 1), Gg + 3 * (na - 1), o, G, S);  // O
-                gr[1] = joint_grad(xC, xA, inv_dpsi, G, S);
-                add_atom(X + 3 * (na - 2), Gg + 3 * (na - 2), o, G, S);  // C
-                // side chain, groups last to first; chi subtrees hold side-chain atoms only
-                float Gs[3] = {0.f, 0.f, 0.f}, Ss[3] = {0.f, 0.f, 0.f};
-                const int nj = tp.njoints[ty];
-                if (nj == 0)
-                    for (int q = 2; q < na - 2; q++) add_atom(X + 3 * q, Gg + 3 * q, o, Gs, Ss);  // Pro ring (none for Gly)
-                // unrolled over the joints: joint kk reads chi angle kk or none (Ala;
-                // topology_layout_ok), so its gradient goes to a register, not a select
-#pragma unroll
-                for (int kk = kMaxScJoints - 1; kk >= 0; kk--) {
-                    if (kk >= nj) continue;
-                    const int f0 = 2 + tp.jfirst[ty][kk], f1 = f0 + tp.jna[ty][kk];
-                    for (int q = f1 - 1; q >= f0; q--) add_atom(X + 3 * q, Gg + 3 * q, o, Gs, Ss);
-                    if (tp.jchi[ty][kk] >= 0) {
-                        const float *pk = X + 3 * f0;
-                        const float *pp = kk == 0 ? X + 3 : X + 3 * (2 + tp.jfirst[ty][kk - 1]);
-                        const float ok_[3] = {pk[0] - o[0], pk[1] - o[1], pk[2] - o[2]};
-                        const float op_[3] = {pp[0] - o[0], pp[1] - o[1], pp[2] - o[2]};
-                        gr[3 + kk] = joint_grad(ok_, op_, 1.f / tp.jd[ty][kk], Gs, Ss);
-                    }
-                }
-#pragma unroll
-                for (int c = 0; c < 3; c++) {
-                    G[c] += Gs[c];
-                    S[c] += Ss[c];
-                }
-                gr[0] = joint_grad(xA, xN, inv_dphi, G, S);
-                add_atom(X + 3, Gg + 3, o, G, S);  // CA
-                add_atom(X, Gg, o, G, S);          // N
+            const bool ok = a2c_mbar_wait(&s_bar[w], parity);
+            if (!__all_sync(0xffffffffu, ok)) {
+                if (lane == 0) a2c_error(a.hdr, TPL_ERR_LOOKBACK_TIMEOUT);
+                (void)a2c_mbar_wait(&s_bar[w], parity);  // bounded: let the copies in flight land
+                failed = true;
             }
-            float later[6], ctot[6];
+            parity ^= 1u;
+        }
+        __syncwarp();  // every lane's word copies have landed
+        // One walk over the residue's atoms, last to first, from G = S = 0.  Every
+        // joint gradient u . (S - o x G) is linear in (G, S), so each joint's share of
+        // its own residue is taken here and the share of the later residues is added
+        // after the scan: complete for the chi joints (side-chain atoms only), and
+        // the own parts of psi and phi.  The walk ends with the residue's totals.
+        float o[3] = {0.f, 0.f, 0.f};  // chunk origin: its first N atom
+        float v[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+        float gr[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+        float xN[3] = {0.f, 0.f, 0.f}, xA[3] = {0.f, 0.f, 0.f}, xC[3] = {0.f, 0.f, 0.f};
+        if (live && !failed) {
 #pragma unroll
-            for (int i = 0; i < 6; i++) later[i] = suffix_excl(v[i], lane, ctot[i]);
-            // the sums over later chunks, moved to this chunk's origin: S_o = S_on + (on - o) x G
-            float Gc[3] = {0.f, 0.f, 0.f}, Sc[3] = {0.f, 0.f, 0.f}, nN[3] = {0.f, 0.f, 0.f};
-            if (k + 1 < nrun) {
-                ring_wait<NW>(k);
-                const float *cin = s_ring[k % NW];
+            for (int c = 0; c < 3; c++) o[c] = sx[c];
+            const float *X = sx + 3 * aoff, *Gg = sg + 3 * aoff;
 #pragma unroll
-                for (int c = 0; c < 3; c++) {
-                    Gc[c] = cin[c];
-                    Sc[c] = cin[3 + c];
-                    nN[c] = cin[6 + c];
-                }
-                const float d[3] = {nN[0] - o[0], nN[1] - o[1], nN[2] - o[2]};
-                float dx[3];
-                cross3(d, Gc, dx);
-#pragma unroll
-                for (int c = 0; c < 3; c++) Sc[c] += dx[c];
+            for (int c = 0; c < 3; c++) {
+                xN[c] = X[c] - o[c];
+                xA[c] = X[3 + c] - o[c];
+                xC[c] = X[3 * (na - 2) + c] - o[c];
             }
-            if (k > 0) {
-                if (lane == 0) {
-                    float *cout = s_ring[(k - 1) % NW];
+            float *G = v, *S = v + 3;
+            add_atom(X + 3 * (na - 1), Gg + 3 * (na - 1), o, G, S);  // O
+            gr[1] = joint_grad(xC, xA, inv_dpsi, G, S);
+            add_atom(X + 3 * (na - 2), Gg + 3 * (na - 2), o, G, S);  // C
+            // side chain, groups last to first; chi subtrees hold side-chain atoms only
+            float Gs[3] = {0.f, 0.f, 0.f}, Ss[3] = {0.f, 0.f, 0.f};
+            RingBwdJoint jt[kMaxScJoints];
 #pragma unroll
-                    for (int c = 0; c < 3; c++) {
-                        cout[c] = Gc[c] + ctot[c];
-                        cout[3 + c] = Sc[c] + ctot[3 + c];
-                        cout[6 + c] = o[c];
-                    }
+            for (int kk = 0; kk < kMaxScJoints; kk++) jt[kk] = sm.topo.joint[ty][kk];
+            if (jt[0].bits == 0)  // no side-chain joint: the Pro ring (nothing for Gly)
+                for (int q = 2; q < na - 2; q++) add_atom(X + 3 * q, Gg + 3 * q, o, Gs, Ss);
+            // unrolled over the joints: joint kk reads chi angle kk or none (Ala;
+            // topology_layout_ok), so its gradient goes to a register, not a select
+#pragma unroll
+            for (int kk = kMaxScJoints - 1; kk >= 0; kk--) {
+                if (jt[kk].bits == 0) continue;
+                const int f0 = 2 + ((jt[kk].bits >> 8) & 0xff), f1 = f0 + (jt[kk].bits & 0xff);
+                for (int q = f1 - 1; q >= f0; q--) add_atom(X + 3 * q, Gg + 3 * q, o, Gs, Ss);
+                if (jt[kk].bits >> 16) {
+                    const float *pk = X + 3 * f0;
+                    const float *pp = kk == 0 ? X + 3 : X + 3 * (2 + ((jt[kk > 0 ? kk - 1 : 0].bits >> 8) & 0xff));
+                    const float ok_[3] = {pk[0] - o[0], pk[1] - o[1], pk[2] - o[2]};
+                    const float op_[3] = {pp[0] - o[0], pp[1] - o[1], pp[2] - o[2]};
+                    gr[3 + kk] = joint_grad(ok_, op_, jt[kk].inv_d, Gs, Ss);
                 }
-                ring_signal<NW>(k - 1);
             }
-            if (live) {
-                // the later residues' share: sums over every atom after this residue
-                const float G[3] = {later[0] + Gc[0], later[1] + Gc[1], later[2] + Gc[2]};
-                const float S[3] = {later[3] + Sc[0], later[4] + Sc[1], later[5] + Sc[2]};
-                if (j + 1 < len) {  // omega_j: the next residue's N joint (the next chunk's first N after lane 31)
-                    const float *X = sx + 3 * aoff;
-                    float xn[3];
 #pragma unroll
-                    for (int c = 0; c < 3; c++) xn[c] = (lane == 31 ? nN[c] : X[3 * na + c]) - o[c];
-                    gr[2] = joint_grad(xn, xC, inv_dom, G, S);
-                }
-                gr[1] += joint_grad(xC, xA, inv_dpsi, G, S);
-                gr[0] += joint_grad(xA, xN, inv_dphi, G, S);
+            for (int c = 0; c < 3; c++) {
+                G[c] += Gs[c];
+                S[c] += Ss[c];
+            }
+            gr[0] = joint_grad(xA, xN, inv_dphi, G, S);
+            add_atom(X + 3, Gg + 3, o, G, S);  // CA
+            add_atom(X, Gg, o, G, S);          // N
+        }
 #pragma unroll
-                for (int q = 0; q < 8; q++) gout[(size_t)q * a.L + j] = gr[q];
+        for (int c = 0; c < 3; c++) o[c] = __shfl_sync(0xffffffffu, o[c], 0);  // lane 0 is live in every chunk but an empty one
+        // the walk was the last to read the buffers: the next chunk's copies may start
+        const bool more = i + 1 < nch || b - (int)gridDim.x >= 0;  // the stream goes on after this chunk
+        const bool first = cb == b_first && i == 0, top = i == 0;   // first of the stream, last chunk of its chain
+        __syncwarp();
+        i += NW;
+        settle();
+        fetch();
+
+        float later[6], ctot[6];
+#pragma unroll
+        for (int q = 0; q < 6; q++) later[q] = suffix_excl(v[q], lane, ctot[q]);
+        float xn[3];  // the next residue's N: the next lane's
+#pragma unroll
+        for (int c = 0; c < 3; c++) xn[c] = __shfl_down_sync(0xffffffffu, xN[c], 1);
+        // the sums over later chunks, moved to this chunk's origin: S_o = S_on + (on - o) x G
+        float Gc[3] = {0.f, 0.f, 0.f}, Sc[3] = {0.f, 0.f, 0.f};
+        if (!first) ring_wait<NW>(w);
+        if (!top) {
+            const float *cin = s_ring[w];
+            float d[3], dx[3];
+#pragma unroll
+            for (int c = 0; c < 3; c++) {
+                Gc[c] = cin[c];
+                Sc[c] = cin[3 + c];
+                d[c] = cin[6 + c] - o[c];
+                if (lane == 31) xn[c] = d[c];  // the next chunk's first N
+            }
+            cross3(d, Gc, dx);
+#pragma unroll
+            for (int c = 0; c < 3; c++) Sc[c] += dx[c];
+        }
+        if (k > 0 && lane == 0) {
+            float *cout = s_ring[(w + 1) % NW];
+#pragma unroll
+            for (int c = 0; c < 3; c++) {
+                cout[c] = Gc[c] + ctot[c];
+                cout[3 + c] = Sc[c] + ctot[3 + c];
+                cout[6 + c] = o[c];
             }
         }
-        // zeros past the chain (and everywhere when the chain was rejected)
-        const int from = nrun > 0 ? len : 0;
-        for (int q = 0; q < 8; q++)
-            for (int i = from + tid; i < a.L; i += NT) gout[(size_t)q * a.L + i] = 0.f;
-        __syncthreads();
+        if (more) ring_signal<NW>((w + 1) % NW);
+        float *gout = a.grad_angles + (size_t)cb * 8 * a.L;
+        if (live && !failed) {
+            // the later residues' share: sums over every atom after this residue
+            const float G[3] = {later[0] + Gc[0], later[1] + Gc[1], later[2] + Gc[2]};
+            const float S[3] = {later[3] + Sc[0], later[4] + Sc[1], later[5] + Sc[2]};
+            if (j + 1 < clen) gr[2] = joint_grad(xn, xC, inv_dom, G, S);  // omega_j
+            gr[1] += joint_grad(xC, xA, inv_dpsi, G, S);
+            gr[0] += joint_grad(xA, xN, inv_dphi, G, S);
+#pragma unroll
+            for (int q = 0; q < 8; q++) gout[(size_t)q * a.L + j] = gr[q];
+        }
+        if (top)  // zeros past the chain (and everywhere when it was refused)
+#pragma unroll 1
+            for (int q = 0; q < 8; q++)
+                zero_span(reinterpret_cast<uint32_t *>(gout) + (size_t)q * a.L + clen, a.L - clen, lane);
     }
 }
 
@@ -1222,7 +1428,7 @@ static int a2c_ring_warps(int B, int chains_per_sm) { return B < chains_per_sm *
 template <int NW>
 static int launch_a2c_fwd_ring(const A2cArgs<float> &a, int B, int renorm, cudaStream_t st) {
     const bool names = a.res_names && a.atom_names;
-    const size_t smem = names ? sizeof(A2cRingSmem<NW>) : a2c_ring_smem_no_names<NW>();
+    const size_t smem = names ? sizeof(A2cRingSmem<NW, true>) : sizeof(A2cRingSmem<NW, false>);
     auto k = names ? a2c_fwd_ring_kernel<NW, true> : a2c_fwd_ring_kernel<NW, false>;
     if (!set_max_dynamic_smem(reinterpret_cast<const void *>(k), (int)smem))
         return TPL_ERR_LAUNCH;
@@ -1235,14 +1441,15 @@ static int launch_a2c_fwd_ring(const A2cArgs<float> &a, int B, int renorm, cudaS
 
 template <int NW>
 static int launch_a2c_bwd_coords_ring(const A2cArgs<float> &a, int B, int L, cudaStream_t st) {
-    const size_t smem = offsetof(A2cBwdRingSmem<NW>, base) + sizeof(int) * (size_t)((L + kA2cChunk - 1) / kA2cChunk + 1);
+    const int max_chunks = std::max(1, (L + kA2cChunk - 1) / kA2cChunk);
+    const size_t smem = offsetof(A2cBwdRingSmem<NW>, base) + sizeof(int) * (size_t)NW * (size_t)(max_chunks + 1);
     auto k = a2c_bwd_coords_ring_kernel<NW>;
     if (!set_max_dynamic_smem(reinterpret_cast<const void *>(k), (int)smem))
         return TPL_ERR_LAUNCH;
     int per_sm = 0;
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, 32 * NW, smem) != cudaSuccess || per_sm < 1) per_sm = 1;
     const int grid = std::min(B, per_sm * device_sm_count());
-    k<<<grid, 32 * NW, smem, st>>>(a, B);
+    k<<<grid, 32 * NW, smem, st>>>(a, B, max_chunks);
     return cudaGetLastError() == cudaSuccess ? TPL_OK : TPL_ERR_LAUNCH;
 }
 
