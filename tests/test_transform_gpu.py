@@ -112,3 +112,45 @@ def test_center_vector_and_scalar_paths(ct, S):
     x[4] += 500.0
     c = ct.Coords2Center()(torch.tensor(x, device="cuda"), torch.tensor(na)).cpu().numpy()
     assert np.abs(c - oracle.coords_center(x, na)).max() <= 1e-6 * np.abs(x).max()
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float64])
+@pytest.mark.parametrize("S,offs", [(1, (0, 0)), (3, (0, 0)), (5, (1, 1)), (127, (0, 0)), (128, (2, 2)), (129, (3, 3)),
+                                    (130, (0, 0)), (131, (0, 1)), (1027, (0, 0))])
+def test_rows_at_every_alignment(ct, dtype, S, offs):
+    """Rows that start at every place of a 16-byte block (odd strides, storage offsets of
+    the input and, through the extension entries, of the output, alike or not) and sizes
+    around the vector groups and warp tiles, with every count from 0 to 9 atoms and a full
+    row: translate, its backward, the centre's backward and the box bit for bit; rotate and
+    centre to the tolerances of the file."""
+    from torchproteinlibrary_gb300 import load_extension
+    fm = load_extension("_FullAtomModel")
+    x, na, T, R = case(dtype, B=14, S=S, seed=S)
+    na[:] = np.minimum(np.arange(14) - 1, S)
+    na[0] = na[13] = S
+    dev, scale = torch.device("cuda"), np.abs(x).max()
+
+    def at(v, off):
+        v = np.asarray(v)
+        t = torch.empty(v.size + off, dtype=dtype, device=dev)[off:].view(v.shape)
+        return t.copy_(torch.tensor(v))
+
+    xt, nat, Tt, Rt = at(x, offs[0]), torch.tensor(na, device=dev), at(T, 0), at(R, 0)
+    out = at(np.full_like(x, 7.0), offs[1])
+    fm.CoordsTranslateGPU_forward(xt, out, Tt, nat)
+    assert np.array_equal(out.cpu().numpy(), oracle.coords_translate(x, T, na))
+    fm.CoordsTranslateGPU_backward(xt, out, Tt, nat)
+    assert np.array_equal(out.cpu().numpy(), oracle.coords_translate(x, None, na))
+    tol = 2e-6 if dtype == torch.float32 else 1e-12
+    fm.CoordsRotateGPU_forward(xt, out, Rt, nat)
+    assert np.abs(out.cpu().numpy() - oracle.coords_rotate(x, R, na)).max() <= tol * scale
+    fm.CoordsRotateGPU_backward(xt, out, Rt, nat)
+    assert np.abs(out.cpu().numpy() - oracle.coords_rotate(x, R, na, transpose=True)).max() <= tol * scale
+    c = ct.Coords2Center()(xt, nat)
+    assert np.abs(c.cpu().numpy() - oracle.coords_center(x, na)).max() <= (1e-6 if dtype == torch.float32 else 1e-12) * scale
+    fm.Coords2CenterGPU_backward(Tt, out, nat)
+    assert np.allclose(out.cpu().numpy(), oracle.coords_center_backward(T, na, S),
+                       rtol=1e-6 if dtype == torch.float32 else 1e-14, atol=0)
+    a, b = ct.getBBox(xt, nat)
+    ra, rb = oracle.coords_bbox(x, na)
+    assert np.array_equal(a.cpu().numpy(), ra) and np.array_equal(b.cpu().numpy(), rb)

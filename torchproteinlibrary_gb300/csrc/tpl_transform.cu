@@ -7,29 +7,25 @@
 // batch_size <= 1024) and sums each centroid serially in one thread; the bounding
 // box runs on the CPU (Layers/FullAtomModel/CoordsTransform/
 // coordsTransform_interface.cpp:175-200, Math/nUtil.cpp:27-57).  Here the
-// elementwise transforms are flat, coalesced, 16-byte-vectorised passes over the
-// whole batch (HBM-bound: 2 x 12 B per atom in FP32), and centroid and box are
-// block reductions, one CTA per chain.
+// elementwise transforms are coalesced, 16-byte-vectorised passes over the batch
+// (HBM-bound: 2 x 12 B per atom in FP32; padding atoms are written, not read), and
+// centroid and box are block reductions, one CTA per chain.
+//
+// A row starts at any place of a 16-byte block (3 * atoms_stride is a multiple of four
+// for one stride in four), so every kernel takes the few elements or atoms before the
+// row's first boundary and after its last one by themselves and moves the rest as
+// vectors.  Scalar passes over such rows had been issue-bound: 4096 rows of 1000..3471
+// atoms, stride 3471 (41 us of HBM traffic each): translate 70 -> 39 us, rotate 54 -> 46 us,
+// box 25 -> 22 us.
 #include <cfloat>
 #include <cmath>
+#include <cstring>
 
 #include "tpl_internal.h"
+#include "tpl_rows.cuh"
 
 namespace tpl {
 namespace {
-
-template <typename T>
-struct Vec16;
-template <>
-struct Vec16<float> {
-    using type = float4;
-    static constexpr int n = 4;
-};
-template <>
-struct Vec16<double> {
-    using type = double2;
-    static constexpr int n = 2;
-};
 
 constexpr int kUnroll = 4;  // vectors in flight per thread in the elementwise passes
 
@@ -50,8 +46,8 @@ __device__ __forceinline__ void store16(T *p, const T (&v)[Vec16<T>::n]) {
 // for e < 3 n_b, 0 after.  Covers translate (add = T), its backward (add = null),
 // and the centre's backward (in = null, add = dL/dcentre, scaled by 1 / n_b).
 // Grid: y over rows (strided), x over pieces of a row, so no thread divides by the
-// row length; VEC: 16-byte vectors inside a row (3 * atoms_stride a multiple of the
-// vector width and 16-byte-aligned rows).
+// row length.  Between the row's first and last 16-byte boundary elements move as
+// vectors when `in` and `out` have the same alignment; the others one by one.
 struct ShiftArgs {
     const void *in;
     void *out;
@@ -62,14 +58,14 @@ struct ShiftArgs {
     int scale_by_count;
 };
 
-template <typename T, bool VEC>
+template <typename T>
 __global__ void __launch_bounds__(256) shift_kernel(ShiftArgs a) {
-    constexpr int N = VEC ? Vec16<T>::n : 1;
-    const T *in = static_cast<const T *>(a.in);
-    T *out = static_cast<T *>(a.out);
+    constexpr int N = Vec16<T>::n;
     const T *add = static_cast<const T *>(a.add);
-    const int nv = a.row / N;  // vectors per row
+    const int step = gridDim.x * blockDim.x, first = blockIdx.x * blockDim.x + threadIdx.x;
     for (int b = blockIdx.y; b < a.B; b += gridDim.y) {
+        const T *in = a.in ? static_cast<const T *>(a.in) + (size_t)b * a.row : nullptr;
+        T *out = static_cast<T *>(a.out) + (size_t)b * a.row;
         const int n = max(0, min(a.num_atoms[b], a.row / 3)), n3 = 3 * n;
         T t[3] = {T(0), T(0), T(0)};
         if (add)
@@ -77,98 +73,139 @@ __global__ void __launch_bounds__(256) shift_kernel(ShiftArgs a) {
                 t[k] = add[3 * (size_t)b + k];
                 if (a.scale_by_count && n > 0) t[k] = t[k] / T(n);
             }
-        const size_t base = (size_t)b * a.row;
+        auto pick = [&](int r) { return r == 0 ? t[0] : (r == 1 ? t[1] : t[2]); };
+        const int off = row_head(out);  // elements of `out` since a 16-byte boundary
+        const int head = in && row_head(in) != off ? a.row : min((N - off) & (N - 1), a.row);
+        const int nv = (a.row - head) / N;
         // kUnroll independent vectors per thread and step: loads issued before use
-        const int step = gridDim.x * blockDim.x;
-        for (int v0 = blockIdx.x * blockDim.x + threadIdx.x; v0 < nv; v0 += kUnroll * step) {
-            T x[kUnroll][Vec16<T>::n];
+        for (int v0 = first; v0 < nv; v0 += kUnroll * step) {
+            T x[kUnroll][N];
 #pragma unroll
             for (int u = 0; u < kUnroll; u++) {
-                const int v = v0 + u * step;
-                if (v >= nv) continue;
-                if (VEC) {
-                    if (in) load16(in + base + (size_t)v * N, x[u]);
-                    else
-                        for (int k = 0; k < N; k++) x[u][k] = T(0);
-                } else {
-                    x[u][0] = in ? __ldcs(in + base + v) : T(0);
-                }
+                const int v = v0 + u * step, e = head + v * N;
+                if (in && v < nv && e < n3) load16(in + e, x[u]);
+                else
+                    for (int k = 0; k < N; k++) x[u][k] = T(0);
             }
 #pragma unroll
             for (int u = 0; u < kUnroll; u++) {
                 const int v = v0 + u * step;
                 if (v >= nv) continue;
+                const int e = head + v * N, r = e % 3;
+                const T te[3] = {pick(r), pick(r == 2 ? 0 : r + 1), pick(r == 0 ? 2 : r - 1)};
 #pragma unroll
-                for (int k = 0; k < N; k++) {
-                    const int e = v * N + k;
-                    x[u][k] = e < n3 ? x[u][k] + t[e % 3] : T(0);
-                }
-                if (VEC) store16(out + base + (size_t)v * N, x[u]);
-                else __stcs(out + base + v, x[u][0]);
+                for (int k = 0; k < N; k++) x[u][k] = e + k < n3 ? x[u][k] + te[k % 3] : T(0);
+                store16(out + e, x[u]);
+            }
+        }
+        // the elements outside the vectors
+        const int rest = a.row - nv * N;
+        for (int i0 = first; i0 < rest; i0 += kUnroll * step) {
+            T x[kUnroll];
+#pragma unroll
+            for (int u = 0; u < kUnroll; u++) {
+                const int i = i0 + u * step, e = i < head ? i : i + nv * N;
+                x[u] = in && i < rest && e < n3 ? __ldcs(in + e) : T(0);
+            }
+#pragma unroll
+            for (int u = 0; u < kUnroll; u++) {
+                const int i = i0 + u * step, e = i < head ? i : i + nv * N;
+                if (i < rest) __stcs(out + e, e < n3 ? x[u] + pick(e % 3) : T(0));
             }
         }
     }
 }
 
 // out[b, atom] = R_b x (or R_b^T x) for atom < n_b, 0 after; R row-major [B, 3, 3].
-// Grid: y over rows (strided), x over atoms of a row.
+// Grid: y over rows (strided), x over pieces of 512 aligned groups of N atoms
+// (tpl_rows.cuh), two tiles of 32 groups per warp whose loads are in flight together (one
+// tile: 54 us; the launch is then bound by the latency of its many short blocks).  A warp loads and stores its tile as 96 vectors in
+// memory order and turns it to one group per lane and back through shared memory: with a
+// group per lane straight from memory every 32-byte sector is written in two pieces
+// (strides of 48 bytes), with an atom per lane in three.  48-byte lane strides are free of
+// bank conflicts.  Atoms outside the groups, and rows whose input and output differ in
+// alignment, are taken one by one.
 template <typename T>
 __global__ void __launch_bounds__(256) rotate_kernel(const T *in, T *out, const T *R, const int *num_atoms, int B,
                                                      int stride, int transpose) {
+    constexpr int N = Vec16<T>::n;
+    using V = typename Vec16<T>::type;
+    __shared__ V s_tile[8][96];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    V *tile = s_tile[w];
     for (int b = blockIdx.y; b < B; b += gridDim.y) {
-        const int n = num_atoms[b];
+        const int n = min(num_atoms[b], stride);
         T m[9];
         for (int k = 0; k < 9; k++) m[k] = R[9 * (size_t)b + (transpose ? 3 * (k % 3) + k / 3 : k)];
         const T *x = in + (size_t)b * 3 * stride;
         T *y = out + (size_t)b * 3 * stride;
-        const int step = gridDim.x * blockDim.x;
-        for (int i0 = blockIdx.x * blockDim.x + threadIdx.x; i0 < stride; i0 += kUnroll * step) {
-            T v[kUnroll][3];
+        auto turn = [&](const T *v, T *r) {
+            const T x0 = v[0], x1 = v[1], x2 = v[2];
+            r[0] = m[0] * x0 + m[1] * x1 + m[2] * x2;
+            r[1] = m[3] * x0 + m[4] * x1 + m[5] * x2;
+            r[2] = m[6] * x0 + m[7] * x1 + m[8] * x2;
+        };
+        const int off = row_head(y);
+        const int head = row_head(x) != off ? stride : min(off, stride);
+        const int ng = (stride - head) / N;
+        const V *src = reinterpret_cast<const V *>(x + 3 * head);  // vector k of group g is 3 g + k
+        V *dst = reinterpret_cast<V *>(y + 3 * head);
+        const int nvec = 3 * ng, live = 3 * (n - head);  // vectors of the groups; values that hold atoms
+        for (int g0 = blockIdx.x * 512 + 32 * w; g0 < ng; g0 += gridDim.x * 512) {
+            V v[2][3];
 #pragma unroll
-            for (int u = 0; u < kUnroll; u++) {  // loads of kUnroll atoms in flight
-                const int i = i0 + u * step;
-                if (i < min(n, stride))
-                    for (int k = 0; k < 3; k++) v[u][k] = __ldcs(x + 3 * i + k);
-            }
+            for (int u = 0; u < 2; u++)
 #pragma unroll
-            for (int u = 0; u < kUnroll; u++) {
-                const int i = i0 + u * step;
-                if (i >= stride) continue;
-                T r0 = T(0), r1 = T(0), r2 = T(0);
-                if (i < n) {
-                    const T x0 = v[u][0], x1 = v[u][1], x2 = v[u][2];
-                    r0 = m[0] * x0 + m[1] * x1 + m[2] * x2;
-                    r1 = m[3] * x0 + m[4] * x1 + m[5] * x2;
-                    r2 = m[6] * x0 + m[7] * x1 + m[8] * x2;
+                for (int q = 0; q < 3; q++) {
+                    const int k = 3 * (g0 + 256 * u) + lane + 32 * q;
+                    if (k < nvec && k * N < live) v[u][q] = __ldcs(src + k);
+                    else memset(&v[u][q], 0, sizeof(V));
                 }
-                __stcs(y + 3 * i, r0);
-                __stcs(y + 3 * i + 1, r1);
-                __stcs(y + 3 * i + 2, r2);
+#pragma unroll
+            for (int u = 0; u < 2; u++) {
+                const int g = g0 + 256 * u;
+                if (3 * g * N < live) {  // the same for the whole warp
+#pragma unroll
+                    for (int q = 0; q < 3; q++) tile[lane + 32 * q] = v[u][q];
+                    __syncwarp();
+                    T p[3 * N];
+                    load_group(reinterpret_cast<const T *>(tile + 3 * lane), p);
+                    const int left = n - head - N * (g + lane);  // atoms from this lane's group on
+#pragma unroll
+                    for (int q = 0; q < N; q++) {
+                        if (q < left) turn(p + 3 * q, p + 3 * q);
+                        else p[3 * q] = p[3 * q + 1] = p[3 * q + 2] = T(0);
+                    }
+                    store_group(reinterpret_cast<T *>(tile + 3 * lane), p);
+                    __syncwarp();
+#pragma unroll
+                    for (int q = 0; q < 3; q++) v[u][q] = tile[lane + 32 * q];
+                    __syncwarp();  // the next tile rewrites it
+                }
+#pragma unroll
+                for (int q = 0; q < 3; q++) {
+                    const int k = 3 * g + lane + 32 * q;
+                    if (k < nvec) __stcs(dst + k, v[u][q]);
+                }
             }
+        }
+        const int rest = stride - N * ng;
+        for (int i0 = blockIdx.x * 256 + threadIdx.x; i0 < rest; i0 += gridDim.x * 256) {
+            const int i = i0 < head ? i0 : i0 + N * ng;
+            T r[3] = {T(0), T(0), T(0)};
+            if (i < n) turn(x + 3 * i, r);
+            for (int k = 0; k < 3; k++) y[3 * i + k] = r[k];
         }
     }
 }
 
 constexpr int kReduceThreads = 256;
 
-template <typename R, typename Op>
-__device__ __forceinline__ R block_reduce(R v, Op op, R *s_warp) {
-#pragma unroll
-    for (int off = 16; off > 0; off >>= 1) v = op(v, __shfl_xor_sync(0xffffffffu, v, off));
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    if (lane == 0) s_warp[w] = v;
-    __syncthreads();
-    R r = s_warp[0];
-    for (int k = 1; k < kReduceThreads / 32; k++) r = op(r, s_warp[k]);
-    __syncthreads();  // s_warp is reused by the next reduction
-    return r;
-}
-
 // Centroid of the first n_b atoms of chain b = blockIdx.x (FP64 accumulation);
 // 0 for an empty chain.
 template <typename T>
 __global__ void __launch_bounds__(kReduceThreads) center_kernel(const T *in, T *center, const int *num_atoms,
-                                                                int stride, int vec) {
+                                                                int stride) {
     constexpr int NW = kReduceThreads / 32;
     __shared__ double s_warp[NW][3];
     const int b = blockIdx.x, lane = threadIdx.x & 31, w = threadIdx.x >> 5;
@@ -179,22 +216,27 @@ __global__ void __launch_bounds__(kReduceThreads) center_kernel(const T *in, T *
     // wherever the chain sits, and GB300's FP64 rate is a small fraction of its FP32 rate
     const T p0 = n > 0 ? x[0] : T(0), p1 = n > 0 ? x[1] : T(0), p2 = n > 0 ? x[2] : T(0);
     T s[3] = {T(0), T(0), T(0)};
-    int i0 = 0;  // first atom of the scalar loop
-    if constexpr (sizeof(T) == 4) {
-        if (vec) {  // 16-byte rows: a thread reads 4 atoms as three float4s, two groups in flight
-            const float4 *x4 = reinterpret_cast<const float4 *>(x);
-            const int ng = n >> 2;
+    // aligned groups of N atoms as three vectors per thread (tpl_rows.cuh), two groups in
+    // flight; then the atoms before and after them
+    constexpr int N = Vec16<T>::n;
+    const int head = max(0, min(row_head(x), n)), ng = max(0, n - head) / N;
+    const T *xg = x + 3 * head;
 #pragma unroll 2
-            for (int g = threadIdx.x; g < ng; g += kReduceThreads) {
-                const float4 a = x4[3 * g], b = x4[3 * g + 1], c = x4[3 * g + 2];
-                s[0] += ((a.x - p0) + (a.w - p0)) + ((b.z - p0) + (c.y - p0));
-                s[1] += ((a.y - p1) + (b.x - p1)) + ((b.w - p1) + (c.z - p1));
-                s[2] += ((a.z - p2) + (b.y - p2)) + ((c.x - p2) + (c.w - p2));
-            }
-            i0 = 4 * ng;
+    for (int g = threadIdx.x; g < ng; g += kReduceThreads) {
+        T v[3 * N];
+        load_group(xg + 3 * N * g, v);
+        if constexpr (N == 4) {
+            s[0] += ((v[0] - p0) + (v[3] - p0)) + ((v[6] - p0) + (v[9] - p0));
+            s[1] += ((v[1] - p1) + (v[4] - p1)) + ((v[7] - p1) + (v[10] - p1));
+            s[2] += ((v[2] - p2) + (v[5] - p2)) + ((v[8] - p2) + (v[11] - p2));
+        } else {
+            s[0] += (v[0] - p0) + (v[3] - p0);
+            s[1] += (v[1] - p1) + (v[4] - p1);
+            s[2] += (v[2] - p2) + (v[5] - p2);
         }
     }
-    for (int i = i0 + threadIdx.x; i < n; i += kReduceThreads) {
+    for (int q = threadIdx.x; q < n - N * ng; q += kReduceThreads) {
+        const int i = q < head ? q : q + N * ng;
         s[0] += x[3 * i] - p0;
         s[1] += x[3 * i + 1] - p1;
         s[2] += x[3 * i + 2] - p2;
@@ -222,27 +264,49 @@ __global__ void __launch_bounds__(kReduceThreads) center_kernel(const T *in, T *
 template <typename T>
 __global__ void __launch_bounds__(kReduceThreads) bbox_kernel(const T *in, T *lo, T *hi, const int *num_atoms,
                                                               int stride) {
-    __shared__ T s_warp[kReduceThreads / 32];
-    const int b = blockIdx.x;
+    constexpr int NW = kReduceThreads / 32, N = Vec16<T>::n;
+    __shared__ T s_warp[NW][6];
+    const int b = blockIdx.x, lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const int n = min(num_atoms[b], stride);
     const T *x = in + (size_t)b * 3 * stride;
     const T inf = (T)INFINITY;
-    T mn[3] = {inf, inf, inf}, mx[3] = {-inf, -inf, -inf};
-    for (int i = threadIdx.x; i < n; i += kReduceThreads)
+    T m[6] = {inf, inf, inf, -inf, -inf, -inf};  // min, max
+    auto add = [&](const T *v) {
+#pragma unroll
         for (int c = 0; c < 3; c++) {
-            const T v = x[3 * i + c];
-            mn[c] = v < mn[c] ? v : mn[c];
-            mx[c] = v > mx[c] ? v : mx[c];
+            m[c] = v[c] < m[c] ? v[c] : m[c];
+            m[3 + c] = v[c] > m[3 + c] ? v[c] : m[3 + c];
         }
-    auto fmin_ = [](T p, T q) { return q < p ? q : p; };
-    auto fmax_ = [](T p, T q) { return q > p ? q : p; };
-    for (int c = 0; c < 3; c++) {
-        const T a = block_reduce<T>(mn[c], fmin_, s_warp);
-        const T z = block_reduce<T>(mx[c], fmax_, s_warp);
-        if (threadIdx.x == 0) {
-            lo[3 * b + c] = a;
-            hi[3 * b + c] = z;
+    };
+    const int head = max(0, min(row_head(x), n)), ng = max(0, n - head) / N;
+    const T *xg = x + 3 * head;
+#pragma unroll 2
+    for (int g = threadIdx.x; g < ng; g += kReduceThreads) {
+        T v[3 * N];
+        load_group(xg + 3 * N * g, v);
+#pragma unroll
+        for (int q = 0; q < N; q++) add(v + 3 * q);
+    }
+    for (int q = threadIdx.x; q < n - N * ng; q += kReduceThreads) add(x + 3 * (q < head ? q : q + N * ng));
+    auto lower = [](T p, T q) { return q < p ? q : p; };
+    auto upper = [](T p, T q) { return q > p ? q : p; };
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1)
+#pragma unroll
+        for (int c = 0; c < 6; c++) {
+            const T o = __shfl_xor_sync(0xffffffffu, m[c], off);
+            m[c] = c < 3 ? lower(m[c], o) : upper(m[c], o);
         }
+    if (lane == 0)
+#pragma unroll
+        for (int c = 0; c < 6; c++) s_warp[w][c] = m[c];
+    __syncthreads();
+    if (threadIdx.x < 6) {
+        const int c = threadIdx.x;
+        T r = s_warp[0][c];
+        for (int k = 1; k < NW; k++) r = c < 3 ? lower(r, s_warp[k][c]) : upper(r, s_warp[k][c]);
+        if (c < 3) lo[3 * b + c] = r;
+        else hi[3 * b + c - 3] = r;
     }
 }
 
@@ -257,8 +321,6 @@ dim3 grid_rows(int B, long long items_per_row) {
     return dim3((unsigned)gx, (unsigned)gy, 1);
 }
 
-bool aligned16(const void *p) { return ((uintptr_t)p & 15u) == 0; }
-
 }  // namespace
 
 template <typename T>
@@ -266,15 +328,8 @@ int coords_shift(const T *in, T *out, const T *add, int scale_by_count, const in
                  cudaStream_t st) {
     if (B == 0 || stride == 0) return TPL_OK;
     ShiftArgs a{in, out, add, num_atoms, B, 3 * stride, scale_by_count};
-    // 16-byte vectors when every row starts 16-byte aligned and holds whole vectors
-    const bool vec = aligned16(out) && (!in || aligned16(in)) && (a.row % Vec16<T>::n == 0) &&
-                     ((a.row * sizeof(T)) % 16 == 0);
-    const int n = vec ? Vec16<T>::n : 1;
-    if (vec) {
-        shift_kernel<T, true><<<grid_rows(B, (a.row / n + kUnroll - 1) / kUnroll), 256, 0, st>>>(a);
-    } else {
-        shift_kernel<T, false><<<grid_rows(B, (a.row + kUnroll - 1) / kUnroll), 256, 0, st>>>(a);
-    }
+    const long long nv = (a.row + Vec16<T>::n - 1) / Vec16<T>::n;
+    shift_kernel<T><<<grid_rows(B, (nv + kUnroll - 1) / kUnroll), 256, 0, st>>>(a);
     return cudaGetLastError() == cudaSuccess ? TPL_OK : TPL_ERR_LAUNCH;
 }
 
@@ -282,16 +337,15 @@ template <typename T>
 int coords_rotate(const T *in, T *out, const T *R, int transpose, const int *num_atoms, int B, int stride,
                   cudaStream_t st) {
     if (B == 0 || stride == 0) return TPL_OK;
-    rotate_kernel<T><<<grid_rows(B, (stride + kUnroll - 1) / kUnroll), 256, 0, st>>>(in, out, R, num_atoms, B, stride,
-                                                                                   transpose);
+    const long long groups = (stride + Vec16<T>::n - 1) / Vec16<T>::n;
+    rotate_kernel<T><<<grid_rows(B, (groups + 1) / 2), 256, 0, st>>>(in, out, R, num_atoms, B, stride, transpose);
     return cudaGetLastError() == cudaSuccess ? TPL_OK : TPL_ERR_LAUNCH;
 }
 
 template <typename T>
 int coords_center(const T *in, T *center, const int *num_atoms, int B, int stride, cudaStream_t st) {
     if (B == 0) return TPL_OK;
-    const int vec = stride % 4 == 0 && (reinterpret_cast<uintptr_t>(in) & 15u) == 0;
-    center_kernel<T><<<B, kReduceThreads, 0, st>>>(in, center, num_atoms, stride, vec);
+    center_kernel<T><<<B, kReduceThreads, 0, st>>>(in, center, num_atoms, stride);
     return cudaGetLastError() == cudaSuccess ? TPL_OK : TPL_ERR_LAUNCH;
 }
 
