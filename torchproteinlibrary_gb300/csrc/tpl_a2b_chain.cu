@@ -460,7 +460,6 @@ __global__ void __launch_bounds__(32 * kWarpsPerCta, fwd_min_blocks(C)) a2b_fwd_
             continue;
         }
         const int j0 = s0 + C * lane;
-        PairFrame tot;
         Frame<float> T;
         if (pf) {
             if (s0 + CH < len) prefetch_angles<C>(abuf + (it ^ 1) * 3 * CH, ang, a.L, s0 + CH, lane);
@@ -472,11 +471,10 @@ __global__ void __launch_bounds__(32 * kWarpsPerCta, fwd_min_blocks(C)) a2b_fwd_
         }
         // lane transforms compose 3C joints: no renormalisation before the scan (the
         // chain frame carried from chunk to chunk is renormalised)
-        const PairFrame E = warp_exclusive_total_pair(to_pair(T), lane, false, tot);
-        // E composes at most 31 renormalised lane transforms: P needs no renormalisation
-        const PairFrame P = compose_pair(F, E);
+        const PairFrame Q = compose_pair(F, warp_inclusive_pair(to_pair(T), lane));
+        const PairFrame P = frame_before(Q, F, lane);
         if ((C * lane) % kRecordStride == 0 && j0 < len) pair_store(rec[j0 / kRecordStride].f, P);
-        F = compose_pair(F, tot);
+        F = shfl_idx_pair(Q, 31);
         if (a.renorm) renormalize_pair(F);
         map_positions<C>(seg, P, j0, len);
         __syncwarp();
@@ -1085,7 +1083,7 @@ __global__ void __launch_bounds__(32 * kRingWarps, ring_fwd_min_blocks(C)) a2b_f
         const int nout = min(CH, a.L - s0);
         const bool live = s0 < len;
         const int j0 = s0 + C * lane;
-        PairFrame E = pair_identity(), tot = pair_identity();
+        PairFrame t = pair_identity();  // prefix of the lane transforms through this lane
         if (live) {  // no renormalisation of the lane transforms (3C joints each), as in a2b_fwd_chain_kernel
             Frame<float> T;
             if (pf) {
@@ -1097,25 +1095,26 @@ __global__ void __launch_bounds__(32 * kRingWarps, ring_fwd_min_blocks(C)) a2b_f
             } else {
                 T = walk_chunk<C, true>(a.bc, ang, a.L, j0, len, vec, seg);
             }
-            E = warp_exclusive_total_pair(to_pair(T), lane, false, tot);
+            t = warp_inclusive_pair(to_pair(T), lane);
         }
         PairFrame F = pair_identity();  // chain frame at the chunk start
         if (k > 0) {
             ring_wait(k);
-            F = carry64 ? pair_load(s_ring64[k & 3]) : pair_load(s_ring[k & 3]);
+            F = carry64 ? pair_load(s_ring64[k & 3]) : pair_load_vec(s_ring[k & 3]);
         }
+        const PairFrame Q = compose_pair(F, t);  // lane 31: the chain frame after the chunk
         if (k + 1 < nchunk) {
             if (carry64) {
                 // the chunk total composes 96C unrenormalised joints: pull it back onto SO(3)
                 // first, or the FP64 product of the totals drifts in scale chunk by chunk
                 // (the FP32 carry below renormalises the carried frame instead)
-                PairFrame t = tot;
-                if (a.renorm) renormalize_pair(t);
-                carry_f64(k > 0 ? s_ring64[k & 3] : nullptr, t, s_ring64[(k + 1) & 3], lane);
+                PairFrame tot = shfl_idx_pair(t, 31);
+                if (a.renorm) renormalize_pair(tot);
+                carry_f64(k > 0 ? s_ring64[k & 3] : nullptr, tot, s_ring64[(k + 1) & 3], lane);
             } else {
-                PairFrame Fn = compose_pair(F, tot);
+                PairFrame Fn = Q;
                 if (a.renorm) renormalize_pair(Fn);
-                if (lane == 0) pair_store(s_ring[(k + 1) & 3], Fn);
+                if (lane == 31) pair_store_vec(s_ring[(k + 1) & 3], Fn);
             }
             ring_signal(k + 1);
         }
@@ -1124,7 +1123,7 @@ __global__ void __launch_bounds__(32 * kRingWarps, ring_fwd_min_blocks(C)) a2b_f
             zero_floats(dst, 9 * nout, lane, vec);
             continue;
         }
-        const PairFrame P = compose_pair(F, E);
+        const PairFrame P = frame_before(Q, F, lane);
         if ((C * lane) % kRecordStride == 0 && j0 < len) pair_store(rec[j0 / kRecordStride].f, P);
         map_positions<C>(seg, P, j0, len);
         __syncwarp();

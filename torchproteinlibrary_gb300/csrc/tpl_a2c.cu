@@ -267,11 +267,10 @@ __device__ __forceinline__ void apply_rx_pair(PairFrame &f, float ca, float sa) 
     f.r2[2] = fmaf(e2, ca, -e1 * sa);
 }
 
-__device__ __forceinline__ void pair_point(const PairFrame &P, float x, float y, float z, float *out) {
-    const float2 xy = __ffma2_rn(P.c[0], f2(x), __ffma2_rn(P.c[1], f2(y), __ffma2_rn(P.c[2], f2(z), P.p)));
-    out[0] = xy.x;
-    out[1] = xy.y;
-    out[2] = fmaf(P.r2[0], x, fmaf(P.r2[1], y, fmaf(P.r2[2], z, P.p2)));
+// frame_point on a PairFrame: x and y of the point, and its z.
+__device__ __forceinline__ float2 pair_point(const PairFrame &P, float x, float y, float z, float &oz) {
+    oz = fmaf(P.r2[0], x, fmaf(P.r2[1], y, fmaf(P.r2[2], z, P.p2)));
+    return __ffma2_rn(P.c[0], f2(x), __ffma2_rn(P.c[1], f2(y), __ffma2_rn(P.c[2], f2(z), P.p)));
 }
 
 // The topology as the chunked float32 kernels read it: one 16-byte shared-memory load
@@ -331,25 +330,19 @@ __device__ __forceinline__ void residue_atoms_pair(const RingTopology &tp, uint3
                                                    const float cs[2], const float sn[2], const float chi_c[5],
                                                    const float chi_s[5], Emit emit) {
     const int ty = info & 0xff, na = (info >> 8) & 0xff, nj = (info >> 16) & 0xff;
-    {
-        const float x[3] = {P.p.x, P.p.y, P.p2};
-        emit(0, x);
-    }
+    emit(0, P.p, P.p2);
     PairFrame F = P;
     apply_backbone<0>(F, cs[0], sn[0]);
-    {
-        const float x[3] = {F.p.x, F.p.y, F.p2};
-        emit(1, x);
-    }
+    emit(1, F.p, F.p2);
     if (info >> 24) {  // Pro
         constexpr float p[9] = {kTopoF32.pro_local[0][0], kTopoF32.pro_local[0][1], kTopoF32.pro_local[0][2],
                                 kTopoF32.pro_local[1][0], kTopoF32.pro_local[1][1], kTopoF32.pro_local[1][2],
                                 kTopoF32.pro_local[2][0], kTopoF32.pro_local[2][1], kTopoF32.pro_local[2][2]};
 #pragma unroll
         for (int a = 0; a < 3; a++) {
-            float x[3];
-            pair_point(F, p[3 * a], p[3 * a + 1], p[3 * a + 2], x);
-            emit(2 + a, x);
+            float z;
+            const float2 xy = pair_point(F, p[3 * a], p[3 * a + 1], p[3 * a + 2], z);
+            emit(2 + a, xy, z);
         }
     }
     if (nj > 0) {
@@ -365,28 +358,22 @@ __device__ __forceinline__ void residue_atoms_pair(const RingTopology &tp, uint3
             const bool fixed = (j.bits >> 16) != 0;
             apply_joint_pair(S, j.cb, j.sb, j.d, k == 0 && fixed ? 1.f : chi_c[k], k == 0 && fixed ? 0.f : chi_s[k]);
             const int f0 = (j.bits >> 8) & 0xff, n = j.bits & 0xff;
-            {  // the group's first atom sits at the joint's origin
-                const float x[3] = {S.p.x, S.p.y, S.p2};
-                emit(2 + f0, x);
-            }
+            emit(2 + f0, S.p, S.p2);  // the group's first atom sits at the joint's origin
             for (int a = 1; a < n; a++) {
                 const RingPoint v = tp.point[ty][f0 + a];
-                float x[3];
-                pair_point(S, v.x, v.y, v.z, x);
-                emit(2 + f0 + a, x);
+                float z;
+                const float2 xy = pair_point(S, v.x, v.y, v.z, z);
+                emit(2 + f0 + a, xy, z);
             }
         }
     }
     PairFrame C = F;
     apply_backbone<1>(C, cs[1], sn[1]);
-    {
-        const float x[3] = {C.p.x, C.p.y, C.p2};
-        emit(na - 2, x);
-    }
+    emit(na - 2, C.p, C.p2);
     constexpr float ox = kTopoF32.o_local[0], oy = kTopoF32.o_local[1], oz = kTopoF32.o_local[2];
-    float x[3];
-    pair_point(C, ox, oy, oz, x);
-    emit(na - 1, x);
+    float z;
+    const float2 xy = pair_point(C, ox, oy, oz, z);
+    emit(na - 1, xy, z);
 }
 
 // Copy n staged values (world coordinates, xyz interleaved) to dst, coalesced.
@@ -620,7 +607,7 @@ __global__ void __launch_bounds__(32 * NW, NW == 4 ? 6 : 3) a2c_fwd_ring_kernel(
     constexpr int NT = 32 * NW;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     A2cRingSmem<NW, NAMES> &sm = *reinterpret_cast<A2cRingSmem<NW, NAMES> *>(smem_raw);
-    __shared__ __align__(16) float s_ring[NW][16];  // chain frame (12) and first atom index
+    __shared__ __align__(16) float s_ring[NW][16];  // chain frame (12, pair_store_vec) and first atom index
 
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
     load_ring_topology<NT>(sm.topo);
@@ -697,8 +684,8 @@ __global__ void __launch_bounds__(32 * NW, NW == 4 ? 6 : 3) a2c_fwd_ring_kernel(
             apply_backbone<1>(t, cs[1], sn[1]);
             apply_backbone<2>(t, cs[2], sn[2]);
         }
-        PairFrame tot;
-        const PairFrame E = warp_exclusive_total_pair(t, lane, renorm != 0, tot);
+        if (renorm) renormalize_pair(t);
+        t = warp_inclusive_pair(t, lane);
         int ci = na;  // atoms of the lanes up to this one
 #pragma unroll
         for (int off = 1; off < 32; off <<= 1) {
@@ -711,35 +698,39 @@ __global__ void __launch_bounds__(32 * NW, NW == 4 ? 6 : 3) a2c_fwd_ring_kernel(
         int abase = 0;                  // first atom of the chunk
         if (cb != (int)blockIdx.x || ck > 0) ring_wait<NW>(w);
         if (ck > 0) {
-            F = pair_load(s_ring[w]);
+            F = pair_load_vec(s_ring[w]);
             abase = __float_as_int(s_ring[w][12]);
         }
-        if (ck + 1 < cnch) {
-            PairFrame Fn = compose_pair(F, tot);
+        const float2 org = F.p;  // the chunk's origin; positions are relative to it
+        const float org2 = F.p2;
+        F.p = make_float2(0.f, 0.f);
+        F.p2 = 0.f;
+        const PairFrame Q = compose_pair(F, t);
+        if (ck + 1 < cnch) {  // lane 31: the chain frame after the chunk
+            PairFrame Fn = Q;
             if (renorm) renormalize_pair(Fn);
-            if (lane == 0) {
-                pair_store(s_ring[(w + 1) % NW], Fn);
+            Fn.p = __fadd2_rn(Fn.p, org);
+            Fn.p2 += org2;
+            if (lane == 31) {
+                pair_store_vec(s_ring[(w + 1) % NW], Fn);
                 s_ring[(w + 1) % NW][12] = __int_as_float(abase + cnt);
             }
         }
         if (ck + 1 < cnch || cb + (int)gridDim.x < nb) ring_signal<NW>((w + 1) % NW);
 
-        const float org[3] = {F.p.x, F.p.y, F.p2};
-        PairFrame Fr = F;  // rotation only: positions relative to the chunk origin
-        Fr.p = make_float2(0.f, 0.f);
-        Fr.p2 = 0.f;
+        const PairFrame P = frame_before(Q, F, lane);  // at this lane's N
         float *out = a.coords + (size_t)cb * 3 * a.maxA;
         float *gdst = out + (size_t)3 * abase;
         float *stg = stage + block_offset(gdst);  // the chunk's values keep their global 16-byte phase
         if (lane == 0) bulk_reads_done();
         __syncwarp();  // the previous chunk has left the staging buffers
         if (live) {
-            const PairFrame P = compose_pair(Fr, E);
             float *dst = stg + 3 * aoff;
-            residue_atoms_pair(tp, info, P, cs, sn, chc, chs, [&](int slot, const float *x) {
-                dst[3 * slot] = x[0] + org[0];
-                dst[3 * slot + 1] = x[1] + org[1];
-                dst[3 * slot + 2] = x[2] + org[2];
+            residue_atoms_pair(tp, info, P, cs, sn, chc, chs, [&](int slot, float2 xy, float z) {
+                xy = __fadd2_rn(xy, org);
+                dst[3 * slot] = xy.x;
+                dst[3 * slot + 1] = xy.y;
+                dst[3 * slot + 2] = z + org2;
             });
             if (NAMES) {
                 uint16_t *code = sm.code[NAMES ? w : 0] + aoff;

@@ -98,29 +98,44 @@ __device__ __forceinline__ PairFrame shfl_idx_pair(const PairFrame &f, int src) 
     return o;
 }
 
-__device__ __forceinline__ void renormalize_pair(PairFrame &g) {
-    Frame<float> f;
-    from_pair(g, f);
-    renormalize(f);
-    g = to_pair(f);
+// renormalize (tpl_common.cuh) on a PairFrame, R <- R (3I - R^T R) / 2: the same chain
+// of operations per output, rows 0 and 1 of the product in pairs.
+__device__ __forceinline__ void renormalize_pair(PairFrame &f) {
+    auto dot = [&](int i, int j) {
+        return fmaf(f.c[i].x, f.c[j].x, fmaf(f.c[i].y, f.c[j].y, f.r2[i] * f.r2[j]));
+    };
+    const float h00 = 1.5f - 0.5f * dot(0, 0), h11 = 1.5f - 0.5f * dot(1, 1), h22 = 1.5f - 0.5f * dot(2, 2);
+    const float h01 = -0.5f * dot(0, 1), h02 = -0.5f * dot(0, 2), h12 = -0.5f * dot(1, 2);
+    const float2 a = f.c[0], b = f.c[1], c = f.c[2];
+    const float a2 = f.r2[0], b2 = f.r2[1], c2 = f.r2[2];
+    f.c[0] = __ffma2_rn(a, f2(h00), __ffma2_rn(b, f2(h01), __fmul2_rn(c, f2(h02))));
+    f.c[1] = __ffma2_rn(a, f2(h01), __ffma2_rn(b, f2(h11), __fmul2_rn(c, f2(h12))));
+    f.c[2] = __ffma2_rn(a, f2(h02), __ffma2_rn(b, f2(h12), __fmul2_rn(c, f2(h22))));
+    f.r2[0] = fmaf(a2, h00, fmaf(b2, h01, c2 * h02));
+    f.r2[1] = fmaf(a2, h01, fmaf(b2, h11, c2 * h12));
+    f.r2[2] = fmaf(a2, h02, fmaf(b2, h12, c2 * h22));
 }
 
-// warp_exclusive_total on PairFrames: the exclusive prefix of the lane transforms in
-// lane order (Kogge-Stone over shuffles), and the warp total.
-__device__ __forceinline__ PairFrame warp_exclusive_total_pair(PairFrame t, int lane, bool renorm,
-                                                               PairFrame &total) {
-    if (renorm) renormalize_pair(t);
+// Inclusive prefix of the lane transforms in lane order (Kogge-Stone over shuffles).
+// The kernels compose the chain frame onto it, Q = F o prefix: lane 31's Q is the frame
+// after the chunk and lane l - 1's the frame at lane l's first joint (frame_before), so
+// one composition serves both.
+__device__ __forceinline__ PairFrame warp_inclusive_pair(PairFrame t, int lane) {
 #pragma unroll
     for (int off = 1; off < kWarp; off <<= 1) {
         const PairFrame o = shfl_up_pair(t, off);
         if (lane >= off) t = compose_pair(o, t);
     }
-    total = shfl_idx_pair(t, 31);
-    PairFrame exc = shfl_up_pair(t, 1);
-    if (lane == 0) exc = pair_identity();
-    return exc;
+    return t;
 }
 
+// Q of the lane before this one; F on lane 0.
+__device__ __forceinline__ PairFrame frame_before(const PairFrame &Q, const PairFrame &F, int lane) {
+    const PairFrame o = shfl_up_pair(Q, 1);
+    return lane == 0 ? F : o;
+}
+
+// A frame as 12 floats, rotation row-major, then the translation.
 __device__ __forceinline__ void pair_store(float *dst, const PairFrame &g) {
     Frame<float> f;
     from_pair(g, f);
@@ -132,6 +147,29 @@ __device__ __forceinline__ PairFrame pair_load(const S *src) {
     Frame<float> f;
     frame_load(f, src);
     return to_pair(f);
+}
+
+// The same as three 16-byte accesses in the registers' own order (the warps' handoff
+// slots), 16-byte aligned.
+__device__ __forceinline__ void pair_store_vec(float *dst, const PairFrame &g) {
+    float4 *d = reinterpret_cast<float4 *>(dst);
+    d[0] = make_float4(g.c[0].x, g.c[0].y, g.c[1].x, g.c[1].y);
+    d[1] = make_float4(g.c[2].x, g.c[2].y, g.p.x, g.p.y);
+    d[2] = make_float4(g.r2[0], g.r2[1], g.r2[2], g.p2);
+}
+__device__ __forceinline__ PairFrame pair_load_vec(const float *src) {
+    const float4 *s = reinterpret_cast<const float4 *>(src);
+    const float4 a = s[0], b = s[1], c = s[2];
+    PairFrame g;
+    g.c[0] = make_float2(a.x, a.y);
+    g.c[1] = make_float2(a.z, a.w);
+    g.c[2] = make_float2(b.x, b.y);
+    g.p = make_float2(b.z, b.w);
+    g.r2[0] = c.x;
+    g.r2[1] = c.y;
+    g.r2[2] = c.z;
+    g.p2 = c.w;
+    return g;
 }
 
 // apply_joint (tpl_common.cuh) on a PairFrame: 9 paired and 9 scalar operations.
