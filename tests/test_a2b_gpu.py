@@ -762,3 +762,40 @@ def test_layer_on_two_streams_concurrently(rm):
         for i in range(2):
             assert torch.equal(outs[i].detach(), ref[i][0])
             assert torch.equal(xs[i].grad, ref[i][1])
+
+
+@pytest.mark.parametrize("scheme", [32, 4])
+@pytest.mark.parametrize("rpt,buffers", [(4, 1), (4, 2), (8, 1)])
+@pytest.mark.parametrize("L,offs", [(133, (0, 0, 0)), (386, (1, 1, 0)), (700, (3, 3, 1)), (387, (0, 1, 2)),
+                                    (700, (0, 0, 3))])
+def test_coordinate_backward_at_every_row_phase(rm, L, offs, rpt, buffers, scheme):
+    """Rows at every 16-byte phase (lengths that are no multiple of four, storage offsets of
+    the coordinates, dL/dx and gradient tensors; the first two alike, so that chunks are
+    shifted to whole blocks, or not, so that they are staged word by word), with lengths
+    around the shifted chunk ends, NaN past each chain: against the oracle, zeros past it."""
+    lens = [L, L - 1, L - 2, L - 3, 128, 127, 126, 125, 124, 5, 4, 3, 2, 1, 0, 129, 130, 131, 132]
+    B = len(lens)
+    ang, lengths, g = make_case(B, L, 900 + L, lengths=lens)
+    gp = g.astype(np.float32)
+    for b, n in enumerate(lengths):
+        gp[b, 9 * n:] = np.nan
+    dev = torch.device("cuda")
+
+    def at(v, off):
+        t = torch.empty(v.size + off, device=dev)[off:].view(v.shape)
+        return t.copy_(torch.tensor(v, dtype=torch.float32))
+
+    ws = torch.zeros(rm.workspace_bytes(B, L), dtype=torch.uint8, device=dev)
+    c = at(np.full((B, 9 * L), np.nan), offs[0])
+    ln = torch.tensor(lengths, device=dev)
+    rm.Angles2BackboneGPU_forward(at(ang, 0), c, ln, ws)
+    for b, n in enumerate(lengths):
+        c[b, 9 * int(n):] = float("nan")
+    gi = at(np.full((B, 3, L), np.nan), offs[2])
+    rm.Angles2BackboneGPU_backward_coords(gi, at(gp, offs[1]), c, ln, ws, rpt, buffers, scheme)
+    assert rm.workspace_status(ws) == 0
+    rc, rg = oracle_ref(ang, lengths, g, True)
+    check(torch.nan_to_num(c).double().cpu().numpy(), gi.double().cpu().numpy(), rc, rg, lengths, L, COORD_TOL_F32,
+          GRAD_TOL_F32)
+    for b, n in enumerate(lengths):
+        assert not gi[b, :, int(n):].any()

@@ -28,6 +28,9 @@
 //   3. each lane walks its residues backwards, accumulating (G, S), and evaluates
 //      dL/dtheta_m = u_m . (S_m - x_m x G_m) for its 3C joints.
 // No CTA-wide barrier, no atomics and no FP64 on this path.
+#include <type_traits>
+
+#include "tpl_async.cuh"
 #include "tpl_common.cuh"
 #include "tpl_internal.h"
 #include "tpl_pair.cuh"
@@ -224,12 +227,6 @@ struct AngBuf {
     static constexpr bool ON = C == 4;
     static constexpr int FLOATS = ON ? 2 * 3 * 32 * C : 0;  // per warp: two chunks of three rows
 };
-__device__ __forceinline__ void cp_async16(float *dst, const float *src) {
-    const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d), "l"(src) : "memory");
-}
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-__device__ __forceinline__ void cp_async_wait1() { asm volatile("cp.async.wait_group 1;" ::: "memory"); }
 
 // Copy the lane's float4s of the chunk starting at s0 (rows phi, psi, omega) into buf
 // (three rows of 32 C floats).  Requires L % 4 == 0 and 16-byte aligned rows.
@@ -707,45 +704,6 @@ __global__ void __launch_bounds__(32 * kWarpsPerCta, bwd_min_blocks(C)) a2b_bwd_
 // sums), a warp suffix scan and a reverse pass over each lane's residues.
 // Positions are taken relative to the chunk's first N atom to keep the sums small.
 
-constexpr unsigned kWaitPolls = 1u << 22;  // bounded mbarrier wait (~0.5 s with back-off)
-
-__device__ __forceinline__ unsigned smem_addr(const void *p) {
-    return static_cast<unsigned>(__cvta_generic_to_shared(p));
-}
-__device__ __forceinline__ void mbar_init(uint64_t *bar) {
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_addr(bar)) : "memory");
-    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-}
-__device__ __forceinline__ void bulk_load_pair(float *dx, const float *sx, float *dg, const float *sg, unsigned bytes,
-                                               uint64_t *bar) {
-    // the buffers were last read through the generic proxy
-    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_addr(bar)), "r"(2 * bytes)
-                 : "memory");
-    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
-                     smem_addr(dx)),
-                 "l"(sx), "r"(bytes), "r"(smem_addr(bar))
-                 : "memory");
-    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
-                     smem_addr(dg)),
-                 "l"(sg), "r"(bytes), "r"(smem_addr(bar))
-                 : "memory");
-}
-// Wait for the phase with the given parity to complete; false after kWaitPolls polls.
-__device__ __forceinline__ bool mbar_wait(uint64_t *bar, unsigned parity) {
-    for (unsigned i = 0; i < kWaitPolls; i++) {
-        unsigned done;
-        asm volatile(
-            "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}"
-            : "=r"(done)
-            : "r"(smem_addr(bar)), "r"(parity)
-            : "memory");
-        if (done) return true;
-        if (i >= 8) __nanosleep(100);
-    }
-    return false;
-}
-
 // The float4s 4q..4q+3 of a lane's staged segment that residue r needs, each
 // fetched once when residues are visited in descending (DESC) or ascending order:
 // a float4 shared with the residue visited before is already in buf.
@@ -759,78 +717,258 @@ __device__ __forceinline__ void fetch_residue(const float *seg, float *buf, int 
         }
 }
 
-constexpr int coords_min_blocks(int C, int NB) { return C * NB >= 16 ? 1 : (C * NB >= 8 ? 3 : 5); }
+constexpr int coords_min_blocks(int C, int NB) { return C * NB >= 16 ? 1 : (C * NB >= 8 ? 3 : 6); }
+
+// A chain's rows of coordinates and dL/dx as the coordinate backwards take them.  A row
+// starts at any 16-byte phase (9 L b floats: phase zero for every chain only when L is a
+// multiple of four), and a lane's C residues (9C floats) should be whole float4s in shared
+// memory, where the bulk copies keep the phase.  9 = 1 (mod 4), so residue j starts a
+// 16-byte block when j = -W (mod 4), W the row's first word counted from a block: the chunks
+// are moved back by s = W residues (slot v of the chain is residue v - s), and the lanes of
+// the first chunk mask the slots below residue 0.  Rows whose coordinates and dL/dx differ
+// in phase (an offset view of one of them) are staged word by word instead, unshifted.
+// GB300, 2048 chains of 100..517 residues, L = 517: 36.1 us staged word by word, 17.0 us
+// shifted.  ALIGNED: every row starts a block (s = 0), and a chunk is copied up to a
+// multiple of four residues, which is inside the row: no words outside the blocks (1024
+// chains of 20..700 residues, L = 700: forward and backward 29.4 against 30.0 us).
+template <int C, bool ALIGNED>
+struct CoordsRow {
+    static constexpr int CH = 32 * C, SEG = 9 * C;
+    const float *x, *g;
+    int len, s;
+    bool bulk;
+    __device__ __forceinline__ CoordsRow(const ChainArgs &a, int b, int l)
+        : x(a.coords + (size_t)b * 9 * a.L), g(a.grad_coords + (size_t)b * 9 * a.L), len(l) {
+        bulk = ALIGNED || block_offset(x) == block_offset(g);
+        s = !ALIGNED && bulk ? block_offset(x) : 0;
+    }
+    __device__ __forceinline__ int nchunk() const { return len > 0 ? (len + s + CH - 1) / CH : 0; }
+    __device__ __forceinline__ int start(int k) const { return k * CH - s; }  // residue of lane 0's first slot
+    __device__ __forceinline__ int origin(int k) const { return ALIGNED ? 0 : 9 * max(0, -start(k)); }  // first N in buf
+    // chunk k into buf: 32 lane segments of coordinates, then of dL/dx
+    __device__ __forceinline__ void issue(int k, float *buf, uint64_t *bar, int lane) const {
+        if constexpr (ALIGNED) {
+            if (lane != 0) return;
+            const int n = 9 * ((min(CH, len - k * CH) + 3) & ~3);
+            async_proxy_fence();  // the buffers were last read through the generic proxy
+            mbar_expect(bar, 8 * n);
+            StageSpan(x + (size_t)9 * k * CH, buf, n).blocks(bar);
+            StageSpan(g + (size_t)9 * k * CH, buf + 32 * SEG, n).blocks(bar);
+        } else {
+            const int at = origin(k), n = 9 * min(len - start(k), CH) - at;
+            const ptrdiff_t from = (ptrdiff_t)9 * start(k) + at;
+            stage_spans(StageSpan(x + from, buf + at, n), StageSpan(g + from, buf + 32 * SEG + at, n), bar, lane);
+        }
+    }
+    // the words outside the blocks of every chunk issued but the newest (all: of every one)
+    __device__ __forceinline__ void wait_words(bool all) const {
+        if constexpr (!ALIGNED) {
+            cp_async_commit();
+            if (all) cp_async_wait_all();
+            else cp_async_wait1();
+        }
+    }
+    __device__ __forceinline__ void stage(int k, float *buf, int lane) const {
+        const int n = 9 * min(CH, len - k * CH);
+        stage_chunk<SEG, SEG>(buf, x + (size_t)9 * k * CH, n, lane, false);
+        stage_chunk<SEG, SEG>(buf + 32 * SEG, g + (size_t)9 * k * CH, n, lane, false);
+    }
+};
+
+template <bool ALIGNED>  // unshifted chunks hold no residue below 0
+__device__ __forceinline__ bool in_chain(int j, int len) {
+    return ALIGNED ? j < len : (unsigned)j < (unsigned)len;
+}
+
+// Lane sums G = sum g and S = sum (x - o) x g over the lane's residues inside the chain.
+template <int C, bool ALIGNED>
+__device__ __forceinline__ void coords_sums(const float *xs, const float *gs, const float (&o)[3], int j0, int len,
+                                            float (&G)[3], float (&S)[3]) {
+    float xb[9 * C], gb[9 * C];
+#pragma unroll
+    for (int r = 0; r < C; r++) {
+        fetch_residue<false>(xs, xb, r, r == 0);
+        fetch_residue<false>(gs, gb, r, r == 0);
+        if (in_chain<ALIGNED>(j0 + r, len)) {
+#pragma unroll
+            for (int at = 0; at < 3; at++) {
+                const float *x = xb + 9 * r + 3 * at, *g = gb + 9 * r + 3 * at;
+                const float xr[3] = {x[0] - o[0], x[1] - o[1], x[2] - o[2]};
+                float xg[3];
+                cross3(xr, g, xg);
+#pragma unroll
+                for (int c = 0; c < 3; c++) {
+                    G[c] += g[c];
+                    S[c] += xg[c];
+                }
+            }
+        }
+    }
+}
+
+// The 3C joint gradients of a lane, backwards over its residues from the sums (G, S) over
+// every later residue; positions relative to o, nxt = N of the residue after the lane's
+// last.  gr: phi, psi, omega; zero outside the chain (stale or padding positions are
+// never stored), and psi and omega of the last residue move nothing.
+template <int C, bool ALIGNED>
+__device__ __forceinline__ void coords_grads(const float *xs, const float *gs, const float (&o)[3], int j0, int len,
+                                             const BondConsts &bc, float (&G)[3], float (&S)[3], float (&nxt)[3],
+                                             float (&gr)[3][C]) {
+    const float inv_d0 = 1.f / bc.d[0], inv_d1 = 1.f / bc.d[1], inv_d2 = 1.f / bc.d[2];
+    float xb[9 * C], gb[9 * C];
+#pragma unroll
+    for (int r = C - 1; r >= 0; r--) {
+        fetch_residue<true>(xs, xb, r, r == C - 1);
+        fetch_residue<true>(gs, gb, r, r == C - 1);
+        const int j = j0 + r;
+        float xN[3], xA[3], xC[3];
+#pragma unroll
+        for (int c = 0; c < 3; c++) {
+            xN[c] = xb[9 * r + c] - o[c];
+            xA[c] = xb[9 * r + 3 + c] - o[c];
+            xC[c] = xb[9 * r + 6 + c] - o[c];
+        }
+        const float *gN = gb + 9 * r, *gA = gb + 9 * r + 3, *gC = gb + 9 * r + 6;
+        const bool in = in_chain<ALIGNED>(j, len), last = j == len - 1;
+        float u[3], tmp[3], cr[3];
+        // omega_j: axis C -> N_{j+1}, through N_{j+1}; moves the atoms after C_j
+#pragma unroll
+        for (int c = 0; c < 3; c++) u[c] = (nxt[c] - xC[c]) * inv_d2;
+        cross3(nxt, G, cr);
+#pragma unroll
+        for (int c = 0; c < 3; c++) tmp[c] = S[c] - cr[c];
+        gr[2][r] = in && !last ? u[0] * tmp[0] + u[1] * tmp[1] + u[2] * tmp[2] : 0.f;
+        // psi_j: axis CA -> C, through C; same atoms
+#pragma unroll
+        for (int c = 0; c < 3; c++) u[c] = (xC[c] - xA[c]) * inv_d1;
+        cross3(xC, G, cr);
+#pragma unroll
+        for (int c = 0; c < 3; c++) tmp[c] = S[c] - cr[c];
+        gr[1][r] = in && !last ? u[0] * tmp[0] + u[1] * tmp[1] + u[2] * tmp[2] : 0.f;
+        if (in) {
+            cross3(xC, gC, cr);
+#pragma unroll
+            for (int c = 0; c < 3; c++) {
+                G[c] += gC[c];
+                S[c] += cr[c];
+            }
+        }
+        // phi_j: axis N -> CA, through CA; moves C_j and everything after
+#pragma unroll
+        for (int c = 0; c < 3; c++) u[c] = (xA[c] - xN[c]) * inv_d0;
+        cross3(xA, G, cr);
+#pragma unroll
+        for (int c = 0; c < 3; c++) tmp[c] = S[c] - cr[c];
+        gr[0][r] = in ? u[0] * tmp[0] + u[1] * tmp[1] + u[2] * tmp[2] : 0.f;
+        if (in) {
+            cross3(xA, gA, cr);
+#pragma unroll
+            for (int c = 0; c < 3; c++) {
+                G[c] += gA[c];
+                S[c] += cr[c];
+            }
+            cross3(xN, gN, cr);
+#pragma unroll
+            for (int c = 0; c < 3; c++) {
+                G[c] += gN[c];
+                S[c] += cr[c];
+            }
+        }
+#pragma unroll
+        for (int c = 0; c < 3; c++) nxt[c] = xN[c];
+    }
+}
+
+// Store a chunk's gradients: float4 rows where they are aligned, else through buf
+// (3 * 32C floats, free once every lane is done with the chunk) as coalesced words.
+// js: residue of lane 0's first slot.
+template <int C, bool ALIGNED>
+__device__ __forceinline__ void store_grads(const ChainArgs &a, float *gout, float *buf, int js, int lane,
+                                            const float (&gr)[3][C]) {
+    if constexpr (ALIGNED) {
+#pragma unroll
+        for (int i = 0; i < C / 4; i++) {
+            const int j = js + C * lane + 4 * i;
+            if (j < a.L)
+#pragma unroll
+                for (int k = 0; k < 3; k++)
+                    __stcs(reinterpret_cast<float4 *>(gout + (size_t)k * a.L + j),
+                           make_float4(gr[k][4 * i], gr[k][4 * i + 1], gr[k][4 * i + 2], gr[k][4 * i + 3]));
+        }
+        return;
+    }
+    __syncwarp();
+#pragma unroll
+    for (int k = 0; k < 3; k++)
+#pragma unroll
+        for (int i = 0; i < C / 4; i++)
+            *reinterpret_cast<float4 *>(buf + 32 * C * k + C * lane + 4 * i) =
+                make_float4(gr[k][4 * i], gr[k][4 * i + 1], gr[k][4 * i + 2], gr[k][4 * i + 3]);
+    __syncwarp();
+#pragma unroll
+    for (int k = 0; k < 3; k++)
+#pragma unroll
+        for (int q = 0; q < C; q++) {
+            const int i = lane + 32 * q;
+            if ((unsigned)(js + i) < (unsigned)a.L) gout[(size_t)k * a.L + js + i] = buf[32 * C * k + i];
+        }
+}
 
 // NB = 1: each chunk's copies are issued and waited for in turn.  NB = 2: two
 // buffer pairs; the copies of the next chunk are in flight while a chunk is
 // evaluated.
-template <int C, int NB>
+template <int C, int NB, bool ALIGNED>
 __global__ void __launch_bounds__(32 * kWarpsPerCta, coords_min_blocks(C, NB)) a2b_bwd_coords_kernel(ChainArgs a) {
-    constexpr int CH = 32 * C, SEG = 9 * C;
+    constexpr int SEG = 9 * C;
     extern __shared__ __align__(16) float s_dyn[];
     __shared__ __align__(8) uint64_t s_bar[kWarpsPerCta][NB];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const int idx = blockIdx.x * kWarpsPerCta + w;
     if (idx >= a.B) return;  // warps are independent
     const int b = a.B - 1 - idx;  // chains last to first, as in a2b_bwd_coords_ring_kernel
-    // per buffer: coordinates of a chunk (contiguous as in the row), then its dL/dx
     float *sbase = s_dyn + (size_t)w * NB * 64 * SEG;
     uint64_t *bars = s_bar[w];
-    const bool vec = a.vec != 0;
-    if (vec && lane == 0)
+    if (lane == 0)
         for (int i = 0; i < NB; i++) mbar_init(&bars[i]);
     __syncwarp();
-    const int len = checked_length(a, b, lane);
-    const float *xin = a.coords + (size_t)b * 9 * a.L;
-    const float *gin = a.grad_coords + (size_t)b * 9 * a.L;
+    const CoordsRow<C, ALIGNED> row(a, b, checked_length(a, b, lane));
     float *gout = a.grad_angles + (size_t)b * 3 * a.L;
-    const float inv_d0 = 1.f / a.bc.d[0], inv_d1 = 1.f / a.bc.d[1], inv_d2 = 1.f / a.bc.d[2];
 
-    const int nchunk = (len + CH - 1) / CH;
-    const int s_end = min(a.L, nchunk * CH);
-    for (int k = 0; k < 3; k++) zero_floats(gout + (size_t)k * a.L + s_end, a.L - s_end, lane, vec && (s_end % 4 == 0));
+    const int nchunk = row.nchunk(), s_end = max(0, min(a.L, row.start(nchunk)));
+    for (int k = 0; k < 3; k++) zero_span(gout + (size_t)k * a.L + s_end, a.L - s_end, lane);
 
     float Gc[3] = {0.f, 0.f, 0.f}, Sc[3] = {0.f, 0.f, 0.f}, oc[3] = {0.f, 0.f, 0.f};  // sums after the chunk
     float nN[3] = {0.f, 0.f, 0.f};  // N of the first residue after the chunk (world)
-    // chunk kk into buffer q: whole residues up to a multiple of 4 (inside the row
-    // since L % 4 == 0), by lane 0
-    auto issue = [&](int kk, int q) {
-        if (lane == 0) {
-            const int n4 = (min(CH, len - kk * CH) + 3) & ~3;
-            float *bx = sbase + (size_t)q * 64 * SEG;
-            bulk_load_pair(bx, xin + (size_t)9 * kk * CH, bx + 32 * SEG, gin + (size_t)9 * kk * CH, 36u * (unsigned)n4,
-                           &bars[q]);
-        }
-    };
     unsigned parity = 0;  // bit q: parity of buffer q's pending phase
-    if (vec && NB == 2 && nchunk > 0) issue(nchunk - 1, 0);
+    if (row.bulk && NB == 2 && nchunk > 0) {
+        row.issue(nchunk - 1, sbase, &bars[0], lane);
+        if (!ALIGNED) cp_async_commit();
+    }
     for (int k = nchunk - 1, it = 0; k >= 0; k--, it++) {
-        const int s0 = k * CH;
-        const int nreal = min(CH, len - s0);
         const int q = NB == 2 ? (it & 1) : 0;
         float *sx = sbase + (size_t)q * 64 * SEG;
-        float *sg = sx + 32 * SEG;
-        const float *xs = sx + lane * SEG, *gs = sg + lane * SEG;
+        const float *xs = sx + lane * SEG, *gs = xs + 32 * SEG;
         __syncwarp();  // the previous chunk's reads of its buffers are done
-        if (vec) {
-            if (NB == 1) issue(k, 0);
-            else if (k > 0) issue(k - 1, q ^ 1);  // prefetch: the other buffer held the previous chunk
+        if (row.bulk) {
+            if (NB == 1) row.issue(k, sx, &bars[0], lane);
+            else if (k > 0) row.issue(k - 1, sbase + (size_t)(q ^ 1) * 64 * SEG, &bars[q ^ 1], lane);  // prefetch
+            row.wait_words(NB == 1);
             const bool ok = mbar_wait(&bars[q], (parity >> q) & 1u);
-            parity ^= 1u << q;
             if (!__all_sync(0xffffffffu, ok)) {
                 if (lane == 0) record_error(a.hdr, TPL_ERR_LOOKBACK_TIMEOUT);
                 // bounded: let the copies in flight land before exiting
-                (void)mbar_wait(&bars[q], ((parity >> q) & 1u) ^ 1u);
+                (void)mbar_wait(&bars[q], (parity >> q) & 1u);
                 if (NB == 2 && k > 0) (void)mbar_wait(&bars[q ^ 1], (parity >> (q ^ 1)) & 1u);
                 return;
             }
+            parity ^= 1u << q;
         } else {
-            stage_chunk<SEG, SEG>(sx, xin + (size_t)9 * s0, 9 * nreal, lane, false);
-            stage_chunk<SEG, SEG>(sg, gin + (size_t)9 * s0, 9 * nreal, lane, false);
-            __syncwarp();
+            row.stage(k, sx, lane);
         }
-        const int j0 = s0 + C * lane;
-        const float o[3] = {sx[0], sx[1], sx[2]};  // chunk origin: its first N atom
+        __syncwarp();  // every lane's words have landed
+        const int j0 = row.start(k) + C * lane;
+        const float *of = sx + row.origin(k);
+        const float o[3] = {of[0], of[1], of[2]};  // chunk origin: its first N atom
         {
             const float d[3] = {oc[0] - o[0], oc[1] - o[1], oc[2] - o[2]};
             float dx[3];
@@ -841,36 +979,8 @@ __global__ void __launch_bounds__(32 * kWarpsPerCta, coords_min_blocks(C, NB)) a
                 oc[i] = o[i];
             }
         }
-        // lane sums about o over the lane's residues below len
         float Gl[3] = {0.f, 0.f, 0.f}, Sl[3] = {0.f, 0.f, 0.f};
-        {
-            float xb[9 * C], gb[9 * C];
-#pragma unroll
-            for (int r = 0; r < C; r++) {
-#pragma unroll
-                for (int q = (9 * r) / 4; q <= (9 * r + 8) / 4; q++)
-                    if (r == 0 || q > (9 * r - 1) / 4) {  // not fetched for residue r - 1
-                        const float4 xv = reinterpret_cast<const float4 *>(xs)[q];
-                        const float4 gv = reinterpret_cast<const float4 *>(gs)[q];
-                        xb[4 * q] = xv.x; xb[4 * q + 1] = xv.y; xb[4 * q + 2] = xv.z; xb[4 * q + 3] = xv.w;
-                        gb[4 * q] = gv.x; gb[4 * q + 1] = gv.y; gb[4 * q + 2] = gv.z; gb[4 * q + 3] = gv.w;
-                    }
-                if (j0 + r < len) {
-#pragma unroll
-                    for (int at = 0; at < 3; at++) {
-                        const float *x = xb + 9 * r + 3 * at, *g = gb + 9 * r + 3 * at;
-                        const float xr[3] = {x[0] - o[0], x[1] - o[1], x[2] - o[2]};
-                        float xg[3];
-                        cross3(xr, g, xg);
-#pragma unroll
-                        for (int c = 0; c < 3; c++) {
-                            Gl[c] += g[c];
-                            Sl[c] += xg[c];
-                        }
-                    }
-                }
-            }
-        }
+        coords_sums<C, ALIGNED>(xs, gs, o, j0, row.len, Gl, Sl);
         float G[3], S[3];
 #pragma unroll
         for (int i = 0; i < 3; i++) {
@@ -884,118 +994,13 @@ __global__ void __launch_bounds__(32 * kWarpsPerCta, coords_min_blocks(C, NB)) a
         float nxt[3];
 #pragma unroll
         for (int c = 0; c < 3; c++) {
-            const float mine = xs[c];
-            const float nb = __shfl_down_sync(0xffffffffu, mine, 1);
-            const float first = __shfl_sync(0xffffffffu, mine, 0);
+            const float nb = __shfl_down_sync(0xffffffffu, xs[c], 1);
             nxt[c] = (lane == 31 ? nN[c] : nb) - o[c];
-            nN[c] = first;
+            nN[c] = o[c];
         }
-        // backwards over the lane's residues, positions relative to o
-        float gph[C], gps[C], gom[C];
-        {
-            float xb[9 * C], gb[9 * C];
-#pragma unroll
-            for (int r = C - 1; r >= 0; r--) {
-#pragma unroll
-                for (int q = (9 * r) / 4; q <= (9 * r + 8) / 4; q++)
-                    if (r == C - 1 || q < (9 * (r + 1)) / 4) {  // not fetched for residue r + 1
-                        const float4 xv = reinterpret_cast<const float4 *>(xs)[q];
-                        const float4 gv = reinterpret_cast<const float4 *>(gs)[q];
-                        xb[4 * q] = xv.x; xb[4 * q + 1] = xv.y; xb[4 * q + 2] = xv.z; xb[4 * q + 3] = xv.w;
-                        gb[4 * q] = gv.x; gb[4 * q + 1] = gv.y; gb[4 * q + 2] = gv.z; gb[4 * q + 3] = gv.w;
-                    }
-                const int j = j0 + r;
-                float xN[3], xA[3], xC[3];
-#pragma unroll
-                for (int c = 0; c < 3; c++) {
-                    xN[c] = xb[9 * r + c] - o[c];
-                    xA[c] = xb[9 * r + 3 + c] - o[c];
-                    xC[c] = xb[9 * r + 6 + c] - o[c];
-                }
-                const float *gN = gb + 9 * r, *gA = gb + 9 * r + 3, *gC = gb + 9 * r + 6;
-                float u[3], tmp[3], cr[3];
-                // omega_j: axis C -> N_{j+1}, through N_{j+1}; moves the atoms after C_j
-#pragma unroll
-                for (int c = 0; c < 3; c++) u[c] = (nxt[c] - xC[c]) * inv_d2;
-                cross3(nxt, G, cr);
-#pragma unroll
-                for (int c = 0; c < 3; c++) tmp[c] = S[c] - cr[c];
-                gom[r] = u[0] * tmp[0] + u[1] * tmp[1] + u[2] * tmp[2];
-                // psi_j: axis CA -> C, through C; same atoms
-#pragma unroll
-                for (int c = 0; c < 3; c++) u[c] = (xC[c] - xA[c]) * inv_d1;
-                cross3(xC, G, cr);
-#pragma unroll
-                for (int c = 0; c < 3; c++) tmp[c] = S[c] - cr[c];
-                gps[r] = u[0] * tmp[0] + u[1] * tmp[1] + u[2] * tmp[2];
-                const bool in = j < len;
-                if (in) {
-                    cross3(xC, gC, cr);
-#pragma unroll
-                    for (int c = 0; c < 3; c++) {
-                        G[c] += gC[c];
-                        S[c] += cr[c];
-                    }
-                }
-                // phi_j: axis N -> CA, through CA; moves C_j and everything after
-#pragma unroll
-                for (int c = 0; c < 3; c++) u[c] = (xA[c] - xN[c]) * inv_d0;
-                cross3(xA, G, cr);
-#pragma unroll
-                for (int c = 0; c < 3; c++) tmp[c] = S[c] - cr[c];
-                gph[r] = u[0] * tmp[0] + u[1] * tmp[1] + u[2] * tmp[2];
-                if (in) {
-                    cross3(xA, gA, cr);
-#pragma unroll
-                    for (int c = 0; c < 3; c++) {
-                        G[c] += gA[c];
-                        S[c] += cr[c];
-                    }
-                    cross3(xN, gN, cr);
-#pragma unroll
-                    for (int c = 0; c < 3; c++) {
-                        G[c] += gN[c];
-                        S[c] += cr[c];
-                    }
-                }
-#pragma unroll
-                for (int c = 0; c < 3; c++) nxt[c] = xN[c];
-            }
-        }
-        // zeros at and past len (stale or padding positions are never stored);
-        // psi and omega of the last residue move nothing
-#pragma unroll
-        for (int r = 0; r < C; r++) {
-            const int j = j0 + r;
-            const bool ok = j < len, last = j == len - 1;
-            gph[r] = ok ? gph[r] : 0.f;
-            gps[r] = ok && !last ? gps[r] : 0.f;
-            gom[r] = ok && !last ? gom[r] : 0.f;
-        }
-        if (vec) {
-#pragma unroll
-            for (int i = 0; i < C / 4; i++) {
-                const int j = j0 + 4 * i;
-                if (j < a.L) {
-                    __stcs(reinterpret_cast<float4 *>(gout + j),
-                           make_float4(gph[4 * i], gph[4 * i + 1], gph[4 * i + 2], gph[4 * i + 3]));
-                    __stcs(reinterpret_cast<float4 *>(gout + a.L + j),
-                           make_float4(gps[4 * i], gps[4 * i + 1], gps[4 * i + 2], gps[4 * i + 3]));
-                    __stcs(reinterpret_cast<float4 *>(gout + 2 * a.L + j),
-                           make_float4(gom[4 * i], gom[4 * i + 1], gom[4 * i + 2], gom[4 * i + 3]));
-                }
-            }
-        } else {
-#pragma unroll
-            for (int r = 0; r < C; r++) {
-                const int j = j0 + r;
-                if (j < a.L) {
-                    gout[j] = gph[r];
-                    gout[a.L + j] = gps[r];
-                    gout[2 * a.L + j] = gom[r];
-                }
-            }
-        }
+        float gr[3][C];
+        coords_grads<C, ALIGNED>(xs, gs, o, j0, row.len, a.bc, G, S, nxt, gr);
+        store_grads<C, ALIGNED>(a, gout, sx, row.start(k), lane, gr);
     }
 }
 
@@ -1135,9 +1140,9 @@ __global__ void __launch_bounds__(32 * kRingWarps, ring_fwd_min_blocks(C)) a2b_f
 // Backward from the coordinates with the ring split of a2b_bwd_coords_kernel: the
 // same per-chunk evaluation, with the carried sums received from the warp of the
 // next chunk instead of kept in registers.
-template <int C, int NB>
+template <int C, int NB, bool ALIGNED>
 __global__ void __launch_bounds__(32 * kRingWarps, coords_min_blocks(C, NB)) a2b_bwd_coords_ring_kernel(ChainArgs a) {
-    constexpr int CH = 32 * C, SEG = 9 * C;
+    constexpr int SEG = 9 * C;
     extern __shared__ __align__(16) float s_dyn[];
     __shared__ __align__(8) uint64_t s_bar[kRingWarps][NB];
     __shared__ __align__(16) float s_ring[kRingWarps][12];
@@ -1147,86 +1152,55 @@ __global__ void __launch_bounds__(32 * kRingWarps, coords_min_blocks(C, NB)) a2b
     const int b = a.B - 1 - (int)blockIdx.x;
     float *sbase = s_dyn + (size_t)w * NB * 64 * SEG;
     uint64_t *bars = s_bar[w];
-    const bool vec = a.vec != 0;
-    if (vec && lane == 0)
+    if (lane == 0)
         for (int i = 0; i < NB; i++) mbar_init(&bars[i]);
     __syncwarp();
-    const int len = checked_length(a, b, lane);
-    const float *xin = a.coords + (size_t)b * 9 * a.L;
-    const float *gin = a.grad_coords + (size_t)b * 9 * a.L;
+    const CoordsRow<C, ALIGNED> row(a, b, checked_length(a, b, lane));
     float *gout = a.grad_angles + (size_t)b * 3 * a.L;
-    const float inv_d0 = 1.f / a.bc.d[0], inv_d1 = 1.f / a.bc.d[1], inv_d2 = 1.f / a.bc.d[2];
 
-    const int nchunk = (len + CH - 1) / CH;
+    const int nchunk = row.nchunk();
     if (w == kRingWarps - 1) {  // gradient rows past the last chunk that holds residues are zero
-        const int s_end = min(a.L, nchunk * CH);
-        for (int k = 0; k < 3; k++)
-            zero_floats(gout + (size_t)k * a.L + s_end, a.L - s_end, lane, vec && (s_end % 4 == 0));
+        const int s_end = max(0, min(a.L, row.start(nchunk)));
+        for (int k = 0; k < 3; k++) zero_span(gout + (size_t)k * a.L + s_end, a.L - s_end, lane);
     }
-    auto issue = [&](int kk, int q) {
-        if (lane == 0) {
-            const int n4 = (min(CH, len - kk * CH) + 3) & ~3;
-            float *bx = sbase + (size_t)q * 64 * SEG;
-            bulk_load_pair(bx, xin + (size_t)9 * kk * CH, bx + 32 * SEG, gin + (size_t)9 * kk * CH, 36u * (unsigned)n4,
-                           &bars[q]);
-        }
-    };
     unsigned parity = 0;  // bit q: parity of buffer q's pending phase
     bool failed = false;  // a bulk copy timed out: the remaining chunks only pass the carry on
     const int first = nchunk - 1 - w;
-    if (vec && NB == 2 && first >= 0) issue(first, 0);
+    if (row.bulk && NB == 2 && first >= 0) {
+        row.issue(first, sbase, &bars[0], lane);
+        if (!ALIGNED) cp_async_commit();
+    }
 #pragma unroll 1
     for (int k = first, it = 0; k >= 0; k -= kRingWarps, it++) {
-        const int s0 = k * CH;
-        const int nreal = min(CH, len - s0);
         const int q = NB == 2 ? (it & 1) : 0;
         float *sx = sbase + (size_t)q * 64 * SEG;
-        float *sg = sx + 32 * SEG;
-        const float *xs = sx + lane * SEG, *gs = sg + lane * SEG;
+        const float *xs = sx + lane * SEG, *gs = xs + 32 * SEG;
         __syncwarp();  // the previous chunk's reads of its buffers are done
-        if (vec && !failed) {
-            if (NB == 1) issue(k, 0);
-            else if (k - kRingWarps >= 0) issue(k - kRingWarps, q ^ 1);
+        if (row.bulk && !failed) {
+            if (NB == 1) row.issue(k, sx, &bars[0], lane);
+            else if (k - kRingWarps >= 0) row.issue(k - kRingWarps, sbase + (size_t)(q ^ 1) * 64 * SEG, &bars[q ^ 1], lane);
+            row.wait_words(NB == 1);
             const bool ok = mbar_wait(&bars[q], (parity >> q) & 1u);
-            parity ^= 1u << q;
             if (!__all_sync(0xffffffffu, ok)) {
                 if (lane == 0) record_error(a.hdr, TPL_ERR_LOOKBACK_TIMEOUT);
                 // bounded: let the copies in flight land before the buffers go unused
-                (void)mbar_wait(&bars[q], ((parity >> q) & 1u) ^ 1u);
+                (void)mbar_wait(&bars[q], (parity >> q) & 1u);
                 if (NB == 2 && k - kRingWarps >= 0) (void)mbar_wait(&bars[q ^ 1], (parity >> (q ^ 1)) & 1u);
                 failed = true;
             }
-        } else if (!vec) {
-            stage_chunk<SEG, SEG>(sx, xin + (size_t)9 * s0, 9 * nreal, lane, false);
-            stage_chunk<SEG, SEG>(sg, gin + (size_t)9 * s0, 9 * nreal, lane, false);
-            __syncwarp();
+            parity ^= 1u << q;
+        } else if (!row.bulk) {
+            row.stage(k, sx, lane);
         }
-        const int j0 = s0 + C * lane;
+        __syncwarp();  // every lane's words have landed
+        const int j0 = row.start(k) + C * lane;
         float o[3] = {0.f, 0.f, 0.f};  // chunk origin: its first N atom
         float Gl[3] = {0.f, 0.f, 0.f}, Sl[3] = {0.f, 0.f, 0.f};
         if (!failed) {
+            const float *of = sx + row.origin(k);
 #pragma unroll
-            for (int c = 0; c < 3; c++) o[c] = sx[c];
-            float xb[9 * C], gb[9 * C];
-#pragma unroll
-            for (int r = 0; r < C; r++) {
-                fetch_residue<false>(xs, xb, r, r == 0);
-                fetch_residue<false>(gs, gb, r, r == 0);
-                if (j0 + r < len) {
-#pragma unroll
-                    for (int at = 0; at < 3; at++) {
-                        const float *x = xb + 9 * r + 3 * at, *g = gb + 9 * r + 3 * at;
-                        const float xr[3] = {x[0] - o[0], x[1] - o[1], x[2] - o[2]};
-                        float xg[3];
-                        cross3(xr, g, xg);
-#pragma unroll
-                        for (int c = 0; c < 3; c++) {
-                            Gl[c] += g[c];
-                            Sl[c] += xg[c];
-                        }
-                    }
-                }
-            }
+            for (int c = 0; c < 3; c++) o[c] = of[c];
+            coords_sums<C, ALIGNED>(xs, gs, o, j0, row.len, Gl, Sl);
         }
         float G[3], S[3], tg[3], ts[3];
 #pragma unroll
@@ -1276,104 +1250,9 @@ __global__ void __launch_bounds__(32 * kRingWarps, coords_min_blocks(C, NB)) a2b
             const float nb = __shfl_down_sync(0xffffffffu, xs[c], 1);
             nxt[c] = (lane == 31 ? nN[c] : nb) - o[c];
         }
-        float gph[C], gps[C], gom[C];
-        {
-            float xb[9 * C], gb[9 * C];
-#pragma unroll
-            for (int r = C - 1; r >= 0; r--) {
-                fetch_residue<true>(xs, xb, r, r == C - 1);
-                fetch_residue<true>(gs, gb, r, r == C - 1);
-                const int j = j0 + r;
-                float xN[3], xA[3], xC[3];
-#pragma unroll
-                for (int c = 0; c < 3; c++) {
-                    xN[c] = xb[9 * r + c] - o[c];
-                    xA[c] = xb[9 * r + 3 + c] - o[c];
-                    xC[c] = xb[9 * r + 6 + c] - o[c];
-                }
-                const float *gN = gb + 9 * r, *gA = gb + 9 * r + 3, *gC = gb + 9 * r + 6;
-                float u[3], tmp[3], cr[3];
-                // omega_j: axis C -> N_{j+1}, through N_{j+1}
-#pragma unroll
-                for (int c = 0; c < 3; c++) u[c] = (nxt[c] - xC[c]) * inv_d2;
-                cross3(nxt, G, cr);
-#pragma unroll
-                for (int c = 0; c < 3; c++) tmp[c] = S[c] - cr[c];
-                gom[r] = u[0] * tmp[0] + u[1] * tmp[1] + u[2] * tmp[2];
-                // psi_j: axis CA -> C, through C
-#pragma unroll
-                for (int c = 0; c < 3; c++) u[c] = (xC[c] - xA[c]) * inv_d1;
-                cross3(xC, G, cr);
-#pragma unroll
-                for (int c = 0; c < 3; c++) tmp[c] = S[c] - cr[c];
-                gps[r] = u[0] * tmp[0] + u[1] * tmp[1] + u[2] * tmp[2];
-                const bool in = j < len;
-                if (in) {
-                    cross3(xC, gC, cr);
-#pragma unroll
-                    for (int c = 0; c < 3; c++) {
-                        G[c] += gC[c];
-                        S[c] += cr[c];
-                    }
-                }
-                // phi_j: axis N -> CA, through CA
-#pragma unroll
-                for (int c = 0; c < 3; c++) u[c] = (xA[c] - xN[c]) * inv_d0;
-                cross3(xA, G, cr);
-#pragma unroll
-                for (int c = 0; c < 3; c++) tmp[c] = S[c] - cr[c];
-                gph[r] = u[0] * tmp[0] + u[1] * tmp[1] + u[2] * tmp[2];
-                if (in) {
-                    cross3(xA, gA, cr);
-#pragma unroll
-                    for (int c = 0; c < 3; c++) {
-                        G[c] += gA[c];
-                        S[c] += cr[c];
-                    }
-                    cross3(xN, gN, cr);
-#pragma unroll
-                    for (int c = 0; c < 3; c++) {
-                        G[c] += gN[c];
-                        S[c] += cr[c];
-                    }
-                }
-#pragma unroll
-                for (int c = 0; c < 3; c++) nxt[c] = xN[c];
-            }
-        }
-        // zeros at and past len; psi and omega of the last residue move nothing
-#pragma unroll
-        for (int r = 0; r < C; r++) {
-            const int j = j0 + r;
-            const bool ok = j < len, last = j == len - 1;
-            gph[r] = ok ? gph[r] : 0.f;
-            gps[r] = ok && !last ? gps[r] : 0.f;
-            gom[r] = ok && !last ? gom[r] : 0.f;
-        }
-        if (vec) {
-#pragma unroll
-            for (int i = 0; i < C / 4; i++) {
-                const int j = j0 + 4 * i;
-                if (j < a.L) {
-                    __stcs(reinterpret_cast<float4 *>(gout + j),
-                           make_float4(gph[4 * i], gph[4 * i + 1], gph[4 * i + 2], gph[4 * i + 3]));
-                    __stcs(reinterpret_cast<float4 *>(gout + a.L + j),
-                           make_float4(gps[4 * i], gps[4 * i + 1], gps[4 * i + 2], gps[4 * i + 3]));
-                    __stcs(reinterpret_cast<float4 *>(gout + 2 * a.L + j),
-                           make_float4(gom[4 * i], gom[4 * i + 1], gom[4 * i + 2], gom[4 * i + 3]));
-                }
-            }
-        } else {
-#pragma unroll
-            for (int r = 0; r < C; r++) {
-                const int j = j0 + r;
-                if (j < a.L) {
-                    gout[j] = gph[r];
-                    gout[a.L + j] = gps[r];
-                    gout[2 * a.L + j] = gom[r];
-                }
-            }
-        }
+        float gr[3][C];
+        coords_grads<C, ALIGNED>(xs, gs, o, j0, row.len, a.bc, G, S, nxt, gr);
+        store_grads<C, ALIGNED>(a, gout, sx, row.start(k), lane, gr);
     }
 }
 
@@ -1485,23 +1364,28 @@ int a2b_backward_coords(float *grad_angles, const float *grad_coords, const floa
     a.coords = const_cast<float *>(coords);  // read only
     a.grad_angles = grad_angles;
     a.grad_coords = grad_coords;
-    a.vec = (L % 4 == 0) && aligned16(coords) && aligned16(grad_angles) && aligned16(grad_coords);
+    a.vec = (L % 4 == 0) && aligned16(coords) && aligned16(grad_angles) && aligned16(grad_coords);  // float4 gradient rows
     const int C = opt.residues_per_thread > 0 ? opt.residues_per_thread : 4;
     const int NB = opt.copy_buffers > 0 ? opt.copy_buffers : 1;
-    constexpr int smem4 = kWarpsPerCta * 64 * 36 * (int)sizeof(float);
-    constexpr int smem8 = kWarpsPerCta * 64 * 72 * (int)sizeof(float);
     // automatic: four warps per chain from 384 residues (three or more 128-residue
     // chunks), one warp per chain for shorter chains (measured on GB300)
-    if (opt.threads_per_cta == kRingWarps || (opt.threads_per_cta == 0 && L >= 384)) {
-        if (C == 4 && NB == 1) return launch_ring(a2b_bwd_coords_ring_kernel<4, 1>, smem4, B, a, st);
-        if (C == 4 && NB == 2) return launch_ring(a2b_bwd_coords_ring_kernel<4, 2>, 2 * smem4, B, a, st);
-        if (C == 8 && NB == 1) return launch_ring(a2b_bwd_coords_ring_kernel<8, 1>, smem8, B, a, st);
-        return TPL_ERR_UNSUPPORTED;
-    }
-    if (C == 4 && NB == 1) return launch_chain(a2b_bwd_coords_kernel<4, 1>, smem4, B, a, st);
-    if (C == 4 && NB == 2) return launch_chain(a2b_bwd_coords_kernel<4, 2>, 2 * smem4, B, a, st);
-    if (C == 8 && NB == 1) return launch_chain(a2b_bwd_coords_kernel<8, 1>, smem8, B, a, st);
-    return TPL_ERR_UNSUPPORTED;
+    const bool ring = opt.threads_per_cta == kRingWarps || (opt.threads_per_cta == 0 && L >= 384);
+    auto launch = [&](auto aligned) {
+        constexpr bool A = decltype(aligned)::value;
+        constexpr int smem4 = kWarpsPerCta * 64 * 36 * (int)sizeof(float);
+        constexpr int smem8 = kWarpsPerCta * 64 * 72 * (int)sizeof(float);
+        if (C == 4 && NB == 1)
+            return ring ? launch_ring(a2b_bwd_coords_ring_kernel<4, 1, A>, smem4, B, a, st)
+                        : launch_chain(a2b_bwd_coords_kernel<4, 1, A>, smem4, B, a, st);
+        if (C == 4 && NB == 2)
+            return ring ? launch_ring(a2b_bwd_coords_ring_kernel<4, 2, A>, 2 * smem4, B, a, st)
+                        : launch_chain(a2b_bwd_coords_kernel<4, 2, A>, 2 * smem4, B, a, st);
+        if (C == 8 && NB == 1)
+            return ring ? launch_ring(a2b_bwd_coords_ring_kernel<8, 1, A>, smem8, B, a, st)
+                        : launch_chain(a2b_bwd_coords_kernel<8, 1, A>, smem8, B, a, st);
+        return (int)TPL_ERR_UNSUPPORTED;
+    };
+    return a.vec ? launch(std::true_type{}) : launch(std::false_type{});
 }
 
 int sincos_poly_f32(const float *a, float *s, float *c, int n, cudaStream_t st) {

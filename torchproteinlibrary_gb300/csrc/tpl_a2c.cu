@@ -29,6 +29,7 @@
 #include <cstddef>
 #include <cstdio>
 
+#include "tpl_async.cuh"
 #include "tpl_common.cuh"
 #include "tpl_internal.h"
 #include "tpl_pair.cuh"
@@ -527,43 +528,6 @@ struct A2cRingSmem {
     uint16_t code[NAMES ? NW : 1][NAMES ? kA2cStageAtoms : 8];
 };
 
-// Word offset of p inside its 16-byte block.
-__device__ __forceinline__ int block_offset(const void *p) { return (int)((reinterpret_cast<uintptr_t>(p) >> 2) & 3u); }
-
-__device__ __forceinline__ void cp_async4(float *dst_smem, const float *src) {
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"((unsigned)__cvta_generic_to_shared(dst_smem)),
-                 "l"(src)
-                 : "memory");
-}
-__device__ __forceinline__ void cp_async_wait_all() {
-    asm volatile("cp.async.commit_group;\ncp.async.wait_group 0;" ::: "memory");
-}
-
-// Store n words to dst from stg = stage + block_offset(dst), stage 16-byte aligned shared
-// memory written by the whole warp before a __syncwarp: the whole 16-byte blocks as one
-// bulk copy by lane 0, the words outside them by the first lanes.  The caller waits for
-// the copy's reads (bulk_reads_done) before it rewrites the buffer.
-__device__ __forceinline__ void bulk_store_span(float *dst, const float *stg, int n, int lane) {
-    const int head = min((4 - block_offset(dst)) & 3, n), body = (n - head) & ~3, tail = n - head - body;
-    if (lane < head) dst[lane] = stg[lane];
-    if (lane < tail) dst[head + body + lane] = stg[head + body + lane];
-    if (lane == 0 && body > 0)
-        asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;\n"
-                     "cp.async.bulk.commit_group;" ::"l"(dst + head),
-                     "r"((unsigned)__cvta_generic_to_shared(stg + head)), "r"(4 * body)
-                     : "memory");
-}
-__device__ __forceinline__ void bulk_reads_done() { asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory"); }
-__device__ __forceinline__ void async_proxy_fence() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
-
-// Zeros to n words from dst, by the warp.
-__device__ __forceinline__ void zero_span(uint32_t *dst, int n, int lane) {
-    const int head = min((4 - block_offset(dst)) & 3, max(n, 0)), nb = (max(n, 0) - head) >> 2;
-    if (lane < head) dst[lane] = 0u;
-    for (int i = lane; i < nb; i += 32) reinterpret_cast<uint4 *>(dst + head)[i] = make_uint4(0u, 0u, 0u, 0u);
-    if (lane < n - head - 4 * nb) dst[head + 4 * nb + lane] = 0u;
-}
-
 // Length of chain b for the chunked kernels, found by each warp for itself: the index of
 // the row's first NUL (at most the row stride), or 0, with the error recorded, when a
 // letter before it is no residue or the chain is longer than L.  atoms(chunk, n) is
@@ -762,7 +726,7 @@ __global__ void __launch_bounds__(32 * NW, NW == 4 ? 6 : 3) a2c_fwd_ring_kernel(
                 if (lane == 0) a2c_error(a.hdr, TPL_ERR_ATOMS);
                 total = a.maxA;
             }
-            zero_span(reinterpret_cast<uint32_t *>(out) + (size_t)3 * total, 3 * (a.maxA - total), lane);
+            zero_span(out + (size_t)3 * total, 3 * (a.maxA - total), lane);
             if (NAMES) {
                 zero_span(rn + total, a.maxA - total, lane);
                 zero_span(an + total, a.maxA - total, lane);
@@ -1120,49 +1084,6 @@ struct A2cBwdRingSmem {
     int base[1];  // per warp: first atom of each chunk, max_chunks + 1 entries (dynamic)
 };
 
-constexpr unsigned kA2cWaitPolls = 1u << 22;  // bounded mbarrier wait (about 0.5 s with the back-off)
-
-__device__ __forceinline__ unsigned smem_u32(const void *p) { return (unsigned)__cvta_generic_to_shared(p); }
-
-// Wait for the mbarrier phase of the given parity; false after kA2cWaitPolls polls.
-__device__ __forceinline__ bool a2c_mbar_wait(uint64_t *bar, unsigned parity) {
-    for (unsigned i = 0; i < kA2cWaitPolls; i++) {
-        unsigned done;
-        asm volatile(
-            "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}"
-            : "=r"(done)
-            : "r"(smem_u32(bar)), "r"(parity)
-            : "memory");
-        if (done) return true;
-        if (i >= 8) __nanosleep(100);
-    }
-    return false;
-}
-
-// The span [src, src + n) and its staging place dst + block_offset(src), dst 16-byte
-// aligned: `head` words before its whole 16-byte blocks, `body` words in them.
-struct StageSpan {
-    const float *src;
-    float *dst;
-    int head, body, tail;
-    __device__ __forceinline__ StageSpan(const float *s, float *row, int n) : src(s), dst(row + block_offset(s)) {
-        head = min((4 - block_offset(s)) & 3, n);
-        body = (n - head) & ~3;
-        tail = n - head - body;
-    }
-    __device__ __forceinline__ void ends(int lane) const {  // word copies outside the blocks (cp.async)
-        if (lane < head) cp_async4(dst + lane, src + lane);
-        if (lane < tail) cp_async4(dst + head + body + lane, src + head + body + lane);
-    }
-    __device__ __forceinline__ void blocks(uint64_t *bar) const {  // the blocks, by one lane
-        if (body > 0)
-            asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
-                             smem_u32(dst + head)),
-                         "l"(src + head), "r"(4 * body), "r"(smem_u32(bar))
-                         : "memory");
-    }
-};
-
 template <int NW>
 __global__ void __launch_bounds__(32 * NW) a2c_bwd_coords_ring_kernel(A2cArgs<float> a, int nb, int max_chunks) {
     constexpr int NT = 32 * NW;
@@ -1177,10 +1098,7 @@ __global__ void __launch_bounds__(32 * NW) a2c_bwd_coords_ring_kernel(A2cArgs<fl
         for (int i = threadIdx.x; i < (int)(sizeof(RingBwdTopology) / 4); i += NT)
             reinterpret_cast<uint32_t *>(&sm.topo)[i] = src[i];
     }
-    if (lane == 0) {
-        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(&s_bar[w])) : "memory");
-        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    }
+    if (lane == 0) mbar_init(&s_bar[w]);
     __syncthreads();
     int *base = sm.base + w * (max_chunks + 1);
     constexpr float inv_dphi = 1.f / kTopoF32.bb_d[0], inv_dpsi = 1.f / kTopoF32.bb_d[1],
@@ -1223,17 +1141,9 @@ __global__ void __launch_bounds__(32 * NW) a2c_bwd_coords_ring_kernel(A2cArgs<fl
         const int k = nch - 1 - i, j = k * kA2cChunk + lane, a0 = base[k], n3 = 3 * (base[k + 1] - a0);
         if (j < len) letter = a.seq[(size_t)b * a.seq_stride + j];
         const size_t at = (size_t)b * 3 * a.maxA + (size_t)3 * a0;
-        const StageSpan sx(a.coords + at, sm.x[w], n3), sg(a.grad_coords + at, sm.g[w], n3);
-        sx.ends(lane);
-        sg.ends(lane);
-        if (lane == 0) {
-            async_proxy_fence();  // the buffers were last read through the generic proxy
-            asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(&s_bar[w])),
-                         "r"(4 * (sx.body + sg.body))
-                         : "memory");
-            sx.blocks(&s_bar[w]);
-            sg.blocks(&s_bar[w]);
-        }
+        const float *x = a.coords + at, *g = a.grad_coords + at;
+        stage_spans(StageSpan(x, sm.x[w] + block_offset(x), n3), StageSpan(g, sm.g[w] + block_offset(g), n3), &s_bar[w],
+                    lane);
     };
     if (b >= 0) {
         enter();
@@ -1258,10 +1168,10 @@ __global__ void __launch_bounds__(32 * NW) a2c_bwd_coords_ring_kernel(A2cArgs<fl
         const float *sx = sm.x[w] + block_offset(a.coords + at), *sg = sm.g[w] + block_offset(a.grad_coords + at);
         if (!failed) {
             cp_async_wait_all();
-            const bool ok = a2c_mbar_wait(&s_bar[w], parity);
+            const bool ok = mbar_wait(&s_bar[w], parity);
             if (!__all_sync(0xffffffffu, ok)) {
                 if (lane == 0) a2c_error(a.hdr, TPL_ERR_LOOKBACK_TIMEOUT);
-                (void)a2c_mbar_wait(&s_bar[w], parity);  // bounded: let the copies in flight land
+                (void)mbar_wait(&s_bar[w], parity);  // bounded: let the copies in flight land
                 failed = true;
             }
             parity ^= 1u;
@@ -1378,7 +1288,7 @@ __global__ void __launch_bounds__(32 * NW) a2c_bwd_coords_ring_kernel(A2cArgs<fl
         if (top)  // zeros past the chain (and everywhere when it was refused)
 #pragma unroll 1
             for (int q = 0; q < 8; q++)
-                zero_span(reinterpret_cast<uint32_t *>(gout) + (size_t)q * a.L + clen, a.L - clen, lane);
+                zero_span(gout + (size_t)q * a.L + clen, a.L - clen, lane);
     }
 }
 
