@@ -799,3 +799,18 @@ def test_coordinate_backward_at_every_row_phase(rm, L, offs, rpt, buffers, schem
           GRAD_TOL_F32)
     for b, n in enumerate(lengths):
         assert not gi[b, :, int(n):].any()
+
+
+@pytest.mark.parametrize("B,L", [(1, 1), (3, 32), (5, 33), (2, 129), (4, 257), (200, 65), (3, 513), (2, 1025), (2, 2049),
+                                 (1, 4100)])
+def test_float64_clusters_and_passes(rm, B, L):
+    """The float64 kernels spread a chain over a cluster of CTAs, one or two residues per
+    lane by batch, and take chains past the cluster's 2048 residues in passes: sizes on both
+    sides of a warp's chunk, of each cluster size and of a pass, with short chains beside the
+    long one and angles beyond the polynomial's range, against the oracle."""
+    lens = np.array([L, max(L - 1, 0), L // 2, 1, 0, min(L, 31), min(L, 64)])[np.arange(B) % 7]
+    ang, lengths, g = make_case(B, L, 700 + L, lengths=lens)
+    ang[0, 0, ::7] += 20000 * np.pi
+    c, gi = run_gpu(rm, ang, lengths, g, torch.float64)
+    rc, rg = oracle_ref(ang, lengths, g, False)
+    check(c, gi, rc, rg, lengths, L, COORD_TOL_F64, GRAD_TOL_F64)

@@ -531,3 +531,24 @@ def test_angles_beyond_the_fast_sincos_range(fm):
     for from_coords in (True, False):
         c, _, _, _, gi = run_gpu(fm, ang, seqs, g, torch.float32, from_coords=from_coords)
         check(c, gi, rc, rg, na, COORD_TOL_F32, GRAD_TOL_F32)
+
+
+@pytest.mark.parametrize("lens", [[1, 31, 32, 33, 0], [64, 65, 63], [128, 129, 200], [257, 256, 40], [513, 512, 3],
+                                  [1100, 20]])
+def test_float64_clusters_and_passes(fm, lens):
+    """The float64 kernels spread a chain over a cluster of CTAs of 64 residues and take
+    chains past 512 residues in passes: lengths on both sides of a warp's chunk, of each
+    cluster size and of a pass, short chains beside long ones: coordinates, names and the
+    gradient against the oracle."""
+    rng = np.random.default_rng(sum(lens))
+    seqs = ["".join(rng.choice(list(AA), n)) for n in lens]
+    ang = rng.uniform(-np.pi, np.pi, (len(lens), 8, max(lens)))
+    rc, rrn, ran, na = oracle.a2c_forward(ang, seqs)
+    g = rng.standard_normal(rc.shape)
+    for b, n in enumerate(na):
+        g[b, 3 * n:] = 0
+    c, rn, an, n_at, gi = run_gpu(fm, ang, seqs, g, torch.float64)
+    np.testing.assert_array_equal(n_at, na)
+    np.testing.assert_array_equal(rn, rrn)
+    np.testing.assert_array_equal(an, ran)
+    check(c, gi, rc, oracle.a2c_backward(g, ang, seqs), na, COORD_TOL_F64, GRAD_TOL_F64)

@@ -1072,209 +1072,6 @@ __global__ void __launch_bounds__(128, warp_tile_min_blocks(R)) a2b_bwd_w_kernel
     finish_launch(&a.hdr->bwd_ticket, &a.hdr->bwd_done, &a.hdr->bwd_epoch);
 }
 
-// ----------------------------------------------------------- plain FP64 form
-// One chain per CTA, one residue per thread per chunk, Hillis-Steele block scan
-// of residue transforms in shared memory, carry between chunks in registers.
-constexpr int kPlainThreads = 256;
-
-struct PlainArgs {
-    const double *angles;
-    const int *lengths;
-    double *coords;
-    double *grad_angles;
-    const double *grad_coords;
-    WsHeader *hdr;
-    TileRecord *rec;
-    int L, nchunks;
-    BondConsts bc;
-};
-
-__device__ __forceinline__ Frame<double> plain_residue(const PlainArgs &a, const double *ang, int j, int len,
-                                                       double cs[3], double sn[3]) {
-    Frame<double> T;
-    frame_identity(T);
-    for (int k = 0; k < 3; k++) {
-        cs[k] = 1.0;
-        sn[k] = 0.0;
-    }
-    if (j < len) {
-        for (int k = 0; k < 3; k++) {
-            if (k == 2 && j == len - 1) break;
-            sincos(ang[(size_t)k * a.L + j], &sn[k], &cs[k]);
-            apply_joint(T, a.bc.cbd[k], a.bc.sbd[k], a.bc.dd[k], cs[k], sn[k]);
-        }
-    }
-    return T;
-}
-
-// Inclusive block scan of frames (Hillis-Steele); returns the exclusive prefix.
-__device__ __forceinline__ Frame<double> plain_block_scan(Frame<double> T, Frame<double> *s, Frame<double> &total) {
-    const int tid = threadIdx.x;
-    s[tid] = T;
-    __syncthreads();
-    for (int off = 1; off < kPlainThreads; off <<= 1) {
-        Frame<double> o;
-        if (tid >= off) o = s[tid - off];
-        __syncthreads();
-        if (tid >= off) {
-            T = compose(o, T);
-            s[tid] = T;
-        }
-        __syncthreads();
-    }
-    Frame<double> exc;
-    if (tid == 0) frame_identity(exc);
-    else exc = s[tid - 1];
-    total = s[kPlainThreads - 1];
-    __syncthreads();
-    return exc;
-}
-
-__global__ void __launch_bounds__(kPlainThreads) a2b_fwd_f64_plain_kernel(PlainArgs a) {
-    __shared__ Frame<double> s_scan[kPlainThreads];
-    const int b = blockIdx.x, tid = threadIdx.x;
-    int len = a.lengths[b];
-    if (len < 0 || len > a.L) {
-        if (tid == 0 && a.hdr) record_error(a.hdr, TPL_ERR_LENGTH);
-        len = max(0, min(len, a.L));
-    }
-    const double *ang = a.angles + (size_t)b * 3 * a.L;
-    double *out = a.coords + (size_t)b * 9 * a.L;
-    Frame<double> carry;
-    frame_identity(carry);
-    for (int s0 = 0; s0 < a.L; s0 += kPlainThreads) {
-        const int j = s0 + tid;
-        double cs[3], sn[3];
-        Frame<double> T = plain_residue(a, ang, j, len, cs, sn);
-        Frame<double> total;
-        Frame<double> exc = plain_block_scan(T, s_scan, total);
-        Frame<double> P = compose(carry, exc);
-        if (j < len) {
-            double *o = out + (size_t)9 * j;
-            for (int q = 0; q < 3; q++) {
-                o[3 * q] = P.p[0]; o[3 * q + 1] = P.p[1]; o[3 * q + 2] = P.p[2];
-                apply_joint(P, a.bc.cbd[q], a.bc.sbd[q], a.bc.dd[q], cs[q], sn[q]);
-            }
-        } else if (j < a.L) {
-            double *o = out + (size_t)9 * j;
-            for (int q = 0; q < 9; q++) o[q] = 0.0;
-        }
-        carry = compose(carry, total);
-    }
-}
-
-__global__ void __launch_bounds__(kPlainThreads) a2b_bwd_f64_plain_kernel(PlainArgs a) {
-    __shared__ Frame<double> s_scan[kPlainThreads];
-    __shared__ double s_sum[kPlainThreads][6];
-    const int b = blockIdx.x, tid = threadIdx.x;
-    int len = a.lengths[b];
-    if (len < 0 || len > a.L) {
-        if (tid == 0 && a.hdr) record_error(a.hdr, TPL_ERR_LENGTH);
-        len = max(0, min(len, a.L));
-    }
-    const double *ang = a.angles + (size_t)b * 3 * a.L;
-    const double *gc = a.grad_coords + (size_t)b * 9 * a.L;
-    double *gout = a.grad_angles + (size_t)b * 3 * a.L;
-    TileRecord *rec = a.rec + (size_t)b * a.nchunks;
-    // pass 1: chunk carries
-    Frame<double> carry;
-    frame_identity(carry);
-    for (int c = 0; c < a.nchunks; c++) {
-        if (tid == 0) frame_store(rec[c].fexc, carry);
-        const int j = c * kPlainThreads + tid;
-        double cs[3], sn[3];
-        Frame<double> T = plain_residue(a, ang, j, len, cs, sn);
-        Frame<double> total;
-        plain_block_scan(T, s_scan, total);
-        carry = compose(carry, total);
-    }
-    __syncthreads();
-    // pass 2: chunks last-first with the running suffix (G, S) about the world origin
-    double Gc[3] = {0, 0, 0}, Sc[3] = {0, 0, 0};
-    for (int c = a.nchunks - 1; c >= 0; c--) {
-        const int j = c * kPlainThreads + tid;
-        double cs[3], sn[3];
-        Frame<double> T = plain_residue(a, ang, j, len, cs, sn);
-        Frame<double> total, start;
-        Frame<double> exc = plain_block_scan(T, s_scan, total);
-        frame_load(start, rec[c].fexc);
-        Frame<double> P = compose(start, exc);
-        double x[3][3], u[3][3], xn[3];
-        double G[3] = {0, 0, 0}, S[3] = {0, 0, 0};
-        if (j < len) {
-            for (int q = 0; q < 3; q++) {
-                for (int k = 0; k < 3; k++) x[q][k] = P.p[k];
-                apply_joint(P, a.bc.cbd[q], a.bc.sbd[q], a.bc.dd[q], cs[q], sn[q]);
-                for (int k = 0; k < 3; k++) u[q][k] = P.r[3 * k];
-            }
-            for (int k = 0; k < 3; k++) xn[k] = P.p[k];
-            for (int q = 0; q < 3; q++) {
-                const double *g = gc + (size_t)9 * j + 3 * q;
-                double xg[3];
-                cross3(x[q], g, xg);
-                for (int k = 0; k < 3; k++) {
-                    G[k] += g[k];
-                    S[k] += xg[k];
-                }
-            }
-        }
-        // exclusive suffix over threads (Hillis-Steele on sums, reversed)
-        double v[6] = {G[0], G[1], G[2], S[0], S[1], S[2]};
-        for (int i = 0; i < 6; i++) s_sum[tid][i] = v[i];
-        __syncthreads();
-        for (int off = 1; off < kPlainThreads; off <<= 1) {
-            double o[6];
-            const bool has = tid + off < kPlainThreads;
-            if (has)
-                for (int i = 0; i < 6; i++) o[i] = s_sum[tid + off][i];
-            __syncthreads();
-            if (has)
-                for (int i = 0; i < 6; i++) {
-                    v[i] += o[i];
-                    s_sum[tid][i] = v[i];
-                }
-            __syncthreads();
-        }
-        double Gr[3], Sr[3], chunk_tot[6];
-        for (int i = 0; i < 6; i++) chunk_tot[i] = s_sum[0][i];
-        for (int k = 0; k < 3; k++) {
-            const double nxt_g = tid + 1 < kPlainThreads ? s_sum[tid + 1][k] : 0.0;
-            const double nxt_s = tid + 1 < kPlainThreads ? s_sum[tid + 1][3 + k] : 0.0;
-            Gr[k] = nxt_g + Gc[k];
-            Sr[k] = nxt_s + Sc[k];
-        }
-        __syncthreads();
-        if (j < len) {
-            double tmp[3], cr[3];
-            cross3(xn, Gr, cr);
-            for (int k = 0; k < 3; k++) tmp[k] = Sr[k] - cr[k];
-            const double gom = u[2][0] * tmp[0] + u[2][1] * tmp[1] + u[2][2] * tmp[2];
-            cross3(x[2], Gr, cr);
-            for (int k = 0; k < 3; k++) tmp[k] = Sr[k] - cr[k];
-            const double gps = u[1][0] * tmp[0] + u[1][1] * tmp[1] + u[1][2] * tmp[2];
-            const double *g = gc + (size_t)9 * j + 6;
-            cross3(x[2], g, cr);
-            for (int k = 0; k < 3; k++) {
-                Gr[k] += g[k];
-                Sr[k] += cr[k];
-            }
-            cross3(x[1], Gr, cr);
-            for (int k = 0; k < 3; k++) tmp[k] = Sr[k] - cr[k];
-            const double gph = u[0][0] * tmp[0] + u[0][1] * tmp[1] + u[0][2] * tmp[2];
-            const bool last = (j == len - 1);
-            gout[j] = gph;
-            gout[(size_t)a.L + j] = last ? 0.0 : gps;
-            gout[(size_t)2 * a.L + j] = last ? 0.0 : gom;
-        } else if (j < a.L) {
-            gout[j] = gout[(size_t)a.L + j] = gout[(size_t)2 * a.L + j] = 0.0;
-        }
-        for (int i = 0; i < 3; i++) {
-            Gc[i] += chunk_tot[i];
-            Sc[i] += chunk_tot[3 + i];
-        }
-    }
-}
-
 // ------------------------------------------------------------------- host side
 template <typename K>
 static int persistent_grid(K kernel, int threads, int items, int max_ctas, int dyn_smem = 0) {
@@ -1454,39 +1251,6 @@ int a2b_backward_f32(float *grad_angles, const float *grad_coords, const float *
         case 8: return launch_bwd<8, 128>(a, opt.max_ctas, st);
     }
     return TPL_ERR_UNSUPPORTED;
-}
-
-int a2b_forward_f64_plain(const double *angles, const int32_t *lengths, double *coords, int B, int L,
-                          cudaStream_t st) {
-    if (B == 0 || L == 0) return TPL_OK;
-    PlainArgs a{};
-    a.angles = angles;
-    a.lengths = lengths;
-    a.coords = coords;
-    a.hdr = nullptr;
-    a.rec = nullptr;
-    a.L = L;
-    a.nchunks = (L + kPlainThreads - 1) / kPlainThreads;
-    a.bc = bond_constants();
-    a2b_fwd_f64_plain_kernel<<<B, kPlainThreads, 0, st>>>(a);
-    return cudaGetLastError() == cudaSuccess ? TPL_OK : TPL_ERR_LAUNCH;
-}
-
-int a2b_backward_f64_plain(double *grad_angles, const double *grad_coords, const double *angles,
-                           const int32_t *lengths, void *ws, int B, int L, cudaStream_t st) {
-    if (B == 0 || L == 0) return TPL_OK;
-    PlainArgs a{};
-    a.angles = angles;
-    a.lengths = lengths;
-    a.grad_angles = grad_angles;
-    a.grad_coords = grad_coords;
-    a.hdr = reinterpret_cast<WsHeader *>(ws);
-    a.rec = reinterpret_cast<TileRecord *>(reinterpret_cast<char *>(ws) + sizeof(WsHeader));
-    a.L = L;
-    a.nchunks = (L + kPlainThreads - 1) / kPlainThreads;
-    a.bc = bond_constants();
-    a2b_bwd_f64_plain_kernel<<<B, kPlainThreads, 0, st>>>(a);
-    return cudaGetLastError() == cudaSuccess ? TPL_OK : TPL_ERR_LAUNCH;
 }
 
 }  // namespace tpl

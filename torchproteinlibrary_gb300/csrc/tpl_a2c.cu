@@ -29,6 +29,7 @@
 #include <cstddef>
 #include <cstdio>
 
+#include "tpl_a2c.cuh"
 #include "tpl_async.cuh"
 #include "tpl_common.cuh"
 #include "tpl_internal.h"
@@ -39,32 +40,6 @@
 namespace tpl {
 
 __device__ const Topology<float> g_topo_f32 = make_topology<float>();
-__device__ const Topology<double> g_topo_f64 = make_topology<double>();
-
-template <typename T>
-__device__ __forceinline__ const Topology<T> &topo_global();
-template <>
-__device__ __forceinline__ const Topology<float> &topo_global<float>() { return g_topo_f32; }
-template <>
-__device__ __forceinline__ const Topology<double> &topo_global<double>() { return g_topo_f64; }
-
-template <typename T>
-struct A2cArgs {
-    const unsigned char *seq;
-    int seq_stride;
-    const T *angles;
-    T *coords;
-    uint32_t *res_names;
-    uint32_t *atom_names;
-    T *grad_angles;
-    const T *grad_coords;
-    WsHeader *hdr;
-    int L, maxA;
-};
-
-__device__ __forceinline__ void a2c_error(WsHeader *h, int code) {
-    if (h) atomicCAS(&h->status, 0u, (unsigned)code);
-}
 
 template <typename T>
 __device__ __forceinline__ void sc(T a, T *s, T *c) { sincos_t(a, s, c); }
@@ -106,7 +81,7 @@ struct A2cSmemBwd {
 // Copy the topology to shared memory and build the letter -> type table.
 template <typename T, int NT>
 __device__ __forceinline__ void load_topology(Topology<T> &dst, signed char *lut) {
-    const uint32_t *src = reinterpret_cast<const uint32_t *>(&topo_global<T>());
+    const uint32_t *src = reinterpret_cast<const uint32_t *>(&g_topo_f32);
     uint32_t *d = reinterpret_cast<uint32_t *>(&dst);
     constexpr int n = sizeof(Topology<T>) / 4;
     static_assert(sizeof(Topology<T>) % 4 == 0, "topology size");
@@ -527,44 +502,6 @@ struct A2cRingSmem {
     A2cRingWarp warp[NW];
     uint16_t code[NAMES ? NW : 1][NAMES ? kA2cStageAtoms : 8];
 };
-
-// Length of chain b for the chunked kernels, found by each warp for itself: the index of
-// the row's first NUL (at most the row stride), or 0, with the error recorded, when a
-// letter before it is no residue or the chain is longer than L.  atoms(chunk, n) is
-// called by the whole warp for every chunk of 32 letters in order, with the atom count of
-// this lane's residue.  table: letter -> word with the atom count in bits 8..15, 0 for
-// what is no residue.
-template <typename Table, typename Atoms>
-__device__ __forceinline__ int ring_chain_length(const A2cArgs<float> &a, int b, const Table *table, int lane,
-                                                 Atoms atoms) {
-    const unsigned char *row = a.seq + (size_t)b * a.seq_stride;
-    int len = a.seq_stride;
-    bool bad = false;
-    for (int j0 = 0; j0 < len; j0 += 128) {
-        unsigned char c[4];
-#pragma unroll
-        for (int u = 0; u < 4; u++) {
-            const int j = j0 + 32 * u + lane;
-            c[u] = j < a.seq_stride ? row[j] : (unsigned char)0;
-        }
-#pragma unroll
-        for (int u = 0; u < 4; u++) {
-            const int j1 = j0 + 32 * u;
-            if (j1 >= len) break;
-            const unsigned nul = __ballot_sync(0xffffffffu, c[u] == 0);
-            if (nul != 0u) len = min(len, j1 + __ffs(nul) - 1);
-            const unsigned info = table[c[u]];
-            const bool in = j1 + lane < len;
-            bad |= __any_sync(0xffffffffu, in && info == 0u);
-            if (j1 < len) atoms(j1 >> 5, in ? (int)((info >> 8) & 0xffu) : 0);
-        }
-    }
-    if (bad || len > a.L) {
-        if (lane == 0) a2c_error(a.hdr, bad ? TPL_ERR_SEQUENCE : TPL_ERR_LENGTH);
-        return 0;
-    }
-    return len;
-}
 
 template <int NW, bool NAMES>
 __global__ void __launch_bounds__(32 * NW, NW == 4 ? 6 : 3) a2c_fwd_ring_kernel(A2cArgs<float> a, int renorm, int nb) {
@@ -1362,7 +1299,7 @@ int a2c_forward(bool f64, const unsigned char *seq, int seq_stride, const void *
     if (f64) {
         A2cArgs<double> a{seq, seq_stride, (const double *)angles, (double *)coords, res_names, atom_names,
                           nullptr, nullptr, (WsHeader *)ws, L, maxA};
-        return launch_a2c_fwd<double, 1, 128>(a, B, renorm, st);
+        return a2c_forward_f64(a, B, renorm != 0, st);
     }
     A2cArgs<float> a{seq, seq_stride, (const float *)angles, (float *)coords, res_names, atom_names,
                      nullptr, nullptr, (WsHeader *)ws, L, maxA};
@@ -1386,7 +1323,7 @@ int a2c_backward(bool f64, void *grad_angles, const void *grad_coords, const uns
     if (f64) {
         A2cArgs<double> a{seq, seq_stride, (const double *)angles, nullptr, nullptr, nullptr,
                           (double *)grad_angles, (const double *)grad_coords, (WsHeader *)ws, L, maxA};
-        return launch_a2c_bwd<double, 1, 128>(a, B, renorm, st);
+        return a2c_backward_f64(a, B, renorm != 0, st);
     }
     A2cArgs<float> a{seq, seq_stride, (const float *)angles, nullptr, nullptr, nullptr, (float *)grad_angles,
                      (const float *)grad_coords, (WsHeader *)ws, L, maxA};
