@@ -111,3 +111,34 @@ def test_long_chain_path(built):
     typed.backward(g)
     ref = oracle.typed_coords_backward(g.cpu().numpy(), rcnt, ridx, xc.shape[1] // 3)
     assert np.array_equal(x.grad.cpu().numpy(), ref)
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float64])
+@pytest.mark.parametrize("pad,na", [(p, [0, 1, 31, 32, 33, 127, 128, 129, 511, 512, 513, 640, 1025]) for p in range(4)] +
+                         [(0, [16384, 3]), (1, [16384, 200]), (0, [20000])])
+def test_groups_and_row_phases(built, dtype, pad, na):
+    """Chains around the 128-atom groups and the split over four warps (eight past 16384
+    atoms of row), rows at every 16-byte phase (odd strides), typed rows narrower than the
+    input rows: counts, offsets, indexes and coordinates against the oracle, bit for bit."""
+    from torchproteinlibrary_gb300 import load_extension
+    fm = load_extension("_FullAtomModel")
+    rng = np.random.default_rng(40 + pad)
+    pairs = [(b"ALA\0", a) for a in (b"N\0\0\0", b"CA\0\0", b"CB\0\0", b"C\0\0\0", b"O\0\0\0")]
+    pairs += [(b"LYS\0", b"NZ\0\0"), (b"CYS\0", b"SG\0\0"), (b"TRP\0", b"NE1\0"), (b"SER\0", b"OG\0\0"),
+              (b"ASP\0", b"OD1\0"), (b"PHE\0", b"CZ\0\0"), (b"ARG\0", b"NH1\0")]
+    na = np.array(na, np.int32)
+    B, S_out = len(na), int(na.max())
+    S = S_out + pad
+    pick = rng.integers(0, len(pairs), (B, S))
+    rn = np.array([[list(pairs[k][0]) for k in row] for row in pick], np.uint8)
+    an = np.array([[list(pairs[k][1]) for k in row] for row in pick], np.uint8)
+    x = rng.standard_normal((B, 3 * S)).astype(np.float32 if dtype == torch.float32 else np.float64)
+    dev = torch.device("cuda")
+    xt, rt, at = torch.tensor(x, device=dev), torch.tensor(rn, device=dev), torch.tensor(an, device=dev)
+    out = torch.full((B, 3 * S_out), float("nan"), dtype=dtype, device=dev)
+    cnt = torch.empty(B, 11, dtype=torch.int32, device=dev)
+    off, idx = torch.empty_like(cnt), torch.full((B, S_out), -7, dtype=torch.int32, device=dev)
+    fm.Coords2TypedCoords_forward(xt, rt, at, torch.tensor(na, device=dev), out, cnt, off, idx)
+    want, wcnt, woff, widx = oracle.typed_coords(x, rn, an, na)
+    assert np.array_equal(cnt.cpu().numpy(), wcnt) and np.array_equal(off.cpu().numpy(), woff)
+    assert np.array_equal(out.cpu().numpy(), want) and np.array_equal(idx.cpu().numpy(), widx)

@@ -9,7 +9,9 @@
 // the atoms of its type before it.  The backward is the inverse gather.  Integer and
 // byte work only; coordinates are copied unchanged.
 #include <cstdint>
+#include <type_traits>
 
+#include "tpl_async.cuh"
 #include "tpl_internal.h"
 
 namespace tpl {
@@ -76,31 +78,42 @@ constexpr TypedName kTypedNames[] = {
 };
 constexpr int kTypedNameCount = sizeof(kTypedNames) / sizeof(TypedName);
 
-// The table as an open-addressing hash of 256 slots (filled at compile time; load
-// factor about 0.4), so that a lookup takes one or two probes instead of a walk
-// over every entry.  A residue word of 0 marks an empty slot.
-constexpr int kHashSlots = 256;
-struct TypedHash {
-    uint32_t res[kHashSlots], atom[kHashSlots];
-    int type[kHashSlots];
+// The names as two tables in which every one has a place of its own (multipliers found by
+// trial; checked at compile time), so that a lookup is one probe of each and no branch:
+// the residue-agnostic names by their atom word, the pairs by both words.
+constexpr int kPairSlots = 512, kPlainSlots = 16;
+struct TypedTables {
+    uint32_t pair[kPairSlots][2];   // residue word | type << 24, atom word; type 0xff in an empty slot
+    uint32_t plain[kPlainSlots][2];  // atom word, type; type 0xffffffff in an empty slot
+    int clashes;
 };
-constexpr uint32_t typed_hash(uint32_t res, uint32_t atom) {
-    return ((res * 0x9E3779B1u) ^ (atom * 0x85EBCA77u)) >> 24;  // top 8 bits
+__host__ __device__ constexpr uint32_t pair_slot(uint32_t res, uint32_t atom) {
+    return ((res * 0x6d30140du) ^ (atom * 0x75d7323u)) >> 23;
 }
-constexpr TypedHash build_typed_hash() {
-    TypedHash h{};
-    for (int i = 0; i < kHashSlots; i++) h.type[i] = -1;
+__host__ __device__ constexpr uint32_t plain_slot(uint32_t atom) { return (atom * 0xed753c7bu) >> 28; }
+constexpr TypedTables build_typed_tables() {
+    TypedTables t{};
+    for (int i = 0; i < kPairSlots; i++) t.pair[i][0] = 0xff000000u;
+    for (int i = 0; i < kPlainSlots; i++) t.plain[i][1] = 0xffffffffu;
     for (int i = 0; i < kTypedNameCount; i++) {
-        uint32_t k = typed_hash(kTypedNames[i].res, kTypedNames[i].atom);
-        while (h.res[k] != 0) k = (k + 1) & (kHashSlots - 1);
-        h.res[k] = kTypedNames[i].res;
-        h.atom[k] = kTypedNames[i].atom;
-        h.type[k] = kTypedNames[i].type;
+        const uint32_t k = pair_slot(kTypedNames[i].res, kTypedNames[i].atom);
+        if (t.pair[k][0] != 0xff000000u) t.clashes++;
+        t.pair[k][0] = kTypedNames[i].res | (uint32_t)kTypedNames[i].type << 24;
+        t.pair[k][1] = kTypedNames[i].atom;
     }
-    return h;
+    // O is not a terminal oxygen (the reference's call passes false)
+    const TypedName plain[6] = {{0, nm("O"), 5}, {0, nm("OXT"), 7}, {0, nm("OT2"), 7},
+                                {0, nm("N"), 1}, {0, nm("C"), 8},   {0, nm("CA"), 10}};
+    for (int i = 0; i < 6; i++) {
+        const uint32_t k = plain_slot(plain[i].atom);
+        if (t.plain[k][1] != 0xffffffffu) t.clashes++;
+        t.plain[k][0] = plain[i].atom;
+        t.plain[k][1] = (uint32_t)plain[i].type;
+    }
+    return t;
 }
-static_assert(kTypedNameCount < kHashSlots / 2, "hash load factor");
-__device__ const TypedHash g_typed_hash = build_typed_hash();
+static_assert(build_typed_tables().clashes == 0, "every name has its own slot");
+__device__ const TypedTables g_typed_tables = build_typed_tables();
 
 // Drop the space bytes of a name word (the reference erases whitespace from the
 // atom name before comparing) and stop at the first NUL.
@@ -128,30 +141,22 @@ __device__ __forceinline__ uint32_t squeeze_fast(uint32_t w) {
     return squeeze(w);
 }
 
-// The 0-based type of an atom, or -1 for a name pair the reference rejects; h is the
-// name hash (global memory, or a copy in shared memory).
-__device__ __forceinline__ int atom_type(uint32_t res, uint32_t atom, const TypedHash &h) {
+// The 0-based type of an atom, or -1 for a name pair the reference rejects; tables in
+// global memory, or a copy in shared memory.
+__device__ __forceinline__ int atom_type(uint32_t res, uint32_t atom, const TypedTables &t) {
     atom = squeeze_fast(atom);
     res = res & 0x00ffffffu;  // the residue is its 3-letter code
-    if (atom == nm("O")) return 5;  // not a terminal oxygen (the reference's call passes false)
-    if (atom == nm("OXT") || atom == nm("OT2")) return 7;
-    if (atom == nm("N")) return 1;
-    if (atom == nm("C")) return 8;
-    if (atom == nm("CA")) return 10;
-    uint32_t k = typed_hash(res, atom);
-    for (int probe = 0; probe < kHashSlots; probe++) {
-        const uint32_t r = h.res[k];
-        if (r == 0u) return -1;
-        if (r == res && h.atom[k] == atom) return h.type[k];
-        k = (k + 1) & (kHashSlots - 1);
-    }
-    return -1;
+    const uint2 p = *reinterpret_cast<const uint2 *>(t.pair[pair_slot(res, atom)]);
+    const uint2 q = *reinterpret_cast<const uint2 *>(t.plain[plain_slot(atom)]);
+    const int by_pair = p.y == atom && (p.x & 0x00ffffffu) == res ? (int)p.x >> 24 : -1;
+    const int by_atom = q.x == atom ? (int)q.y : -1;
+    return by_atom >= 0 ? by_atom : by_pair;
 }
-__device__ __forceinline__ int atom_type(uint32_t res, uint32_t atom) { return atom_type(res, atom, g_typed_hash); }
+__device__ __forceinline__ int atom_type(uint32_t res, uint32_t atom) { return atom_type(res, atom, g_typed_tables); }
 
 // Input rows hold in_stride atoms (coordinates and names); typed rows and atom
 // indexes hold out_stride slots.  One CTA per chain, for chains too long for
-// typed_fwd_seg_kernel's type cache: the scatter pass looks the types up again.
+// typed_fwd_group_kernel's codes: the scatter pass looks the types up again.
 template <typename T>
 __global__ void __launch_bounds__(kTypedThreads) typed_fwd_kernel(const T *coords, const uint32_t *res_names,
                                                                   const uint32_t *atom_names, const int *num_atoms,
@@ -232,131 +237,205 @@ __global__ void __launch_bounds__(kTypedThreads) typed_fwd_kernel(const T *coord
     }
 }
 
-// The same regrouping by four warps per chain with three CTA barriers in all: each
-// warp takes a quarter of the chain's 32-atom tiles.  Pass 1 types the atoms of the
-// warp's tiles and counts them per type (per tile, __match_any_sync groups the lanes
-// of each type and the lowest of them adds their number); after a barrier every warp
-// knows where its atoms of each type start (the type's offset plus the counts of the
-// earlier warps), and pass 2 scatters its tiles in order: an atom's slot is its
-// type's next free slot plus its rank among the tile's atoms of that type, so the
-// order within a type is the input order.  Both passes load kTypedUnroll tiles
-// before working on them, so that a warp has several tiles' loads in flight.  Pass
-// 1's types stay in shared memory (in_stride bytes) for pass 2, and the name hash is
-// copied there too.  GB300, 4096 chains of U{50..500} residues: 0.158 -> 0.145 ms
-// against typed_fwd_kernel, which keeps chains of more than kTypeCacheMax atoms.
-constexpr int kTypedWarps = 4;  // warps per chain
+// The same regrouping by NW = 4 or 8 warps per chain with two CTA barriers, for chains whose
+// per-atom codes fit in shared memory.  Each warp takes an equal run of the chain's 32-atom
+// tiles.  Pass 1 types the atoms and ranks each among the warp's atoms of its type (per
+// tile, __match_any_sync groups the lanes of each type); type and rank stay in shared
+// memory, and with them how many atoms of each type came before every group of 128.  After
+// a barrier every warp knows where its atoms of each type start (the type's offset plus
+// the earlier warps' counts): an atom's slot is that plus its rank, so the order within a
+// type is the input order.  Pass 2 takes the groups in turn: the atoms' places when the
+// group is ordered by type, and its slots, go to shared memory, the coordinates come there
+// by cp.async one group ahead, and consecutive lanes write consecutive words of a type's
+// run.
+//
+// What bounds it is instruction issue and the sectors written: an atom scattered straight
+// to its slot costs three partial sectors of coordinates and one of index.  GB300, 4096
+// chains of U{50..500} residues (72 us of HBM traffic): 142 us with scattered stores, a
+// probed name hash and ranks found twice (73 M warp instructions, 21.7 M sector writes);
+// 102 us (63 M, 17.0 M).  Ordering the groups without keeping the ranks was slower than
+// scattering (160 us, 101 M).
 constexpr int kTypedUnroll = 4;
+constexpr int kTypedGroup = 32 * kTypedUnroll;  // atoms ordered and written together
+constexpr int kTypedMaxAtoms = 32768;           // 16-bit codes: ranks below 4096 with NW = 4 up to 16384 atoms, 8 past that
 
+// Groups of one warp's share of a row, and the dynamic shared memory: per warp two groups'
+// coordinates, codes (16 bits per atom), and per warp the counts before each group and
+// after the last.
+constexpr int typed_groups(int in_stride, int nw) {
+    return (((in_stride + 31) / 32 + nw - 1) / nw + kTypedUnroll - 1) / kTypedUnroll;
+}
 template <typename T>
-__global__ void __launch_bounds__(32 * kTypedWarps) typed_fwd_seg_kernel(
+constexpr int kRawWords = 3 * kTypedGroup * (int)sizeof(T) / 4 + 4;  // 4 words for the 16-byte phase
+template <typename T>
+constexpr size_t typed_smem(int in_stride, int nw) {
+    return 8 * (size_t)nw * kRawWords<T> +
+           2 * ((size_t)in_stride + (size_t)nw * (typed_groups(in_stride, nw) + 1) * kTypes);
+}
+
+// Copy the n words at src to dst, shared memory of the same 16-byte phase, by the warp
+// with cp.async (not committed).
+__device__ __forceinline__ void stage_words(float *dst, const float *src, int n, int lane) {
+    const StageSpan sp(src, dst, n);
+    sp.ends(lane);
+    for (int i = 4 * lane; i < sp.body; i += 128) cp_async16(dst + sp.head + i, src + sp.head + i);
+}
+
+template <typename T, int NW>
+__global__ void __launch_bounds__(32 * NW) typed_fwd_group_kernel(
     const T *__restrict__ coords, const uint32_t *__restrict__ res_names, const uint32_t *__restrict__ atom_names,
     const int *__restrict__ num_atoms, int in_stride, int out_stride, T *__restrict__ out,
     int *__restrict__ n_of_type, int *__restrict__ offsets, int *__restrict__ atom_index, WsHeader *hdr) {
-    extern __shared__ signed char s_ty[];
-    __shared__ int s_cnt[kTypedWarps][kTypes];
-    __shared__ int s_ntyped;
-    __shared__ TypedHash s_hash;
+    constexpr int kWords = sizeof(T) / 4;
+    extern __shared__ __align__(16) unsigned char s_dyn[];
+    uint16_t *s_code = reinterpret_cast<uint16_t *>(s_dyn + 8 * NW * kRawWords<T>);  // by atom: rank << 4 | type (15: none)
+    __shared__ int s_cnt[NW][kTypes];
+    __shared__ __align__(16) TypedTables s_tab;
+    __shared__ uint32_t s_perm[NW][kTypedGroup];  // by place in the group: 3 * slot << 9 | 3 * atom of the group
+    __shared__ int2 s_at[NW][16];                 // per type: place and slot of rank 0
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, b = blockIdx.x;
     {
-        const uint32_t *src = reinterpret_cast<const uint32_t *>(&g_typed_hash);
-        uint32_t *dst = reinterpret_cast<uint32_t *>(&s_hash);
-        for (int i = threadIdx.x; i < (int)(sizeof(TypedHash) / 4); i += 32 * kTypedWarps) dst[i] = src[i];
+        const uint32_t *src = reinterpret_cast<const uint32_t *>(&g_typed_tables);
+        uint32_t *dst = reinterpret_cast<uint32_t *>(&s_tab);
+        for (int i = threadIdx.x; i < (int)(sizeof(TypedTables) / 4); i += 32 * NW) dst[i] = src[i];
     }
     const int n = max(0, min(num_atoms[b], min(in_stride, out_stride)));
     const size_t row = (size_t)b * in_stride, orow = (size_t)b * out_stride;
     const uint32_t *rn = res_names + row, *an = atom_names + row;
     const unsigned below = (1u << lane) - 1u;
-    const int ntiles = (n + 31) >> 5, per = (ntiles + kTypedWarps - 1) / kTypedWarps;
-    const int t0 = min(ntiles, w * per), t1 = min(ntiles, t0 + per);
+    const int ntiles = (n + 31) >> 5, per = (ntiles + NW - 1) / NW;
+    const int a0 = min(n, 32 * w * per), a1 = min(n, a0 + 32 * per);  // this warp's atoms
+    uint16_t *s_before = s_code + in_stride + w * (typed_groups(in_stride, NW) + 1) * kTypes;
+    int *cnt = s_cnt[w];
+    if (lane < kTypes) cnt[lane] = 0;
 
-    if (lane < kTypes) s_cnt[w][lane] = 0;
-    __syncthreads();  // the hash copy and the zeroed counts
-    bool bad = false;
-    for (int tb = t0; tb < t1; tb += kTypedUnroll) {
-        uint32_t r[kTypedUnroll], a[kTypedUnroll];
-#pragma unroll
-        for (int u = 0; u < kTypedUnroll; u++) {
-            const int j = 32 * (tb + u) + lane;
-            const bool in = tb + u < t1 && j < n;
-            r[u] = in ? rn[j] : 0u;
-            a[u] = in ? an[j] : 0u;
+    const float *src = reinterpret_cast<const float *>(coords + 3 * row);
+    float *s_raw = reinterpret_cast<float *>(s_dyn) + 2 * w * kRawWords<T>;  // two groups' coordinates
+    auto fetch = [&](int j0, int q) {
+        if (j0 < a1) {
+            const float *from = src + (size_t)3 * kWords * j0;
+            stage_words(s_raw + q * kRawWords<T> + block_offset(from), from, 3 * kWords * min(kTypedGroup, a1 - j0), lane);
         }
+        cp_async_commit();
+    };
+    fetch(a0, 0);  // the first group's coordinates arrive during pass 1
+    __syncthreads();  // the tables and the zeroed counts
+    bool bad = false;
+    uint16_t *before = s_before;
+    uint32_t r[kTypedUnroll], a[kTypedUnroll];  // the next group's names, loaded one group ahead (115 -> 102 us)
+    auto names = [&](int j0) {
 #pragma unroll
         for (int u = 0; u < kTypedUnroll; u++) {
-            const int j = 32 * (tb + u) + lane;
-            const bool in = tb + u < t1 && j < n;
-            const int t = in ? atom_type(r[u], a[u], s_hash) : -2;  // -1: a name pair the reference rejects
-            if (in) s_ty[j] = (signed char)t;
+            const int j = j0 + 32 * u + lane;
+            r[u] = j < a1 ? rn[j] : 0u;
+            a[u] = j < a1 ? an[j] : 0u;
+        }
+    };
+    names(a0);
+    for (int j0 = a0; j0 < a1; j0 += kTypedGroup, before += kTypes) {
+        uint32_t res[kTypedUnroll], atom[kTypedUnroll];
+#pragma unroll
+        for (int u = 0; u < kTypedUnroll; u++) {
+            res[u] = r[u];
+            atom[u] = a[u];
+        }
+        names(j0 + kTypedGroup);
+        if (lane < kTypes) before[lane] = (uint16_t)cnt[lane];
+#pragma unroll
+        for (int u = 0; u < kTypedUnroll; u++) {
+            const int j = j0 + 32 * u + lane;
+            const int t = j < a1 ? atom_type(res[u], atom[u], s_tab) : -2;  // -1: a name pair the reference rejects
             bad |= t == -1;
-            // the lanes of each type: the lowest of them adds their number
             const unsigned m = __match_any_sync(0xffffffffu, t);
-            if (t >= 0 && (m & below) == 0u) s_cnt[w][t] += __popc(m);
+            const int c = t >= 0 ? cnt[t] : 0;
+            __syncwarp();
+            if (t >= 0 && (m & below) == 0u) cnt[t] = c + __popc(m);
+            if (j < a1) s_code[j] = (uint16_t)(t >= 0 ? (c + __popc(m & below)) << 4 | t : 15);
             __syncwarp();
         }
     }
+    if (lane < kTypes) before[lane] = (uint16_t)cnt[lane];
     if (bad) atomicCAS(&hdr->status, 0u, (unsigned)TPL_ERR_ATOM_TYPE);
     __syncthreads();
     // lane k < kTypes: the type's total, its offset, and this warp's first slot of it
-    int tot = 0, before = 0;
+    int tot = 0, earlier = 0;
     if (lane < kTypes)
 #pragma unroll
-        for (int v = 0; v < kTypedWarps; v++) {
+        for (int v = 0; v < NW; v++) {
             const int c = s_cnt[v][lane];
             tot += c;
-            before += v < w ? c : 0;
+            earlier += v < w ? c : 0;
         }
-    int inc = tot;
+    auto scan = [&](int v) {  // inclusive over lanes 0 .. 15
 #pragma unroll
-    for (int off = 1; off < 16; off <<= 1) {
-        const int v = __shfl_up_sync(0xffffffffu, inc, off);
-        if (lane >= off) inc += v;
-    }
-    const int type_off = inc - tot;
+        for (int off = 1; off < 16; off <<= 1) {
+            const int o = __shfl_up_sync(0xffffffffu, v, off);
+            if (lane >= off) v += o;
+        }
+        return v;
+    };
+    const int inc = scan(tot), type_off = inc - tot, slot0 = type_off + earlier;
+    const int ntyped = __shfl_sync(0xffffffffu, inc, kTypes - 1);
     if (w == 0 && lane < kTypes) {
         n_of_type[(size_t)b * kTypes + lane] = tot;
         offsets[(size_t)b * kTypes + lane] = type_off;
     }
-    if (w == 0 && lane == kTypes - 1) s_ntyped = inc;
-    __syncthreads();  // every warp has read the counts
-    int *s_next = s_cnt[w];  // reused: this warp's next free slot of each type
-    if (lane < kTypes) s_next[lane] = type_off + before;
-    __syncwarp();
 
-    for (int tb = t0; tb < t1; tb += kTypedUnroll) {
-        T x[kTypedUnroll][3];
-        int ty[kTypedUnroll];
+    uint32_t *perm = s_perm[w];
+    T *o = out + 3 * orow;
+    before = s_before;
+    // word e = lane + 32 i of a group's coordinates belongs to place e / 3: 32 (i / 3) plus
+    // one of three values per lane
+    int at[3], x[3];
+#pragma unroll
+    for (int k = 0; k < 3; k++) {
+        at[k] = (lane + 32 * k) / 3;
+        x[k] = (lane + 32 * k) % 3;
+    }
+    for (int j0 = a0, q = 0; j0 < a1; j0 += kTypedGroup, q ^= 1, before += kTypes) {
+        __syncwarp();  // every lane is done with the group before
+        fetch(j0 + kTypedGroup, q ^ 1);
+        // lane k < kTypes: the type's run in the group ordered by type
+        const int b0 = lane < kTypes ? before[lane] : 0, c = lane < kTypes ? before[kTypes + lane] - b0 : 0;
+        const int run = scan(c), in_group = __shfl_sync(0xffffffffu, run, kTypes - 1);
+        if (lane < kTypes) s_at[w][lane] = make_int2(run - c - b0, slot0);
+        __syncwarp();
 #pragma unroll
         for (int u = 0; u < kTypedUnroll; u++) {
-            const int j = 32 * (tb + u) + lane;
-            const bool in = tb + u < t1 && j < n;
-            const T *src = coords + 3 * (row + j);
+            const int j = j0 + 32 * u + lane;
+            const int code = j < a1 ? s_code[j] : 15, t = code & 15, rank = code >> 4;
+            if (t != 15) {
+                const int2 p = s_at[w][t];
+                perm[p.x + rank] = (uint32_t)(3 * (p.y + rank)) << 9 | (uint32_t)(3 * (32 * u + lane));
+            }
+        }
+        cp_async_wait1();  // this group's coordinates
+        __syncwarp();
+        const T *raw = reinterpret_cast<const T *>(s_raw + q * kRawWords<T> + block_offset(src + (size_t)3 * kWords * j0));
 #pragma unroll
-            for (int c = 0; c < 3; c++) x[u][c] = in ? src[c] : T(0);
-            ty[u] = in ? (int)s_ty[j] : -2;
+        for (int i = 0; i < 3 * kTypedUnroll; i++) {
+            if (lane + 32 * i < 3 * in_group) {
+                const uint32_t p = perm[32 * (i / 3) + at[i % 3]];
+                o[(p >> 9) + x[i % 3]] = raw[(p & 511u) + x[i % 3]];
+            }
         }
 #pragma unroll
         for (int u = 0; u < kTypedUnroll; u++) {
-            const int j = 32 * (tb + u) + lane, t = ty[u];
-            const unsigned m = __match_any_sync(0xffffffffu, t);
-            if (t >= 0) {
-                const int slot = s_next[t] + __popc(m & below);
-                T *dst = out + 3 * (orow + slot);
-                dst[0] = x[u][0];
-                dst[1] = x[u][1];
-                dst[2] = x[u][2];
-                atom_index[orow + slot] = j;
+            if (32 * u + lane < in_group) {
+                const uint32_t p = perm[32 * u + lane];
+                // thirds of multiples of three below 2^17 and 2^9
+                atom_index[orow + ((p >> 9) * 43691u >> 17)] = j0 + (int)((p & 511u) * 171u >> 9);
             }
-            __syncwarp();
-            if (t >= 0 && (m & below) == 0u) s_next[t] += __popc(m);
-            __syncwarp();
         }
     }
-    __syncthreads();
-    // slots past the typed atoms are zero, as in the reference's zero-filled outputs
-    const int ntyped = s_ntyped;
-    T *o = out + 3 * orow;
-    for (int e = 3 * ntyped + threadIdx.x; e < 3 * out_stride; e += 32 * kTypedWarps) o[e] = T(0);
-    for (int q = ntyped + threadIdx.x; q < out_stride; q += 32 * kTypedWarps) atom_index[orow + q] = 0;
+    // slots past the typed atoms are zero, as in the reference's zero-filled outputs; a
+    // share of each span per warp
+    auto zeros = [&](void *p, int words) {
+        const int share = (words + NW - 1) / NW;
+        zero_span(static_cast<uint32_t *>(p) + w * share, min(share, words - w * share), lane);
+    };
+    zeros(out + 3 * (orow + ntyped), 3 * kWords * (out_stride - ntyped));
+    zeros(atom_index + orow + ntyped, out_stride - ntyped);
 }
 
 // grad_flat[atom_index[s]] = grad_typed[s] for the typed slots, zero elsewhere;
@@ -432,7 +511,6 @@ __global__ void __launch_bounds__(kTypedThreads) typed_bwd_gather_kernel(const T
 }
 
 constexpr int kGatherMaxAtoms = 16384;  // 64 KB of slots per CTA
-constexpr int kTypeCacheMax = 32768;    // typed_fwd_seg_kernel's type cache: one byte per input atom
 
 }  // namespace
 
@@ -441,19 +519,24 @@ int typed_forward(bool f64, const void *coords, const uint32_t *res_names, const
                   int *atom_index, void *ws, cudaStream_t st) {
     if (B == 0) return TPL_OK;
     WsHeader *hdr = reinterpret_cast<WsHeader *>(ws);
-    if (in_stride <= kTypeCacheMax) {  // four warps per chain, types cached in shared memory
-        const size_t smem = (size_t)in_stride;
-        auto launch_s = [&](auto kernel, auto *out_t, auto *coords_t) -> int {
-            if (smem > 48 * 1024 && !set_max_dynamic_smem(reinterpret_cast<const void *>(kernel), (int)smem))
-                return TPL_ERR_LAUNCH;
-            kernel<<<B, 32 * kTypedWarps, smem, st>>>(coords_t, res_names, atom_names, num_atoms, in_stride,
-                                                       out_stride, out_t, n_of_type, offsets, atom_index, hdr);
+    if (in_stride <= kTypedMaxAtoms) {
+        auto launch = [&](auto nw, auto *out_t, auto *coords_t) -> int {
+            constexpr int NW = decltype(nw)::value;
+            using T = std::remove_pointer_t<decltype(out_t)>;
+            auto kernel = typed_fwd_group_kernel<T, NW>;
+            const size_t smem = typed_smem<T>(in_stride, NW);
+            if (!set_max_dynamic_smem(reinterpret_cast<const void *>(kernel), (int)smem)) return TPL_ERR_LAUNCH;
+            kernel<<<B, 32 * NW, smem, st>>>(coords_t, res_names, atom_names, num_atoms, in_stride, out_stride, out_t,
+                                             n_of_type, offsets, atom_index, hdr);
             return cudaGetLastError() == cudaSuccess ? (int)TPL_OK : (int)TPL_ERR_LAUNCH;
         };
-        if (f64)
-            return launch_s(typed_fwd_seg_kernel<double>, static_cast<double *>(out),
-                            static_cast<const double *>(coords));
-        return launch_s(typed_fwd_seg_kernel<float>, static_cast<float *>(out), static_cast<const float *>(coords));
+        auto pick = [&](auto *out_t, auto *coords_t) -> int {
+            // four warps' ranks fit the codes up to 16384 atoms
+            return in_stride <= kTypedMaxAtoms / 2 ? launch(std::integral_constant<int, 4>{}, out_t, coords_t)
+                                                   : launch(std::integral_constant<int, 8>{}, out_t, coords_t);
+        };
+        return f64 ? pick(static_cast<double *>(out), static_cast<const double *>(coords))
+                   : pick(static_cast<float *>(out), static_cast<const float *>(coords));
     }
     // longer chains: one CTA per chain, the types looked up again in the scatter pass
     if (f64)
