@@ -39,6 +39,13 @@ def _check(t, what, device):
             raise Exception(f"Coords2TypedCoordsFunction: {what} Nan")
 
 
+def _max_atoms(num_atoms):
+    known = getattr(num_atoms, "_tpl_max_atoms", None)  # Angles2Coords' counts carry their maximum
+    if known is not None:
+        return known
+    return int(torch.max(num_atoms)) if num_atoms.numel() else 0
+
+
 class Coords2TypedCoordsFunction(Function):
     """coordinates -> coordinates arranged in atom types function"""
 
@@ -50,9 +57,7 @@ class Coords2TypedCoordsFunction(Function):
             raise RuntimeError("Coords2TypedCoords: this build has no CPU path; move the tensors to a CUDA device")
         x = input_coords.contiguous()
         dev = x.device
-        max_num_atoms = getattr(num_atoms, "_tpl_max_atoms", None)  # Angles2Coords' counts carry their maximum
-        if max_num_atoms is None:
-            max_num_atoms = int(torch.max(num_atoms)) if num_atoms.numel() else 0
+        max_num_atoms = _max_atoms(num_atoms)
         B = x.size(0)
         na = num_atoms.to(device=dev, dtype=torch.int32).contiguous()
         rn = input_resnames.to(dev).contiguous()
@@ -84,4 +89,9 @@ class Coords2TypedCoords(Module):
         super(Coords2TypedCoords, self).__init__()
 
     def forward(self, input_coords, input_resnames, input_atomnames, num_atoms):
+        if (input_coords.dim() == 2 and input_coords.is_cuda and os.environ.get("TPL_CHECK_NAN", "0") != "1"
+                and not torch.jit.is_tracing() and not torch._C._are_functorch_transforms_active()):
+            # the same entries through the extension's C++ autograd function: no Python frame
+            return tuple(_FullAtomModel.typed_coords_autograd(input_coords, input_resnames, input_atomnames, num_atoms,
+                                                              _max_atoms(num_atoms)))
         return Coords2TypedCoordsFunction.apply(input_coords, input_resnames, input_atomnames, num_atoms)

@@ -18,6 +18,9 @@ Differences from the reference:
     check raises).
   * The NaN checks that force a host sync after every call run only when
     TPL_CHECK_NAN=1.
+  * The modules and getBBox run the extension's C++ autograd functions (the same entries);
+    with TPL_CHECK_NAN=1, under torch.jit.trace and under functorch transforms they run the
+    Python functions below.
 """
 import math
 import os
@@ -39,11 +42,22 @@ def _check(t, what):
         raise Exception(f"{what} Nan")
 
 
-def _coords(x, what):
+def _native():
+    """Whether the extension's C++ autograd functions may take a call: the NaN check, tracing
+    and functorch transforms go through the Python functions, which those see as such."""
+    return not (os.environ.get("TPL_CHECK_NAN", "0") == "1" or torch.jit.is_tracing()
+                or torch._C._are_functorch_transforms_active())
+
+
+def _check_coords(x, what):
     if x.dim() != 2:
         raise ValueError(f'{what}: ', 'Incorrect input size:', x.size())
     if not x.is_cuda:
         raise RuntimeError(f"{what}: this build has no CPU path; move the tensors to a CUDA device")
+
+
+def _coords(x, what):
+    _check_coords(x, what)
     return x.contiguous()
 
 
@@ -53,6 +67,9 @@ def _num_atoms(num_atoms, device):
 
 def getBBox(input_coords, num_atoms):
     """Per-chain bounding box: a = min, b = max over the first num_atoms[b] atoms."""
+    if _native():
+        _check_coords(input_coords, "getBBox")
+        return tuple(_FullAtomModel.bbox(input_coords, num_atoms))
     x = _coords(input_coords, "getBBox")
     a = torch.empty(x.size(0), 3, dtype=x.dtype, device=x.device)
     b = torch.empty_like(a)
@@ -120,6 +137,9 @@ class CoordsTranslate(Module):
         super(CoordsTranslate, self).__init__()
 
     def forward(self, input_coords, T, num_atoms):
+        if _native():
+            _check_coords(input_coords, "CoordsTranslateFunction")
+            return _FullAtomModel.coords_translate_autograd(input_coords, T, num_atoms)
         return CoordsTranslateFunction.apply(input_coords, T, num_atoms)
 
 
@@ -152,6 +172,9 @@ class CoordsRotate(Module):
         super(CoordsRotate, self).__init__()
 
     def forward(self, input_coords, R, num_atoms):
+        if _native():
+            _check_coords(input_coords, "CoordsRotateFunction")
+            return _FullAtomModel.coords_rotate_autograd(input_coords, R, num_atoms)
         return CoordsRotateFunction.apply(input_coords, R, num_atoms)
 
 
@@ -183,4 +206,7 @@ class Coords2Center(Module):
         super(Coords2Center, self).__init__()
 
     def forward(self, input_coords, num_atoms):
+        if _native():
+            _check_coords(input_coords, "Coords2CenterFunction")
+            return _FullAtomModel.coords_center_autograd(input_coords, num_atoms)
         return Coords2CenterFunction.apply(input_coords, num_atoms)

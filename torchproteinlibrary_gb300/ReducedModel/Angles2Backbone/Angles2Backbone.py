@@ -58,13 +58,18 @@ def new_workspace(batch, max_len, device, residues_per_thread=-1, threads_per_ct
                        dtype=torch.uint8, device=device)
 
 
-def _shared_workspace(batch, max_len, device, fwd_opts):
+def _shared_workspace(batch, max_len, device, fwd_opts, private=False):
     """A zeroed-once workspace per (device, current stream, shape, options), kept for
     reuse by later calls (at most _WS_CACHE_SIZE of them).  A graph being captured
-    gets one of its own."""
+    gets one of its own; private: no caller can reach it to read its status word."""
     if torch.cuda.is_current_stream_capturing():
+        if private and fwd_opts[1] in (4, 32):
+            # one CTA or one warp per chain keeps no look-back words there that must start
+            # from zero: no memset in the graph (13 MB, 3 us, at 4096 x 1000)
+            return torch.empty(int(_ReducedModel.workspace_bytes(batch, max_len, *fwd_opts)), dtype=torch.uint8,
+                               device=device)
         return new_workspace(batch, max_len, device, *fwd_opts)
-    key = (device.index, torch.cuda.current_stream(device).cuda_stream, batch, max_len) + tuple(fwd_opts)
+    key = (device.index, torch._C._cuda_getCurrentRawStream(device.index), batch, max_len) + tuple(fwd_opts)
     ws = _WS_CACHE.get(key)
     if ws is None:
         ws = new_workspace(batch, max_len, device, *fwd_opts)
@@ -151,5 +156,5 @@ class Angles2Backbone(Module):
         dev = input.device
         tuned = autotune.options_for(dev, batch_size, max_len)
         fwd_opts, bwd_opts = tuned if tuned is not None else ((-1, -1), (-1, -1, -1))
-        ws = _shared_workspace(batch_size, max_len, dev, fwd_opts)
+        ws = _shared_workspace(batch_size, max_len, dev, fwd_opts, private=True)
         return _ReducedModel.angles2backbone_autograd(input, angles_length, ws, list(fwd_opts), list(bwd_opts))
