@@ -374,23 +374,17 @@ struct FwdStage {
     __device__ static __forceinline__ int lane_offset(int l) { return l * SEG + GAP * (l >> 2); }
 };
 
-// store_chunk for the FwdStage layout: float4 q of the chunk (floats 4q..4q+3, in lane
-// segment floor(4q / SEG)) is staged at float 4q + GAP floor(q / SEG).
-__device__ __forceinline__ void st_evict_last(float4 *p, float4 v, uint64_t pol) {
-    asm volatile("st.global.L2::cache_hint.v4.f32 [%0], {%1, %2, %3, %4}, %5;" ::"l"(p), "f"(v.x), "f"(v.y), "f"(v.z),
-                 "f"(v.w), "l"(pol)
-                 : "memory");
-}
-
 // The coordinates are stored with an L2 evict-last hint: the layer's backward reads
 // them back (chains last to first, so the rows written last come first), and the rows
 // still in L2 save their DRAM reads (GB300, 4096 x 1000: backward 0.0601 -> 0.0580 ms
 // in the step; evict-first stores kept fewer of them).
 //
-// At C = 4 the staging layout is the chunk's own order (no gaps), so an aligned chunk
-// leaves as one bulk copy issued by lane 0; the warp waits for its reads of the buffer
+// The staging layout is the chunk's own order but for the gaps (none at C = 4, one after
+// every four lanes at C = 8), so an aligned chunk leaves as one bulk copy, or as eight of
+// 1152 bytes, each issued by a lane; the warp waits for their reads of the buffer
 // (store_reads_done) when the next chunk is about to rewrite it (a2b_fwd_ring_kernel<4>,
-// 4096 x 1000: 56.9 -> 51.3 us, issue active 60 -> 69 %).
+// 4096 x 1000: 56.9 -> 51.3 us, issue active 60 -> 69 %; a2b_fwd_ring_kernel<8>, against
+// 16-byte stores: 56 -> 45.6 us).
 template <int C>
 __device__ __forceinline__ void store_chunk_fwd(float *dst, const float *stage, int n, int lane, bool vec) {
     using S = FwdStage<C>;
@@ -398,21 +392,15 @@ __device__ __forceinline__ void store_chunk_fwd(float *dst, const float *stage, 
     if (vec) {
         uint64_t pol;
         asm volatile("createpolicy.fractional.L2::evict_last.b64 %0, 1.0;" : "=l"(pol));
-        if constexpr (S::GAP == 0) {
-            async_proxy_fence();
-            __syncwarp();
-            if (lane == 0)
-                asm volatile("cp.async.bulk.global.shared::cta.bulk_group.L2::cache_hint [%0], [%1], %2, %3;\n"
-                             "cp.async.bulk.commit_group;" ::"l"(dst),
-                             "r"(smem_addr(stage)), "r"(4 * n), "l"(pol)
-                             : "memory");
-            return;
-        }
+        constexpr int RUN = S::GAP == 0 ? 32 * SEG : 4 * SEG;  // floats without a gap
+        async_proxy_fence();
         __syncwarp();
-#pragma unroll 2
-        for (int q = lane; 4 * q < n; q += 32)
-            st_evict_last(reinterpret_cast<float4 *>(dst) + q,
-                          *reinterpret_cast<const float4 *>(stage + 4 * q + S::GAP * (q / SEG)), pol);
+        const int f = RUN * lane;  // lanes past the last run have nothing left
+        if (f < n)
+            asm volatile("cp.async.bulk.global.shared::cta.bulk_group.L2::cache_hint [%0], [%1], %2, %3;\n"
+                         "cp.async.bulk.commit_group;" ::"l"(dst + f),
+                         "r"(smem_addr(stage + f + S::GAP * lane)), "r"(4 * min(RUN, n - f)), "l"(pol)
+                         : "memory");
     } else {
         __syncwarp();
         for (int f = lane; f < n; f += 32) {
@@ -421,10 +409,9 @@ __device__ __forceinline__ void store_chunk_fwd(float *dst, const float *stage, 
         }
     }
 }
-// Before the staging buffer is rewritten, or the kernel ends.
-template <int C>
-__device__ __forceinline__ void store_reads_done(int lane) {
-    if (FwdStage<C>::GAP == 0 && lane == 0) bulk_reads_done();
+// Before the staging buffer is rewritten, or the kernel ends: by the lanes that copied.
+__device__ __forceinline__ void store_reads_done() {
+    bulk_reads_done();
     __syncwarp();
 }
 
@@ -480,7 +467,7 @@ __global__ void __launch_bounds__(32 * kWarpsPerCta, fwd_min_blocks(C)) a2b_fwd_
             continue;
         }
         const int j0 = s0 + C * lane;
-        store_reads_done<C>(lane);  // the walk rewrites the staging buffer
+        store_reads_done();  // the walk rewrites the staging buffer
         Frame<float> T;
         if (pf) {
             if (s0 + CH < len) prefetch_angles<C>(abuf + (it ^ 1) * 3 * CH, ang, a.L, s0 + CH, lane);
@@ -500,7 +487,7 @@ __global__ void __launch_bounds__(32 * kWarpsPerCta, fwd_min_blocks(C)) a2b_fwd_
         map_positions<C>(seg, P, j0, len);
         store_chunk_fwd<C>(dst, stage, 9 * nout, lane, vec);
     }
-    store_reads_done<C>(lane);
+    store_reads_done();
 }
 
 template <int C>
@@ -1113,7 +1100,7 @@ __global__ void __launch_bounds__(32 * kRingWarps, ring_fwd_min_blocks(C)) a2b_f
         const int j0 = s0 + C * lane;
         PairFrame t = pair_identity();  // prefix of the lane transforms through this lane
         if (live) {  // no renormalisation of the lane transforms (3C joints each), as in a2b_fwd_chain_kernel
-            store_reads_done<C>(lane);  // the walk rewrites the staging buffer
+            store_reads_done();  // the walk rewrites the staging buffer
             Frame<float> T;
             if (pf) {
                 const int sn = s0 + kRingWarps * CH;
@@ -1157,7 +1144,7 @@ __global__ void __launch_bounds__(32 * kRingWarps, ring_fwd_min_blocks(C)) a2b_f
         map_positions<C>(seg, P, j0, len);
         store_chunk_fwd<C>(dst, stage, 9 * nout, lane, vec);
     }
-    store_reads_done<C>(lane);
+    store_reads_done();
 }
 
 // Backward from the coordinates with the ring split of a2b_bwd_coords_kernel: the

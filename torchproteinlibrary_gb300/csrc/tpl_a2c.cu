@@ -971,6 +971,8 @@ __device__ __forceinline__ float suffix_excl(float v, int lane, float &total) {
     return inc - v;
 }
 
+// The cross product on its own, then added: accumulated straight into S it would save three
+// additions but chain two FMAs per atom (4096 x 500: 144 -> 157 us).
 __device__ __forceinline__ void add_atom(const float *xs, const float *gs, const float *o, float *G, float *S) {
     const float xr[3] = {xs[0] - o[0], xs[1] - o[1], xs[2] - o[2]};
     float xg[3];
