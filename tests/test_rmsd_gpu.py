@@ -173,3 +173,30 @@ def test_atom_groups_at_every_alignment_and_block_size(built, dtype, B, N, offs)
         want = float(w[b]) * grads[b, :3 * n]
         scale = np.abs(want).max()
         assert np.abs(g[b, :3 * n] - want).max() <= (1e-3 if dtype == torch.float32 else 1e-8) * scale
+
+
+@pytest.mark.parametrize("half", [0, 1])
+def test_two_chains_per_cta(built, half):
+    """Large batches solve two chains per warp, one on each half: an odd batch (the last CTA
+    has one chain), and next to an ordinary chain one that takes the degenerate solve (a
+    rigid copy of a collinear set), an empty one and a one-atom one, on either half.
+    Tolerance as for the other batches: 1e-4 of the largest value in float32."""
+    from torchproteinlibrary_gb300.RMSD import Coords2RMSD
+    rng = np.random.default_rng(7 + half)
+    B, N = 4 * torch.cuda.get_device_properties(0).multi_processor_count + 5, 37
+    B += 1 - B % 2
+    na = rng.integers(9, N + 1, B).astype(np.int32)
+    src = rng.standard_normal((B, 3 * N)) * 10 + 30
+    dst = rng.standard_normal((B, 3 * N)) * 10 - 20
+    for b in range(half, B - 1, 14):
+        line = np.outer(np.arange(N), [1.0, 2.0, -0.5])
+        src[b], dst[b] = line.ravel(), line[::-1].ravel()
+    na[half + 2:B - 1:14] = 0
+    na[half + 4:B - 1:14] = 1
+    r = Coords2RMSD()(torch.tensor(src, dtype=torch.float32).cuda(), torch.tensor(dst, dtype=torch.float32).cuda(),
+                      torch.tensor(na))
+    src, dst = src.astype(np.float32).astype(np.float64), dst.astype(np.float32).astype(np.float64)
+    ref, _, _ = oracle.rmsd(src, dst, na)
+    ok = na > 1
+    assert np.abs(r.double().cpu().numpy() - ref)[ok].max() <= 1e-4 * ref[ok].max()
+    assert r[torch.tensor(na == 0)].eq(0).all()

@@ -9,7 +9,7 @@
 // correlation R_ab = sum x_a y_b and R2 = sum |x|^2 + |y|^2 (sums in the coordinate
 // type per thread and per warp, in FP64 across the warps), the 4x4 matrix T (same
 // layout as the reference), its largest eigenpair by the characteristic-polynomial
-// method on one warp (key_eigen_warp), U from the unit quaternion, UT = U^T and
+// method on one warp (key_eigen_halves), U from the unit quaternion, UT = U^T and
 // rmsd = sqrt((R2 - 2 |lambda_max| + 1e-10) / N).  The backward is one launch with
 // one thread per group of atoms (chains on x, blocks of groups on y):
 // dL/dx_i = g (x_i - UT y_i) / (rmsd N) on the centred coordinates.
@@ -19,7 +19,8 @@
 // for 16 cycles whether one lane or 32 take part.  A form with every warp's partial sums
 // converted and the solve written for one lane spent about 280 of them per chain (ncu:
 // FP64 pipe 73 % busy; 4096 chains of 400..2303 atoms, 20 us of HBM traffic: 90 us per
-// layer call); this one about 100, and reads the coordinates once: 45 us.
+// layer call); this one, which solves two chains with the same instructions and reads the
+// coordinates once, about 45: 37 us.
 #include <cmath>
 #include <cstring>
 
@@ -79,7 +80,7 @@ __device__ __forceinline__ double det3(double a, double b, double c, double d, d
 }
 
 // Largest eigenpair of the symmetric 4x4 K by cyclic Jacobi rotations in FP64, on one
-// thread: the fallback of key_eigen_warp for a near-multiple largest root (collinear
+// thread: the fallback of key_eigen_halves for a near-multiple largest root (collinear
 // or otherwise degenerate structures, two-atom chains), where Newton on the quartic
 // converges only linearly and stalls at about the square root of the rounding error.
 // Rotation (p, r) with t = sgn(theta) / (|theta| + sqrt(theta^2 + 1)),
@@ -131,17 +132,16 @@ __device__ __forceinline__ void jacobi_top_eigenpair(const double *K, double *a,
     for (int k = 0; k < 4; k++) q[k] = v[4 * k + best];
 }
 
-// The eigenvector of key_eigen_warp<true>, in FP32: the largest row of the cofactor
+// The eigenvector of key_eigen_halves<true>, in FP32: the largest row of the cofactor
 // matrix of M = K - l I (entries of order one, in shared memory), one cofactor per
-// lane.  The root itself stays FP64: when the top two eigenvalues nearly meet it is
-// ill-conditioned, and an all-FP32 solve moved it by up to 3e-5 relative (a 2.4e-4
+// lane of each half warp.  The root itself stays FP64: when the top two eigenvalues nearly
+// meet it is ill-conditioned, and an all-FP32 solve moved it by up to 3e-5 relative (a 2.4e-4
 // gradient error on one of 256 training-step chains), where this form matches the
 // FP64 solve to 1e-5 of the largest gradient.
 __device__ void eigvec_f32(const float *sM, double (&q)[4]) {
-    const int lane = threadIdx.x & 31;
-    float cf = 0.f;
-    if (lane < 16) {
-        const int i = lane >> 2, j = lane & 3;
+    float cf;
+    {
+        const int i = (threadIdx.x & 15) >> 2, j = threadIdx.x & 3;
         float m[9];  // rows but i, columns but j
 #pragma unroll
         for (int t = 0; t < 9; t++) m[t] = sM[4 * (t / 3 + (t / 3 >= i)) + t % 3 + (t % 3 >= j)];
@@ -153,9 +153,9 @@ __device__ void eigvec_f32(const float *sM, double (&q)[4]) {
     nrm += __shfl_xor_sync(0xffffffffu, nrm, 1);
     nrm += __shfl_xor_sync(0xffffffffu, nrm, 2);
     int best = 0;
-    float bn = __shfl_sync(0xffffffffu, nrm, 0);
+    float bn = __shfl_sync(0xffffffffu, nrm, 0, 16);
     for (int i = 1; i < 4; i++) {
-        const float v = __shfl_sync(0xffffffffu, nrm, 4 * i);
+        const float v = __shfl_sync(0xffffffffu, nrm, 4 * i, 16);
         if (v > bn) {
             bn = v;
             best = i;
@@ -164,7 +164,7 @@ __device__ void eigvec_f32(const float *sM, double (&q)[4]) {
     const bool ok = bn > 1e-30f;
     const float inv = ok ? rsqrtf(bn) : 0.f;
 #pragma unroll
-    for (int k = 0; k < 4; k++) q[k] = (double)(__shfl_sync(0xffffffffu, cf, 4 * best + k) * inv);
+    for (int k = 0; k < 4; k++) q[k] = (double)(__shfl_sync(0xffffffffu, cf, 4 * best + k, 16) * inv);
     if (!ok) {
         q[0] = 1.0;
         q[1] = q[2] = q[3] = 0.0;
@@ -202,43 +202,50 @@ __device__ __forceinline__ double negate_if(double v, bool neg) {  // on the sig
 //   * R (nine doubles, shared memory) and e0 = (sum |x|^2 + |y|^2) / 2 >= l_max come
 //     scaled by unit_scale(), so nothing is divided to bring them to order one.
 //   * FP64 instructions are few: one entry of K per lane (two additions), |R|^2 as a
-//     shuffle sum, the cofactor expansion of det K along row 0 on four lanes.
+//     shuffle sum, the cofactor expansion of det K along row 0 on four lanes and det R on
+//     four others in the same instructions.
 //   * Newton's method from e0 descends monotonically to the largest root.  It runs in
 //     FP32 and is then polished by three FP64 Newton steps whose quotient uses an FP32
 //     reciprocal (each step gains about seven digits).
 //   * The eigenvector is the largest row of the cofactor matrix of K - l I (rank one
 //     for a simple root), one cofactor per lane.
 //   * F32_VEC (float32 inputs): the eigenvector in FP32 instead (eigvec_f32).
-// sK: 16 doubles of scratch, sM: 16 floats, s_jac: 32 doubles.  Executed by a full
-// warp; every lane returns l (scaled) and the unit q (q = 1, 0, 0, 0 when every
-// cofactor vanishes).
+// Executed by a full warp whose halves of 16 lanes each solve a problem of their own (an
+// FP64 instruction costs the same for both): sR, e0 and the scratch sK (16 doubles), sM
+// (16 floats) and s_jac (32 doubles) are the half's; every lane of it returns its l
+// (scaled) and unit q (q = 1, 0, 0, 0 when every cofactor vanishes).
 template <bool F32_VEC>
-__device__ void key_eigen_warp(const double *sR, double e0, double *sK, float *sM, double *s_jac, double &l,
-                               double (&q)[4]) {
-    const int lane = threadIdx.x & 31, e = lane & 15;
+__device__ void key_eigen_halves(const double *sR, double e0, double *sK, float *sM, double *s_jac, double &l,
+                                 double (&q)[4]) {
+    const int e = threadIdx.x & 15;
     constexpr uint64_t kA = pack_nibbles(kKeyA), kB = pack_nibbles(kKeyB);
     const bool diag = (e >> 2) == (e & 3);
     double k = negate_if(sR[(kA >> (4 * e)) & 15], (kKeyNegA >> e) & 1u) +
                negate_if(sR[(kB >> (4 * e)) & 15], (kKeyNegB >> e) & 1u);
     if (diag) k += negate_if(sR[8], (kKeyNegC >> e) & 1u);
-    if (lane < 16) sK[e] = k;
+    sK[e] = k;
     double t2 = e < 9 ? sR[e] : 0.0;
     t2 *= t2;
 #pragma unroll
     for (int off = 8; off > 0; off >>= 1) t2 += __shfl_xor_sync(0xffffffffu, t2, off);
     const double c2 = -2.0 * t2;
-    const double c1 = -8.0 * det3(sR[0], sR[1], sR[2], sR[3], sR[4], sR[5], sR[6], sR[7], sR[8]);
     __syncwarp();
-    double c0;
+    double c0, c1;
     {
-        const int j = lane & 3;
-        const int ca = j == 0 ? 1 : 0, cb = j <= 1 ? 2 : 1, cc = j <= 2 ? 3 : 2;
-        c0 = negate_if(sK[j], j & 1) * det3(sK[4 + ca], sK[4 + cb], sK[4 + cc], sK[8 + ca], sK[8 + cb], sK[8 + cc],
-                                            sK[12 + ca], sK[12 + cb], sK[12 + cc]);
-        c0 += __shfl_xor_sync(0xffffffffu, c0, 1);
-        c0 += __shfl_xor_sync(0xffffffffu, c0, 2);
+        const int j = e & 3;  // lanes 0..3: the minor of K without row 0 and column j; 4..7: R
+        double m[9];
+#pragma unroll
+        for (int t = 0; t < 9; t++)
+            m[t] = *((e & 4) ? sR + t : sK + 4 * (1 + t / 3) + t % 3 + (t % 3 >= j));
+        const double d = det3(m[0], m[1], m[2], m[3], m[4], m[5], m[6], m[7], m[8]);
+        double s = negate_if(sK[j], j & 1) * d;
+        s += __shfl_xor_sync(0xffffffffu, s, 1);
+        s += __shfl_xor_sync(0xffffffffu, s, 2);
+        c0 = __shfl_sync(0xffffffffu, s, 0, 16);
+        c1 = -8.0 * __shfl_sync(0xffffffffu, d, 4, 16);
     }
     l = 0.0;
+    bool simple = true;
     if (e0 > 0.0) {
         const float e0f = (float)e0, a2 = (float)c2, a1 = (float)c1, a0 = (float)c0;
         float s = e0f * 1.0000002f;  // not below e0
@@ -268,55 +275,59 @@ __device__ void key_eigen_warp(const double *sR, double e0, double *sK, float *s
         // a simple root has converged by the third polish step (each gains about
         // seven digits); a near-multiple one (the top eigenvalues of K nearly or
         // exactly equal) converges only linearly: a last step above 1e-10 of e0 sends
-        // the chain to the Jacobi solve (the same decision on every lane)
-        if (!(fabsf(corr) <= 1e-10f * e0f)) {
-            double lj = 0.0, qj[4] = {1.0, 0.0, 0.0, 0.0};
-            if (lane == 0) jacobi_top_eigenpair(sK, s_jac, s_jac + 16, lj, qj);
-            l = __shfl_sync(0xffffffffu, lj, 0);
-#pragma unroll
-            for (int i = 0; i < 4; i++) q[i] = __shfl_sync(0xffffffffu, qj[i], 0);
-            return;
-        }
+        // the chain to the Jacobi solve (the same decision on every lane of the half)
+        simple = fabsf(corr) <= 1e-10f * e0f;
     }
+    __syncwarp();
     if (F32_VEC) {
         if (diag) k -= l;
-        if (lane < 16) sM[e] = (float)k;
+        sM[e] = (float)k;
         __syncwarp();
         eigvec_f32(sM, q);
-        return;
-    }
-    // cofactor (i, j) of M = K - l I on lane 4 i + j
-    double cof = 0.0;
-    if (lane < 16) {
-        const int i = lane >> 2, j = lane & 3;
+    } else {
+        // cofactor (i, j) of M = K - l I on lane 4 i + j
+        const int i = e >> 2, j = e & 3;
         double m[9];  // rows but i, columns but j
 #pragma unroll
         for (int t = 0; t < 9; t++) {
             const int r = t / 3 + (t / 3 >= i), c = t % 3 + (t % 3 >= j);
             m[t] = sK[4 * r + c] - (r == c ? l : 0.0);
         }
-        cof = det3(m[0], m[1], m[2], m[3], m[4], m[5], m[6], m[7], m[8]);
+        double cof = det3(m[0], m[1], m[2], m[3], m[4], m[5], m[6], m[7], m[8]);
         if ((i + j) & 1) cof = -cof;
-    }
-    // squared norm of the row of this lane (lanes 4 i .. 4 i + 3)
-    double nrm = cof * cof;
-    nrm += __shfl_xor_sync(0xffffffffu, nrm, 1);
-    nrm += __shfl_xor_sync(0xffffffffu, nrm, 2);
-    int best = 0;
-    double bn = __shfl_sync(0xffffffffu, nrm, 0);
-    for (int i = 1; i < 4; i++) {
-        const double v = __shfl_sync(0xffffffffu, nrm, 4 * i);
-        if (v > bn) {
-            bn = v;
-            best = i;
+        // squared norm of the row of this lane (lanes 4 i .. 4 i + 3)
+        double nrm = cof * cof;
+        nrm += __shfl_xor_sync(0xffffffffu, nrm, 1);
+        nrm += __shfl_xor_sync(0xffffffffu, nrm, 2);
+        int best = 0;
+        double bn = __shfl_sync(0xffffffffu, nrm, 0, 16);
+        for (int r = 1; r < 4; r++) {
+            const double v = __shfl_sync(0xffffffffu, nrm, 4 * r, 16);
+            if (v > bn) {
+                bn = v;
+                best = r;
+            }
+        }
+        const double inv = bn > 1e-300 ? 1.0 / sqrt(bn) : 0.0;
+#pragma unroll
+        for (int r = 0; r < 4; r++) q[r] = __shfl_sync(0xffffffffu, cof, 4 * best + r, 16) * inv;
+        if (!(bn > 1e-300)) {
+            q[0] = 1.0;
+            q[1] = q[2] = q[3] = 0.0;
         }
     }
-    const double inv = bn > 1e-300 ? 1.0 / sqrt(bn) : 0.0;
+    if (__any_sync(0xffffffffu, !simple)) {
+        double lj = 0.0, qj[4] = {1.0, 0.0, 0.0, 0.0};
+        if (!simple && e == 0) jacobi_top_eigenpair(sK, s_jac, s_jac + 16, lj, qj);
+        __syncwarp();
+        lj = __shfl_sync(0xffffffffu, lj, 0, 16);
 #pragma unroll
-    for (int i = 0; i < 4; i++) q[i] = __shfl_sync(0xffffffffu, cof, 4 * best + i) * inv;
-    if (!(bn > 1e-300)) {
-        q[0] = 1.0;
-        q[1] = q[2] = q[3] = 0.0;
+        for (int i = 0; i < 4; i++) qj[i] = __shfl_sync(0xffffffffu, qj[i], 0, 16);
+        if (!simple) {
+            l = lj;
+#pragma unroll
+            for (int i = 0; i < 4; i++) q[i] = qj[i];
+        }
     }
 }
 
@@ -335,15 +346,12 @@ __device__ __forceinline__ void store_ut(T *ut, T q0, T q1, T q2, T q3) {
 }
 
 template <typename T>
-__device__ __forceinline__ int checked_atoms(const RmsdArgs<T> &a, int b) {
+__device__ __forceinline__ int checked_atoms(const RmsdArgs<T> &a, int b, bool reports) {
     const int n = a.num_atoms[b];
     if (n >= 0 && n <= a.atoms_stride) return n;
-    if (threadIdx.x == 0 && a.hdr) atomicCAS(&a.hdr->status, 0u, (unsigned)TPL_ERR_ATOMS);
+    if (reports && a.hdr) atomicCAS(&a.hdr->status, 0u, (unsigned)TPL_ERR_ATOMS);
     return max(0, min(n, a.atoms_stride));
 }
-
-// One value of x0 / x1 / x2 by index, in registers.
-__device__ __forceinline__ float pick3(int i, float x0, float x1, float x2) { return i == 0 ? x0 : (i == 1 ? x1 : x2); }
 
 constexpr int kRmsdSums = 16;  // R (row-major), R2, sum x, sum y
 
@@ -354,16 +362,34 @@ constexpr int kRmsdSums = 16;  // R (row-major), R2, sum x, sum y
 // sums keep the size, and the rounding, of centred ones, and the second read of every
 // coordinate goes.  Atoms are read as float4 groups (tpl_rows.cuh) where both rows
 // have the same alignment.
-template <int NT>
-__global__ void __launch_bounds__(NT) rmsd_fwd_f32_kernel(RmsdArgs<float> a) {
-    constexpr int NW = NT / 32;
-    __shared__ __align__(8) float s_red[4 * NW][kRmsdSums];
-    __shared__ double s_R[9], s_K[16], s_jac[32];
-    __shared__ float s_M[16];
-    const int b = blockIdx.x, tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
-    const int n = checked_atoms(a, b);
+//
+// NC = 1 or 2 chains per CTA, NT threads each; the first warp then solves for both, one per
+// half, as an FP64 instruction costs the same for 16 lanes or 32.
+template <int NT, int NC>
+__global__ void __launch_bounds__(NT * NC) rmsd_fwd_f32_kernel(RmsdArgs<float> a, int nb) {
+    constexpr int LR = NT > 64 ? 8 : 4;  // lanes summed in FP32
+    constexpr int ROWS = NT / LR;
+    __shared__ __align__(16) float s_red[NC][ROWS][kRmsdSums];
+    __shared__ double s_R[2][9], s_K[2][16], s_jac[2][32];
+    __shared__ float s_M[2][16], s_c[NC][6];
+    __shared__ int s_n[NC];
+    const int ch = NC == 1 ? 0 : threadIdx.x / NT, tid = threadIdx.x - ch * NT, lane = tid & 31, w = tid >> 5;
+    const int b = min(NC * (int)blockIdx.x + ch, nb - 1);
+    const bool own = NC * (int)blockIdx.x + ch < nb;  // false: the last CTA's half without a chain
+    const int n = own ? checked_atoms(a, b, tid == 0) : 0;
     const float *x = a.src + (size_t)b * 3 * a.atoms_stride;
     const float *y = a.dst + (size_t)b * 3 * a.atoms_stride;
+    // The thread's first group is asked for before the centres are known: a small batch
+    // then waits for memory once less.  (Not in the form for large batches, where it takes
+    // 16 more registers.)
+    constexpr bool kAhead = NC == 1;
+    const int head = row_head(x), ng = head == row_head(y) ? max(0, n - head) >> 2 : 0;
+    const float *xg = x + 3 * head, *yg = y + 3 * head;
+    float xv[12], yv[12];
+    if (kAhead && tid < ng) {
+        load_group(xg + 12 * tid, xv);
+        load_group(yg + 12 * tid, yv);
+    }
     float c[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};  // provisional centres, the same on every thread
     if (a.center && n > 0) {
         const size_t i = (size_t)n * (2 * (lane & 15) + 1) / 32;
@@ -393,39 +419,38 @@ __global__ void __launch_bounds__(NT) rmsd_fwd_f32_kernel(RmsdArgs<float> a) {
         }
         s[9] += xi[0] * xi[0] + xi[1] * xi[1] + xi[2] * xi[2] + yi[0] * yi[0] + yi[1] * yi[1] + yi[2] * yi[2];
     };
-    int i0 = 0;  // first atom of the scalar loop; the atoms before the groups come last
-    const int head = row_head(x);
-    int nhead = 0;
-    if (head == row_head(y) && n > head) {
-        const int ng = (n - head) >> 2;
-        const float *xg = x + 3 * head, *yg = y + 3 * head;
+    auto add_group = [&]() {
+        float s[kRmsdSums];  // the group's own sums first: fewer roundings at the size of the running sums
+#pragma unroll
+        for (int k = 0; k < kRmsdSums; k++) s[k] = 0.f;
+#pragma unroll
+        for (int q = 0; q < 4; q++) add(s, xv + 3 * q, yv + 3 * q);
+#pragma unroll
+        for (int k = 0; k < kRmsdSums; k++) v[k] += s[k];
+    };
+    if (kAhead && tid < ng) add_group();
 #pragma unroll 2
-        for (int g = tid; g < ng; g += NT) {
-            float xv[12], yv[12];
-            load_group(xg + 12 * g, xv);
-            load_group(yg + 12 * g, yv);
-            float s[kRmsdSums];  // the group's own sums first: fewer roundings at the size of the running sums
-#pragma unroll
-            for (int k = 0; k < kRmsdSums; k++) s[k] = 0.f;
-#pragma unroll
-            for (int q = 0; q < 4; q++) add(s, xv + 3 * q, yv + 3 * q);
-#pragma unroll
-            for (int k = 0; k < kRmsdSums; k++) v[k] += s[k];
-        }
-        i0 = head + 4 * ng;
-        nhead = head;
+    for (int g = kAhead ? tid + NT : tid; g < ng; g += NT) {
+        load_group(xg + 12 * g, xv);
+        load_group(yg + 12 * g, yv);
+        add_group();
     }
+    // the atoms before the groups come after the last group's
+    const int i0 = ng > 0 ? head + 4 * ng : 0, nhead = ng > 0 ? head : 0;
     for (int i = i0 + tid - nhead; i < n; i += NT) {
         const int at = i < i0 ? i - i0 + nhead : i;  // the nhead atoms before the groups, then the rest
         add(v, x + 3 * at, y + 3 * at);
     }
-    // Sums over eight lanes: a lane hands half of its values to its partner and keeps the
-    // sums of the other half, so that 16 values take 14 shuffles.  The four sums of a
-    // warp and the warps are then added in FP64: FP32 additions of ever larger sums up to
-    // the whole warp were most of the rounding error (rmsd against FP64, 4096 chains of
-    // 400..2303 atoms: 1.4e-6 with all five levels in FP32).
+    // Sums over LR lanes: a lane hands half of its values to its partner and keeps the sums
+    // of the other half, so that 16 values take 14 shuffles (12 for four lanes).  The sums of
+    // a warp's groups and the warps are then added in more than FP32: FP32 additions of ever
+    // larger sums up to the whole warp were most of the rounding error (rmsd against FP64,
+    // 4096 chains of 400..2303 atoms: 1.4e-6 with all five levels in FP32; the fewer threads
+    // a chain has, the larger its threads' sums, hence four lanes for 64).
+    constexpr int LEFT = kRmsdSums / LR;  // values a lane is left with
+    static_assert((LR == 8 || LR == 4) && LEFT * LR == kRmsdSums && ROWS * LR == NT, "rows of s_red");
 #pragma unroll
-    for (int off = 16, h = kRmsdSums / 2; h > 1; off >>= 1, h >>= 1) {
+    for (int off = 16, h = kRmsdSums / 2; h >= LEFT; off >>= 1, h >>= 1) {
         const bool up = (lane & off) != 0;
 #pragma unroll
         for (int k = 0; k < h; k++) {
@@ -433,59 +458,76 @@ __global__ void __launch_bounds__(NT) rmsd_fwd_f32_kernel(RmsdArgs<float> a) {
             v[k] = keep + __shfl_xor_sync(0xffffffffu, give, off);
         }
     }
-    // values 2 (lane >> 2) and the next, summed over the lanes with this lane's low bits
-    *reinterpret_cast<float2 *>(&s_red[4 * w + (lane & 3)][2 * (lane >> 2)]) = make_float2(v[0], v[1]);
-    __syncthreads();
-    if (w != 0) return;
-
-    // warp 0, in FP64: value lane & 15 over the warps, then moved to the true centroids
-    const int k = lane & 15;
-    double d = 0.0;
+    // values LEFT (lane / LR) and the next ones, summed over the lanes with this lane's low bits
+    if constexpr (LEFT == 2)
+        *reinterpret_cast<float2 *>(&s_red[ch][4 * w + (lane & 3)][2 * (lane >> 2)]) = make_float2(v[0], v[1]);
+    else
+        *reinterpret_cast<float4 *>(&s_red[ch][8 * w + (lane & 7)][4 * (lane >> 3)]) =
+            make_float4(v[0], v[1], v[2], v[3]);
+    if (tid == 0) {
+        s_n[ch] = n;
 #pragma unroll
-    for (int i = 0; i < 2 * NW; i++) d += (double)s_red[2 * NW * (lane >> 4) + i][k];
-    d += __shfl_xor_sync(0xffffffffu, d, 16);
+        for (int k = 0; k < 6; k++) s_c[ch][k] = c[k];
+    }
+    __syncthreads();
+    if (threadIdx.x >= 32) return;
+
+    // The first warp: value k of chain h on lane 16 h + k (one chain: half the rows on each
+    // half).  The rows are added exactly but for the last bits of a two-float sum (Knuth's
+    // two-sum; 47 bits), which costs three FP64 instructions instead of two a row, then moved
+    // to the true centroids in FP64.
+    const int half = lane >> 4, h = NC == 1 ? 0 : half, k = lane & 15;
+    const int bh = NC * (int)blockIdx.x + h, nh = s_n[h];
+    const bool writes = NC == 1 ? half == 0 : bh < nb;
+    constexpr int R = NC == 1 ? ROWS / 2 : ROWS;
+    float hi = 0.f, lo = 0.f;
+#pragma unroll
+    for (int i = 0; i < R; i++) {
+        const float u = s_red[h][(NC == 1 ? R * half : 0) + i][k], t = hi + u, z = t - hi;
+        lo += (hi - (t - z)) + (u - z);
+        hi = t;
+    }
+    double d = (double)hi + (fabsf(hi) <= 3.402823466e38f ? (double)lo : 0.0);  // an infinite sum stays one
+    if (NC == 1) d += __shfl_xor_sync(0xffffffffu, d, 16);
     if (a.center) {
         double rn = 0.0;  // 1 / n: an FP32 reciprocal and one Newton step
-        if (n > 0) {
-            rn = (double)(1.f / (float)n);
-            rn = fma(rn, fma(-(double)n, rn, 1.0), rn);
+        if (nh > 0) {
+            rn = (double)(1.f / (float)nh);
+            rn = fma(rn, fma(-(double)nh, rn, 1.0), rn);
         }
         const double m = d * rn;  // lanes 10 .. 15: the centroids from the provisional centres
-        if (lane >= 10 && lane < 16 && a.centroids) {
-            const float c_k = k < 13 ? pick3(k - 10, c[0], c[1], c[2]) : pick3(k - 13, c[3], c[4], c[5]);
-            a.centroids[6 * b + k - 10] = (double)c_k + m;
-        }
-        const double sx = __shfl_sync(0xffffffffu, d, 10 + (k < 9 ? k / 3 : 0));
-        const double my = __shfl_sync(0xffffffffu, m, 13 + (k < 9 ? k % 3 : 0));
+        if (k >= 10 && writes && a.centroids) a.centroids[6 * bh + k - 10] = (double)s_c[h][k - 10] + m;
+        const double sx = __shfl_sync(0xffffffffu, d, 10 + (k < 9 ? k / 3 : 0), 16);
+        const double my = __shfl_sync(0xffffffffu, m, 13 + (k < 9 ? k % 3 : 0), 16);
         double sq = k >= 10 ? d * m : 0.0;
 #pragma unroll
         for (int off = 8; off > 0; off >>= 1) sq += __shfl_xor_sync(0xffffffffu, sq, off);
         d -= k < 9 ? sx * my : sq;
-    } else if (lane < 6 && a.centroids) {
-        a.centroids[6 * b + lane] = 0.0;
+    } else if (k < 6 && writes && a.centroids) {
+        a.centroids[6 * bh + k] = 0.0;
     }
-    const double r2 = __shfl_sync(0xffffffffu, d, 9);
+    const double r2 = __shfl_sync(0xffffffffu, d, 9, 16);
     double scale, inv;
     unit_scale(0.5 * r2, scale, inv);
-    if (lane < 9) s_R[lane] = d * scale;
+    if (k < 9) s_R[half][k] = d * scale;
     __syncwarp();
     double l, q[4];
-    key_eigen_warp<true>(s_R, 0.5 * r2 * scale, s_K, s_M, s_jac, l, q);
-    if (lane != 0) return;
-    store_ut(a.ut + (size_t)9 * b, (float)q[0], (float)q[1], (float)q[2], (float)q[3]);
-    const float msd = n > 0 ? (float)(r2 - 2.0 * fabs(l * inv) + 1e-10) * (1.f / (float)n) : 0.f;
-    a.rmsd[b] = sqrtf(msd > 0.f ? msd : 0.f);
+    key_eigen_halves<true>(s_R[half], 0.5 * r2 * scale, s_K[half], s_M[half], s_jac[half], l, q);
+    if (k != 0 || !writes) return;
+    store_ut(a.ut + (size_t)9 * bh, (float)q[0], (float)q[1], (float)q[2], (float)q[3]);
+    const float msd = nh > 0 ? (float)(r2 - 2.0 * fabs(l * inv) + 1e-10) * (1.f / (float)nh) : 0.f;
+    a.rmsd[bh] = sqrtf(msd > 0.f ? msd : 0.f);
 }
 
 // float64 forward: two passes (centroids, then the correlation), everything in FP64.
 __global__ void __launch_bounds__(kRmsdThreads) rmsd_fwd_f64_kernel(RmsdArgs<double> a) {
     __shared__ double s_red[kRmsdWarps * 10];
     __shared__ double s_out[10];
-    __shared__ double s_R[9], s_K[16];
-    __shared__ double s_jac[32];  // scratch of the Jacobi fallback
+    __shared__ double s_R[9], s_K[2][16];
+    __shared__ double s_jac[2][32];  // scratch of the Jacobi fallback
     __shared__ double s_c[6];     // centroids (src, dst)
     const int b = blockIdx.x, tid = threadIdx.x;
-    const int n = checked_atoms(a, b);
+    const int n = checked_atoms(a, b, tid == 0);
     const double *x = a.src + (size_t)b * 3 * a.atoms_stride;
     const double *y = a.dst + (size_t)b * 3 * a.atoms_stride;
     if (a.center) {
@@ -524,7 +566,8 @@ __global__ void __launch_bounds__(kRmsdThreads) rmsd_fwd_f64_kernel(RmsdArgs<dou
     if (tid < 9) s_R[tid] = s_out[tid] * scale;
     __syncwarp();
     double l, q[4];
-    key_eigen_warp<false>(s_R, 0.5 * r2 * scale, s_K, nullptr, s_jac, l, q);
+    const int half = tid >> 4;  // both halves solve the same chain
+    key_eigen_halves<false>(s_R, 0.5 * r2 * scale, s_K[half], nullptr, s_jac[half], l, q);
     if (tid != 0) return;
     store_ut(a.ut + (size_t)9 * b, q[0], q[1], q[2], q[3]);
     const double msd = n > 0 ? (r2 - 2.0 * fabs(l * inv) + 1e-10) / (double)n : 0.0;
@@ -598,12 +641,15 @@ static int rmsd_fwd_launch(const T *src, const T *dst, const int *num_atoms, int
         // Threads per chain: with few chains per SM the longest chain's loads bound the
         // launch (256 chains of 50..500 residues, training step as a graph: 65.7 / 66.6 /
         // 68.9 us at 512 / 256 / 128 threads); with many, a CTA holds its registers while
-        // its first warp solves, so small CTAs keep more chains' loads in flight (4096
-        // chains of 400..2303 atoms: 116 / 60 / 42 us; 64 threads: 46 us).
+        // its first warp solves, so small CTAs keep more chains' loads in flight, and two
+        // chains share a solve (forward of 4096 chains of up to 2303 atoms, threads x chains:
+        // 128 x 1 42.9 us, 128 x 2 45.2, 64 x 1 40.3, 64 x 2 32.9, 32 x 2 31.7; of 1200
+        // chains 20.0 / 12.9 / 14.3 / 12.8 / 15.4; of 620 chains 11.8 with 64 x 2 and 11.3
+        // with 256 x 1).
         const int sms = device_sm_count();
-        if (B <= 2 * sms) rmsd_fwd_f32_kernel<512><<<B, 512, 0, st>>>(a);
-        else if (B <= 4 * sms) rmsd_fwd_f32_kernel<256><<<B, 256, 0, st>>>(a);
-        else rmsd_fwd_f32_kernel<128><<<B, 128, 0, st>>>(a);
+        if (B <= 2 * sms) rmsd_fwd_f32_kernel<512, 1><<<B, 512, 0, st>>>(a, B);
+        else if (B <= 4 * sms) rmsd_fwd_f32_kernel<256, 1><<<B, 256, 0, st>>>(a, B);
+        else rmsd_fwd_f32_kernel<64, 2><<<B / 2 + B % 2, 128, 0, st>>>(a, B);
     } else {
         rmsd_fwd_f64_kernel<<<B, kRmsdThreads, 0, st>>>(a);
     }
