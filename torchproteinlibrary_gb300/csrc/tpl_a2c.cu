@@ -466,6 +466,53 @@ __global__ void __launch_bounds__(NT) a2c_fwd_kernel(A2cArgs<T> a, int renorm) {
     (void)lane;
 }
 
+// ---------------------------------------------------------- handoffs of a chain
+// The frame a warp hands to the next chunk's, F o T for the frame F it has received and its
+// chunk's transform T, one entry per lane (lanes 0..11 in pair_store_vec's order).  The
+// handoffs of a chain run one after another, so what lies between a warp's wait and its
+// signal is the latency of a small batch: an entry is three fused multiply-adds on values
+// one shared-memory read away, and T is renormalised before the wait instead of F o T after
+// it.  Whole frames composed, renormalised and stored by one lane: 530 cycles a handoff
+// against 490 (8 chains of 256 residues), 61.0 against 60.1 us a training step of 256 chains,
+// 291.8 against 289.5 us for 4096 x 500.  (The Angles2Backbone forward, whose chunks are
+// shorter work, loses 1.5 % by it.  Barrier numbers from a register, instead of the switch,
+// take a handoff to 410 cycles but reserve all 16 barriers of a CTA: 10 % slower at 4096
+// chains.)
+// Lane e holds row i, column j (3: the translation): e = 2 j + i for i < 2, 8 + j for i = 2.
+__device__ __forceinline__ float3 carry_column(float *scratch, const PairFrame &T, int lane) {
+    if (lane == 31) pair_store_vec(scratch, T);
+    __syncwarp();
+    const int j = lane < 8 ? lane >> 1 : (lane & 3);
+    return make_float3(scratch[2 * j], scratch[2 * j + 1], scratch[8 + j]);
+}
+// F from a handoff slot.
+__device__ __forceinline__ float carry_product(const float *slot, float3 t, int lane) {
+    const float *f = slot + (lane < 8 ? (lane & 1) : 8);
+    const int step = lane < 8 ? 2 : 1;
+    const float v = fmaf(f[0], t.x, fmaf(f[step], t.y, f[2 * step] * t.z)), p = f[3 * step];
+    return ((0x8c0 >> lane) & 1) ? v + p : v;  // lanes 6, 7 and 11: the translation
+}
+// F the identity.
+__device__ __forceinline__ float carry_first(float3 t, int lane) {
+    return lane >= 8 ? t.z : ((lane & 1) ? t.y : t.x);
+}
+
+// What a backward hands on (G, S and an origin) as three 16-byte accesses.
+__device__ __forceinline__ void store_sums(float *slot, float g0, float g1, float g2, float s0, float s1, float s2,
+                                           const float *o) {
+    float4 *d = reinterpret_cast<float4 *>(slot);
+    d[0] = make_float4(g0, g1, g2, s0);
+    d[1] = make_float4(s1, s2, o[0], o[1]);
+    d[2] = make_float4(o[2], 0.f, 0.f, 0.f);
+}
+__device__ __forceinline__ void load_sums(const float *slot, float (&v)[9]) {
+    const float4 *s = reinterpret_cast<const float4 *>(slot);
+    const float4 a = s[0], b = s[1];
+    v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w;
+    v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
+    v[8] = slot[8];
+}
+
 // ------------------------------------------ forward, four or eight warps per chain
 // Chunks of 32 residues, one per lane, dealt round the NW = 4 or 8 warps of a CTA.  A
 // CTA takes chains b, b + grid, ... (persistent: the topology loads once) and their
@@ -509,6 +556,7 @@ __global__ void __launch_bounds__(32 * NW, NW == 4 ? 6 : 3) a2c_fwd_ring_kernel(
     extern __shared__ __align__(16) unsigned char smem_raw[];
     A2cRingSmem<NW, NAMES> &sm = *reinterpret_cast<A2cRingSmem<NW, NAMES> *>(smem_raw);
     __shared__ __align__(16) float s_ring[NW][16];  // chain frame (12, pair_store_vec) and first atom index
+    __shared__ __align__(16) float s_total[NW][12];  // carry_column
 
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const RingTopology &tp = sm.topo;
@@ -609,6 +657,13 @@ __global__ void __launch_bounds__(32 * NW, NW == 4 ? 6 : 3) a2c_fwd_ring_kernel(
         }
         const int cnt = __shfl_sync(0xffffffffu, ci, 31), aoff = ci - na;
 
+        const bool hands = ck + 1 < cnch;  // the chain goes on after this chunk
+        float3 tc = make_float3(0.f, 0.f, 0.f);
+        if (hands) {
+            PairFrame T = t;  // lane 31: the chunk's transform
+            if (renorm) renormalize_pair(T);
+            tc = carry_column(s_total[w], T, lane);
+        }
         PairFrame F = pair_identity();  // chain frame at the chunk start
         int abase = 0;                  // first atom of the chunk
         if (cb != (int)blockIdx.x || ck > 0) ring_wait<NW>(w);
@@ -616,22 +671,17 @@ __global__ void __launch_bounds__(32 * NW, NW == 4 ? 6 : 3) a2c_fwd_ring_kernel(
             F = pair_load_vec(s_ring[w]);
             abase = __float_as_int(s_ring[w][12]);
         }
+        if (hands) {
+            float *next = s_ring[(w + 1) % NW];
+            const float v = ck > 0 ? carry_product(s_ring[w], tc, lane) : carry_first(tc, lane);
+            if (lane < 13) next[lane] = lane < 12 ? v : __int_as_float(abase + cnt);
+        }
+        if (hands || cb + (int)gridDim.x < nb) ring_signal<NW>((w + 1) % NW);
         const float2 org = F.p;  // the chunk's origin; positions are relative to it
         const float org2 = F.p2;
         F.p = make_float2(0.f, 0.f);
         F.p2 = 0.f;
         const PairFrame Q = compose_pair(F, t);
-        if (ck + 1 < cnch) {  // lane 31: the chain frame after the chunk
-            PairFrame Fn = Q;
-            if (renorm) renormalize_pair(Fn);
-            Fn.p = __fadd2_rn(Fn.p, org);
-            Fn.p2 += org2;
-            if (lane == 31) {
-                pair_store_vec(s_ring[(w + 1) % NW], Fn);
-                s_ring[(w + 1) % NW][12] = __int_as_float(abase + cnt);
-            }
-        }
-        if (ck + 1 < cnch || cb + (int)gridDim.x < nb) ring_signal<NW>((w + 1) % NW);
 
         const PairFrame P = frame_before(Q, F, lane);  // at this lane's N
         float *out = a.coords + (size_t)cb * 3 * a.maxA;
@@ -1042,7 +1092,7 @@ __global__ void __launch_bounds__(32 * NW) a2c_bwd_coords_ring_kernel(A2cArgs<fl
     constexpr int NT = 32 * NW;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     A2cBwdRingSmem<NW> &sm = *reinterpret_cast<A2cBwdRingSmem<NW> *>(smem_raw);
-    __shared__ __align__(16) float s_ring[NW][12];
+    __shared__ __align__(16) float s_ring[NW][12];  // G, S, the chunk's first N
     __shared__ __align__(8) uint64_t s_bar[NW];
 
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -1204,28 +1254,23 @@ __global__ void __launch_bounds__(32 * NW) a2c_bwd_coords_ring_kernel(A2cArgs<fl
         float Gc[3] = {0.f, 0.f, 0.f}, Sc[3] = {0.f, 0.f, 0.f};
         if (!first) ring_wait<NW>(w);
         if (!top) {
-            const float *cin = s_ring[w];
+            float c9[9];
+            load_sums(s_ring[w], c9);
             float d[3], dx[3];
 #pragma unroll
             for (int c = 0; c < 3; c++) {
-                Gc[c] = cin[c];
-                Sc[c] = cin[3 + c];
-                d[c] = cin[6 + c] - o[c];
+                Gc[c] = c9[c];
+                Sc[c] = c9[3 + c];
+                d[c] = c9[6 + c] - o[c];
                 if (lane == 31) xn[c] = d[c];  // the next chunk's first N
             }
             cross3(d, Gc, dx);
 #pragma unroll
             for (int c = 0; c < 3; c++) Sc[c] += dx[c];
         }
-        if (k > 0 && lane == 0) {
-            float *cout = s_ring[(w + 1) % NW];
-#pragma unroll
-            for (int c = 0; c < 3; c++) {
-                cout[c] = Gc[c] + ctot[c];
-                cout[3 + c] = Sc[c] + ctot[3 + c];
-                cout[6 + c] = o[c];
-            }
-        }
+        if (k > 0 && lane == 0)
+            store_sums(s_ring[(w + 1) % NW], Gc[0] + ctot[0], Gc[1] + ctot[1], Gc[2] + ctot[2], Sc[0] + ctot[3],
+                       Sc[1] + ctot[4], Sc[2] + ctot[5], o);
         if (more) ring_signal<NW>((w + 1) % NW);
         float *gout = a.grad_angles + (size_t)cb * 8 * a.L;
         if (live && !failed) {

@@ -49,21 +49,26 @@ __device__ __forceinline__ int ring_chain_length(const A2cArgs<T> &a, int b, con
     int len = a.seq_stride;
     bool bad = false;
     for (int j0 = 0;;) {
+        // votes and lookups of all pieces side by side: none waits for the one before
+        uint32_t info[U];
+#pragma unroll
+        for (int u = U - 1; u >= 0; u--) {
+            const unsigned nul = __ballot_sync(0xffffffffu, c[u] == 0);
+            info[u] = table[c[u]];
+            if (nul != 0u) len = min(a.seq_stride, j0 + 32 * u + __ffs(nul) - 1);
+        }
 #pragma unroll
         for (int u = 0; u < U; u++) {
             const int j1 = j0 + 32 * u;
-            if (j1 >= len) break;
-            const unsigned nul = __ballot_sync(0xffffffffu, c[u] == 0);
-            if (nul != 0u) len = min(len, j1 + __ffs(nul) - 1);
-            const unsigned info = table[c[u]];
             const bool in = j1 + lane < len;
-            bad |= __any_sync(0xffffffffu, in && info == 0u);
-            if (j1 < len) atoms(j1 >> 5, in ? (int)((info >> 8) & 0xffu) : 0);
+            bad |= in && info[u] == 0u;
+            if (j1 < len) atoms(j1 >> 5, in ? (int)((info[u] >> 8) & 0xffu) : 0);
         }
         j0 += 32 * U;
         if (j0 >= len) break;
         load_letters(a, b, j0, lane, c);
     }
+    bad = __any_sync(0xffffffffu, bad);
     if (bad || len > a.L) {
         if (lane == 0) a2c_error(a.hdr, bad ? TPL_ERR_SEQUENCE : TPL_ERR_LENGTH);
         return 0;
