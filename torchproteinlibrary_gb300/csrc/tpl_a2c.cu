@@ -591,7 +591,7 @@ __global__ void __launch_bounds__(32 * NW, NW == 4 ? 6 : 3) a2c_fwd_ring_kernel(
     // padded to L), together with the letters and the topology: a small batch waits for
     // memory once (32 residues 6.7 -> 6.2 us, 256 x 50..500 15.9 -> 15.4 us with names).
     {
-        unsigned char c[kFirstLetters];
+        unsigned char c[kFirstLetters][4];
         if (b < nb) {
             load_letters(a, b, 0, lane, c);
             fetch(a.L);
@@ -1096,6 +1096,9 @@ __global__ void __launch_bounds__(32 * NW) a2c_bwd_coords_ring_kernel(A2cArgs<fl
     __shared__ __align__(8) uint64_t s_bar[NW];
 
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int b_first = nb - 1 - (int)blockIdx.x;
+    unsigned char c_first[kFirstLetters][4];  // of the first chain, asked for together with the topology
+    if (b_first >= 0) load_letters(a, b_first, 0, lane, c_first);
     {
         const uint32_t *src = reinterpret_cast<const uint32_t *>(&g_ring_bwd_topo);
         for (int i = threadIdx.x; i < (int)(sizeof(RingBwdTopology) / 4); i += NT)
@@ -1109,16 +1112,25 @@ __global__ void __launch_bounds__(32 * NW) a2c_bwd_coords_ring_kernel(A2cArgs<fl
 
     // the warp's next chunk: the i-th of chain b counted from its last (length len, nch
     // chunks; an empty or refused chain has one, which writes its zeros)
-    const int b_first = nb - 1 - (int)blockIdx.x;
     int b = b_first, i = w, len = 0, nch = 0;
     unsigned char letter = 0;
-    auto enter = [&]() {
+    auto enter = [&](auto &letters) {
         int run = 0;
         __syncwarp();  // every lane has read the bases of the chain before
-        len = ring_chain_length(a, b, sm.topo.letter, lane, [&](int c, int n) {
-            if (lane == 0 && c <= max_chunks) base[c] = run;
-            run += __reduce_add_sync(0xffffffffu, n);
+        len = ring_chain_length(a, b, sm.topo.letter, lane, letters, [&](int c, int n) {
+#pragma unroll
+            for (int off = 1; off < 8; off <<= 1) n += __shfl_xor_sync(0xffffffffu, n, off);
+            int inc = n;  // atoms of the chunks up to this lane's
+#pragma unroll
+            for (int off = 8; off < 32; off <<= 1) {
+                const int v = __shfl_up_sync(0xffffffffu, inc, off);
+                if (lane >= off) inc += v;
+            }
+            c += lane >> 3;
+            if ((lane & 7) == 0 && c <= max_chunks) base[c] = run + inc - n;
+            run += __shfl_sync(0xffffffffu, inc, 31);
         });
+        __syncwarp();  // what follows writes some of the same entries
         if (len > 0 && run > a.maxA) {  // a chain whose atoms overflow the rows gets zeros
             if (lane == 0) a2c_error(a.hdr, TPL_ERR_ATOMS);
             len = 0;
@@ -1135,7 +1147,9 @@ __global__ void __launch_bounds__(32 * NW) a2c_bwd_coords_ring_kernel(A2cArgs<fl
             i -= nch;
             b -= (int)gridDim.x;
             if (b < 0) break;
-            enter();
+            unsigned char c[1][4];
+            load_letters(a, b, 0, lane, c);
+            enter(c);
         }
     };
     bool failed = false;  // a bulk copy timed out: the remaining chunks only pass the carry on
@@ -1149,7 +1163,7 @@ __global__ void __launch_bounds__(32 * NW) a2c_bwd_coords_ring_kernel(A2cArgs<fl
                     lane);
     };
     if (b >= 0) {
-        enter();
+        enter(c_first);
         settle();
         fetch();
     }

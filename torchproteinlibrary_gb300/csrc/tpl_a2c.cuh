@@ -25,46 +25,56 @@ __device__ __forceinline__ void a2c_error(WsHeader *h, int code) {
     if (h) atomicCAS(&h->status, 0u, (unsigned)code);
 }
 
-// U pieces of 32 letters of chain b's row from letter j0 on, all loads in flight at once;
-// 0 past the row.
+// A lane's letters of U blocks of 128 of chain b's row, from letter j0 on: four of each, all
+// loads in flight at once; 0 past the row.
 template <int U, typename T>
-__device__ __forceinline__ void load_letters(const A2cArgs<T> &a, int b, int j0, int lane, unsigned char (&c)[U]) {
+__device__ __forceinline__ void load_letters(const A2cArgs<T> &a, int b, int j0, int lane, unsigned char (&c)[U][4]) {
     const unsigned char *row = a.seq + (size_t)b * a.seq_stride;
 #pragma unroll
-    for (int u = 0; u < U; u++) {
-        const int j = j0 + 32 * u + lane;
-        c[u] = j < a.seq_stride ? row[j] : (unsigned char)0;
-    }
+    for (int v = 0; v < U; v++)
+#pragma unroll
+        for (int u = 0; u < 4; u++) {
+            const int j = j0 + 128 * v + 4 * lane + u;
+            c[v][u] = j < a.seq_stride ? row[j] : (unsigned char)0;
+        }
 }
 
 // Length of chain b for the kernels whose warps find it each for itself: the index of
 // the row's first NUL (at most the row stride), or 0, with the error recorded, when a
-// letter before it is no residue or the chain is longer than L.  atoms(chunk, n) is
-// called by the whole warp for every chunk of 32 letters in order, with the atom count of
-// this lane's residue.  table: letter -> word with the atom count in bits 8..15, 0 for
-// what is no residue.  c: the row's first U pieces (load_letters).
+// letter before it is no residue or the chain is longer than L.  A lane looks at four
+// letters of every 128, so that a chain costs few instructions; atoms(chunk, n) is called
+// by the whole warp for every 128 letters in order, with the number of the first of their
+// four chunks of 32 and the atoms of this lane's four residues (lanes 8 g .. 8 g + 7: chunk
+// + g).  table: letter -> word with the atom count in bits 8..15, 0 for what is no residue.
+// c: the row's first U blocks (load_letters).
 template <int U, typename T, typename Table, typename Atoms>
 __device__ __forceinline__ int ring_chain_length(const A2cArgs<T> &a, int b, const Table *table, int lane,
-                                                 unsigned char (&c)[U], Atoms atoms) {
+                                                 unsigned char (&c)[U][4], Atoms atoms) {
     int len = a.seq_stride;
     bool bad = false;
+#pragma unroll 1
     for (int j0 = 0;;) {
-        // votes and lookups of all pieces side by side: none waits for the one before
-        uint32_t info[U];
 #pragma unroll
-        for (int u = U - 1; u >= 0; u--) {
-            const unsigned nul = __ballot_sync(0xffffffffu, c[u] == 0);
-            info[u] = table[c[u]];
-            if (nul != 0u) len = min(a.seq_stride, j0 + 32 * u + __ffs(nul) - 1);
-        }
+        for (int v = 0; v < U; v++, j0 += 128) {
+            if (j0 >= len) break;
+            const int j = j0 + 4 * lane;
+            unsigned nul = 0;
 #pragma unroll
-        for (int u = 0; u < U; u++) {
-            const int j1 = j0 + 32 * u;
-            const bool in = j1 + lane < len;
-            bad |= in && info[u] == 0u;
-            if (j1 < len) atoms(j1 >> 5, in ? (int)((info[u] >> 8) & 0xffu) : 0);
+            for (int u = 0; u < 4; u++) nul |= c[v][u] == 0 ? 1u << u : 0u;
+            const unsigned lanes = __ballot_sync(0xffffffffu, nul != 0);
+            if (lanes != 0u) {
+                const int l = __ffs(lanes) - 1;
+                len = min(len, j0 + 4 * l + __ffs(__shfl_sync(0xffffffffu, nul, l)) - 1);
+            }
+            int n = 0;
+#pragma unroll
+            for (int u = 0; u < 4; u++) {
+                const unsigned info = j + u < len ? table[c[v][u]] : 0x100u;
+                bad |= info == 0u;
+                n += j + u < len ? (int)((info >> 8) & 0xffu) : 0;
+            }
+            atoms(j0 >> 5, n);
         }
-        j0 += 32 * U;
         if (j0 >= len) break;
         load_letters(a, b, j0, lane, c);
     }
@@ -78,13 +88,13 @@ __device__ __forceinline__ int ring_chain_length(const A2cArgs<T> &a, int b, con
 template <typename T, typename Table, typename Atoms>
 __device__ __forceinline__ int ring_chain_length(const A2cArgs<T> &a, int b, const Table *table, int lane,
                                                  Atoms atoms) {
-    unsigned char c[4];
+    unsigned char c[1][4];
     load_letters(a, b, 0, lane, c);
     return ring_chain_length(a, b, table, lane, c, atoms);
 }
-// Pieces a kernel asks for before it does anything else: its first chain's length then
+// Blocks a kernel asks for before it does anything else: its first chain's length then
 // waits for memory once, not once every 128 letters.
-constexpr int kFirstLetters = 16;
+constexpr int kFirstLetters = 4;
 
 // float64 launchers (tpl_f64.cu).
 int a2c_forward_f64(const A2cArgs<double> &a, int B, bool renorm, cudaStream_t st);
