@@ -814,3 +814,34 @@ def test_float64_clusters_and_passes(rm, B, L):
     c, gi = run_gpu(rm, ang, lengths, g, torch.float64)
     rc, rg = oracle_ref(ang, lengths, g, False)
     check(c, gi, rc, rg, lengths, L, COORD_TOL_F64, GRAD_TOL_F64)
+
+
+@pytest.mark.parametrize("per_sm,L", [(1, 64), (2, 513), (5, 300), (5, 700), (6, 513), (7, 129), (8, 128), (8, 129),
+                                      (8, 257), (9, 320), (9, 384), (9, 767), (9, 768)])
+def test_automatic_scheme_is_one_of_the_schemes(built, per_sm, L):
+    """The built-in choice on both sides of its lines in chains per SM and residues: with
+    every option left at 0 the results are bit for bit those of one explicit choice, and that
+    choice is the one the rule states."""
+    from torchproteinlibrary_gb300 import load_extension
+    rm = load_extension("_ReducedModel")
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    B = per_sm * sms - 3 if per_sm < 9 else 8 * sms
+    g = torch.Generator("cuda").manual_seed(L)
+    ang = (torch.rand(B, 3, L, device="cuda", generator=g) * 2 - 1) * 3.1
+    lens = torch.randint(1, L + 1, (B,), device="cuda", generator=g, dtype=torch.int32)
+    up = torch.randn(B, 9 * L, device="cuda", generator=g)
+    ws = torch.zeros(rm.workspace_bytes(B, L), dtype=torch.uint8, device="cuda")
+
+    def both(fwd, bwd):
+        coords, grad = torch.empty(B, 9 * L, device="cuda"), torch.empty(B, 3, L, device="cuda")
+        rm.Angles2BackboneGPU_forward(ang, coords, lens, ws, *fwd)
+        rm.Angles2BackboneGPU_backward_coords(grad, up, coords, lens, ws, *bwd)
+        return coords, grad
+
+    ring = L >= 384 or B < 8 * sms
+    eight = (L >= 768 or (L > 512 and B < 6 * sms)) if ring else 128 < L <= 256
+    bring = L >= 384 or B < 6 * sms
+    want = both((8 if eight else 4, 4 if ring else 32), (4, 2 if bring and B <= 2 * sms else 1, 4 if bring else 32))
+    got = both((0, 0), (0, 0, 0))
+    assert torch.equal(got[0], want[0])
+    assert torch.equal(got[1], want[1])

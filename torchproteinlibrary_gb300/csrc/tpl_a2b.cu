@@ -1109,14 +1109,21 @@ static int num_sms() { return device_sm_count(); }
 // GB300 (4-residue-per-lane and 8-residue-per-lane chunks, one warp or one CTA of
 // four warps per chain, warp tiles; batches of 32 to 16384 chains of 64 to 1000
 // residues):
-//   * max_len >= 384: one CTA of four warps per chain (the chunks of a chain run on
-//     four warps at once), 8 residues per lane from max_len 768 and 4 below;
-//   * shorter chains: one warp per chain with 4 residues per lane when the batch
-//     gives every SM two chains, else one CTA of four warps per chain;
+//   * max_len >= 384, or fewer than eight chains per SM: one CTA of four warps per chain
+//     (the chunks of a chain run on four warps at once).  Forward, four warps / one warp, us:
+//     1024 chains of 64 residues 4.0 / 4.5, of 256 5.9 / 6.2; 2048 of 64 6.7 / 6.5, of 256
+//     9.5 / 8.8, of 384 12.0 / 12.9.  Four residues per lane, as four chunks of 128 then take
+//     512 residues in one round of the warps; eight above 768 residues, and above 512 while
+//     the batch leaves SMs short of warps (four / eight residues: 512 chains of 700 8.0 / 7.1,
+//     2048 of 700 18.1 / 18.8, 304 of 1000 7.0 / 6.0, 4096 of 1000 49.8 / 45.8);
+//   * else one warp per chain, with eight residues per lane where a chunk of 256 holds the
+//     chain but one of 128 does not (4096 chains of 256: four / eight residues 14.3 / 13.4, of
+//     128 9.1 / 12.6, of 320 18.7 / 20.7);
 //   * fewer than two chains per SM and chains over 4096 residues: warp tiles, whose
 //     look-back spreads one chain over many warps.
 // An explicit residues_per_thread of 4 or 8 is kept; 1 or 2 selects warp tiles.
-// The forward and the backward of one shape make the same choice.
+// The forward and the recomputing backward of one shape agree on whether a chain is split
+// into tiles; the frames recorded for the backward serve any chunk size.
 static bool use_chain_scheme(const tpl_options &opt, int B, int L) {
     if (opt.threads_per_cta == 32 || opt.threads_per_cta == 4) return true;
     if (opt.threads_per_cta != 0) return false;
@@ -1125,12 +1132,17 @@ static bool use_chain_scheme(const tpl_options &opt, int B, int L) {
     return !(B < 2 * num_sms() && L > 4096);
 }
 
-static tpl_options chain_options(const tpl_options &opt, int B, int L) {
+static tpl_options chain_options(const tpl_options &opt, int B, int L, bool forward) {
     tpl_options o = opt;
     if (o.threads_per_cta == 0) {
-        const bool ring = L >= 384 || B < 2 * num_sms();
+        const bool ring = L >= 384 || B < 8 * num_sms();
         o.threads_per_cta = ring ? 4 : 32;
-        if (o.residues_per_thread == 0) o.residues_per_thread = (ring && L >= 768) ? 8 : 4;
+        if (o.residues_per_thread == 0) {
+            const bool eight = !forward ? L >= 768
+                               : ring   ? L >= 768 || (L > 512 && B < 6 * num_sms())
+                                        : L > 128 && L <= 256;
+            o.residues_per_thread = eight ? 8 : 4;
+        }
     }
     if (o.residues_per_thread == 0) o.residues_per_thread = 8;
     return o;
@@ -1204,7 +1216,7 @@ int a2b_forward_f32(const float *angles, const int32_t *lengths, float *coords, 
                     const tpl_options &opt, cudaStream_t st) {
     if (B == 0 || L == 0) return TPL_OK;
     if (use_chain_scheme(opt, B, L))
-        return a2b_forward_chain(angles, lengths, coords, ws, B, L, chain_options(opt, B, L), st);
+        return a2b_forward_chain(angles, lengths, coords, ws, B, L, chain_options(opt, B, L, true), st);
     A2bShape s = a2b_shape(opt, false);
     A2bArgs a = make_args(angles, lengths, ws, B, L, s.R * s.NT, opt);
     a.coords = coords;
@@ -1230,7 +1242,8 @@ int a2b_backward_f32(float *grad_angles, const float *grad_coords, const float *
                      void *ws, int B, int L, const tpl_options &opt, cudaStream_t st) {
     if (B == 0 || L == 0) return TPL_OK;
     if (use_chain_scheme(opt, B, L))
-        return a2b_backward_chain(grad_angles, grad_coords, angles, lengths, ws, B, L, chain_options(opt, B, L), st);
+        return a2b_backward_chain(grad_angles, grad_coords, angles, lengths, ws, B, L, chain_options(opt, B, L, false),
+                                  st);
     A2bShape s = a2b_shape(opt, true);
     A2bArgs a = make_args(angles, lengths, ws, B, L, s.R * s.NT, opt);
     a.grad_angles = grad_angles;

@@ -1376,10 +1376,15 @@ int a2b_backward_coords(float *grad_angles, const float *grad_coords, const floa
     a.grad_coords = grad_coords;
     a.vec = (L % 4 == 0) && aligned16(coords) && aligned16(grad_angles) && aligned16(grad_coords);  // float4 gradient rows
     const int C = opt.residues_per_thread > 0 ? opt.residues_per_thread : 4;
-    const int NB = opt.copy_buffers > 0 ? opt.copy_buffers : 1;
-    // automatic: four warps per chain from 384 residues (three or more 128-residue
-    // chunks), one warp per chain for shorter chains (measured on GB300)
-    const bool ring = opt.threads_per_cta == kRingWarps || (opt.threads_per_cta == 0 && L >= 384);
+    // automatic: four warps per chain from 384 residues (three or more 128-residue chunks) or
+    // below six chains per SM, else one warp per chain (four warps / one warp, us: 800 chains
+    // of 256 residues 4.7 / 5.2, 1024 6.2 / 5.3, 2048 of 384 10.2 / 9.4, of 512 11.4 / 11.9);
+    // two chunk buffers per warp where shared memory holds two CTAs with them on every SM
+    // and the batch has no more (304 chains of 700: one / two buffers 5.9 / 5.6; 512: 6.9 / 8.4)
+    const int sms = device_sm_count();
+    const bool ring =
+        opt.threads_per_cta == kRingWarps || (opt.threads_per_cta == 0 && (L >= 384 || B < 6 * sms));
+    const int NB = opt.copy_buffers > 0 ? opt.copy_buffers : (ring && C == 4 && B <= 2 * sms ? 2 : 1);
     auto launch = [&](auto aligned) {
         constexpr bool A = decltype(aligned)::value;
         constexpr int smem4 = kWarpsPerCta * 64 * 36 * (int)sizeof(float);
