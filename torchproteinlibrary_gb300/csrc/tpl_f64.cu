@@ -83,12 +83,71 @@ __device__ __forceinline__ void sincos_f64(double a, double *s, double *c) {
     *c = __hiloint2double(__double2hiint(cc) ^ (int)(((q + 1u) << 30) & 0x80000000u), __double2loint(cc));
 }
 
+// Inclusive prefix of the lane transforms.  At level off the lanes with that bit compose the
+// prefix of the block before them onto their own; the lanes without it have nothing to do,
+// so each works for the lane off above it: a composition's four columns (three of the
+// rotation, and the translation) are two each, 18 FP64 instructions a level for the warp
+// where a lane on its own would take 36.
+__device__ __forceinline__ FrameD scan_inclusive(FrameD t, int lane) {
+#pragma unroll
+    for (int off = 1; off < 32; off <<= 1) {
+        const bool owner = (lane & off) != 0;
+        const int src = (lane & ~(2 * off - 1)) | (off - 1);  // last lane of the block before
+        double a[9], ap[3], x[6];                             // the prefix; this lane's two columns of t
+#pragma unroll
+        for (int i = 0; i < 9; i++) a[i] = __shfl_sync(0xffffffffu, t.r[i], src);
+#pragma unroll
+        for (int i = 0; i < 3; i++) ap[i] = __shfl_sync(0xffffffffu, t.p[i], src);
+#pragma unroll
+        for (int i = 0; i < 3; i++) {
+            const double c2 = __shfl_xor_sync(0xffffffffu, t.r[3 * i + 2], off);
+            const double cp = __shfl_xor_sync(0xffffffffu, t.p[i], off);
+            x[i] = owner ? t.r[3 * i] : c2;
+            x[3 + i] = owner ? t.r[3 * i + 1] : cp;
+        }
+        double y[6];
+#pragma unroll
+        for (int i = 0; i < 3; i++) {
+            y[i] = fma(a[3 * i], x[0], fma(a[3 * i + 1], x[1], a[3 * i + 2] * x[2]));
+            y[3 + i] = fma(a[3 * i], x[3], fma(a[3 * i + 1], x[4], fma(a[3 * i + 2], x[5], owner ? 0.0 : ap[i])));
+        }
+#pragma unroll
+        for (int i = 0; i < 3; i++) {
+            const double c2 = __shfl_xor_sync(0xffffffffu, y[i], off);
+            const double cp = __shfl_xor_sync(0xffffffffu, y[3 + i], off);
+            if (owner) {
+                t.r[3 * i] = y[i];
+                t.r[3 * i + 1] = y[3 + i];
+                t.r[3 * i + 2] = c2;
+                t.p[i] = cp;
+            }
+        }
+    }
+    return t;
+}
+
 // Exclusive prefix of the lane transforms; lane 31's inclusive one is left in t.
 __device__ __forceinline__ FrameD scan_exclusive(FrameD &t, int lane) {
-    t = warp_scan_frames(t, lane);
+    t = scan_inclusive(t, lane);
     FrameD e = shfl_up_frame(t, 1);
     if (lane == 0) frame_identity(e);
     return e;
+}
+
+// apply_joint on the identity, without the products by its zeros and ones.
+__device__ __forceinline__ void first_joint(FrameD &f, double cb, double sb, double d, double ca, double sa) {
+    f.r[0] = cb;
+    f.r[1] = sb * sa;
+    f.r[2] = sb * ca;
+    f.r[3] = 0.0;
+    f.r[4] = ca;
+    f.r[5] = -sa;
+    f.r[6] = -sb;
+    f.r[7] = cb * sa;
+    f.r[8] = cb * ca;
+    f.p[0] = d * cb;
+    f.p[1] = 0.0;
+    f.p[2] = -(d * sb);
 }
 
 // What the chunks of a pass tell one another: the chunk's transform, its atoms, and its
@@ -269,7 +328,8 @@ __device__ __forceinline__ FrameD walk(const BackboneArgs &a, const double *ang,
             if (k == 2 && j == len - 1) break;
             double s, c;
             sincos_f64(ang[(size_t)k * a.L + j], &s, &c);
-            apply_joint(f, a.bc.cbd[k], a.bc.sbd[k], a.bc.dd[k], c, s);
+            if (r == 0 && k == 0) first_joint(f, a.bc.cbd[k], a.bc.sbd[k], a.bc.dd[k], c, s);
+            else apply_joint(f, a.bc.cbd[k], a.bc.sbd[k], a.bc.dd[k], c, s);
         }
     }
     return f;
@@ -301,8 +361,15 @@ __global__ void __launch_bounds__(32 * NW, 4) a2b_fwd_f64_kernel(BackboneArgs a)
                 for (int r = 0; r < R; r++)
                     if (j0 + r < len)
 #pragma unroll
-                        for (int k = 0; k < 3; k++) frame_point(P, pos[r][3 * k], pos[r][3 * k + 1], pos[r][3 * k + 2],
-                                                                out + (size_t)9 * (j0 + r) + 3 * k);
+                        for (int k = 0; k < 3; k++) {
+                            double *o = out + (size_t)9 * (j0 + r) + 3 * k;
+                            if (r == 0 && k == 0) {  // the lane's origin
+#pragma unroll
+                                for (int i = 0; i < 3; i++) o[i] = P.p[i];
+                            } else {
+                                frame_point(P, pos[r][3 * k], pos[r][3 * k + 1], pos[r][3 * k + 2], o);
+                            }
+                        }
             }
             if (p0 + cap < len) F = ch.prefix(F, ch.nc, n);
             ch.sync();  // every CTA has read the slots: the next pass, or a CTA's exit, may follow
@@ -331,7 +398,7 @@ __global__ void __launch_bounds__(32 * NW, 3) a2b_bwd_f64_kernel(BackboneArgs a)
         frame_identity(F);
         for (int p = 0; p + 1 < npass; p++) {
             FrameD t = walk<R, false>(a, ang, p * cap + (32 * ch.c + ch.lane) * R, len, nullptr);
-            ch.publish(warp_scan_frames(t, ch.lane), 0);
+            ch.publish(scan_inclusive(t, ch.lane), 0);
             F = ch.prefix(F, ch.nc, n);
             if (ch.c == 0 && ch.lane == 0) frame_store(rec[p + 1].fexc, F);
             ch.sync();
@@ -380,11 +447,16 @@ __global__ void __launch_bounds__(32 * NW, 3) a2b_bwd_f64_kernel(BackboneArgs a)
                 if (j0 + r < len)
 #pragma unroll
                     for (int k = 0; k < 3; k++) {
+                        double g[3];
+                        load3(gin + (size_t)9 * (j0 + r) + 3 * k, g);
+                        if (r == 0 && k == 0) {  // the lane's origin: zero, and no moment
+#pragma unroll
+                            for (int i = 0; i < 3; i++) v6[i] += g[i];
+                            continue;
+                        }
                         rot(W, pos[r] + 3 * k, y);
 #pragma unroll
                         for (int i = 0; i < 3; i++) pos[r][3 * k + i] = y[i];
-                        double g[3];
-                        load3(gin + (size_t)9 * (j0 + r) + 3 * k, g);
                         add_moment(y, g, v6, v6 + 3);
                     }
             move_origin(P, v6, v6 + 3);  // about the pass start
@@ -488,7 +560,8 @@ __device__ __forceinline__ FrameD load_residue(const A2cArgs<double> &a, int b, 
             const double v = k == 2 && j == len - 1 ? 0.0 : ang[(size_t)k * a.L];
             sincos_f64(v, &q.sn[k], &q.cs[k]);
         }
-        backbone_joint<0>(t, q.cs[0], q.sn[0]);
+        constexpr double cb = kTopo.bb_cb[0], sb = kTopo.bb_sb[0], d = kTopo.bb_d[0];
+        first_joint(t, cb, sb, d, q.cs[0], q.sn[0]);
         backbone_joint<1>(t, q.cs[1], q.sn[1]);
         backbone_joint<2>(t, q.cs[2], q.sn[2]);
     }
@@ -630,7 +703,7 @@ __global__ void __launch_bounds__(32 * NW) a2c_bwd_f64_kernel(A2cArgs<double> a,
             FrameD t = load_residue<3>(a, b, p * cap + 32 * ch.c + ch.lane, len, renorm, q);
             int chunk_atoms;
             atoms_exclusive((int)(q.info >> 8), ch.lane, chunk_atoms);
-            ch.publish(warp_scan_frames(t, ch.lane), chunk_atoms);
+            ch.publish(scan_inclusive(t, ch.lane), chunk_atoms);
             F = ch.prefix(F, ch.nc, total);
             if (threadIdx.x == 0) {
                 s_frame[p + 1] = F;
