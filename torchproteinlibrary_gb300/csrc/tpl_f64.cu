@@ -5,12 +5,14 @@
 // FP64 instructions bound these kernels: GB300 issues two FP64 lanes per cycle and SM, so
 // one warp instruction holds an SM's FP64 pipe for 16 cycles however many lanes take
 // part.  Hence
-//   * few FP64 instructions: sines from a 28-instruction polynomial (sincos_f64), one
-//     Kogge-Stone scan over a warp (36 instructions a level) instead of one over a block,
+//   * few FP64 instructions: sines from a 28-instruction polynomial (sincos_f64), one scan
+//     over a warp (18 instructions a level, scan_inclusive) instead of one over a block,
 //     and joints walked once (the backbone's local positions stay in registers);
 //   * full warps: R residues per lane share one scan, frames of earlier chunks are composed
-//     one matrix entry per lane (three instructions a chunk), and warps whose chunk holds no
-//     residue of the chain only pass the barriers;
+//     one matrix entry per lane (three instructions a chunk), lanes that a scan has no work
+//     for take half of their neighbours', and warps whose chunk holds no residue of the chain
+//     only pass the barriers; four CTAs of the backbone kernels per SM, whose spills cost
+//     nothing beside the FP64 pipe (backward, three: 256 chains 96.3 against 86.6 us);
 //   * every SM: a chain's chunks of 32 R residues are spread over the CTAs of a cluster of
 //     1 to 8, which exchange one frame (and, backward, six sums) per chunk through
 //     distributed shared memory.  A chain longer than the cluster's capacity is taken in
@@ -18,10 +20,10 @@
 // Positions are kept relative to the pass's first joint, in world orientation.
 //
 // GB300, against one CTA per chain with block-wide scans (forward, backward): Angles2Backbone
-// 256 chains of 60..350 residues 124 -> 64 us, 268 -> 107 us; Angles2Coords 64 chains of 150
-// residues 132 -> 50 us, 293 -> 70 us, where a warp's own FP64 instructions are what is
-// waited for.  Errors against 64-bit plain torch are no larger than before (6.5e-15 and
-// 4.3e-15 relative).
+// 256 chains of 60..350 residues 124 -> 54 us, 268 -> 87 us; Angles2Coords 64 chains of 150
+// residues 132 -> 49 us, 293 -> 70 us, where a warp's own FP64 instructions are what is
+// waited for.  Errors against 64-bit plain torch are no larger than before (6.4e-15 and
+// 4.2e-15 relative).
 #include <cooperative_groups.h>
 
 #include <algorithm>
@@ -240,17 +242,36 @@ struct Chain {
     }
 };
 
-// Sum over lanes above this one (exclusive suffix) of v, and the warp total.
-__device__ __forceinline__ double suffix_excl(double v, int lane, double &total) {
-    double inc = v;
+// Sums of six values over the lanes above this one, and over the warp, with the halves of
+// the lanes working for one another as in scan_inclusive: at level off a lane without that
+// bit adds the sum of the block after it, three values itself and three on the lane off
+// above it.
+__device__ __forceinline__ void suffix_excl(const double (&v)[6], int lane, double (&suf)[6], double (&total)[6]) {
+    double t[6];
+#pragma unroll
+    for (int i = 0; i < 6; i++) t[i] = v[i];
 #pragma unroll
     for (int off = 1; off < 32; off <<= 1) {
-        const double o = __shfl_down_sync(0xffffffffu, inc, off);
-        if (lane + off < 32) inc += o;
+        const bool owner = (lane & off) == 0;
+        const int src = (lane & ~(2 * off - 1)) | off;  // first lane of the block after
+#pragma unroll
+        for (int i = 0; i < 3; i++) {
+            const double b0 = __shfl_sync(0xffffffffu, t[i], src), b1 = __shfl_sync(0xffffffffu, t[3 + i], src);
+            const double x = __shfl_xor_sync(0xffffffffu, t[3 + i], off);
+            const double y = (owner ? t[i] : x) + (owner ? b0 : b1);
+            const double z = __shfl_xor_sync(0xffffffffu, y, off);
+            if (owner) {
+                t[i] = y;
+                t[3 + i] = z;
+            }
+        }
     }
-    total = __shfl_sync(0xffffffffu, inc, 0);
-    const double e = __shfl_down_sync(0xffffffffu, inc, 1);
-    return lane == 31 ? 0.0 : e;
+#pragma unroll
+    for (int i = 0; i < 6; i++) {
+        total[i] = __shfl_sync(0xffffffffu, t[i], 0);
+        const double e = __shfl_down_sync(0xffffffffu, t[i], 1);
+        suf[i] = lane == 31 ? 0.0 : e;
+    }
 }
 
 // R v of a frame's rotation.
@@ -383,7 +404,7 @@ __global__ void __launch_bounds__(32 * NW, 4) a2b_fwd_f64_kernel(BackboneArgs a)
 }
 
 template <int R, int NW>
-__global__ void __launch_bounds__(32 * NW, 3) a2b_bwd_f64_kernel(BackboneArgs a) {
+__global__ void __launch_bounds__(32 * NW, 4) a2b_bwd_f64_kernel(BackboneArgs a) {
     __shared__ ChunkSlots<NW> s_slots;
     Chain<NW> ch(&s_slots);
     const int b = ch.chain(), len = backbone_length(a, b), cap = ch.nc * 32 * R;
@@ -460,8 +481,7 @@ __global__ void __launch_bounds__(32 * NW, 3) a2b_bwd_f64_kernel(BackboneArgs a)
                         add_moment(y, g, v6, v6 + 3);
                     }
             move_origin(P, v6, v6 + 3);  // about the pass start
-#pragma unroll
-            for (int i = 0; i < 6; i++) suf[i] = suffix_excl(v6[i], ch.lane, tot[i]);
+            suffix_excl(v6, ch.lane, suf, tot);
         }
         ch.publish_sums(tot);
         double after, whole;
@@ -484,16 +504,16 @@ __global__ void __launch_bounds__(32 * NW, 3) a2b_bwd_f64_kernel(BackboneArgs a)
                     const double *gj = gin + (size_t)9 * j;  // read again: kept, it would cost a CTA per SM
                     double u[3], g[3];
 #pragma unroll
-                    for (int i = 0; i < 3; i++) u[i] = (nxt[i] - xC[i]) * a.inv_d[2];
-                    const double om = end ? 0.0 : joint_gradient(u, nxt, G, S);
+                    for (int i = 0; i < 3; i++) u[i] = nxt[i] - xC[i];
+                    const double om = end ? 0.0 : a.inv_d[2] * joint_gradient(u, nxt, G, S);
 #pragma unroll
-                    for (int i = 0; i < 3; i++) u[i] = (xC[i] - xA[i]) * a.inv_d[1];
-                    const double ps = end ? 0.0 : joint_gradient(u, xC, G, S);
+                    for (int i = 0; i < 3; i++) u[i] = xC[i] - xA[i];
+                    const double ps = end ? 0.0 : a.inv_d[1] * joint_gradient(u, xC, G, S);
                     load3(gj + 6, g);
                     add_moment(xC, g, G, S);
 #pragma unroll
-                    for (int i = 0; i < 3; i++) u[i] = (xA[i] - xN[i]) * a.inv_d[0];
-                    const double ph = joint_gradient(u, xA, G, S);
+                    for (int i = 0; i < 3; i++) u[i] = xA[i] - xN[i];
+                    const double ph = a.inv_d[0] * joint_gradient(u, xA, G, S);
                     load3(gj + 3, g);
                     add_moment(xA, g, G, S);
                     load3(gj, g);
@@ -826,8 +846,7 @@ __global__ void __launch_bounds__(32 * NW) a2c_bwd_f64_kernel(A2cArgs<double> a,
         double suf[6] = {0, 0, 0, 0, 0, 0}, tot[6] = {0, 0, 0, 0, 0, 0}, after, whole;
         if (c0 < len) {
             move_origin(P, v6, v6 + 3);  // about the pass start
-#pragma unroll
-            for (int i = 0; i < 6; i++) suf[i] = suffix_excl(v6[i], ch.lane, tot[i]);
+            suffix_excl(v6, ch.lane, suf, tot);
         }
         ch.publish_sums(tot);
         ch.sums_after(min(ch.nc, (len - p0 + 31) / 32) - 1, after, whole);
@@ -904,10 +923,10 @@ constexpr int kBackboneWarps = 4, kAtomWarps = 2;
 
 // Residues per lane of the backbone kernels: two share a scan; one where the batch leaves
 // FP64 pipes idle and the walk's length is what is waited for (forward + backward, one
-// against two: 32 x 64 residues 40 / 58 us, 64 x 128 45 / 59, 64 x 300 66 / 64, 256 x 350
-// 190 / 186, 1024 x 1000 1685 / 1162).
+// against two: 32 x 64 residues 34 / 52 us, 64 x 128 38 / 53, 64 x 300 54 / 57, 128 x 200
+// 57 / 57, 256 x 350 149 / 143, 1024 x 1000 1254 / 981).
 bool one_per_lane(int B, int L) {
-    return (long long)B * L <= 64ll * device_sm_count() && L <= kMaxCluster * 32 * kBackboneWarps;
+    return (long long)B * L <= 128ll * device_sm_count() && L <= kMaxCluster * 32 * kBackboneWarps;
 }
 
 }  // namespace
