@@ -1332,11 +1332,12 @@ static int launch_a2c_bwd(const A2cArgs<T> &a, int B, int renorm, cudaStream_t s
     return cudaGetLastError() == cudaSuccess ? TPL_OK : TPL_ERR_LAUNCH;
 }
 
-// Warps per chain of the float32 kernels: eight while the batch leaves SMs short of
-// chains, four once every SM has several (GB300, forward without names, 0.099 against
-// 0.109 ms at 1024 x 1000 residues and 0.188 against 0.170 ms at 4096 x 500; with
-// names or in the backward the crossing comes at about half the batch).
-static int a2c_ring_warps(int B, int chains_per_sm) { return B < chains_per_sm * device_sm_count() ? 8 : 4; }
+// Warps per chain of the float32 kernels: eight while the batch leaves SMs short of chains,
+// four once every SM has several.  GB300, eight / four warps, us, chains of U{50..500}
+// residues: forward with names 700 chains 25.9 / 28.0, 1024 37.2 / 38.9, 1500 49.0 / 48.6
+// (without names the same line); backward, of whose CTAs of eight warps two fit an SM, 256
+// chains 14.9 / 17.9, 400 22.0 / 20.5, 512 24.1 / 21.5.
+static int a2c_ring_warps(int B, int chains_per_sm) { return B <= chains_per_sm * device_sm_count() ? 8 : 4; }
 
 // The resident CTAs, at most one per chain (a batch of one per SM need not ask).
 template <typename K>
@@ -1394,7 +1395,7 @@ int a2c_forward(bool f64, const unsigned char *seq, int seq_stride, const void *
         case 256: return launch_a2c_fwd<float, 1, 256>(a, B, renorm, st);
         case 512: return launch_a2c_fwd<float, 1, 512>(a, B, renorm, st);
     }
-    return a2c_ring_warps(B, res_names && atom_names ? 4 : 8) == 8 ? launch_a2c_fwd_ring<8>(a, B, renorm, st)
+    return a2c_ring_warps(B, 8) == 8 ? launch_a2c_fwd_ring<8>(a, B, renorm, st)
                                                                     : launch_a2c_fwd_ring<4>(a, B, renorm, st);
 }
 
@@ -1421,7 +1422,7 @@ int a2c_backward_coords(float *grad_angles, const float *grad_coords, const floa
     if (B == 0) return TPL_OK;
     A2cArgs<float> a{seq, seq_stride, nullptr, const_cast<float *>(coords), nullptr, nullptr, grad_angles, grad_coords,
                      (WsHeader *)ws, L, maxA};
-    return a2c_ring_warps(B, 4) == 8 ? launch_a2c_bwd_coords_ring<8>(a, B, L, st)
+    return a2c_ring_warps(B, 2) == 8 ? launch_a2c_bwd_coords_ring<8>(a, B, L, st)
                                      : launch_a2c_bwd_coords_ring<4>(a, B, L, st);
 }
 
