@@ -435,6 +435,17 @@ __device__ __forceinline__ int checked_length(const ChainArgs &a, int b, int lan
 constexpr int fwd_min_blocks(int C) { return C >= 8 ? 5 : 7; }
 constexpr int bwd_min_blocks(int C) { return C >= 8 ? 2 : 4; }
 
+// A lane's transform as the scan takes it.  24 joints (C = 8) drift from SO(3) enough to
+// show in the coordinates, so they are pulled back (1000 residues, against FP64: 1.27e-6 ->
+// 1.07e-6 of the coordinates' norm, C = 4 1.15e-6; 45.7 -> 46.1 us at 4096 chains); 12
+// (C = 4) are left to the chain frame's renormalisation from chunk to chunk.
+template <int C>
+__device__ __forceinline__ PairFrame lane_transform(const Frame<float> &T, int renorm) {
+    PairFrame t = to_pair(T);
+    if (C == 8 && renorm) renormalize_pair(t);
+    return t;
+}
+
 template <int C>
 __global__ void __launch_bounds__(32 * kWarpsPerCta, fwd_min_blocks(C)) a2b_fwd_chain_kernel(ChainArgs a) {
     constexpr int CH = 32 * C;
@@ -477,9 +488,7 @@ __global__ void __launch_bounds__(32 * kWarpsPerCta, fwd_min_blocks(C)) a2b_fwd_
         } else {
             T = walk_chunk<C, C != 4>(a.bc, ang, a.L, j0, len, vec, seg);
         }
-        // lane transforms compose 3C joints: no renormalisation before the scan (the
-        // chain frame carried from chunk to chunk is renormalised)
-        const PairFrame Q = compose_pair(F, warp_inclusive_pair(to_pair(T), lane));
+        const PairFrame Q = compose_pair(F, warp_inclusive_pair(lane_transform<C>(T, a.renorm), lane));
         const PairFrame P = frame_before(Q, F, lane);
         if ((C * lane) % kRecordStride == 0 && j0 < len) pair_store(rec[j0 / kRecordStride].f, P);
         F = shfl_idx_pair(Q, 31);
@@ -1099,7 +1108,7 @@ __global__ void __launch_bounds__(32 * kRingWarps, ring_fwd_min_blocks(C)) a2b_f
         const bool live = s0 < len;
         const int j0 = s0 + C * lane;
         PairFrame t = pair_identity();  // prefix of the lane transforms through this lane
-        if (live) {  // no renormalisation of the lane transforms (3C joints each), as in a2b_fwd_chain_kernel
+        if (live) {
             store_reads_done();  // the walk rewrites the staging buffer
             Frame<float> T;
             if (pf) {
@@ -1111,7 +1120,7 @@ __global__ void __launch_bounds__(32 * kRingWarps, ring_fwd_min_blocks(C)) a2b_f
             } else {
                 T = walk_chunk<C, true>(a.bc, ang, a.L, j0, len, vec, seg);
             }
-            t = warp_inclusive_pair(to_pair(T), lane);
+            t = warp_inclusive_pair(lane_transform<C>(T, a.renorm), lane);
         }
         PairFrame F = pair_identity();  // chain frame at the chunk start
         if (k > 0) {
