@@ -62,7 +62,8 @@ typedef struct tpl_options {
                                   k % 4, the chain frame handed from warp to warp in shared memory
                                   (same records); 1 = warp-granular tiles of 32 R residues joined by
                                   look-back; 128 = CTA tiles of 128 R residues.  Angles2Coords
-                                  reads it as its threads per chain (0 = 256, 128, 256, 512). */
+                                  reads it as warps per chain (4, 8; 0 = by the batch) or threads per
+                                  chain (128, 256, 512). */
     int fp64_carry_min_len;    /* chains at least this long compose inter-tile carries in FP64.
                                   Tile schemes: 0 = default (always), -1 = never.  Four warps per
                                   chain: a positive length hands the chain frame from warp to warp
@@ -131,8 +132,8 @@ int tpl_a2b_backward_coords_f32(float *grad_angles, const float *grad_coords, co
                                 const int32_t *lengths, void *workspace, size_t workspace_bytes, int batch,
                                 int max_len, const tpl_options *opt, void *stream);
 
-/* Angles2Backbone forward, plain FP64 form: one chain per CTA, one launch.
- * Same contract as tpl_a2b_forward_f32 in double precision; replaces
+/* Angles2Backbone forward, plain FP64 form: one thread-block cluster per chain, one
+ * launch.  Same contract as tpl_a2b_forward_f32 in double precision; replaces
  * Angles2BackboneCPU_forward (angles2backbone_interface.cpp:60-80) on the GPU.
  * Needs no workspace. */
 int tpl_a2b_forward_f64(const double *angles, const int32_t *lengths, double *coords, int batch, int max_len,

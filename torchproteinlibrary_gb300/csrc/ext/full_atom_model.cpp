@@ -736,7 +736,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
                         "threads_per_cta of Angles2Coords must be 0, 4, 8, 128, 256 or 512");
             g_a2c_opt.threads_per_cta = (int)threads_per_cta;
         },
-        "Angles2Coords float32 forward: threads per chain (0 = 256; 256 or 512 = 1 residue each; 128 = 2 each; "
+        "Angles2Coords float32 forward: threads per chain (0 = by the batch; 256 or 512 = 1 residue each; 128 = 2 each; "
         "4 or 8 = four or eight warps per chain, chunks of 32 residues)",
         py::arg("threads_per_cta") = 0);
     m.def("get_options", []() { return (int64_t)g_a2c_opt.threads_per_cta; }, "Angles2Coords threads per chain");

@@ -136,7 +136,7 @@ bool options_ok(const tpl_options &o) {
 
 size_t a2b_ws(int B, int L, const tpl_options &o) {
     const int tile = a2b_tile_for(o);
-    const int plain_chunk = 256;  // the plain FP64 backward keeps one record per 256-residue chunk
+    const int plain_chunk = 256;  // room for a record per 256 residues in the FP64 backward
     const int smallest = tile < plain_chunk ? tile : plain_chunk;
     return ws_bytes_for(B, (L + smallest - 1) / smallest);
 }

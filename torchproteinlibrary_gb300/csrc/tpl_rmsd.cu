@@ -20,7 +20,7 @@
 // converted and the solve written for one lane spent about 280 of them per chain (ncu:
 // FP64 pipe 73 % busy; 4096 chains of 400..2303 atoms, 20 us of HBM traffic: 90 us per
 // layer call); this one, which solves two chains with the same instructions and reads the
-// coordinates once, about 45: 37 us.
+// coordinates once, about 45 (FP64 pipe 26 % busy): 37 us.
 #include <cmath>
 #include <cstring>
 

@@ -4,10 +4,11 @@
 // Reference: Layers/FullAtomModel/Coords2TypedCoords/coords2typedcoords_interface.cpp
 // runs on the CPU, one OpenMP task per chain, with string compares per atom.  Here
 // one CTA per chain classifies its atoms from the packed 4-byte name words that
-// Angles2Coords writes, counts them per type, and scatters coordinates in a stable
-// order: per 256-atom tile, one warp ballot per type gives each atom its rank among
-// the atoms of its type before it.  The backward is the inverse gather.  Integer and
-// byte work only; coordinates are copied unchanged.
+// Angles2Coords writes, one probe of a perfect hash each, ranks every atom among those of
+// its type, and moves the coordinates in input order within each type, groups of 128 atoms
+// ordered in shared memory first so that a type's run is written by consecutive lanes
+// (typed_fwd_group_kernel; rows past 32 768 atoms take typed_fwd_kernel).  The backward is
+// the inverse gather.  Integer and byte work only; coordinates are copied unchanged.
 #include <cstdint>
 #include <type_traits>
 
