@@ -419,7 +419,7 @@ def time_plain_fp64(rm, ang, lengths, up, dev, steps):
     torch.cuda.synchronize(dev)
     ms = s.elapsed_time(e) / steps
     return {"value": B * L_RES / (ms / 1e3), "unit": "residues/s", "ms_per_step": ms, "steps": steps,
-            "dtype": "f64", "form": "one chain per CTA, FP64, one launch per pass"}
+            "dtype": "f64", "form": "one cluster per chain, FP64, one launch per pass"}
 
 
 def time_e2e(layer, ang_np, len_np, up_np, dev, steps):

@@ -16,7 +16,7 @@
 // row's first boundary and after its last one by themselves and moves the rest as
 // vectors.  Scalar passes over such rows had been issue-bound: 4096 rows of 1000..3471
 // atoms, stride 3471 (41 us of HBM traffic each): translate 70 -> 39 us, rotate 54 -> 46 us,
-// box 25 -> 22 us.
+// box 26 -> 21 us.
 #include <cfloat>
 #include <cmath>
 #include <cstring>
@@ -199,20 +199,23 @@ __global__ void __launch_bounds__(256) rotate_kernel(const T *in, T *out, const 
     }
 }
 
-constexpr int kReduceThreads = 256;
+// Threads per chain of the two reductions: a thread's loads are what is waited for, and more
+// small CTAs keep more of them in flight (4096 rows of 1157..3471 atoms, 256 / 128 threads:
+// centre 24.7 / 22.1 us, box 22.4 / 21.1; a launch of 4000 atoms each 35.3 / 33.9 and 33.1 / 32.4).
+constexpr int kReduceThreads = 128;
 
 // Centroid of the first n_b atoms of chain b = blockIdx.x (FP64 accumulation);
 // 0 for an empty chain.
 template <typename T>
 __global__ void __launch_bounds__(kReduceThreads) center_kernel(const T *in, T *center, const int *num_atoms,
                                                                 int stride) {
-    constexpr int NW = kReduceThreads / 32;
-    __shared__ double s_warp[NW][3];
-    const int b = blockIdx.x, lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    constexpr int ROWS = kReduceThreads / 8;
+    __shared__ T s_sum[ROWS][3];
+    const int b = blockIdx.x, lane = threadIdx.x & 31;
     const int n = min(num_atoms[b], stride);  // a count past the row is clamped to it
     const T *x = in + (size_t)b * 3 * stride;
-    // offsets from the chain's first atom, summed in the coordinate type per thread and
-    // per warp and in FP64 across the warps: the offsets stay of the chain's own extent
+    // offsets from the chain's first atom, summed in the coordinate type per thread and over
+    // eight lanes and in FP64 across those: the offsets stay of the chain's own extent
     // wherever the chain sits, and GB300's FP64 rate is a small fraction of its FP32 rate
     const T p0 = n > 0 ? x[0] : T(0), p1 = n > 0 ? x[1] : T(0), p2 = n > 0 ? x[2] : T(0);
     T s[3] = {T(0), T(0), T(0)};
@@ -242,20 +245,26 @@ __global__ void __launch_bounds__(kReduceThreads) center_kernel(const T *in, T *
         s[2] += x[3 * i + 2] - p2;
     }
 #pragma unroll
-    for (int off = 16; off > 0; off >>= 1)
+    for (int off = 4; off > 0; off >>= 1)
 #pragma unroll
         for (int c = 0; c < 3; c++) s[c] += __shfl_xor_sync(0xffffffffu, s[c], off);
-    if (lane == 0)
+    if ((lane & 7) == 0)
 #pragma unroll
-        for (int c = 0; c < 3; c++) s_warp[w][c] = (double)s[c];
+        for (int c = 0; c < 3; c++) s_sum[threadIdx.x >> 3][c] = s[c];
     __syncthreads();
-    if (threadIdx.x < 3) {
-        const int c = threadIdx.x;
-        double t = 0.0;
+    if (threadIdx.x >= 32) return;
+    static_assert(ROWS <= 32, "one sum per lane");
+    double t[3];
 #pragma unroll
-        for (int q = 0; q < NW; q++) t += s_warp[q][c];
-        const double pc = c == 0 ? (double)p0 : (c == 1 ? (double)p1 : (double)p2);
-        center[3 * b + c] = n > 0 ? (T)(pc + t / n) : T(0);
+    for (int c = 0; c < 3; c++) t[c] = lane < ROWS ? (double)s_sum[lane][c] : 0.0;
+#pragma unroll
+    for (int off = ROWS / 2; off > 0; off >>= 1)
+#pragma unroll
+        for (int c = 0; c < 3; c++) t[c] += __shfl_xor_sync(0xffffffffu, t[c], off);
+    if (lane < 3) {
+        const double v = lane == 0 ? t[0] : (lane == 1 ? t[1] : t[2]);
+        const double p = lane == 0 ? (double)p0 : (lane == 1 ? (double)p1 : (double)p2);
+        center[3 * b + lane] = n > 0 ? (T)(p + v / n) : T(0);
     }
 }
 
