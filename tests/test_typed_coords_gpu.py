@@ -142,3 +142,37 @@ def test_groups_and_row_phases(built, dtype, pad, na):
     want, wcnt, woff, widx = oracle.typed_coords(x, rn, an, na)
     assert np.array_equal(cnt.cpu().numpy(), wcnt) and np.array_equal(off.cpu().numpy(), woff)
     assert np.array_equal(out.cpu().numpy(), want) and np.array_equal(idx.cpu().numpy(), widx)
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float64])
+@pytest.mark.parametrize("pad", range(4))
+def test_four_warps_in_large_batches(built, dtype, pad):
+    """Batches of four chains per SM and more take four warps per chain: the same chains over
+    and over, lengths around the tiles and groups, rows at every 16-byte phase, bit for bit."""
+    from torchproteinlibrary_gb300 import load_extension
+    fm = load_extension("_FullAtomModel")
+    rng = np.random.default_rng(60 + pad)
+    pairs = [(b"GLY\0", a) for a in (b"N\0\0\0", b"CA\0\0", b"C\0\0\0", b"O\0\0\0")]
+    pairs += [(b"LYS\0", b"NZ\0\0"), (b"MET\0", b"SD\0\0"), (b"HIS\0", b"CG\0\0"), (b"THR\0", b"OG1\0")]
+    na = np.array([0, 1, 31, 33, 127, 128, 129, 511, 512, 513, 641], np.int32)
+    S_out = int(na.max())
+    S = S_out + pad
+    pick = rng.integers(0, len(pairs), (len(na), S))
+    rn = np.array([[list(pairs[k][0]) for k in row] for row in pick], np.uint8)
+    an = np.array([[list(pairs[k][1]) for k in row] for row in pick], np.uint8)
+    x = rng.standard_normal((len(na), 3 * S)).astype(np.float32 if dtype == torch.float32 else np.float64)
+    want, wcnt, woff, widx = oracle.typed_coords(x, rn, an, na)
+    reps = 4 * torch.cuda.get_device_properties(0).multi_processor_count // len(na) + 1
+    dev = torch.device("cuda")
+
+    def rows(v):
+        t = torch.tensor(v, device=dev)
+        return t.repeat(reps, *[1] * (t.dim() - 1))
+
+    B = reps * len(na)
+    out = torch.full((B, 3 * S_out), float("nan"), dtype=dtype, device=dev)
+    cnt = torch.empty(B, 11, dtype=torch.int32, device=dev)
+    off, idx = torch.empty_like(cnt), torch.full((B, S_out), -7, dtype=torch.int32, device=dev)
+    fm.Coords2TypedCoords_forward(rows(x), rows(rn), rows(an), rows(na), out, cnt, off, idx)
+    for got, ref in ((out, want), (cnt, wcnt), (off, woff), (idx, widx)):
+        assert torch.equal(got, rows(ref).to(got.dtype))

@@ -254,7 +254,7 @@ __global__ void __launch_bounds__(kTypedThreads) typed_fwd_kernel(const T *coord
 // to its slot costs three partial sectors of coordinates and one of index.  GB300, 4096
 // chains of U{50..500} residues (72 us of HBM traffic): 142 us with scattered stores, a
 // probed name hash and ranks found twice (73 M warp instructions, 21.7 M sector writes);
-// 102 us (63 M, 17.0 M).  Ordering the groups without keeping the ranks was slower than
+// 102 us with four warps per chain (63 M, 17.0 M), 98 with eight.  Ordering the groups without keeping the ranks was slower than
 // scattering (160 us, 101 M).
 constexpr int kTypedUnroll = 4;
 constexpr int kTypedGroup = 32 * kTypedUnroll;  // atoms ordered and written together
@@ -532,9 +532,14 @@ int typed_forward(bool f64, const void *coords, const uint32_t *res_names, const
             return cudaGetLastError() == cudaSuccess ? (int)TPL_OK : (int)TPL_ERR_LAUNCH;
         };
         auto pick = [&](auto *out_t, auto *coords_t) -> int {
-            // four warps' ranks fit the codes up to 16384 atoms
-            return in_stride <= kTypedMaxAtoms / 2 ? launch(std::integral_constant<int, 4>{}, out_t, coords_t)
-                                                   : launch(std::integral_constant<int, 8>{}, out_t, coords_t);
+            // Eight warps per chain for rows past 3500 atoms, where a chain's codes are most of
+            // the shared memory and more warps share them, and for batches below four chains per
+            // SM; past 16384 atoms four warps' ranks would not fit the codes either.  Eight /
+            // four, us: 4096 chains of 2745 atoms 68.4 / 66.2, of 4465 98.2 / 102.7; 256 of 2250
+            // 11.7 / 15.3; 512 of 4465 23.8 / 25.6.
+            const bool eight = in_stride > 3500 || B < 4 * device_sm_count();
+            return eight ? launch(std::integral_constant<int, 8>{}, out_t, coords_t)
+                         : launch(std::integral_constant<int, 4>{}, out_t, coords_t);
         };
         return f64 ? pick(static_cast<double *>(out), static_cast<const double *>(coords))
                    : pick(static_cast<float *>(out), static_cast<const float *>(coords));
