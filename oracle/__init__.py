@@ -34,7 +34,7 @@ def reference_dir() -> str | None:
     """The reference checkout that the oracle's reference builds read: the
     TPL_REFERENCE_DIR environment variable, else the REF default of
     oracle/Makefile (the one place that names the conventional location).
-    None when that directory does not exist (e.g. on a machine without it)."""
+    None when that directory does not exist or is empty (e.g. on a machine without it)."""
     d = os.environ.get("TPL_REFERENCE_DIR")
     if not d:
         with open(os.path.join(HERE, "Makefile")) as f:
@@ -42,7 +42,7 @@ def reference_dir() -> str | None:
                 if line.startswith("REF") and "?=" in line:
                     d = line.split("?=", 1)[1].strip()
                     break
-    return d if d and os.path.isdir(d) else None
+    return d if d and os.path.isdir(d) and os.listdir(d) else None
 
 
 def build(ref_dir: str | None = None) -> None:
