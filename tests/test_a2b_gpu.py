@@ -816,8 +816,9 @@ def test_float64_clusters_and_passes(rm, B, L):
     check(c, gi, rc, rg, lengths, L, COORD_TOL_F64, GRAD_TOL_F64)
 
 
-@pytest.mark.parametrize("per_sm,L", [(1, 64), (2, 513), (5, 300), (5, 700), (6, 513), (7, 129), (8, 128), (8, 129),
-                                      (8, 257), (9, 320), (9, 384), (9, 767), (9, 768)])
+@pytest.mark.parametrize("per_sm,L", [(1, 64), (2, 513), (2, 516), (5, 300), (5, 700), (6, 516), (7, 132), (8, 128),
+                                      (8, 132), (9, 132), (9, 256), (9, 260), (9, 129), (9, 320), (9, 384), (9, 764),
+                                      (9, 768), (9, 769)])
 def test_automatic_scheme_is_one_of_the_schemes(built, per_sm, L):
     """The built-in choice on both sides of its lines in chains per SM and residues: with
     every option left at 0 the results are bit for bit those of one explicit choice, and that
@@ -839,9 +840,36 @@ def test_automatic_scheme_is_one_of_the_schemes(built, per_sm, L):
         return coords, grad
 
     ring = L >= 384 or B < 8 * sms
-    eight = (L >= 768 or (L > 512 and B < 6 * sms)) if ring else 128 < L <= 256
+    eight = L % 4 == 0 and ((L >= 768 or (L > 512 and B < 6 * sms)) if ring else 128 < L <= 256)
     bring = L >= 384 or B < 6 * sms
     want = both((8 if eight else 4, 4 if ring else 32), (4, 2 if bring and B <= 2 * sms else 1, 4 if bring else 32))
     got = both((0, 0), (0, 0, 0))
     assert torch.equal(got[0], want[0])
     assert torch.equal(got[1], want[1])
+
+
+@pytest.mark.parametrize("L,off", [(1, 0), (3, 1), (5, 2), (127, 0), (128, 1), (129, 3), (130, 0), (385, 0), (514, 0),
+                                   (515, 2), (517, 1), (600, 3), (1027, 0)])
+def test_forward_rows_at_every_phase(built, L, off):
+    """The four-warp forward with four residues per lane on rows that start anywhere in a
+    16-byte block (odd L: every phase within a batch; storage `off` values into an
+    allocation) gives, bit for bit, what it gives on aligned rows: lengths 0 and up, chunk
+    edges, the zeros past each chain, and not a word outside the rows."""
+    from torchproteinlibrary_gb300 import load_extension
+    rm = load_extension("_ReducedModel")
+    B, LA = 13, (L + 3) // 4 * 4
+    g = torch.Generator("cuda").manual_seed(100 + L)
+    ang = torch.zeros(B, 3, LA, device="cuda")
+    ang[:, :, :L] = (torch.rand(B, 3, L, device="cuda", generator=g) * 2 - 1) * 3.1
+    lens = torch.randint(0, L + 1, (B,), device="cuda", generator=g, dtype=torch.int32)
+    lens[0], lens[1] = L, 0
+    ws = torch.zeros(rm.workspace_bytes(B, LA, 4, 4), dtype=torch.uint8, device="cuda")
+    want = torch.empty(B, 9 * LA, device="cuda")
+    rm.Angles2BackboneGPU_forward(ang, want, lens, ws, 4, 4)
+    a = torch.full((B * 3 * L + off,), float("nan"), device="cuda")
+    a[off:] = ang[:, :, :L].reshape(-1)
+    c = torch.full((B * 9 * L + off + 8,), 7.0, device="cuda")
+    got = c[off:off + B * 9 * L].view(B, 9 * L)
+    rm.Angles2BackboneGPU_forward(a[off:].view(B, 3, L), got, lens, ws, 4, 4)
+    assert torch.equal(got, want[:, :9 * L])
+    assert (c[:off] == 7).all() and (c[off + B * 9 * L:] == 7).all()

@@ -226,11 +226,16 @@ def options_for(device, batch: int, max_len: int):
         return hit
     name = torch.cuda.get_device_name(device)
     bucket = _bucket(batch, max_len)
-    entry = _load_cache().get(f"{name}|{bucket}|v2") or _shipped_table(name).get(bucket)
+    own = _load_cache().get(f"{name}|{bucket}|v2")
+    entry = own or _shipped_table(name).get(bucket)
     res = None
     if entry and "backward_coords" in entry:
         try:
             res = _entry_options(entry)
+            if not own and max_len % 4:
+                # the table is tuned on rows of whole 16-byte blocks; others take the built-in
+                # forward (1024 x 999: 15.2 us, with the bucket's eight residues per lane 16.8)
+                res = ((0, 0), res[1])
         except (KeyError, TypeError, ValueError):
             res = None
     _LOOKUP[key] = res

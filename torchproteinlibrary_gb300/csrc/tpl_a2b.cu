@@ -1119,6 +1119,9 @@ static int num_sms() { return device_sm_count(); }
 //   * else one warp per chain, with eight residues per lane where a chunk of 256 holds the
 //     chain but one of 128 does not (4096 chains of 256: four / eight residues 14.3 / 13.4, of
 //     128 9.1 / 12.6, of 320 18.7 / 20.7);
+//   * rows off 16-byte boundaries (max_len no multiple of four): always four residues per
+//     lane, whose chunks leave as bulk copies whatever the row's phase (four / eight, four
+//     warps per chain: 1024 chains of 999 15.2 / 16.8, 2048 of 517 18.6 / 21.9);
 //   * fewer than two chains per SM and chains over 4096 residues: warp tiles, whose
 //     look-back spreads one chain over many warps.
 // An explicit residues_per_thread of 4 or 8 is kept; 1 or 2 selects warp tiles.
@@ -1138,9 +1141,10 @@ static tpl_options chain_options(const tpl_options &opt, int B, int L, bool forw
         const bool ring = L >= 384 || B < 8 * num_sms();
         o.threads_per_cta = ring ? 4 : 32;
         if (o.residues_per_thread == 0) {
-            const bool eight = !forward ? L >= 768
-                               : ring   ? L >= 768 || (L > 512 && B < 6 * num_sms())
-                                        : L > 128 && L <= 256;
+            const bool eight = !forward     ? L >= 768
+                               : L % 4 != 0 ? false
+                               : ring       ? L >= 768 || (L > 512 && B < 6 * num_sms())
+                                            : L > 128 && L <= 256;
             o.residues_per_thread = eight ? 8 : 4;
         }
     }
