@@ -850,8 +850,9 @@ def test_automatic_scheme_is_one_of_the_schemes(built, per_sm, L):
 
 @pytest.mark.parametrize("L,off", [(1, 0), (3, 1), (5, 2), (127, 0), (128, 1), (129, 3), (130, 0), (385, 0), (514, 0),
                                    (515, 2), (517, 1), (600, 3), (1027, 0)])
-def test_forward_rows_at_every_phase(built, L, off):
-    """The four-warp forward with four residues per lane on rows that start anywhere in a
+@pytest.mark.parametrize("cta", [4, 32])
+def test_forward_rows_at_every_phase(built, cta, L, off):
+    """The four-warp and one-warp forwards with four residues per lane on rows that start anywhere in a
     16-byte block (odd L: every phase within a batch; storage `off` values into an
     allocation) gives, bit for bit, what it gives on aligned rows: lengths 0 and up, chunk
     edges, the zeros past each chain, and not a word outside the rows."""
@@ -863,13 +864,13 @@ def test_forward_rows_at_every_phase(built, L, off):
     ang[:, :, :L] = (torch.rand(B, 3, L, device="cuda", generator=g) * 2 - 1) * 3.1
     lens = torch.randint(0, L + 1, (B,), device="cuda", generator=g, dtype=torch.int32)
     lens[0], lens[1] = L, 0
-    ws = torch.zeros(rm.workspace_bytes(B, LA, 4, 4), dtype=torch.uint8, device="cuda")
+    ws = torch.zeros(rm.workspace_bytes(B, LA, 4, cta), dtype=torch.uint8, device="cuda")
     want = torch.empty(B, 9 * LA, device="cuda")
-    rm.Angles2BackboneGPU_forward(ang, want, lens, ws, 4, 4)
+    rm.Angles2BackboneGPU_forward(ang, want, lens, ws, 4, cta)
     a = torch.full((B * 3 * L + off,), float("nan"), device="cuda")
     a[off:] = ang[:, :, :L].reshape(-1)
     c = torch.full((B * 9 * L + off + 8,), 7.0, device="cuda")
     got = c[off:off + B * 9 * L].view(B, 9 * L)
-    rm.Angles2BackboneGPU_forward(a[off:].view(B, 3, L), got, lens, ws, 4, 4)
+    rm.Angles2BackboneGPU_forward(a[off:].view(B, 3, L), got, lens, ws, 4, cta)
     assert torch.equal(got, want[:, :9 * L])
     assert (c[:off] == 7).all() and (c[off + B * 9 * L:] == 7).all()

@@ -429,7 +429,8 @@ __device__ __forceinline__ void store_chunk_fwd(float *dst, const float *stage, 
 // written last; the groups of four points go last to first, so that nothing is overwritten
 // before it is read.  Forward of 1024 chains of up to 517 residues, against scalar stores and
 // angles loaded as they are used: 10.5 -> 9.1 us, 2048 of up to 999 26.1 -> 23.9; 4096 of 385
-// each 27.0 -> 27.8.
+// each 27.0 -> 27.8 (four warps per chain); 4096 of up to 255 16.6 -> 15.1, 16384 of up to 65
+// 27.8 -> 26.1 (one warp).
 template <int P>
 __device__ __forceinline__ void map_points_shifted(float *seg, const Frame<float> &F, int nvalid) {
     float next[4] = {0.f, 0.f, 0.f, 0.f}, tail[4];
@@ -526,14 +527,16 @@ __device__ __forceinline__ PairFrame lane_transform(const Frame<float> &T, int r
     return t;
 }
 
-template <int C>
+// SHIFT: rows of any alignment (C = 4), as in a2b_fwd_ring_kernel.
+template <int C, bool SHIFT>
 __global__ void __launch_bounds__(32 * kWarpsPerCta, fwd_min_blocks(C)) a2b_fwd_chain_kernel(ChainArgs a) {
-    constexpr int CH = 32 * C;
+    static_assert(!SHIFT || C == 4, "the shifted stage is laid out for four residues a lane");
+    constexpr int CH = 32 * C, STAGE = FwdStage<C>::FLOATS + (SHIFT ? 4 : 0);
     extern __shared__ __align__(16) float s_dyn[];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const int b = blockIdx.x * kWarpsPerCta + w;
     if (b >= a.B) return;  // warps are independent: no CTA-wide barrier follows
-    float *stage = s_dyn + w * FwdStage<C>::FLOATS;
+    float *stage = s_dyn + w * STAGE;
     float *seg = stage + FwdStage<C>::lane_offset(lane);
     const int len = checked_length(a, b, lane);
     const float *ang = a.angles + (size_t)b * 3 * a.L;
@@ -543,10 +546,14 @@ __global__ void __launch_bounds__(32 * kWarpsPerCta, fwd_min_blocks(C)) a2b_fwd_
 
     PairFrame F = pair_identity();  // chain frame at the chunk start (world)
     constexpr bool PF = AngBuf<C>::ON;
-    float *abuf = s_dyn + kWarpsPerCta * FwdStage<C>::FLOATS + w * AngBuf<C>::FLOATS;
-    const bool pf = PF && vec;
+    float *abuf = s_dyn + kWarpsPerCta * STAGE + w * AngBuf<C>::FLOATS;
+    const bool pf = PF && (SHIFT || vec);
+    auto prefetch = [&](float *buf, int s0) {
+        if constexpr (SHIFT) prefetch_angles_words<C>(buf, ang, a.L, s0, lane);
+        else prefetch_angles<C>(buf, ang, a.L, s0, lane);
+    };
     if (pf) {
-        if (len > 0) prefetch_angles<C>(abuf, ang, a.L, 0, lane);
+        if (len > 0) prefetch(abuf, 0);
         cp_async_commit();
     }
     int it = 0;
@@ -554,14 +561,15 @@ __global__ void __launch_bounds__(32 * kWarpsPerCta, fwd_min_blocks(C)) a2b_fwd_
         const int nout = min(CH, a.L - s0);
         float *dst = out + (size_t)9 * s0;
         if (s0 >= len) {
-            zero_floats(dst, 9 * nout, lane, vec);
+            if constexpr (SHIFT) zero_span(dst, 9 * nout, lane);
+            else zero_floats(dst, 9 * nout, lane, vec);
             continue;
         }
         const int j0 = s0 + C * lane;
         store_reads_done();  // the walk rewrites the staging buffer
         Frame<float> T;
         if (pf) {
-            if (s0 + CH < len) prefetch_angles<C>(abuf + (it ^ 1) * 3 * CH, ang, a.L, s0 + CH, lane);
+            if (s0 + CH < len) prefetch(abuf + (it ^ 1) * 3 * CH, s0 + CH);
             cp_async_commit();
             cp_async_wait1();  // this chunk's copies (all groups but the newest) have landed
             T = walk_chunk_smem<C, C != 4>(a.bc, abuf + it * 3 * CH, lane, j0, len, seg);
@@ -573,8 +581,14 @@ __global__ void __launch_bounds__(32 * kWarpsPerCta, fwd_min_blocks(C)) a2b_fwd_
         if ((C * lane) % kRecordStride == 0 && j0 < len) pair_store(rec[j0 / kRecordStride].f, P);
         F = shfl_idx_pair(Q, 31);
         if (a.renorm) renormalize_pair(F);
-        map_positions<C>(seg, P, j0, len);
-        store_chunk_fwd<C>(dst, stage, 9 * nout, lane, vec);
+        if constexpr (SHIFT) {
+            const int phase = block_offset(dst);
+            map_positions_shifted(seg, P, len - j0, phase);
+            store_span_fwd(dst, stage + phase, 9 * nout, lane);
+        } else {
+            map_positions<C>(seg, P, j0, len);
+            store_chunk_fwd<C>(dst, stage, 9 * nout, lane, vec);
+        }
     }
     store_reads_done();
 }
@@ -1445,14 +1459,18 @@ int a2b_forward_chain(const float *angles, const int32_t *lengths, float *coords
     const bool ring = opt.threads_per_cta == kRingWarps;
     const int carry_bytes = a.fp64_min > 0 ? kRingWarps * 12 * (int)sizeof(double) : 0;  // FP64 carry slots
     switch (C) {
-        case 4:
-            if (ring && !a.vec)
-                return launch_ring(a2b_fwd_ring_kernel<4, true>, fwd_smem<4>() + 16 * kRingWarps + carry_bytes, B, a, st);
-            return ring ? launch_ring(a2b_fwd_ring_kernel<4, false>, fwd_smem<4>() + carry_bytes, B, a, st)
-                        : launch_chain(a2b_fwd_chain_kernel<4>, fwd_smem<4>(), B, a, st);
+        case 4: {
+            constexpr int smem = fwd_smem<4>(), shift = 16 * kRingWarps;  // four words a warp for the phase
+            static_assert(kRingWarps == kWarpsPerCta, "warps per CTA");
+            if (!a.vec)
+                return ring ? launch_ring(a2b_fwd_ring_kernel<4, true>, smem + shift + carry_bytes, B, a, st)
+                            : launch_chain(a2b_fwd_chain_kernel<4, true>, smem + shift, B, a, st);
+            return ring ? launch_ring(a2b_fwd_ring_kernel<4, false>, smem + carry_bytes, B, a, st)
+                        : launch_chain(a2b_fwd_chain_kernel<4, false>, smem, B, a, st);
+        }
         case 8:
             return ring ? launch_ring(a2b_fwd_ring_kernel<8, false>, fwd_smem<8>() + carry_bytes, B, a, st)
-                        : launch_chain(a2b_fwd_chain_kernel<8>, fwd_smem<8>(), B, a, st);
+                        : launch_chain(a2b_fwd_chain_kernel<8, false>, fwd_smem<8>(), B, a, st);
     }
     return TPL_ERR_UNSUPPORTED;
 }
