@@ -552,3 +552,60 @@ def test_float64_clusters_and_passes(fm, lens):
     np.testing.assert_array_equal(rn, rrn)
     np.testing.assert_array_equal(an, ran)
     check(c, gi, rc, oracle.a2c_backward(g, ang, seqs), na, COORD_TOL_F64, GRAD_TOL_F64)
+
+
+def _ring_angles(fm, n, points):
+    """n (phi, psi) pairs, omega = pi, whose helix of residues has next to no rise, so that a
+    chain of any length stays within some ten Angstrom: for n values of phi the psi of the
+    least rise among points values, from float64 chains of six glycines."""
+    dev = torch.device("cuda")
+    phi = torch.linspace(-3.0, 3.0, n, dtype=torch.float64, device=dev).repeat_interleave(points)
+    psi = torch.linspace(-np.pi, np.pi, points, dtype=torch.float64, device=dev).repeat(n)
+    ang = torch.zeros(n * points, 8, 6, dtype=torch.float64, device=dev)
+    ang[:, 0], ang[:, 1], ang[:, 2] = phi[:, None], psi[:, None], np.pi
+    seq = torch.full((n * points, 7), ord("G"), dtype=torch.uint8, device=dev)
+    seq[:, 6] = 0
+    coords = torch.empty(n * points, 72, dtype=torch.float64, device=dev)
+    e = torch.empty(0, dtype=torch.uint8, device=dev)
+    fm.Angles2Coords_forward(seq, ang, coords, e, e)
+    N = coords.view(-1, 6, 4, 3)[:, :, 0]
+    bend = N[:, 2:] - 2 * N[:, 1:-1] + N[:, :-2]  # normal to the axis
+    axis = torch.linalg.cross(bend[:, 1], bend[:, 2])
+    rise = ((N[:, 3] - N[:, 2]) * axis).sum(-1).abs() / axis.norm(dim=-1).clamp_min(1e-9)
+    rise[bend[:, 1].norm(dim=-1) < 0.5] = 1e9  # straight: no ring
+    best = rise.view(n, points).argmin(1) + torch.arange(n, device=dev) * points
+    assert rise[best].max() < 1e-2
+    return phi[best], psi[best]
+
+
+@pytest.mark.parametrize("warps", [4, 8])
+def test_carried_frame_stays_a_rotation(fm, warps):
+    """The frame handed from chunk to chunk is renormalised, so its departure from a rotation
+    does not grow along the chain.  Every residue of a chain has the same angles, so every
+    chunk of 32 is placed from the same local positions and only the carried frame differs:
+    distances within the last of 512 chunks over those within the first.  In a ring
+    conformation coordinates stay below 16 A: four roundings of half an ulp of 9.5e-7 in each
+    coordinate at either end are 8e-7 of a distance (one standard deviation of them 2e-7 at
+    4 A, in either chunk), and a renormalised frame is a rotation to 2e-7: 2e-6 for the
+    largest of 2e5 distances of 4 A and more."""
+    dev = torch.device("cuda")
+    B, L = 24, 512 * 32
+    phi, psi = _ring_angles(fm, B, 20001)
+    ang = torch.zeros(B, 8, L, device=dev)
+    ang[:, 0], ang[:, 1], ang[:, 2] = phi.float()[:, None], psi.float()[:, None], np.pi
+    seq = torch.full((B, L + 1), ord("G"), dtype=torch.uint8, device=dev)
+    seq[:, L] = 0
+    e = torch.empty(0, dtype=torch.uint8, device=dev)
+    c = torch.empty(B, 12 * L, device=dev)
+    fm.set_options(warps)
+    try:
+        fm.Angles2Coords_forward(seq, ang, c, e, e)
+    finally:
+        fm.set_options(0)
+    assert fm.workspace_status(0) == 0 and c.abs().max() < 16.0
+    x = c.view(B, 512, 128, 3)[:, [0, -1]].double()
+    first, last = (x[:, :, :, None] - x[:, :, None, :]).norm(dim=-1).unbind(1)
+    far = first > 4.0
+    assert far.any(dim=(1, 2)).all()
+    err = (last / first - 1.0).abs()[far].max().item()
+    assert err <= 2e-6, err

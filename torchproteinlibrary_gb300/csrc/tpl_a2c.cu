@@ -467,36 +467,6 @@ __global__ void __launch_bounds__(NT) a2c_fwd_kernel(A2cArgs<T> a, int renorm) {
 }
 
 // ---------------------------------------------------------- handoffs of a chain
-// The frame a warp hands to the next chunk's, F o T for the frame F it has received and its
-// chunk's transform T, one entry per lane (lanes 0..11 in pair_store_vec's order).  The
-// handoffs of a chain run one after another, so what lies between a warp's wait and its
-// signal is the latency of a small batch: an entry is three fused multiply-adds on values
-// one shared-memory read away, and T is renormalised before the wait instead of F o T after
-// it.  Whole frames composed, renormalised and stored by one lane: 530 cycles a handoff
-// against 490 (8 chains of 256 residues), 61.0 against 60.1 us a training step of 256 chains,
-// 291.8 against 289.5 us for 4096 x 500.  (The Angles2Backbone forward, whose chunks are
-// shorter work, loses 1.5 % by it.  Barrier numbers from a register, instead of the switch,
-// take a handoff to 410 cycles but reserve all 16 barriers of a CTA: 10 % slower at 4096
-// chains.)
-// Lane e holds row i, column j (3: the translation): e = 2 j + i for i < 2, 8 + j for i = 2.
-__device__ __forceinline__ float3 carry_column(float *scratch, const PairFrame &T, int lane) {
-    if (lane == 31) pair_store_vec(scratch, T);
-    __syncwarp();
-    const int j = lane < 8 ? lane >> 1 : (lane & 3);
-    return make_float3(scratch[2 * j], scratch[2 * j + 1], scratch[8 + j]);
-}
-// F from a handoff slot.
-__device__ __forceinline__ float carry_product(const float *slot, float3 t, int lane) {
-    const float *f = slot + (lane < 8 ? (lane & 1) : 8);
-    const int step = lane < 8 ? 2 : 1;
-    const float v = fmaf(f[0], t.x, fmaf(f[step], t.y, f[2 * step] * t.z)), p = f[3 * step];
-    return ((0x8c0 >> lane) & 1) ? v + p : v;  // lanes 6, 7 and 11: the translation
-}
-// F the identity.
-__device__ __forceinline__ float carry_first(float3 t, int lane) {
-    return lane >= 8 ? t.z : ((lane & 1) ? t.y : t.x);
-}
-
 // What a backward hands on (G, S and an origin) as three 16-byte accesses.
 __device__ __forceinline__ void store_sums(float *slot, float g0, float g1, float g2, float s0, float s1, float s2,
                                            const float *o) {
@@ -556,7 +526,6 @@ __global__ void __launch_bounds__(32 * NW, NW == 4 ? 6 : 3) a2c_fwd_ring_kernel(
     extern __shared__ __align__(16) unsigned char smem_raw[];
     A2cRingSmem<NW, NAMES> &sm = *reinterpret_cast<A2cRingSmem<NW, NAMES> *>(smem_raw);
     __shared__ __align__(16) float s_ring[NW][16];  // chain frame (12, pair_store_vec) and first atom index
-    __shared__ __align__(16) float s_total[NW][12];  // carry_column
 
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const RingTopology &tp = sm.topo;
@@ -657,13 +626,6 @@ __global__ void __launch_bounds__(32 * NW, NW == 4 ? 6 : 3) a2c_fwd_ring_kernel(
         }
         const int cnt = __shfl_sync(0xffffffffu, ci, 31), aoff = ci - na;
 
-        const bool hands = ck + 1 < cnch;  // the chain goes on after this chunk
-        float3 tc = make_float3(0.f, 0.f, 0.f);
-        if (hands) {
-            PairFrame T = t;  // lane 31: the chunk's transform
-            if (renorm) renormalize_pair(T);
-            tc = carry_column(s_total[w], T, lane);
-        }
         PairFrame F = pair_identity();  // chain frame at the chunk start
         int abase = 0;                  // first atom of the chunk
         if (cb != (int)blockIdx.x || ck > 0) ring_wait<NW>(w);
@@ -671,17 +633,28 @@ __global__ void __launch_bounds__(32 * NW, NW == 4 ? 6 : 3) a2c_fwd_ring_kernel(
             F = pair_load_vec(s_ring[w]);
             abase = __float_as_int(s_ring[w][12]);
         }
-        if (hands) {
-            float *next = s_ring[(w + 1) % NW];
-            const float v = ck > 0 ? carry_product(s_ring[w], tc, lane) : carry_first(tc, lane);
-            if (lane < 13) next[lane] = lane < 12 ? v : __int_as_float(abase + cnt);
-        }
-        if (hands || cb + (int)gridDim.x < nb) ring_signal<NW>((w + 1) % NW);
         const float2 org = F.p;  // the chunk's origin; positions are relative to it
         const float org2 = F.p2;
         F.p = make_float2(0.f, 0.f);
         F.p2 = 0.f;
         const PairFrame Q = compose_pair(F, t);
+        // Lane 31's Q is the frame the next chunk starts from.  It is the frame handed on that
+        // is pulled back to a rotation, at every handoff, so that a chain's rounding does not
+        // add up to a scale however many chunks it has.  (Only the chunk's own transform
+        // renormalised, before the wait: 61.0 -> 60.1 us a training step of 256 chains, but the
+        // scale drifts: distances within a chunk 3.2e-6 off after 64 chunks of a ring
+        // conformation and 2.3e-5 after 512, where they are 4e-7 off with it.)
+        if (ck + 1 < cnch) {
+            PairFrame Fn = Q;
+            if (renorm) renormalize_pair(Fn);
+            Fn.p = __fadd2_rn(Fn.p, org);
+            Fn.p2 += org2;
+            if (lane == 31) {
+                pair_store_vec(s_ring[(w + 1) % NW], Fn);
+                s_ring[(w + 1) % NW][12] = __int_as_float(abase + cnt);
+            }
+        }
+        if (ck + 1 < cnch || cb + (int)gridDim.x < nb) ring_signal<NW>((w + 1) % NW);
 
         const PairFrame P = frame_before(Q, F, lane);  // at this lane's N
         float *out = a.coords + (size_t)cb * 3 * a.maxA;
