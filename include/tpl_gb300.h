@@ -336,6 +336,9 @@ int tpl_pdb_read_batch(const char *const *filenames, int batch, int max_atoms, d
  * Taylor series), for n device floats on `stream`. */
 int tpl_sincos_f32(const float *a, float *s, float *c, int n, void *stream);
 
+/* The same for the FP64 kernels (the library's sincos beyond |a| = 1e4). */
+int tpl_sincos_f64(const double *a, double *s, double *c, int n, void *stream);
+
 /* Coords2RMSD forward: least RMSD between src and dst after optimal superposition
  * (quaternion method), per chain.  Replaces Coords2RMSDGPU_forward
  * (Layers/RMSD/Coords2RMSD/coords2rmsd_interface.cpp:52-111); center = 1 also folds

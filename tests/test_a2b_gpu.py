@@ -874,3 +874,38 @@ def test_forward_rows_at_every_phase(built, cta, L, off):
     rm.Angles2BackboneGPU_forward(a[off:].view(B, 3, L), got, lens, ws, 4, cta)
     assert torch.equal(got, want[:, :9 * L])
     assert (c[:off] == 7).all() and (c[off + B * 9 * L:] == 7).all()
+
+
+def test_sincos_f64_error_bound(built):
+    """The float64 kernels' own sin/cos against extended precision (longdouble: 64 bits of
+    significand at least), relative to the result: on [-pi, pi], up to the switch to the
+    library's function at 1e4 and past it, on the doubles next to multiples of pi/2, where the
+    result is the reduced argument itself, and near them; infinities and NaN give NaN.  The
+    bound: half an ulp of the reduced argument, half an ulp of the last addition and a tenth
+    for what is added there; the library's own bound is 2."""
+    from torchproteinlibrary_gb300 import capi
+    lib = capi.lib()
+    dev = torch.device("cuda")
+    rng = np.random.default_rng(14)
+    k = rng.integers(-6366, 6367, 100000)
+    multiples = k * (np.pi / 2)
+    x = np.concatenate([rng.uniform(-np.pi, np.pi, 200000), rng.uniform(-1e4, 1e4, 200000),
+                        multiples, np.nextafter(multiples, np.inf), np.nextafter(multiples, -np.inf),
+                        multiples + rng.uniform(-1, 1, k.size) * 2.0 ** rng.integers(-50, 0, k.size),
+                        rng.uniform(-1, 1, 10000) * 2.0 ** rng.integers(-60, 0, 10000),
+                        np.array([0.0, np.pi / 4, -np.pi / 4, np.pi / 2, -np.pi, 1e4, -1e4,
+                                  np.nextafter(1e4, 2e4), -np.nextafter(1e4, 2e4), 1e6, -1e15])])
+    special = np.array([np.inf, -np.inf, np.nan])
+    a = torch.tensor(np.concatenate([x, special]), device=dev)
+    s, c = torch.empty_like(a), torch.empty_like(a)
+    capi.check(lib.tpl_sincos_f64(a.data_ptr(), s.data_ptr(), c.data_ptr(), a.numel(), capi.stream_ptr()), "sincos")
+    torch.cuda.synchronize()
+    assert torch.isnan(s[-3:]).all() and torch.isnan(c[-3:]).all()
+    inside = np.abs(x) <= 1e4
+    xl = x.astype(np.longdouble)
+    for got, ref in ((s, np.sin(xl)), (c, np.cos(xl))):
+        got = got[:-3].cpu().numpy()
+        ulp = np.spacing(np.abs(ref).astype(np.float64)).astype(np.longdouble)
+        err = np.abs(got - ref) / ulp
+        assert err[inside].max() <= 1.1, (float(err[inside].max()), float(x[inside][err[inside].argmax()]))
+        assert err[~inside].max() <= 2.0

@@ -172,6 +172,11 @@ int tpl_sincos_f32(const float *a, float *s, float *c, int n, void *stream) {
     return sincos_poly_f32(a, s, c, n, (cudaStream_t)stream);
 }
 
+int tpl_sincos_f64(const double *a, double *s, double *c, int n, void *stream) {
+    if (n < 0 || (n > 0 && (!a || !s || !c))) return TPL_ERR_ARGUMENT;
+    return sincos_poly_f64(a, s, c, n, (cudaStream_t)stream);
+}
+
 size_t tpl_a2b_workspace_bytes(int batch, int max_len, const tpl_options *opt) {
     if (batch < 0 || max_len < 0) return 0;
     return a2b_ws(batch, max_len, resolve(opt));

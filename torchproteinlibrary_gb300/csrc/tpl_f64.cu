@@ -5,7 +5,7 @@
 // FP64 instructions bound these kernels: GB300 issues two FP64 lanes per cycle and SM, so
 // one warp instruction holds an SM's FP64 pipe for 16 cycles however many lanes take
 // part.  Hence
-//   * few FP64 instructions: sines from a 28-instruction polynomial (sincos_f64), one scan
+//   * few FP64 instructions: sines from a 29-instruction polynomial (sincos_f64), one scan
 //     over a warp (18 instructions a level, scan_inclusive) instead of one over a block,
 //     and joints walked once (the backbone's local positions stay in registers);
 //   * full warps: R residues per lane share one scan, frames of earlier chunks are composed
@@ -47,11 +47,14 @@ __device__ __noinline__ double2 sincos_any(double a) {
 }
 
 // sin and cos without the library's branches: Cody-Waite reduction by pi/2 (rounded by
-// adding 1.5 * 2^52, whose sum's low bits are the quadrant; pi/2 as two doubles, the
+// adding 1.5 * 2^52, whose sum's low bits are the quadrant; pi/2 as three doubles, the
 // rounding of the reduced argument kept as rl), then the Taylor series of sin to r^17 and
-// of cos to r^16 (truncation below 1e-17 on |r| <= pi/4), corrected to first order in rl.
-// Below one ulp of the result's binade for |a| <= 1e4; larger arguments, infinities and
-// NaN go to sincos.
+// of cos to r^16 (truncation below 1e-17 on |r| <= pi/4), with rl taken into what is added
+// last to r and to 1.  Against 113-bit sines (five million arguments, those next to
+// multiples of pi/2 among them) within 0.97 ulp of the result for |a| <= 1e4, 9.4e-17
+// absolute.  (Two terms of pi/2, and rl added to r and to 1 before the series: one
+// instruction less, 1.47 ulp and 1.3e-16, but 296 ulp next to multiples of pi/2.)  Larger
+// arguments, infinities and NaN go to sincos.
 __device__ __forceinline__ void sincos_f64(double a, double *s, double *c) {
     if (!(fabs(a) <= 1.0e4)) {
         const double2 v = sincos_any(a);
@@ -59,9 +62,14 @@ __device__ __forceinline__ void sincos_f64(double a, double *s, double *c) {
         *c = v.y;
         return;
     }
-    constexpr double kShift = 6755399441055744.0, kHi = 1.5707963267948966, kLo = 6.123233995736766e-17;
+    constexpr double kShift = 6755399441055744.0;
+    constexpr double kHi = 1.5707963267948966, kMid = 6.123233995736766e-17, kLo = -1.4973849048591833e-33;
     const double t = fma(a, 0.63661977236758134, kShift), k = t - kShift;
-    const double rh = fma(-k, kHi, a), r = fma(-k, kLo, rh), rl = fma(-k, kLo, rh - r);
+    // rh is exact; below 2^-40 (by the exponent bits) rh - r no longer is, and r's rounding
+    // is half an ulp of the result
+    const double rh = fma(-k, kHi, a), r = fma(-k, kMid, rh);
+    const bool tiny = (unsigned)(__double2hiint(r) & 0x7fffffff) < 0x3d700000u;
+    const double rl = fma(-k, kLo, tiny ? 0.0 : fma(-k, kMid, rh - r));
     const double r2 = r * r;
     double ps = fma(r2, 1.0 / 355687428096000.0, -1.0 / 1307674368000.0);
     ps = fma(ps, r2, 1.0 / 6227020800.0);
@@ -77,8 +85,7 @@ __device__ __forceinline__ void sincos_f64(double a, double *s, double *c) {
     pc = fma(pc, r2, -1.0 / 720.0);
     pc = fma(pc, r2, 1.0 / 24.0);
     pc = fma(pc, r2, -0.5);
-    const double c0 = fma(pc, r2, 1.0);
-    const double sr = fma(ps * r2, r, fma(rl, c0, r)), cr = fma(pc, r2, fma(-rl, r, 1.0));
+    const double cr = fma(fma(pc, r, -rl), r, 1.0), sr = r + fma(ps * r2, r, rl * cr);
     const unsigned q = (unsigned)__double2loint(t);
     const double ss = (q & 1u) ? cr : sr, cc = (q & 1u) ? sr : cr;
     *s = __hiloint2double(__double2hiint(ss) ^ (int)((q << 30) & 0x80000000u), __double2loint(ss));
@@ -891,6 +898,12 @@ __global__ void __launch_bounds__(32 * NW) a2c_bwd_f64_kernel(A2cArgs<double> a,
         for (int k = 0; k < 8; k++) gout[(size_t)k * a.L + i] = 0.0;
 }
 
+// sincos_f64 as the kernels above evaluate it, for the tests.
+__global__ void sincos_f64_kernel(const double *a, double *s, double *c, int n) {
+    const int i = (int)(blockIdx.x * blockDim.x + threadIdx.x);
+    if (i < n) sincos_f64(a[i], s + i, c + i);
+}
+
 // ------------------------------------------------------------------ host side
 constexpr int kMaxCluster = 8;  // the portable cluster size
 
@@ -964,6 +977,12 @@ int a2b_backward_f64_plain(double *grad_angles, const double *grad_coords, const
     if (one_per_lane(B, L))
         return launch_cluster(a2b_bwd_f64_kernel<1, NW>, B, cluster_size(L, 32 * NW), 32 * NW, 0, st, a);
     return launch_cluster(a2b_bwd_f64_kernel<2, NW>, B, cluster_size(L, 64 * NW), 32 * NW, 0, st, a);
+}
+
+int sincos_poly_f64(const double *a, double *s, double *c, int n, cudaStream_t st) {
+    if (n <= 0) return TPL_OK;
+    sincos_f64_kernel<<<(unsigned)((n + 255ll) / 256), 256, 0, st>>>(a, s, c, n);
+    return cudaGetLastError() == cudaSuccess ? TPL_OK : TPL_ERR_LAUNCH;
 }
 
 int a2c_forward_f64(const A2cArgs<double> &a, int B, bool renorm, cudaStream_t st) {

@@ -81,6 +81,7 @@ int a2b_chain_record_stride();
 int a2b_backward_coords(float *grad_angles, const float *grad_coords, const float *coords, const int32_t *lengths,
                         void *ws, int B, int L, const tpl_options &opt, cudaStream_t st);
 int sincos_poly_f32(const float *a, float *s, float *c, int n, cudaStream_t st);
+int sincos_poly_f64(const double *a, double *s, double *c, int n, cudaStream_t st);  // tpl_f64.cu
 size_t a2b_ws(int B, int L, const tpl_options &o);  // workspace bytes of the FP32 Angles2Backbone entries
 tpl_options resolve(const tpl_options *opt);
 bool options_ok(const tpl_options &o);
