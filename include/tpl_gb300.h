@@ -205,7 +205,8 @@ int tpl_a2c_backward_f64(double *grad_angles, const double *grad_coords, const u
  * gradient's error against FP64 is about 1e-5 of its largest entry, since the axes
  * come from FP32 coordinate differences.  The workspace only needs its status word
  * (>= 64 bytes, zeroed once).  Eight warps share a chain on chunks of 32 residues
- * below 4 x (number of SMs) chains, four from there. */
+ * up to 2 x (number of SMs) chains, four from there.  max_len up to 1.1 million: the first
+ * atom of every chunk is kept in shared memory; TPL_ERR_UNSUPPORTED past that. */
 int tpl_a2c_backward_coords_f32(float *grad_angles, const float *grad_coords, const float *coords,
                                 const uint8_t *sequences, int seq_stride, void *workspace, size_t workspace_bytes,
                                 int batch, int max_len, int max_atoms, void *stream);

@@ -609,3 +609,37 @@ def test_carried_frame_stays_a_rotation(fm, warps):
     assert far.any(dim=(1, 2)).all()
     err = (last / first - 1.0).abs()[far].max().item()
     assert err <= 2e-6, err
+
+
+@pytest.mark.parametrize("max_len", [144384, 144385, 1100000])
+def test_backward_of_long_rows(fm, max_len):
+    """Rows as long as eight warps' tables of first atoms fit the shared memory, a chunk
+    longer (the warps then share one), and near the limit: the float32 backward from the
+    coordinates against the oracle, zeros past every chain, an empty chain; then a batch
+    with a chain that is refused and one whose atoms overflow the rows."""
+    rng = np.random.default_rng(17)
+    seqs = ["".join(rng.choice(list(AA), n)) for n in (700, 33, 0, 1, 257)]
+    L = 700
+    ang = rng.uniform(-np.pi, np.pi, (len(seqs), 8, L)).astype(np.float32).astype(np.float64)
+    rc, _, _, na = oracle.a2c_forward(ang, seqs)
+    g = rng.standard_normal(rc.shape).astype(np.float32).astype(np.float64)
+    for b, n in enumerate(na):
+        g[b, 3 * n:] = 0
+    rg = oracle.a2c_backward(g, ang, seqs)
+    long = np.zeros((len(seqs), 8, max_len), np.float32)
+    long[:, :, :L] = ang
+    c, _, _, _, gi = run_gpu(fm, long, seqs, g, torch.float32, from_coords=True)
+    assert not gi[:, :, L:].any()
+    check(c, gi[:, :, :L], rc, rg, na, COORD_TOL_F32, GRAD_TOL_F32)
+
+    from torchproteinlibrary_gb300.FullAtomModel.Angles2Coords import convertStringList
+    dev = torch.device("cuda")
+    slots = 3600
+    bad = ["G" * 900, "G" * 500 + "X" + "G" * 100, "W" * 700]  # 4 and 14 atoms a residue: 3600, refused, 9800
+    for refused, status in ((bad[:2], -5), (bad[::2], -7)):
+        ga = torch.full((2, 8, max_len), float("nan"), device=dev)
+        fm.Angles2Coords_backward_coords(torch.ones(2, 3 * slots, device=dev), ga, convertStringList(refused).to(dev),
+                                         torch.randn(2, 3 * slots, device=dev))
+        assert fm.workspace_status(0) == status
+        assert torch.all(ga[1] == 0) and torch.all(ga[0, :, 900:] == 0)
+        assert torch.isfinite(ga[0]).all() and torch.any(ga[0] != 0)

@@ -1040,7 +1040,9 @@ __device__ __forceinline__ void add_atom(const float *xs, const float *gs, const
 // The kernel: chunks of 32 residues, one per lane, last chunk first, dealt round NW = 4 or
 // 8 warps as one stream over the CTA's chains, as in a2c_fwd_ring_kernel (chains last to
 // first: the first CTAs read the rows the forward wrote last, which may still be in L2).
-// A warp finds the first atom of every chunk itself as it reads a chain's sequence.  Per
+// A warp finds the first atom of every chunk itself as it reads a chain's sequence (4 bytes a
+// chunk and warp; where that does not fit the shared memory, past 140 000 residues with eight
+// warps, a CTA takes one chain and its warps share one table).  Per
 // chunk it receives the atom range of coordinates and dL/dx in shared memory (one bulk
 // copy each of their whole 16-byte blocks, word copies of the ragged ends), walks each
 // lane's residue, suffix-scans the sums over the warp and takes the sums over later chunks
@@ -1073,11 +1075,13 @@ struct A2cBwdRingSmem {
     alignas(16) float x[NW][kA2cStageAtoms * 3 + 4];  // 4 words of slack for the 16-byte phase of the source
     alignas(16) float g[NW][kA2cStageAtoms * 3 + 4];
     RingBwdTopology topo;
-    int base[1];  // per warp: first atom of each chunk, max_chunks + 1 entries (dynamic)
+    int base[1];  // first atom of each chunk, max_chunks + 1 entries per warp, or for all of them (dynamic)
 };
 
+// shared_bases: one table for the CTA; the grid is then the batch.
 template <int NW>
-__global__ void __launch_bounds__(32 * NW) a2c_bwd_coords_ring_kernel(A2cArgs<float> a, int nb, int max_chunks) {
+__global__ void __launch_bounds__(32 * NW) a2c_bwd_coords_ring_kernel(A2cArgs<float> a, int nb, int max_chunks,
+                                                                      bool shared_bases) {
     constexpr int NT = 32 * NW;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     A2cBwdRingSmem<NW> &sm = *reinterpret_cast<A2cBwdRingSmem<NW> *>(smem_raw);
@@ -1095,7 +1099,7 @@ __global__ void __launch_bounds__(32 * NW) a2c_bwd_coords_ring_kernel(A2cArgs<fl
     }
     if (lane == 0) mbar_init(&s_bar[w]);
     __syncthreads();
-    int *base = sm.base + w * (max_chunks + 1);
+    int *base = sm.base + (shared_bases ? 0 : w * (max_chunks + 1));
     constexpr float inv_dphi = 1.f / kTopoF32.bb_d[0], inv_dpsi = 1.f / kTopoF32.bb_d[1],
                     inv_dom = 1.f / kTopoF32.bb_d[2];
 
@@ -1153,6 +1157,7 @@ __global__ void __launch_bounds__(32 * NW) a2c_bwd_coords_ring_kernel(A2cArgs<fl
     };
     if (b >= 0) {
         enter(c_first);
+        if (shared_bases) __syncthreads();  // the warps write the same entries, in their own time
         settle();
         fetch();
     }
@@ -1347,12 +1352,18 @@ static int launch_a2c_fwd_ring(const A2cArgs<float> &a, int B, int renorm, cudaS
 template <int NW>
 static int launch_a2c_bwd_coords_ring(const A2cArgs<float> &a, int B, int L, cudaStream_t st) {
     const int max_chunks = std::max(1, (L + kA2cChunk - 1) / kA2cChunk);
-    const size_t smem = offsetof(A2cBwdRingSmem<NW>, base) + sizeof(int) * (size_t)NW * (size_t)(max_chunks + 1);
     auto k = a2c_bwd_coords_ring_kernel<NW>;
-    if (!set_max_dynamic_smem(reinterpret_cast<const void *>(k), (int)smem))
-        return TPL_ERR_LAUNCH;
-    const int grid = ring_grid(k, 32 * NW, smem, B);
-    k<<<grid, 32 * NW, smem, st>>>(a, B, max_chunks);
+    size_t smem = 0;
+    auto fits = [&](int tables) {
+        smem = offsetof(A2cBwdRingSmem<NW>, base) + sizeof(int) * (size_t)tables * (size_t)(max_chunks + 1);
+        if (smem <= (1u << 30) && set_max_dynamic_smem(reinterpret_cast<const void *>(k), (int)smem)) return true;
+        (void)cudaGetLastError();  // a size past the limit is no failure yet
+        return false;
+    };
+    const bool shared_bases = !fits(NW);
+    if (shared_bases && !fits(1)) return TPL_ERR_UNSUPPORTED;
+    const int grid = shared_bases ? B : ring_grid(k, 32 * NW, smem, B);
+    k<<<grid, 32 * NW, smem, st>>>(a, B, max_chunks, shared_bases);
     return cudaGetLastError() == cudaSuccess ? TPL_OK : TPL_ERR_LAUNCH;
 }
 
