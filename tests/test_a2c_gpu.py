@@ -643,3 +643,24 @@ def test_backward_of_long_rows(fm, max_len):
         assert fm.workspace_status(0) == status
         assert torch.all(ga[1] == 0) and torch.all(ga[0, :, 900:] == 0)
         assert torch.isfinite(ga[0]).all() and torch.any(ga[0] != 0)
+
+
+@pytest.mark.parametrize("chi", [3, 4, 5, 6, 7])
+def test_float64_nan_side_chain_angle(fm, chi):
+    """A NaN chi angle in float64 reaches every atom that the oracle has NaN, the first atom
+    of the joint's group among them (the only one of Lys' fifth), and no other; the gradient
+    is NaN for the residue's phi and whatever moves it, and finite for the residues after."""
+    seqs = ["GG" + r + "GG" for r in "KRWSVM"]
+    rng = np.random.default_rng(chi)
+    ang = rng.uniform(-np.pi, np.pi, (len(seqs), 8, 5))
+    ang[:, chi, 2] = np.nan
+    rc, _, _, na = oracle.a2c_forward(ang, seqs)
+    g = rng.standard_normal(rc.shape)
+    c, _, _, _, gi = run_gpu(fm, ang, seqs, g, torch.float64)
+    np.testing.assert_array_equal(np.isnan(c), np.isnan(rc))
+    for b, n in enumerate(na):
+        if np.isnan(rc[b, :3 * n]).any():
+            assert np.isnan(gi[b, 0, :3]).all() and np.isnan(gi[b, 1, :2]).all() and np.isnan(gi[b, 2, :2]).all()
+            assert np.isfinite(gi[b, :, 3:]).all()
+        else:
+            assert np.isfinite(gi[b]).all()

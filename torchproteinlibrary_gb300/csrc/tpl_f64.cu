@@ -596,6 +596,14 @@ __device__ __forceinline__ FrameD load_residue(const A2cArgs<double> &a, int b, 
     return t;
 }
 
+// The first atom of a side-chain group: the group's origin, but with the product by its zero
+// local position, so that a NaN angle makes it NaN as it does the group's other atoms (it is
+// the only one of Lys' fifth).
+__device__ __forceinline__ void group_origin(const FrameD &f, double *x) {
+#pragma unroll
+    for (int i = 0; i < 3; i++) x[i] = fma(f.r[3 * i + 1], 0.0, f.p[i]);
+}
+
 // Atoms of the lanes before this one, and of the warp.
 __device__ __forceinline__ int atoms_exclusive(int na, int lane, int &total) {
     int inc = na;
@@ -670,7 +678,9 @@ __global__ void __launch_bounds__(32 * NW) a2c_fwd_f64_kernel(A2cArgs<double> a,
                 apply_joint(S, g_topo.jcb[ty][k], g_topo.jsb[ty][k], g_topo.jd[ty][k], fixed ? 1.0 : q.cs[3 + k],
                             fixed ? 0.0 : q.sn[3 + k]);
                 const int f0 = g_topo.jfirst[ty][k];
-                emit(2 + f0, S.p);  // the group's first atom sits at the joint's origin
+                double first[3];
+                group_origin(S, first);
+                emit(2 + f0, first);
                 for (int m = 1; m < g_topo.jna[ty][k]; m++) {
                     const double *v = g_topo.sc[ty][f0 + m];
                     local(S, v[0], v[1], v[2], 2 + f0 + m);
@@ -824,7 +834,9 @@ __global__ void __launch_bounds__(32 * NW) a2c_bwd_f64_kernel(A2cArgs<double> a,
                     chi[k] = -joint_gradient(ju[k], S.p, Gsc, Ssc);  // less the atoms before the group
                 }
                 const int f0 = g_topo.jfirst[ty][k];
-                take(2 + f0, S.p, Gsc, Ssc);
+                double first[3];
+                group_origin(S, first);
+                take(2 + f0, first, Gsc, Ssc);
                 for (int m = 1; m < g_topo.jna[ty][k]; m++) {
                     const double *v = g_topo.sc[ty][f0 + m];
                     double x[3];
