@@ -9,6 +9,7 @@
 // ordered in shared memory first so that a type's run is written by consecutive lanes
 // (typed_fwd_group_kernel; rows past 32 768 atoms take typed_fwd_kernel).  The backward is
 // the inverse gather.  Integer and byte work only; coordinates are copied unchanged.
+#include <cstddef>
 #include <cstdint>
 #include <type_traits>
 
@@ -83,7 +84,7 @@ constexpr int kTypedNameCount = sizeof(kTypedNames) / sizeof(TypedName);
 // trial; checked at compile time), so that a lookup is one probe of each and no branch:
 // the residue-agnostic names by their atom word, the pairs by both words.
 constexpr int kPairSlots = 512, kPlainSlots = 16;
-struct TypedTables {
+struct alignas(8) TypedTables {  // an entry is read as one 8-byte word
     uint32_t pair[kPairSlots][2];   // residue word | type << 24, atom word; type 0xff in an empty slot
     uint32_t plain[kPlainSlots][2];  // atom word, type; type 0xffffffff in an empty slot
     int clashes;
@@ -114,6 +115,8 @@ constexpr TypedTables build_typed_tables() {
     return t;
 }
 static_assert(build_typed_tables().clashes == 0, "every name has its own slot");
+static_assert(alignof(TypedTables) >= sizeof(uint2) && offsetof(TypedTables, plain) % sizeof(uint2) == 0,
+              "entries on 8-byte boundaries, in global memory too");
 __device__ const TypedTables g_typed_tables = build_typed_tables();
 
 // Drop the space bytes of a name word (the reference erases whitespace from the
