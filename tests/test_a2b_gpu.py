@@ -909,3 +909,41 @@ def test_sincos_f64_error_bound(built):
         err = np.abs(got - ref) / ulp
         assert err[inside].max() <= 1.1, (float(err[inside].max()), float(x[inside][err[inside].argmax()]))
         assert err[~inside].max() <= 2.0
+
+
+def test_tuning_beside_a_thread_that_allocates(built):
+    """The autotuner's sweeps while another thread of the program allocates device memory and
+    gives it back: neither sees an error."""
+    import threading
+
+    from torchproteinlibrary_gb300 import autotune
+    dev = torch.device("cuda")
+    B, L = 64, 96
+    ang = torch.rand(B, 3, L, device=dev) * 6 - 3
+    lengths = torch.full((B,), L, dtype=torch.int32, device=dev)
+    up = torch.randn(B, 9 * L, device=dev)
+    stop, errors, rounds = threading.Event(), [], [0]
+
+    def allocate():
+        try:
+            while not stop.is_set():
+                torch.empty(48 << 20, dtype=torch.uint8, device=dev)
+                torch.cuda.empty_cache()
+                rounds[0] += 1
+        except RuntimeError as e:
+            errors.append(e)
+
+    t = threading.Thread(target=allocate)
+    t.start()
+    try:
+        while rounds[0] == 0 and not errors:
+            pass
+        for _ in range(10):
+            fwd = autotune.sweep(ang, lengths, up, candidates=((4, 32), (4, 4)), steps=5)
+            bwd = autotune.sweep_backward_coords(ang, lengths, up, candidates=((4, 1, 32),), steps=5)
+    finally:
+        stop.set()
+        t.join()
+    assert not errors and rounds[0] > 1
+    assert len(fwd) == 2 and len(bwd) == 1
+    assert all(0.0 < ms < 1.0 for ms in [r["fwd_ms"] for r in fwd] + [r["bwd_ms"] for r in fwd + bwd])

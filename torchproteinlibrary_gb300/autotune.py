@@ -65,23 +65,24 @@ def _save_cache(d: dict) -> None:
         pass
 
 
-def _replay_ms(device, fn, calls):
-    """Mean milliseconds of fn in a CUDA graph of `calls` of them.  Issued one by one, a small
-    shape's calls would be timed by the host (6 us each on GB300, more than the kernels)."""
-    for _ in range(2):
+def _queued_ms(device, fn, calls):
+    """Mean device milliseconds of fn.  The calls are queued behind 20 us a call of waiting
+    on the device: issued against an idle device a small shape's calls would be timed by the
+    host (6 us each on GB300, more than the kernels).  No graph: a capture would refuse other
+    threads' allocations while it lasts."""
+    total = 0.0
+    with torch.cuda.device(device):
         fn()
-    graph = torch.cuda.CUDAGraph()
-    with torch.cuda.device(device), torch.cuda.graph(graph):
-        for _ in range(calls):
-            fn()
-    graph.replay()
-    e = [torch.cuda.Event(enable_timing=True) for _ in range(2)]
-    e[0].record()
-    for _ in range(3):
-        graph.replay()
-    e[1].record()
-    torch.cuda.synchronize(device)
-    return e[0].elapsed_time(e[1]) / (3 * calls)
+        for _ in range(3):
+            e = [torch.cuda.Event(enable_timing=True) for _ in range(2)]
+            torch.cuda._sleep(40000 * calls)
+            e[0].record()
+            for _ in range(calls):
+                fn()
+            e[1].record()
+            e[1].synchronize()
+            total += e[0].elapsed_time(e[1])
+    return total / (3 * calls)
 
 
 def _time_options(rm, opts, ang, lengths, up, steps):
@@ -92,8 +93,8 @@ def _time_options(rm, opts, ang, lengths, up, steps):
     coords = torch.empty(B, 9 * L, device=ang.device)
     gang = torch.empty(B, 3, L, device=ang.device)
     none = torch.empty(0, device=ang.device)
-    f = _replay_ms(ang.device, lambda: rm.Angles2BackboneGPU_forward(ang, coords, lengths, ws), steps)
-    b = _replay_ms(ang.device, lambda: rm.Angles2BackboneGPU_backward(gang, up, ang, lengths, ws, none), steps)
+    f = _queued_ms(ang.device, lambda: rm.Angles2BackboneGPU_forward(ang, coords, lengths, ws), steps)
+    b = _queued_ms(ang.device, lambda: rm.Angles2BackboneGPU_backward(gang, up, ang, lengths, ws, none), steps)
     return f, b, coords, gang
 
 
@@ -149,7 +150,7 @@ def sweep_backward_coords(ang, lengths, up, candidates=COORDS_BWD_CANDIDATES, st
     try:
         for c, nb, sch in candidates:
             rm.set_backward_options(c, nb, sch)
-            ms = _replay_ms(ang.device,
+            ms = _queued_ms(ang.device,
                             lambda: rm.Angles2BackboneGPU_backward_coords(gang, up, coords, lengths, ws), steps)
             _, _, grel = _errors(rm, ang, lengths, up, coords, gang)
             out.append({"residues_per_thread": c, "copy_buffers": nb, "threads_per_cta": sch,
