@@ -88,6 +88,12 @@ int tpl_version(void);
  * `batch` chains stored with stride `max_len` (host). */
 size_t tpl_a2b_workspace_bytes(int batch, int max_len, const tpl_options *opt);
 
+/* 1 when the Angles2Backbone FP32 forward of this shape and these options splits chains
+ * into tiles, whose look-back words in the workspace must start from zero; 0 when it
+ * uses one warp or one CTA per chain, which keep only the status word and frames
+ * written before they are read there (host). */
+int tpl_a2b_workspace_zeroed(int batch, int max_len, const tpl_options *opt);
+
 /* Zero a workspace before its first use, or after an error (enqueued on stream). */
 int tpl_workspace_init(void *workspace, size_t workspace_bytes, void *stream);
 

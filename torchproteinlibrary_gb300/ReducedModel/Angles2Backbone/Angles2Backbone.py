@@ -63,9 +63,10 @@ def _shared_workspace(batch, max_len, device, fwd_opts, private=False):
     reuse by later calls (at most _WS_CACHE_SIZE of them).  A graph being captured
     gets one of its own; private: no caller can reach it to read its status word."""
     if torch.cuda.is_current_stream_capturing():
-        if private and fwd_opts[1] in (4, 32):
-            # one CTA or one warp per chain keeps no look-back words there that must start
-            # from zero: no memset in the graph (13 MB, 3 us, at 4096 x 1000)
+        if private and not _ReducedModel.workspace_zeroed(batch, max_len, *fwd_opts, device.index):
+            # one CTA or one warp per chain (named by the options or resolved to by the
+            # library's rule) keeps no look-back words there that must start from zero: no
+            # memset in the graph (13 MB, 3 us, at 4096 x 1000)
             return torch.empty(int(_ReducedModel.workspace_bytes(batch, max_len, *fwd_opts)), dtype=torch.uint8,
                                device=device)
         return new_workspace(batch, max_len, device, *fwd_opts)

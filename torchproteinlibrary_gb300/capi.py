@@ -27,6 +27,7 @@ _SIGNATURES = {
     "tpl_status_string": (ctypes.c_char_p, [_i]),
     "tpl_version": (_i, []),
     "tpl_a2b_workspace_bytes": (_sz, [_i, _i, _vp]),
+    "tpl_a2b_workspace_zeroed": (_i, [_i, _i, _vp]),
     "tpl_workspace_init": (_i, [_vp, _sz, _vp]),
     "tpl_workspace_status": (_i, [_vp, _vp, ctypes.POINTER(_i)]),
     "tpl_a2b_forward_f32": (_i, [_vp, _vp, _vp, _vp, _sz, _i, _i, _vp, _vp]),

@@ -204,6 +204,12 @@ int64_t workspace_bytes(int64_t B, int64_t L, int64_t residues_per_thread, int64
     return (int64_t)ws_bytes(B, L, call_options(residues_per_thread, threads_per_cta));
 }
 
+bool workspace_zeroed(int64_t B, int64_t L, int64_t residues_per_thread, int64_t threads_per_cta, int64_t device) {
+    const at::cuda::CUDAGuard guard((c10::DeviceIndex)device);
+    const tpl_options o = call_options(residues_per_thread, threads_per_cta);
+    return tpl_a2b_workspace_zeroed((int)B, (int)L, &o) != 0;
+}
+
 int64_t workspace_status(torch::Tensor A) {
     check_cuda(A, "A");
     const at::cuda::CUDAGuard guard(A.device());
@@ -247,6 +253,10 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
     m.def("Angles2BackboneCPU_backward", &no_cpu_path_bwd, "not available: no CPU path");
     m.def("workspace_bytes", &workspace_bytes, "bytes of the A workspace for (batch, max_len)", py::arg("batch"),
           py::arg("max_len"), py::arg("residues_per_thread") = -1, py::arg("threads_per_cta") = -1);
+    m.def("workspace_zeroed", &workspace_zeroed,
+          "whether the float32 forward of this shape and options needs a workspace that starts from zero",
+          py::arg("batch"), py::arg("max_len"), py::arg("residues_per_thread"), py::arg("threads_per_cta"),
+          py::arg("device"));
     m.def("workspace_status", &workspace_status, "synchronise and read the first device-detected error");
     m.def("set_options", &set_options, "tuning knobs", py::arg("residues_per_thread") = 0,
           py::arg("fp64_carry_min_len") = 0, py::arg("renormalize") = 0, py::arg("max_ctas") = 0,

@@ -1135,6 +1135,8 @@ static bool use_chain_scheme(const tpl_options &opt, int B, int L) {
     return !(B < 2 * num_sms() && L > 4096);
 }
 
+bool a2b_tiled(const tpl_options &opt, int B, int L) { return !use_chain_scheme(opt, B, L); }
+
 static tpl_options chain_options(const tpl_options &opt, int B, int L, bool forward) {
     tpl_options o = opt;
     if (o.threads_per_cta == 0) {

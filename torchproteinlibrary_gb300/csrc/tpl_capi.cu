@@ -182,6 +182,10 @@ size_t tpl_a2b_workspace_bytes(int batch, int max_len, const tpl_options *opt) {
     return a2b_ws(batch, max_len, resolve(opt));
 }
 
+int tpl_a2b_workspace_zeroed(int batch, int max_len, const tpl_options *opt) {
+    return a2b_tiled(resolve(opt), batch, max_len) ? 1 : 0;
+}
+
 int tpl_workspace_init(void *workspace, size_t workspace_bytes, void *stream) {
     if (!workspace || workspace_bytes < sizeof(WsHeader)) return TPL_ERR_WORKSPACE;
     cudaError_t e = cudaMemsetAsync(workspace, 0, workspace_bytes, (cudaStream_t)stream);

@@ -69,6 +69,7 @@ int a2b_forward_f64_plain(const double *angles, const int32_t *lengths, double *
 int a2b_backward_f64_plain(double *grad_angles, const double *grad_coords, const double *angles,
                            const int32_t *lengths, void *ws, int B, int L, cudaStream_t st);
 int a2b_tile_for(const tpl_options &opt);
+bool a2b_tiled(const tpl_options &opt, int B, int L);  // whether the FP32 entries split chains into tiles
 // One warp per chain (tpl_a2b_chain.cu; threads_per_cta = 32, residues_per_thread 4 or 8).
 // The forward records the chain frame every a2b_chain_record_stride() residues in
 // the workspace; the backward starts its chunks from those records.
