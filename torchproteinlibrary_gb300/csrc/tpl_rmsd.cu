@@ -11,7 +11,7 @@
 // layout as the reference), its largest eigenpair by the characteristic-polynomial
 // method on one warp (key_eigen_halves), U from the unit quaternion, UT = U^T and
 // rmsd = sqrt((R2 - 2 |lambda_max| + 1e-10) / N).  The backward is one launch with
-// one thread per group of atoms (chains on x, blocks of groups on y):
+// one thread per atom (chains on x, blocks of atoms on y):
 // dL/dx_i = g (x_i - UT y_i) / (rmsd N) on the centred coordinates.
 //
 // What bounds the float32 forward is the FP64 pipe: GB300 issues two FP64 lanes per
@@ -576,6 +576,10 @@ __global__ void __launch_bounds__(kRmsdThreads) rmsd_fwd_f64_kernel(RmsdArgs<dou
         for (int k = 0; k < 6; k++) a.centroids[6 * b + k] = s_c[k];
 }
 
+// One atom per thread: a block's life is two memory latencies, and small blocks of few
+// registers overlap them best.  (Groups of four atoms as 16-byte vectors, a thread each:
+// 20000 chains of 1000 atoms 210 -> 151 us, but 4096 of 2300 71 -> 81, of 200 8 -> 14, 256 of
+// 2300 5.4 -> 6.9, float64 4096 of 20 14 -> 24.)
 template <typename T>
 __global__ void __launch_bounds__(kRmsdThreads) rmsd_bwd_kernel(RmsdArgs<T> a) {
     const int b = blockIdx.x, tid = threadIdx.x;
@@ -597,38 +601,20 @@ __global__ void __launch_bounds__(kRmsdThreads) rmsd_bwd_kernel(RmsdArgs<T> a) {
     for (int k = 0; k < 6; k++) c[k] = s_c[k];
     for (int k = 0; k < 9; k++) U[k] = s_U[k];
     const T scale = s_scale;
-    // one group of N atoms per thread: chains on x, blocks of groups on y; group 0 is the
-    // row's unaligned head, and whole groups move as 16-byte vectors (tpl_rows.cuh)
-    constexpr int N = Vec16<T>::n;
-    const int head = row_head(x);
-    const bool vec = head == row_head(y) && head == row_head(gx);
-    const int i0 = head + N * ((int)(blockIdx.y * kRmsdThreads + tid) - 1);
-    auto atom = [&](const T *xa, const T *ya, T *g) {
-        const T xi[3] = {xa[0] - c[0], xa[1] - c[1], xa[2] - c[2]}, yi[3] = {ya[0] - c[3], ya[1] - c[4], ya[2] - c[5]};
-#pragma unroll
-        for (int k = 0; k < 3; k++)
-            g[k] = scale * (xi[k] - (U[3 * k] * yi[0] + U[3 * k + 1] * yi[1] + U[3 * k + 2] * yi[2]));
-    };
-    if (vec && i0 >= 0 && i0 + N <= a.atoms_stride) {
-        T g[3 * N];
-#pragma unroll
-        for (int k = 0; k < 3 * N; k++) g[k] = T(0);
-        if (i0 < n) {
-            T xv[3 * N], yv[3 * N];
-            load_group(x + 3 * i0, xv);
-            load_group(y + 3 * i0, yv);
-#pragma unroll
-            for (int q = 0; q < N; q++)
-                if (i0 + q < n) atom(xv + 3 * q, yv + 3 * q, g + 3 * q);
+    // one atom per thread: chains on x, blocks of atoms on y
+    const int i = blockIdx.y * kRmsdThreads + tid;
+    if (i < a.atoms_stride) {
+        if (i < n) {
+            T xi[3], yi[3];
+            for (int k = 0; k < 3; k++) {
+                xi[k] = x[3 * i + k] - c[k];
+                yi[k] = y[3 * i + k] - c[3 + k];
+            }
+            for (int k = 0; k < 3; k++)
+                gx[3 * i + k] = scale * (xi[k] - (U[3 * k] * yi[0] + U[3 * k + 1] * yi[1] + U[3 * k + 2] * yi[2]));
+        } else {
+            gx[3 * i] = gx[3 * i + 1] = gx[3 * i + 2] = T(0);
         }
-        store_group(gx + 3 * i0, g);
-        return;
-    }
-    for (int i = max(i0, 0); i < min(i0 + N, a.atoms_stride); i++) {
-        T g[3] = {T(0), T(0), T(0)};
-        if (i < n) atom(x + 3 * i, y + 3 * i, g);
-#pragma unroll
-        for (int k = 0; k < 3; k++) gx[3 * i + k] = g[k];
     }
 }
 
@@ -663,10 +649,8 @@ static int rmsd_bwd_launch(const T *grad_rmsd, const T *src, const T *dst, const
     if (B == 0) return TPL_OK;
     RmsdArgs<T> a{src, dst, num_atoms, stride, center, const_cast<T *>(rmsd), const_cast<T *>(ut),
                   const_cast<double *>(centroids), grad_rmsd, grad_src, nullptr};
-    if ((max(stride, 1) + kRmsdThreads - 1) / kRmsdThreads > 65535) return TPL_ERR_UNSUPPORTED;
-    constexpr int N = Vec16<T>::n;
-    const int groups = (max(stride, 1) + N - 1) / N + 1;  // the head and the aligned groups
-    const int ablocks = (groups + kRmsdThreads - 1) / kRmsdThreads;
+    const int ablocks = (max(stride, 1) + kRmsdThreads - 1) / kRmsdThreads;
+    if (ablocks > 65535) return TPL_ERR_UNSUPPORTED;
     rmsd_bwd_kernel<T><<<dim3((unsigned)B, (unsigned)ablocks), kRmsdThreads, 0, st>>>(a);
     return cudaGetLastError() == cudaSuccess ? TPL_OK : TPL_ERR_LAUNCH;
 }
