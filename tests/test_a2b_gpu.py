@@ -947,3 +947,39 @@ def test_tuning_beside_a_thread_that_allocates(built):
     assert not errors and rounds[0] > 1
     assert len(fwd) == 2 and len(bwd) == 1
     assert all(0.0 < ms < 1.0 for ms in [r["fwd_ms"] for r in fwd] + [r["bwd_ms"] for r in fwd + bwd])
+
+
+@pytest.mark.parametrize("B,L,off", [(900, 640, 1), (40, 1000, 2), (2048, 200, 3), (64, 999, 0)])
+def test_rows_off_16_byte_boundaries_take_four_residues_a_lane(rm, B, L, off):
+    """Rows that start off a 16-byte boundary, by their length or as a view into an allocation,
+    take four residues per lane in the forward whatever the table holds for the bucket or
+    the built-in rule for an aligned row of the length: the layer and the extension's
+    automatic choice equal that choice made explicitly, bit for bit, and the same options
+    on an aligned copy.  A copy of the view takes the aligned rows' options again."""
+    from torchproteinlibrary_gb300 import autotune
+    from torchproteinlibrary_gb300.ReducedModel import Angles2Backbone
+    g = torch.Generator("cuda").manual_seed(L)
+    buf = (torch.rand(B * 3 * L + 4, device="cuda", generator=g) * 2 - 1) * 3.1
+    view = buf[off:off + B * 3 * L].view(B, 3, L)
+    lens = torch.randint(1, L + 1, (B,), device="cuda", generator=g, dtype=torch.int32)
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    automatic = 4 if L >= 384 or B < 8 * sms else 32
+
+    def forward(a, rpt, cta):
+        ws = torch.zeros(rm.workspace_bytes(B, L, rpt, cta), dtype=torch.uint8, device="cuda")
+        c = torch.empty(B, 9 * L, device="cuda")
+        rm.Angles2BackboneGPU_forward(a, c, lens, ws, rpt, cta)
+        return c
+
+    want = forward(view, 4, automatic)
+    assert torch.equal(forward(view, 0, 0), want)
+    if off:
+        assert torch.equal(forward(view.clone(), 4, automatic), want)
+    tuned = autotune.options_for(view.device, B, L, False)
+    if tuned is not None:
+        (rpt, cta), _ = tuned
+        assert rpt == 4 and cta in (4, 32)
+        assert torch.equal(Angles2Backbone()(view, lens), forward(view, rpt, cta))
+        if off:
+            (rpt, cta), _ = autotune.options_for(view.device, B, L)
+            assert torch.equal(Angles2Backbone()(view.clone(), lens), forward(view.clone(), rpt, cta))

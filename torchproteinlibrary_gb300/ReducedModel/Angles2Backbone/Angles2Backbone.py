@@ -96,7 +96,8 @@ class Angles2BackboneGPUFunction(Function):
         dev = input_angles.device
         coords = torch.empty(batch_size, 9 * max_len, dtype=input_angles.dtype, device=dev)
         f32 = input_angles.dtype == torch.float32
-        tuned = autotune.options_for(dev, batch_size, max_len) if f32 and dev.type == "cuda" else None
+        tuned = (autotune.options_for(dev, batch_size, max_len, input_angles.data_ptr() % 16 == 0)
+                 if f32 and dev.type == "cuda" else None)
         fwd_opts, bwd_opts = tuned if tuned is not None else ((-1, -1), (-1, -1, -1))
         ctx.from_coords = Angles2BackboneGPUFunction.backward_from_coords and f32
         if ctx.from_coords:
@@ -155,7 +156,9 @@ class Angles2Backbone(Module):
         # frame in the backward
         batch_size, _, max_len = input.shape
         dev = input.device
-        tuned = autotune.options_for(dev, batch_size, max_len)
+        # (angles that are not contiguous are copied to an allocation of their own)
+        tuned = autotune.options_for(dev, batch_size, max_len,
+                                     not input.is_contiguous() or input.data_ptr() % 16 == 0)
         fwd_opts, bwd_opts = tuned if tuned is not None else ((-1, -1), (-1, -1, -1))
         ws = _shared_workspace(batch_size, max_len, dev, fwd_opts, private=True)
         return _ReducedModel.angles2backbone_autograd(input, angles_length, ws, list(fwd_opts), list(bwd_opts))

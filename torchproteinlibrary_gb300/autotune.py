@@ -216,12 +216,14 @@ def _entry_options(entry: dict):
             (int(bc["residues_per_thread"]), int(bc.get("copy_buffers", 0)), int(bc.get("threads_per_cta", 0))))
 
 
-def options_for(device, batch: int, max_len: int):
+def options_for(device, batch: int, max_len: int, aligned: bool = True):
     """((residues_per_thread, threads_per_cta) of the forward, (residues_per_thread,
     copy_buffers, threads_per_cta) of the backward from coordinates) tuned for this
     shape's bucket on this GPU, or None (the library's built-in rule then applies).
-    Looked up once per (device, batch, max_len) in the process."""
-    key = (device.index, int(batch), int(max_len))
+    aligned: whether the angles start on a 16-byte boundary.  Looked up once per
+    arguments in the process."""
+    aligned = bool(aligned) and max_len % 4 == 0  # every row does
+    key = (device.index, int(batch), int(max_len), aligned)
     hit = _LOOKUP.get(key, False)
     if hit is not False:
         return hit
@@ -233,10 +235,11 @@ def options_for(device, batch: int, max_len: int):
     if entry and "backward_coords" in entry:
         try:
             res = _entry_options(entry)
-            if not own and max_len % 4:
-                # the table is tuned on rows of whole 16-byte blocks; others take the built-in
-                # forward (1024 x 999: 15.2 us, with the bucket's eight residues per lane 16.8)
-                res = ((0, 0), res[1])
+            if not own and not aligned and res[0][1] in (4, 32):
+                # the table is tuned on rows that start on 16-byte boundaries; on others only
+                # chunks of four residues a lane leave as bulk copies (forward, with the
+                # bucket's eight: 1024 x 999 15.2 / 16.8 us, 8000 x 200 24.0 / 29.3)
+                res = ((4, res[0][1]), res[1])
         except (KeyError, TypeError, ValueError):
             res = None
     _LOOKUP[key] = res

@@ -1119,9 +1119,10 @@ static int num_sms() { return device_sm_count(); }
 //   * else one warp per chain, with eight residues per lane where a chunk of 256 holds the
 //     chain but one of 128 does not (4096 chains of 256: four / eight residues 14.3 / 13.4, of
 //     128 9.1 / 12.6, of 320 18.7 / 20.7);
-//   * rows off 16-byte boundaries (max_len no multiple of four): always four residues per
-//     lane, whose chunks leave as bulk copies whatever the row's phase (four / eight, four
-//     warps per chain: 1024 chains of 999 15.2 / 16.8, 2048 of 517 18.6 / 21.9);
+//   * rows off 16-byte boundaries (max_len no multiple of four, or angles or coordinates that
+//     start off one): always four residues per lane, whose chunks leave as bulk copies
+//     whatever the row's phase (four / eight, four warps per chain: 1024 chains of 999 15.2 /
+//     16.8, 2048 of 517 18.6 / 21.9; 900 of 640 a word into an allocation 9.3 / 12.9);
 //   * fewer than two chains per SM and chains over 4096 residues: warp tiles, whose
 //     look-back spreads one chain over many warps.
 // An explicit residues_per_thread of 4 or 8 is kept; 1 or 2 selects warp tiles.
@@ -1137,16 +1138,16 @@ static bool use_chain_scheme(const tpl_options &opt, int B, int L) {
 
 bool a2b_tiled(const tpl_options &opt, int B, int L) { return !use_chain_scheme(opt, B, L); }
 
-static tpl_options chain_options(const tpl_options &opt, int B, int L, bool forward) {
+static tpl_options chain_options(const tpl_options &opt, int B, int L, bool forward, bool aligned) {
     tpl_options o = opt;
     if (o.threads_per_cta == 0) {
         const bool ring = L >= 384 || B < 8 * num_sms();
         o.threads_per_cta = ring ? 4 : 32;
         if (o.residues_per_thread == 0) {
-            const bool eight = !forward     ? L >= 768
-                               : L % 4 != 0 ? false
-                               : ring       ? L >= 768 || (L > 512 && B < 6 * num_sms())
-                                            : L > 128 && L <= 256;
+            const bool eight = !forward   ? L >= 768
+                               : !aligned ? false
+                               : ring     ? L >= 768 || (L > 512 && B < 6 * num_sms())
+                                          : L > 128 && L <= 256;
             o.residues_per_thread = eight ? 8 : 4;
         }
     }
@@ -1221,8 +1222,9 @@ static int launch_bwd(A2bArgs &a, int max_ctas, cudaStream_t st) {
 int a2b_forward_f32(const float *angles, const int32_t *lengths, float *coords, void *ws, int B, int L,
                     const tpl_options &opt, cudaStream_t st) {
     if (B == 0 || L == 0) return TPL_OK;
+    const bool aligned = a2b_rows_aligned(angles, coords, L);
     if (use_chain_scheme(opt, B, L))
-        return a2b_forward_chain(angles, lengths, coords, ws, B, L, chain_options(opt, B, L, true), st);
+        return a2b_forward_chain(angles, lengths, coords, ws, B, L, chain_options(opt, B, L, true, aligned), st);
     A2bShape s = a2b_shape(opt, false);
     A2bArgs a = make_args(angles, lengths, ws, B, L, s.R * s.NT, opt);
     a.coords = coords;
@@ -1248,8 +1250,8 @@ int a2b_backward_f32(float *grad_angles, const float *grad_coords, const float *
                      void *ws, int B, int L, const tpl_options &opt, cudaStream_t st) {
     if (B == 0 || L == 0) return TPL_OK;
     if (use_chain_scheme(opt, B, L))
-        return a2b_backward_chain(grad_angles, grad_coords, angles, lengths, ws, B, L, chain_options(opt, B, L, false),
-                                  st);
+        return a2b_backward_chain(grad_angles, grad_coords, angles, lengths, ws, B, L,
+                                  chain_options(opt, B, L, false, false), st);
     A2bShape s = a2b_shape(opt, true);
     A2bArgs a = make_args(angles, lengths, ws, B, L, s.R * s.NT, opt);
     a.grad_angles = grad_angles;

@@ -1449,12 +1449,16 @@ int launch_ring(K kernel, int smem, int B, const ChainArgs &a, cudaStream_t st) 
 
 int a2b_chain_record_stride() { return kRecordStride; }
 
+bool a2b_rows_aligned(const float *angles, const float *coords, int L) {
+    return L % 4 == 0 && aligned16(angles) && aligned16(coords);
+}
+
 int a2b_forward_chain(const float *angles, const int32_t *lengths, float *coords, void *ws, int B, int L,
                       const tpl_options &opt, cudaStream_t st) {
     if (B == 0 || L == 0) return TPL_OK;
     ChainArgs a = chain_args(angles, lengths, ws, B, L, opt);
     a.coords = coords;
-    a.vec = (L % 4 == 0) && aligned16(angles) && aligned16(coords);
+    a.vec = a2b_rows_aligned(angles, coords, L);
     const int C = opt.residues_per_thread > 0 ? opt.residues_per_thread : 8;
     const bool ring = opt.threads_per_cta == kRingWarps;
     const int carry_bytes = a.fp64_min > 0 ? kRingWarps * 12 * (int)sizeof(double) : 0;  // FP64 carry slots

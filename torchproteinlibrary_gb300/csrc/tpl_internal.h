@@ -78,6 +78,9 @@ int a2b_forward_chain(const float *angles, const int32_t *lengths, float *coords
 int a2b_backward_chain(float *grad_angles, const float *grad_coords, const float *angles, const int32_t *lengths,
                        void *ws, int B, int L, const tpl_options &opt, cudaStream_t st);
 int a2b_chain_record_stride();
+// Whether every row of angles and of coordinates starts on a 16-byte boundary: what the
+// choice of residues per lane and the forward's kernels go by.
+bool a2b_rows_aligned(const float *angles, const float *coords, int L);
 // Backward from the forward's output coordinates (no re-walk; tpl_a2b_chain.cu).
 int a2b_backward_coords(float *grad_angles, const float *grad_coords, const float *coords, const int32_t *lengths,
                         void *ws, int B, int L, const tpl_options &opt, cudaStream_t st);
