@@ -200,3 +200,30 @@ def test_two_chains_per_cta(built, half):
     ok = na > 1
     assert np.abs(r.double().cpu().numpy() - ref)[ok].max() <= 1e-4 * ref[ok].max()
     assert r[torch.tensor(na == 0)].eq(0).all()
+
+
+@pytest.mark.parametrize("B", [20, 400, 700])
+def test_sampled_atoms_that_are_outliers(built, B):
+    """The float32 forward takes its sums from a centre found on 16 atoms spread over the
+    chain: coils of 2300 atoms that have those 16 moved 300 A away, as the only ones, in every
+    block size of the forward, next to ordinary chains.  The float32 tolerances of this file
+    (rmsd 1e-4 relative, gradients 1e-3 of the largest)."""
+    from torchproteinlibrary_gb300.RMSD import Coords2RMSD
+    rng = np.random.default_rng(23)
+    K, N = 20, 2300
+    pick = [N * (2 * i + 1) // 32 for i in range(16)]
+    src = np.cumsum(rng.standard_normal((K, N, 3)), 1) * 0.7
+    src -= src.mean(1, keepdims=True)
+    src[::2, pick] += rng.permuted(np.tile([300.0, 0.0, 0.0], (K // 2, 1, 1)), axis=2)
+    dst = np.stack([s @ random_rotation(rng).T for s in src]) + rng.standard_normal(src.shape) * 1.2
+    src, dst = (v.reshape(K, -1).astype(np.float32) for v in (src, dst))
+    na = np.full(K, N, np.int32)
+    ref, _, gref = oracle.rmsd(src.astype(np.float64), dst.astype(np.float64), na)
+    x = torch.tensor(src, device="cuda").repeat(B // K, 1).requires_grad_()
+    y = torch.tensor(dst, device="cuda").repeat(B // K, 1)
+    r = Coords2RMSD()(x, y, torch.tensor(na).repeat(B // K))
+    g, = torch.autograd.grad(r.sum(), x)
+    err = np.abs(r.detach().double().cpu().numpy().reshape(-1, K) / ref - 1.0).max()
+    assert err <= 1e-4, err
+    ge = np.abs(g.double().cpu().numpy().reshape(-1, K, 3 * N) - gref).max() / np.abs(gref).max()
+    assert ge <= 1e-3, ge

@@ -355,12 +355,40 @@ __device__ __forceinline__ int checked_atoms(const RmsdArgs<T> &a, int b, bool r
 
 constexpr int kRmsdSums = 16;  // R (row-major), R2, sum x, sum y
 
+// Value k of the 16 sums of a chain of n atoms again, from the centres c: one lane a value,
+// four atoms in FP32 at a time.  Rare, and so out of the way of the kernel's registers.
+__device__ __forceinline__ double sum_again(const float *x, const float *y, int n, const float *c, int k) {
+    // what the value is a sum of: components p and r (3..5: y) multiplied, or p alone
+    const int p = k < 9 ? k / 3 : k - 10, r = k < 9 ? 3 + k % 3 : -1;
+    auto at = [&](int i, int q) { return (q < 3 ? x[3 * i + q] : y[3 * i + q - 3]) - c[q]; };
+    double d = 0.0;
+#pragma unroll 1
+    for (int i0 = 0; i0 < n; i0 += 4) {
+        float s = 0.f;
+#pragma unroll 1
+        for (int i = i0; i < min(i0 + 4, n); i++) {
+            if (k == 9) {
+#pragma unroll 1
+                for (int q = 0; q < 6; q++) s = fmaf(at(i, q), at(i, q), s);
+            } else {
+                s = fmaf(at(i, p), r < 0 ? 1.f : at(i, r), s);
+            }
+        }
+        d += (double)s;
+    }
+    return d;
+}
+
 // float32 forward: one pass over the chain.  Both sets are taken relative to a
 // provisional centre, the mean of 16 atoms spread over the chain, and the sums are
 // moved to the true centroids afterwards in FP64 (R - n cx cy^T and so on): the
-// provisional centre is off by about a quarter of the radius of gyration, so the
-// sums keep the size, and the rounding, of centred ones, and the second read of every
-// coordinate goes.  Atoms are read as float4 groups (tpl_rows.cuh) where both rows
+// provisional centre is off by a quarter of the radius of gyration where the 16 atoms are
+// drawn like the others (a twentieth along a coil), so the sums keep the size, and the
+// rounding, of centred ones, and the second read of every coordinate goes.  Where they are
+// not, and the shift makes up more than a third of sum |x|^2 + |y|^2 (of independent points
+// one chain in 1e8), the sums are taken again from the centroids found (sum_again; a coil of
+// 2300 atoms whose sampled ones are 300 A off: 8e-4 relative without, 7e-6 with).  Atoms are
+// read as float4 groups (tpl_rows.cuh) where both rows
 // have the same alignment.
 //
 // NC = 1 or 2 chains per CTA, NT threads each; the first warp then solves for both, one per
@@ -495,14 +523,24 @@ __global__ void __launch_bounds__(NT * NC) rmsd_fwd_f32_kernel(RmsdArgs<float> a
             rn = (double)(1.f / (float)nh);
             rn = fma(rn, fma(-(double)nh, rn, 1.0), rn);
         }
-        const double m = d * rn;  // lanes 10 .. 15: the centroids from the provisional centres
-        if (k >= 10 && writes && a.centroids) a.centroids[6 * bh + k - 10] = (double)s_c[h][k - 10] + m;
-        const double sx = __shfl_sync(0xffffffffu, d, 10 + (k < 9 ? k / 3 : 0), 16);
-        const double my = __shfl_sync(0xffffffffu, m, 13 + (k < 9 ? k % 3 : 0), 16);
-        double sq = k >= 10 ? d * m : 0.0;
+#pragma unroll 1
+        for (bool first = true;; first = false) {
+            const double m = d * rn;  // lanes 10 .. 15: the centroids from the provisional centres
+            if (k >= 10 && writes && a.centroids) a.centroids[6 * bh + k - 10] = (double)s_c[h][k - 10] + m;
+            const double sx = __shfl_sync(0xffffffffu, d, 10 + (k < 9 ? k / 3 : 0), 16);
+            const double my = __shfl_sync(0xffffffffu, m, 13 + (k < 9 ? k % 3 : 0), 16);
+            double sq = k >= 10 ? d * m : 0.0;
 #pragma unroll
-        for (int off = 8; off > 0; off >>= 1) sq += __shfl_xor_sync(0xffffffffu, sq, off);
-        d -= k < 9 ? sx * my : sq;
+            for (int off = 8; off > 0; off >>= 1) sq += __shfl_xor_sync(0xffffffffu, sq, off);
+            if (!first || !__any_sync(0xffffffffu, k == 9 && 3.0 * sq > d)) {
+                d -= k < 9 ? sx * my : sq;
+                break;
+            }
+            if (k >= 10 && writes) s_c[h][k - 10] = (float)((double)s_c[h][k - 10] + m);
+            __syncwarp();
+            const size_t row = (size_t)min(bh, nb - 1) * 3 * a.atoms_stride;
+            d = sum_again(a.src + row, a.dst + row, nh, s_c[h], k);
+        }
     } else if (k < 6 && writes && a.centroids) {
         a.centroids[6 * bh + k] = 0.0;
     }
