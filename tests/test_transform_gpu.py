@@ -154,3 +154,54 @@ def test_rows_at_every_alignment(ct, dtype, S, offs):
     a, b = ct.getBBox(xt, nat)
     ra, rb = oracle.coords_bbox(x, na)
     assert np.array_equal(a.cpu().numpy(), ra) and np.array_equal(b.cpu().numpy(), rb)
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float64])
+@pytest.mark.parametrize("S,offs", [(299, (0, 0)), (301, (1, 1)), (1499, (0, 0)), (1500, (2, 2)), (1501, (0, 0)),
+                                    (1502, (3, 3)), (1503, (0, 1)), (12001, (0, 0))])
+def test_large_batches(ct, dtype, S, offs):
+    """Batches large enough for what small ones do not take: shifts as vectors between the
+    boundaries of rows that start anywhere, rotations in tiles (float32), reductions by 128
+    threads; rows on both sides of each line and at every 16-byte phase, input and output in
+    different phases, counts from none to 9 atoms and full rows.  Translate, the two shift
+    backwards and the box bit for bit; rotate and centre to the tolerances of the file."""
+    from torchproteinlibrary_gb300 import load_extension
+    fm = load_extension("_FullAtomModel")
+    K, B = 17, 3400 if S < 12000 else 700
+    x, na, T, R = case(dtype, B=K, S=S, seed=S)
+    na[:] = np.minimum(np.arange(K) - 1, S)
+    na[0], na[11:] = S, [S, S - 1, S - 2, S - 3, S - 5, S // 2]
+    dev, scale = torch.device("cuda"), np.abs(x).max()
+    rows = torch.arange(B, device=dev) % K
+
+    def at(v, off):
+        v = torch.tensor(np.asarray(v), device=dev)
+        t = torch.empty(B * v[0].numel() + off, dtype=dtype, device=dev)[off:].view(B, *v.shape[1:])
+        return t.copy_(v[rows])
+
+    def same(got, want):
+        return torch.equal(got, torch.tensor(want, device=dev)[rows])
+
+    def error(got, want):
+        return (got - torch.tensor(want, device=dev)[rows]).abs().max().item()
+
+    xt, nat, Tt, Rt = at(x, offs[0]), torch.tensor(na, device=dev)[rows].contiguous(), at(T, 0), at(R, 0)
+    out = at(np.full_like(x, 7.0), offs[1])
+    fm.CoordsTranslateGPU_forward(xt, out, Tt, nat)
+    assert same(out, oracle.coords_translate(x, T, na))
+    fm.CoordsTranslateGPU_backward(xt, out, Tt, nat)
+    assert same(out, oracle.coords_translate(x, None, na))
+    tol = 2e-6 if dtype == torch.float32 else 1e-12
+    for call, transpose in ((fm.CoordsRotateGPU_forward, False), (fm.CoordsRotateGPU_backward, True)):
+        out.fill_(7.0)
+        call(xt, out, Rt, nat)
+        assert error(out, oracle.coords_rotate(x, R, na, transpose=transpose)) <= tol * scale
+        assert not out[1].any()
+    c = ct.Coords2Center()(xt, nat)
+    assert error(c, oracle.coords_center(x, na)) <= (1e-6 if dtype == torch.float32 else 1e-12) * scale
+    fm.Coords2CenterGPU_backward(Tt, out, nat)
+    want = torch.tensor(oracle.coords_center_backward(T, na, S), device=dev)[rows]
+    assert torch.allclose(out, want, rtol=1e-6 if dtype == torch.float32 else 1e-14, atol=0)
+    lo, hi = ct.getBBox(xt, nat)
+    rlo, rhi = oracle.coords_bbox(x, na)
+    assert same(lo, rlo) and same(hi, rhi)

@@ -12,14 +12,15 @@
 // centroid and box are block reductions, one CTA per chain.
 //
 // A row starts at any place of a 16-byte block (3 * atoms_stride is a multiple of four
-// for one stride in four), so every kernel takes the few elements or atoms before the
-// row's first boundary and after its last one by themselves and moves the rest as
-// vectors.  Scalar passes over such rows had been issue-bound: 4096 rows of 1000..3471
-// atoms, stride 3471 (41 us of HBM traffic each): translate 70 -> 39 us, rotate 54 -> 46 us,
-// box 26 -> 21 us.
+// for one stride in four), so kernels that have enough to move take the few elements or
+// atoms before the row's first boundary and after its last one by themselves and move the
+// rest as vectors.  Scalar passes over such rows had been issue-bound: 4096 rows of
+// 1000..3471 atoms, stride 3471 (41 us of HBM traffic each): translate 70 -> 39 us, rotate 54
+// -> 46 us, box 26 -> 21 us.
 #include <cfloat>
 #include <cmath>
 #include <cstring>
+#include <type_traits>
 
 #include "tpl_internal.h"
 #include "tpl_rows.cuh"
@@ -46,8 +47,10 @@ __device__ __forceinline__ void store16(T *p, const T (&v)[Vec16<T>::n]) {
 // for e < 3 n_b, 0 after.  Covers translate (add = T), its backward (add = null),
 // and the centre's backward (in = null, add = dL/dcentre, scaled by 1 / n_b).
 // Grid: y over rows (strided), x over pieces of a row, so no thread divides by the
-// row length.  Between the row's first and last 16-byte boundary elements move as
-// vectors when `in` and `out` have the same alignment; the others one by one.
+// row length; VEC: 16-byte vectors inside a row (rows that start on a 16-byte boundary and
+// hold whole vectors), else element by element.  In float64 SCALE says whether there is
+// anything to scale: a translation that shares the code computes the division too (GB300, 4096
+// rows of 4000 atoms: 284 -> 98 us).
 struct ShiftArgs {
     const void *in;
     void *out;
@@ -58,8 +61,60 @@ struct ShiftArgs {
     int scale_by_count;
 };
 
-template <typename T>
+template <typename T, bool VEC, bool SCALE>
 __global__ void __launch_bounds__(256) shift_kernel(ShiftArgs a) {
+    constexpr int N = VEC ? Vec16<T>::n : 1;
+    const T *in = static_cast<const T *>(a.in);
+    T *out = static_cast<T *>(a.out);
+    const T *add = static_cast<const T *>(a.add);
+    const int nv = a.row / N;  // vectors per row
+    for (int b = blockIdx.y; b < a.B; b += gridDim.y) {
+        const int n = max(0, min(a.num_atoms[b], a.row / 3)), n3 = 3 * n;
+        T t[3] = {T(0), T(0), T(0)};
+        if (add)
+            for (int k = 0; k < 3; k++) {
+                t[k] = add[3 * (size_t)b + k];
+                if ((sizeof(T) == 8 ? SCALE : a.scale_by_count != 0) && n > 0) t[k] = t[k] / T(n);
+            }
+        const size_t base = (size_t)b * a.row;
+        // kUnroll independent vectors per thread and step: loads issued before use
+        const int step = gridDim.x * blockDim.x;
+        for (int v0 = blockIdx.x * blockDim.x + threadIdx.x; v0 < nv; v0 += kUnroll * step) {
+            T x[kUnroll][Vec16<T>::n];
+#pragma unroll
+            for (int u = 0; u < kUnroll; u++) {
+                const int v = v0 + u * step;
+                if (v >= nv) continue;
+                if (VEC) {
+                    if (in && v * N < n3) load16(in + base + (size_t)v * N, x[u]);
+                    else
+                        for (int k = 0; k < N; k++) x[u][k] = T(0);
+                } else {
+                    x[u][0] = in && v < n3 ? __ldcs(in + base + v) : T(0);
+                }
+            }
+#pragma unroll
+            for (int u = 0; u < kUnroll; u++) {
+                const int v = v0 + u * step;
+                if (v >= nv) continue;
+#pragma unroll
+                for (int k = 0; k < N; k++) {
+                    const int e = v * N + k;
+                    x[u][k] = e < n3 ? x[u][k] + t[e % 3] : T(0);
+                }
+                if (VEC) store16(out + base + (size_t)v * N, x[u]);
+                else __stcs(out + base + v, x[u][0]);
+            }
+        }
+    }
+}
+
+// Eight blocks per SM in float32: short rows leave most of a block idle (16000 rows of 20
+// atoms, 38 registers: 17 -> 20 us).
+// The same for rows that start anywhere: vectors between the row's first and last 16-byte
+// boundary where `in` and `out` have the same phase, the elements outside them by themselves.
+template <typename T, bool SCALE>
+__global__ void __launch_bounds__(256, sizeof(T) == 4 ? 8 : 6) shift_rows_kernel(ShiftArgs a) {
     constexpr int N = Vec16<T>::n;
     const T *add = static_cast<const T *>(a.add);
     const int step = gridDim.x * blockDim.x, first = blockIdx.x * blockDim.x + threadIdx.x;
@@ -71,7 +126,7 @@ __global__ void __launch_bounds__(256) shift_kernel(ShiftArgs a) {
         if (add)
             for (int k = 0; k < 3; k++) {
                 t[k] = add[3 * (size_t)b + k];
-                if (a.scale_by_count && n > 0) t[k] = t[k] / T(n);
+                if (SCALE && n > 0) t[k] = t[k] / T(n);
             }
         auto pick = [&](int r) { return r == 0 ? t[0] : (r == 1 ? t[1] : t[2]); };
         const int off = row_head(out);  // elements of `out` since a 16-byte boundary
@@ -83,7 +138,8 @@ __global__ void __launch_bounds__(256) shift_kernel(ShiftArgs a) {
 #pragma unroll
             for (int u = 0; u < kUnroll; u++) {
                 const int v = v0 + u * step, e = head + v * N;
-                if (in && v < nv && e < n3) load16(in + e, x[u]);
+                if (v >= nv) continue;
+                if (in && e < n3) load16(in + e, x[u]);
                 else
                     for (int k = 0; k < N; k++) x[u][k] = T(0);
             }
@@ -91,10 +147,9 @@ __global__ void __launch_bounds__(256) shift_kernel(ShiftArgs a) {
             for (int u = 0; u < kUnroll; u++) {
                 const int v = v0 + u * step;
                 if (v >= nv) continue;
-                const int e = head + v * N, r = e % 3;
-                const T te[3] = {pick(r), pick(r == 2 ? 0 : r + 1), pick(r == 0 ? 2 : r - 1)};
+                const int e = head + v * N;
 #pragma unroll
-                for (int k = 0; k < N; k++) x[u][k] = e + k < n3 ? x[u][k] + te[k % 3] : T(0);
+                for (int k = 0; k < N; k++) x[u][k] = e + k < n3 ? x[u][k] + t[(e + k) % 3] : T(0);
                 store16(out + e, x[u]);
             }
         }
@@ -117,6 +172,49 @@ __global__ void __launch_bounds__(256) shift_kernel(ShiftArgs a) {
 }
 
 // out[b, atom] = R_b x (or R_b^T x) for atom < n_b, 0 after; R row-major [B, 3, 3].
+// Grid: y over rows (strided), x over atoms of a row.
+template <typename T>
+__global__ void __launch_bounds__(256) rotate_kernel(const T *in, T *out, const T *R, const int *num_atoms, int B,
+                                                     int stride, int transpose) {
+    for (int b = blockIdx.y; b < B; b += gridDim.y) {
+        const int n = num_atoms[b];
+        T m[9];
+        for (int k = 0; k < 9; k++) m[k] = R[9 * (size_t)b + (transpose ? 3 * (k % 3) + k / 3 : k)];
+        const T *x = in + (size_t)b * 3 * stride;
+        T *y = out + (size_t)b * 3 * stride;
+        const int step = gridDim.x * blockDim.x;
+        for (int i0 = blockIdx.x * blockDim.x + threadIdx.x; i0 < stride; i0 += kUnroll * step) {
+            T v[kUnroll][3];
+#pragma unroll
+            for (int u = 0; u < kUnroll; u++) {  // loads of kUnroll atoms in flight
+                const int i = i0 + u * step;
+                if (i < min(n, stride))
+                    for (int k = 0; k < 3; k++) v[u][k] = __ldcs(x + 3 * i + k);
+            }
+#pragma unroll
+            for (int u = 0; u < kUnroll; u++) {
+                const int i = i0 + u * step;
+                if (i >= stride) continue;
+                T r0 = T(0), r1 = T(0), r2 = T(0);
+                if (i < n) {
+                    const T x0 = v[u][0], x1 = v[u][1], x2 = v[u][2];
+                    r0 = m[0] * x0 + m[1] * x1 + m[2] * x2;
+                    r1 = m[3] * x0 + m[4] * x1 + m[5] * x2;
+                    r2 = m[6] * x0 + m[7] * x1 + m[8] * x2;
+                }
+                __stcs(y + 3 * i, r0);
+                __stcs(y + 3 * i + 1, r1);
+                __stcs(y + 3 * i + 2, r2);
+            }
+        }
+    }
+}
+
+// The same for float32 batches that pass through more memory than L2 holds (129 MB), on rows
+// of three quarters of a block's atoms at least: there the partial sectors cost, and the
+// tiles' latency does not (one atom per thread / tiles, us: 4096 rows of 3471 atoms 56.9 / 52.7,
+// ragged 51.2 / 44.2; 1000 rows, 83 MB, 12.0 / 12.7; 16000 of 1001 62.7 / 67.5; float64, bound by
+// its arithmetic, 4096 of 3471 226 / 236).
 // Grid: y over rows (strided), x over pieces of 512 aligned groups of N atoms
 // (tpl_rows.cuh), two tiles of 32 groups per warp whose loads are in flight together (one
 // tile: 54 us; the launch is then bound by the latency of its many short blocks).  A warp loads and stores its tile as 96 vectors in
@@ -125,9 +223,9 @@ __global__ void __launch_bounds__(256) shift_kernel(ShiftArgs a) {
 // (strides of 48 bytes), with an atom per lane in three.  48-byte lane strides are free of
 // bank conflicts.  Atoms outside the groups, and rows whose input and output differ in
 // alignment, are taken one by one.
-template <typename T>
-__global__ void __launch_bounds__(256) rotate_kernel(const T *in, T *out, const T *R, const int *num_atoms, int B,
-                                                     int stride, int transpose) {
+__global__ void __launch_bounds__(256) rotate_tiles_kernel(const float *in, float *out, const float *R,
+                                                           const int *num_atoms, int B, int stride, int transpose) {
+    using T = float;
     constexpr int N = Vec16<T>::n;
     using V = typename Vec16<T>::type;
     __shared__ V s_tile[8][96];
@@ -199,33 +297,56 @@ __global__ void __launch_bounds__(256) rotate_kernel(const T *in, T *out, const 
     }
 }
 
-// Threads per chain of the two reductions: a thread's loads are what is waited for, and more
-// small CTAs keep more of them in flight (4096 rows of 1157..3471 atoms, 256 / 128 threads:
-// centre 24.7 / 22.1 us, box 22.4 / 21.1; a launch of 4000 atoms each 35.3 / 33.9 and 33.1 / 32.4).
-constexpr int kReduceThreads = 128;
+// Threads per chain NT of the two reductions: a thread's loads are what is waited for.  Where
+// the batch fills the GPU more small CTAs keep more of them in flight, 128 threads each; a
+// smaller batch waits for its longest chain, and long rows for themselves: 256.  256 / 128
+// threads, us: float32 4096 rows of 1157..3471 atoms centre 24.7 / 22.1, box 22.4 / 21.1; 450 of
+// 20001 15.4 / 26.9, 19.3 / 29.1; 800 of 20001 centre 27.0 / 30.7.  In float64 the reduction's
+// own additions weigh more: box of 150 rows of 20001 45 / 66, of 300 84 / 90, of 450 121 / 118,
+// of 300 of 4000 22.6 / 20.7; centre of 150 of 20001 40.4 / 44.6, of 600 6.2 / 5.4.
+template <typename T>
+static bool wide_reduction(int B, int stride, bool box) {
+    const int sms = device_sm_count();
+    const bool lng = stride > 12000;
+    if (sizeof(T) == 4) return lng || B <= 4 * sms;
+    return lng ? !box || B <= 2 * sms : B <= sms && (box || stride > 2000);
+}
 
 // Centroid of the first n_b atoms of chain b = blockIdx.x (FP64 accumulation);
 // 0 for an empty chain.
-template <typename T>
-__global__ void __launch_bounds__(kReduceThreads) center_kernel(const T *in, T *center, const int *num_atoms,
-                                                                int stride) {
-    constexpr int ROWS = kReduceThreads / 8;
-    __shared__ T s_sum[ROWS][3];
+// (32 registers in float32: 2000 chains of 4000 atoms are one wave of CTAs of 128 threads then,
+// 10.4 us, and two with 40, 15.0)
+template <typename T, int NT>
+__global__ void __launch_bounds__(NT, (sizeof(T) == 4 ? 2048 : 1536) / NT) center_kernel(const T *in, T *center, const int *num_atoms, int stride) {
+    // lanes summed in the coordinate type: fewer where a thread has more atoms
+    constexpr int LR = NT == 128 ? 8 : 32, ROWS = NT / LR;
+    // (float64 sums where few rows are left: the conversions are then those of many warps)
+    using Sum = std::conditional_t<ROWS <= 8, double, T>;
+    __shared__ Sum s_sum[ROWS][3];
     const int b = blockIdx.x, lane = threadIdx.x & 31;
     const int n = min(num_atoms[b], stride);  // a count past the row is clamped to it
     const T *x = in + (size_t)b * 3 * stride;
     // offsets from the chain's first atom, summed in the coordinate type per thread and over
-    // eight lanes and in FP64 across those: the offsets stay of the chain's own extent
+    // LR lanes and in FP64 across those: the offsets stay of the chain's own extent
     // wherever the chain sits, and GB300's FP64 rate is a small fraction of its FP32 rate
     const T p0 = n > 0 ? x[0] : T(0), p1 = n > 0 ? x[1] : T(0), p2 = n > 0 ? x[2] : T(0);
     T s[3] = {T(0), T(0), T(0)};
     // aligned groups of N atoms as three vectors per thread (tpl_rows.cuh), two groups in
-    // flight; then the atoms before and after them
+    // flight; the few atoms before and after them, loaded first, are added last
     constexpr int N = Vec16<T>::n;
     const int head = max(0, min(row_head(x), n)), ng = max(0, n - head) / N;
     const T *xg = x + 3 * head;
+    const int q = threadIdx.x;
+    const bool outside = q < n - N * ng;  // at most 2 (N - 1)
+    T o[3] = {p0, p1, p2};
+    if (outside) {
+        const T *xo = x + 3 * (q < head ? q : q + N * ng);
+        o[0] = xo[0];
+        o[1] = xo[1];
+        o[2] = xo[2];
+    }
 #pragma unroll 2
-    for (int g = threadIdx.x; g < ng; g += kReduceThreads) {
+    for (int g = threadIdx.x; g < ng; g += NT) {
         T v[3 * N];
         load_group(xg + 3 * N * g, v);
         if constexpr (N == 4) {
@@ -238,22 +359,31 @@ __global__ void __launch_bounds__(kReduceThreads) center_kernel(const T *in, T *
             s[2] += (v[2] - p2) + (v[5] - p2);
         }
     }
-    for (int q = threadIdx.x; q < n - N * ng; q += kReduceThreads) {
-        const int i = q < head ? q : q + N * ng;
-        s[0] += x[3 * i] - p0;
-        s[1] += x[3 * i + 1] - p1;
-        s[2] += x[3 * i + 2] - p2;
+    if (outside) {
+        s[0] += o[0] - p0;
+        s[1] += o[1] - p1;
+        s[2] += o[2] - p2;
     }
 #pragma unroll
-    for (int off = 4; off > 0; off >>= 1)
+    for (int off = LR / 2; off > 0; off >>= 1)
 #pragma unroll
         for (int c = 0; c < 3; c++) s[c] += __shfl_xor_sync(0xffffffffu, s[c], off);
-    if ((lane & 7) == 0)
+    if (lane % LR == 0)
 #pragma unroll
-        for (int c = 0; c < 3; c++) s_sum[threadIdx.x >> 3][c] = s[c];
+        for (int c = 0; c < 3; c++) s_sum[threadIdx.x / LR][c] = (Sum)s[c];
     __syncthreads();
     if (threadIdx.x >= 32) return;
-    static_assert(ROWS <= 32, "one sum per lane");
+    if constexpr (ROWS <= 8) {  // a sum a lane
+        if (lane < 3) {
+            double t = 0.0;
+#pragma unroll
+            for (int q = 0; q < ROWS; q++) t += s_sum[q][lane];
+            const double p = lane == 0 ? (double)p0 : (lane == 1 ? (double)p1 : (double)p2);
+            center[3 * b + lane] = n > 0 ? (T)(p + t / n) : T(0);
+        }
+        return;
+    }
+    static_assert(ROWS <= 32, "a row a lane");
     double t[3];
 #pragma unroll
     for (int c = 0; c < 3; c++) t[c] = lane < ROWS ? (double)s_sum[lane][c] : 0.0;
@@ -270,10 +400,9 @@ __global__ void __launch_bounds__(kReduceThreads) center_kernel(const T *in, T *
 
 // Axis-aligned bounding box of the first n_b atoms of chain b: lo = min, hi = max
 // per coordinate (+inf / -inf for an empty chain, as Math/nUtil.cpp:27-57).
-template <typename T>
-__global__ void __launch_bounds__(kReduceThreads) bbox_kernel(const T *in, T *lo, T *hi, const int *num_atoms,
-                                                              int stride) {
-    constexpr int NW = kReduceThreads / 32, N = Vec16<T>::n;
+template <typename T, int NT>
+__global__ void __launch_bounds__(NT, (sizeof(T) == 4 ? 2048 : 1536) / NT) bbox_kernel(const T *in, T *lo, T *hi, const int *num_atoms, int stride) {
+    constexpr int NW = NT / 32, N = Vec16<T>::n;
     __shared__ T s_warp[NW][6];
     const int b = blockIdx.x, lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const int n = min(num_atoms[b], stride);
@@ -289,14 +418,23 @@ __global__ void __launch_bounds__(kReduceThreads) bbox_kernel(const T *in, T *lo
     };
     const int head = max(0, min(row_head(x), n)), ng = max(0, n - head) / N;
     const T *xg = x + 3 * head;
+    const int q = threadIdx.x;
+    const bool outside = q < n - N * ng;  // the atoms before and after the groups, at most 2 (N - 1)
+    T o[3];
+    if (outside) {
+        const T *xo = x + 3 * (q < head ? q : q + N * ng);
+        o[0] = xo[0];
+        o[1] = xo[1];
+        o[2] = xo[2];
+    }
 #pragma unroll 2
-    for (int g = threadIdx.x; g < ng; g += kReduceThreads) {
+    for (int g = threadIdx.x; g < ng; g += NT) {
         T v[3 * N];
         load_group(xg + 3 * N * g, v);
 #pragma unroll
-        for (int q = 0; q < N; q++) add(v + 3 * q);
+        for (int i = 0; i < N; i++) add(v + 3 * i);
     }
-    for (int q = threadIdx.x; q < n - N * ng; q += kReduceThreads) add(x + 3 * (q < head ? q : q + N * ng));
+    if (outside) add(o);
     auto lower = [](T p, T q) { return q < p ? q : p; };
     auto upper = [](T p, T q) { return q > p ? q : p; };
 #pragma unroll
@@ -332,13 +470,30 @@ dim3 grid_rows(int B, long long items_per_row) {
 
 }  // namespace
 
+// Rows that cannot move as vectors throughout: the vectors between the boundaries cost a
+// second round of loads for the elements outside them, which only pays where there is enough
+// to move. Elements / vectors, us: float32 4096 rows of 101 atoms 6.0 / 6.4, of 401 11.4 / 8.8;
+// 64 of 2001 2.8 / 3.0, 150 3.5 / 3.1; float64 1000 of 1001 8.6 / 8.9, 4096 34.9 / 32.9.
+template <typename T, bool SCALE>
+static void launch_shift(const ShiftArgs &a, cudaStream_t st) {
+    constexpr int N = Vec16<T>::n;
+    auto grid = [&](int per_item) { return grid_rows(a.B, ((a.row + per_item - 1) / per_item + kUnroll - 1) / kUnroll); };
+    auto aligned16 = [](const void *p) { return ((uintptr_t)p & 15u) == 0; };
+    if (a.row % N == 0 && aligned16(a.out) && aligned16(a.in))
+        shift_kernel<T, true, SCALE && sizeof(T) == 8><<<grid(N), 256, 0, st>>>(a);
+    else if (a.row < 900 || (long long)a.B * a.row < (sizeof(T) == 4 ? 600000 : 6000000))
+        shift_kernel<T, false, SCALE && sizeof(T) == 8><<<grid(1), 256, 0, st>>>(a);
+    else
+        shift_rows_kernel<T, SCALE><<<grid(N), 256, 0, st>>>(a);
+}
+
 template <typename T>
 int coords_shift(const T *in, T *out, const T *add, int scale_by_count, const int *num_atoms, int B, int stride,
                  cudaStream_t st) {
     if (B == 0 || stride == 0) return TPL_OK;
-    ShiftArgs a{in, out, add, num_atoms, B, 3 * stride, scale_by_count};
-    const long long nv = (a.row + Vec16<T>::n - 1) / Vec16<T>::n;
-    shift_kernel<T><<<grid_rows(B, (nv + kUnroll - 1) / kUnroll), 256, 0, st>>>(a);
+    const ShiftArgs a{in, out, add, num_atoms, B, 3 * stride, scale_by_count};
+    if (scale_by_count) launch_shift<T, true>(a, st);
+    else launch_shift<T, false>(a, st);
     return cudaGetLastError() == cudaSuccess ? TPL_OK : TPL_ERR_LAUNCH;
 }
 
@@ -346,22 +501,32 @@ template <typename T>
 int coords_rotate(const T *in, T *out, const T *R, int transpose, const int *num_atoms, int B, int stride,
                   cudaStream_t st) {
     if (B == 0 || stride == 0) return TPL_OK;
-    const long long groups = (stride + Vec16<T>::n - 1) / Vec16<T>::n;
-    rotate_kernel<T><<<grid_rows(B, (groups + 1) / 2), 256, 0, st>>>(in, out, R, num_atoms, B, stride, transpose);
+    if constexpr (sizeof(T) == 4) {
+        if (stride >= 1500 && (long long)B * stride >= 5000000) {
+            const long long groups = (stride + Vec16<T>::n - 1) / Vec16<T>::n;
+            rotate_tiles_kernel<<<grid_rows(B, (groups + 1) / 2), 256, 0, st>>>(in, out, R, num_atoms, B, stride,
+                                                                               transpose);
+            return cudaGetLastError() == cudaSuccess ? TPL_OK : TPL_ERR_LAUNCH;
+        }
+    }
+    rotate_kernel<T><<<grid_rows(B, (stride + kUnroll - 1) / kUnroll), 256, 0, st>>>(in, out, R, num_atoms, B, stride,
+                                                                                   transpose);
     return cudaGetLastError() == cudaSuccess ? TPL_OK : TPL_ERR_LAUNCH;
 }
 
 template <typename T>
 int coords_center(const T *in, T *center, const int *num_atoms, int B, int stride, cudaStream_t st) {
     if (B == 0) return TPL_OK;
-    center_kernel<T><<<B, kReduceThreads, 0, st>>>(in, center, num_atoms, stride);
+    if (wide_reduction<T>(B, stride, false)) center_kernel<T, 256><<<B, 256, 0, st>>>(in, center, num_atoms, stride);
+    else center_kernel<T, 128><<<B, 128, 0, st>>>(in, center, num_atoms, stride);
     return cudaGetLastError() == cudaSuccess ? TPL_OK : TPL_ERR_LAUNCH;
 }
 
 template <typename T>
 int coords_bbox(const T *in, T *lo, T *hi, const int *num_atoms, int B, int stride, cudaStream_t st) {
     if (B == 0) return TPL_OK;
-    bbox_kernel<T><<<B, kReduceThreads, 0, st>>>(in, lo, hi, num_atoms, stride);
+    if (wide_reduction<T>(B, stride, true)) bbox_kernel<T, 256><<<B, 256, 0, st>>>(in, lo, hi, num_atoms, stride);
+    else bbox_kernel<T, 128><<<B, 128, 0, st>>>(in, lo, hi, num_atoms, stride);
     return cudaGetLastError() == cudaSuccess ? TPL_OK : TPL_ERR_LAUNCH;
 }
 
