@@ -176,3 +176,49 @@ def test_four_warps_in_large_batches(built, dtype, pad):
     fm.Coords2TypedCoords_forward(rows(x), rows(rn), rows(an), rows(na), out, cnt, off, idx)
     for got, ref in ((out, want), (cnt, wcnt), (off, woff), (idx, widx)):
         assert torch.equal(got, rows(ref).to(got.dtype))
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float64])
+@pytest.mark.parametrize("S", [1, 31, 33, 128, 599, 600, 601])
+def test_short_rows_in_large_batches(built, dtype, S):
+    """Batches of three chains per SM and more take the scattering kernel on rows of up to 600
+    atoms: one chain fewer and that many, rows on both sides of the line, counts from none
+    to all of the row, typed rows narrower than the input rows, a name pair without a type
+    (left out and reported); bit for bit against the oracle."""
+    from torchproteinlibrary_gb300 import load_extension
+    fm = load_extension("_FullAtomModel")
+    rng = np.random.default_rng(S)
+    pairs = [(b"GLY\0", a) for a in (b"N\0\0\0", b"CA\0\0", b"C\0\0\0", b"O\0\0\0")]
+    pairs += [(b"LYS\0", b"NZ\0\0"), (b"MET\0", b"SD\0\0"), (b"HIS\0", b"CG\0\0"), (b"THR\0", b"OG1\0")]
+    K, S_out = 19, max(1, S - 1)
+    na = rng.integers(0, S_out + 1, K).astype(np.int32)
+    na[:3] = 0, S_out, min(1, S_out)
+    pick = rng.integers(0, len(pairs), (K, S))
+    rn = np.array([[list(pairs[k][0]) for k in row] for row in pick], np.uint8)
+    an = np.array([[list(pairs[k][1]) for k in row] for row in pick], np.uint8)
+    x = rng.standard_normal((K, 3 * S)).astype(np.float32 if dtype == torch.float32 else np.float64)
+    want, wcnt, woff, widx = oracle.typed_coords(x, rn, an, na)
+    wide = want.shape[1] // 3
+    dev = torch.device("cuda")
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    for B in (3 * sms - 1, 3 * sms):
+        at = torch.arange(B, device=dev) % K
+
+        def rows(v):
+            return torch.tensor(v, device=dev)[at].contiguous()
+
+        out = torch.full((B, 3 * S_out), float("nan"), dtype=dtype, device=dev)
+        cnt = torch.empty(B, 11, dtype=torch.int32, device=dev)
+        off, idx = torch.empty_like(cnt), torch.full((B, S_out), -7, dtype=torch.int32, device=dev)
+        fm.Coords2TypedCoords_forward(rows(x), rows(rn), rows(an), rows(na), out, cnt, off, idx)
+        assert fm.workspace_status(0) == 0
+        assert torch.equal(cnt, rows(wcnt)) and torch.equal(off, rows(woff))
+        assert torch.equal(out[:, :3 * wide], rows(want)) and not out[:, 3 * wide:].any()
+        assert torch.equal(idx[:, :wide], rows(widx).to(torch.int32)) and not idx[:, wide:].any()
+        if S == 33:
+            bad = an.copy()
+            bad[1, 4] = list(b"QQ\0\0")
+            out.fill_(float("nan"))
+            fm.Coords2TypedCoords_forward(rows(x), rows(rn), rows(bad), rows(na), out, cnt, off, idx)
+            assert fm.workspace_status(0) != 0
+            assert int(cnt[1].sum()) == int(na[1]) - 1 and int(cnt[0].sum()) == 0 and torch.isfinite(out).all()

@@ -7,7 +7,8 @@
 // Angles2Coords writes, one probe of a perfect hash each, ranks every atom among those of
 // its type, and moves the coordinates in input order within each type, groups of 128 atoms
 // ordered in shared memory first so that a type's run is written by consecutive lanes
-// (typed_fwd_group_kernel; rows past 32 768 atoms take typed_fwd_kernel).  The backward is
+// (typed_fwd_group_kernel; short rows in large batches take typed_fwd_scatter_kernel, rows
+// past 32 768 atoms typed_fwd_kernel).  The backward is
 // the inverse gather.  Integer and byte work only; coordinates are copied unchanged.
 #include <cstddef>
 #include <cstdint>
@@ -442,6 +443,128 @@ __global__ void __launch_bounds__(32 * NW) typed_fwd_group_kernel(
     zeros(atom_index + orow + ntyped, out_stride - ntyped);
 }
 
+// Short rows in batches that fill the GPU: the same two passes, but the types are found again
+// tile by tile and the coordinates go straight to their slots.  A warp has a tile or a few
+// there, so ordering and staging them costs more than the partial sectors of scattered
+// stores, and this form's small shared memory keeps twice the chains on an SM.  GB300,
+// scattered / ordered, us: float32 16000 chains of up to 100 atoms 31 / 48, of up to 400
+// 51 / 66, 4096 of 600 each 30 / 34, of 800 each 41 / 38; 300 of 400 5.1 / 4.7; float64 16000 of
+// up to 100 36 / 63.
+constexpr int kTypedScatterWarps = 4;
+constexpr int kTypedScatterAtoms = 600;
+
+template <typename T>
+__global__ void __launch_bounds__(32 * kTypedScatterWarps) typed_fwd_scatter_kernel(
+    const T *__restrict__ coords, const uint32_t *__restrict__ res_names, const uint32_t *__restrict__ atom_names,
+    const int *__restrict__ num_atoms, int in_stride, int out_stride, T *__restrict__ out,
+    int *__restrict__ n_of_type, int *__restrict__ offsets, int *__restrict__ atom_index, WsHeader *hdr) {
+    extern __shared__ signed char s_ty[];
+    __shared__ int s_cnt[kTypedScatterWarps][kTypes];
+    __shared__ int s_ntyped;
+    __shared__ TypedTables s_tab;
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, b = blockIdx.x;
+    {
+        const uint32_t *src = reinterpret_cast<const uint32_t *>(&g_typed_tables);
+        uint32_t *dst = reinterpret_cast<uint32_t *>(&s_tab);
+        for (int i = threadIdx.x; i < (int)(sizeof(TypedTables) / 4); i += 32 * kTypedScatterWarps) dst[i] = src[i];
+    }
+    const int n = max(0, min(num_atoms[b], min(in_stride, out_stride)));
+    const size_t row = (size_t)b * in_stride, orow = (size_t)b * out_stride;
+    const uint32_t *rn = res_names + row, *an = atom_names + row;
+    const unsigned below = (1u << lane) - 1u;
+    const int ntiles = (n + 31) >> 5, per = (ntiles + kTypedScatterWarps - 1) / kTypedScatterWarps;
+    const int t0 = min(ntiles, w * per), t1 = min(ntiles, t0 + per);
+
+    if (lane < kTypes) s_cnt[w][lane] = 0;
+    __syncthreads();  // the tables' copy and the zeroed counts
+    bool bad = false;
+    for (int tb = t0; tb < t1; tb += kTypedUnroll) {
+        uint32_t r[kTypedUnroll], a[kTypedUnroll];
+#pragma unroll
+        for (int u = 0; u < kTypedUnroll; u++) {
+            const int j = 32 * (tb + u) + lane;
+            const bool in = tb + u < t1 && j < n;
+            r[u] = in ? rn[j] : 0u;
+            a[u] = in ? an[j] : 0u;
+        }
+#pragma unroll
+        for (int u = 0; u < kTypedUnroll; u++) {
+            const int j = 32 * (tb + u) + lane;
+            const bool in = tb + u < t1 && j < n;
+            const int t = in ? atom_type(r[u], a[u], s_tab) : -2;  // -1: a name pair the reference rejects
+            if (in) s_ty[j] = (signed char)t;
+            bad |= t == -1;
+            // the lanes of each type: the lowest of them adds their number
+            const unsigned m = __match_any_sync(0xffffffffu, t);
+            if (t >= 0 && (m & below) == 0u) s_cnt[w][t] += __popc(m);
+            __syncwarp();
+        }
+    }
+    if (bad) atomicCAS(&hdr->status, 0u, (unsigned)TPL_ERR_ATOM_TYPE);
+    __syncthreads();
+    // lane k < kTypes: the type's total, its offset, and this warp's first slot of it
+    int tot = 0, before = 0;
+    if (lane < kTypes)
+#pragma unroll
+        for (int v = 0; v < kTypedScatterWarps; v++) {
+            const int c = s_cnt[v][lane];
+            tot += c;
+            before += v < w ? c : 0;
+        }
+    int inc = tot;
+#pragma unroll
+    for (int off = 1; off < 16; off <<= 1) {
+        const int v = __shfl_up_sync(0xffffffffu, inc, off);
+        if (lane >= off) inc += v;
+    }
+    const int type_off = inc - tot;
+    if (w == 0 && lane < kTypes) {
+        n_of_type[(size_t)b * kTypes + lane] = tot;
+        offsets[(size_t)b * kTypes + lane] = type_off;
+    }
+    if (w == 0 && lane == kTypes - 1) s_ntyped = inc;
+    __syncthreads();  // every warp has read the counts
+    int *s_next = s_cnt[w];  // reused: this warp's next free slot of each type
+    if (lane < kTypes) s_next[lane] = type_off + before;
+    __syncwarp();
+
+    for (int tb = t0; tb < t1; tb += kTypedUnroll) {
+        T x[kTypedUnroll][3];
+        int ty[kTypedUnroll];
+#pragma unroll
+        for (int u = 0; u < kTypedUnroll; u++) {
+            const int j = 32 * (tb + u) + lane;
+            const bool in = tb + u < t1 && j < n;
+            const T *src = coords + 3 * (row + j);
+#pragma unroll
+            for (int c = 0; c < 3; c++) x[u][c] = in ? src[c] : T(0);
+            ty[u] = in ? (int)s_ty[j] : -2;
+        }
+#pragma unroll
+        for (int u = 0; u < kTypedUnroll; u++) {
+            const int j = 32 * (tb + u) + lane, t = ty[u];
+            const unsigned m = __match_any_sync(0xffffffffu, t);
+            if (t >= 0) {
+                const int slot = s_next[t] + __popc(m & below);
+                T *dst = out + 3 * (orow + slot);
+                dst[0] = x[u][0];
+                dst[1] = x[u][1];
+                dst[2] = x[u][2];
+                atom_index[orow + slot] = j;
+            }
+            __syncwarp();
+            if (t >= 0 && (m & below) == 0u) s_next[t] += __popc(m);
+            __syncwarp();
+        }
+    }
+    __syncthreads();
+    // slots past the typed atoms are zero, as in the reference's zero-filled outputs
+    const int ntyped = s_ntyped;
+    T *o = out + 3 * orow;
+    for (int e = 3 * ntyped + threadIdx.x; e < 3 * out_stride; e += 32 * kTypedScatterWarps) o[e] = T(0);
+    for (int q = ntyped + threadIdx.x; q < out_stride; q += 32 * kTypedScatterWarps) atom_index[orow + q] = 0;
+}
+
 // grad_flat[atom_index[s]] = grad_typed[s] for the typed slots, zero elsewhere;
 // grad_flat rows hold in_stride atoms, grad_typed rows out_stride slots.
 template <typename T>
@@ -535,6 +658,13 @@ int typed_forward(bool f64, const void *coords, const uint32_t *res_names, const
             return cudaGetLastError() == cudaSuccess ? (int)TPL_OK : (int)TPL_ERR_LAUNCH;
         };
         auto pick = [&](auto *out_t, auto *coords_t) -> int {
+            if (in_stride <= kTypedScatterAtoms && B >= 3 * device_sm_count()) {
+                using T = std::remove_pointer_t<decltype(out_t)>;
+                typed_fwd_scatter_kernel<T><<<B, 32 * kTypedScatterWarps, in_stride, st>>>(
+                    coords_t, res_names, atom_names, num_atoms, in_stride, out_stride, out_t, n_of_type, offsets,
+                    atom_index, hdr);
+                return cudaGetLastError() == cudaSuccess ? (int)TPL_OK : (int)TPL_ERR_LAUNCH;
+            }
             // Eight warps per chain for rows past 3500 atoms, where a chain's codes are most of
             // the shared memory and more warps share them, and for batches below four chains per
             // SM; past 16384 atoms four warps' ranks would not fit the codes either.  Eight /
