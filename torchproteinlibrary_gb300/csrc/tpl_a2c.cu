@@ -41,50 +41,46 @@ namespace tpl {
 
 __device__ const Topology<float> g_topo_f32 = make_topology<float>();
 
-template <typename T>
-__device__ __forceinline__ void sc(T a, T *s, T *c) { sincos_t(a, s, c); }
-// float angles: the register polynomial of the Angles2Backbone kernels (about one
-// ulp, no special-function unit; sincosf beyond |a| = 1e4)
-template <>
-__device__ __forceinline__ void sc<float>(float a, float *s, float *c) { sincos_poly(a, s, c); }
+// The register polynomial of the Angles2Backbone kernels (about one ulp, no special-function
+// unit; sincosf beyond |a| = 1e4).
+__device__ __forceinline__ void sc(float a, float *s, float *c) { sincos_poly(a, s, c); }
 
-template <typename T>
-__device__ __forceinline__ void renorm_if(Frame<T> &f, bool on) {
+__device__ __forceinline__ void renorm_if(Frame<float> &f, bool on) {
     if (on) renormalize(f);
 }
 
 // Shared-memory layout of the tile buffers (dynamic).
-template <typename T, int TILE>
+template <int TILE>
 struct A2cSmem {
-    Topology<T> topo;
-    T ang[8][TILE];
-    T xyz[TILE * kMaxResAtoms * 3];
+    Topology<float> topo;
+    float ang[8][TILE];
+    float xyz[TILE * kMaxResAtoms * 3];
     signed char type[TILE];
     signed char lut[256];
 };
 
 // The forward also stages the tile's residue and atom names, so that they leave
 // with the coordinates' coalesced store instead of per-residue scattered writes.
-template <typename T, int TILE>
+template <int TILE>
 struct A2cSmemFwd {
-    A2cSmem<T, TILE> f;
+    A2cSmem<TILE> f;
     uint32_t res_name[TILE * kMaxResAtoms];
     uint32_t atom_name[TILE * kMaxResAtoms];
 };
 
-template <typename T, int TILE>
+template <int TILE>
 struct A2cSmemBwd {
-    A2cSmem<T, TILE> f;
-    T g[TILE * kMaxResAtoms * 3];
+    A2cSmem<TILE> f;
+    float g[TILE * kMaxResAtoms * 3];
 };
 
 // Copy the topology to shared memory and build the letter -> type table.
-template <typename T, int NT>
-__device__ __forceinline__ void load_topology(Topology<T> &dst, signed char *lut) {
+template <int NT>
+__device__ __forceinline__ void load_topology(Topology<float> &dst, signed char *lut) {
     const uint32_t *src = reinterpret_cast<const uint32_t *>(&g_topo_f32);
     uint32_t *d = reinterpret_cast<uint32_t *>(&dst);
-    constexpr int n = sizeof(Topology<T>) / 4;
-    static_assert(sizeof(Topology<T>) % 4 == 0, "topology size");
+    constexpr int n = sizeof(Topology<float>) / 4;
+    static_assert(sizeof(Topology<float>) % 4 == 0, "topology size");
     for (int i = threadIdx.x; i < n; i += NT) d[i] = src[i];
     for (int i = threadIdx.x; i < 256; i += NT) lut[i] = (signed char)residue_type((unsigned char)i);
 }
@@ -111,20 +107,20 @@ __device__ __forceinline__ int chain_length(const unsigned char *row, int stride
 
 // Per-thread scan state for one tile: backbone aggregate of the thread's
 // residues, its exclusive prefix inside the warp, atom counts.
-template <typename T, int R, int NT>
+template <int R, int NT>
 struct TileScan {
-    T cs[R][3], sn[R][3];
-    Frame<T> exc;     // exclusive prefix inside the warp
+    float cs[R][3], sn[R][3];
+    Frame<float> exc;     // exclusive prefix inside the warp
     int cnt_exc;      // atoms before this thread inside the warp
     int cnt_own;      // atoms of this thread
 };
 
-template <typename T, int R, int NT>
-__device__ __forceinline__ void a2c_tile_scan(const Topology<T> &tp, const T (*ang)[R * NT],
+template <int R, int NT>
+__device__ __forceinline__ void a2c_tile_scan(const Topology<float> &tp, const float (*ang)[R * NT],
                                               const signed char *type, int n, bool chain_end, bool renorm,
-                                              TileScan<T, R, NT> &ts, Frame<T> *s_wtot, int *s_wcnt) {
+                                              TileScan<R, NT> &ts, Frame<float> *s_wtot, int *s_wcnt) {
     const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
-    Frame<T> agg;
+    Frame<float> agg;
     frame_identity(agg);
     int cnt = 0;
 #pragma unroll
@@ -132,8 +128,8 @@ __device__ __forceinline__ void a2c_tile_scan(const Topology<T> &tp, const T (*a
         const int j = tid * R + r;
 #pragma unroll
         for (int k = 0; k < 3; k++) {
-            ts.cs[r][k] = T(1);
-            ts.sn[r][k] = T(0);
+            ts.cs[r][k] = 1.f;
+            ts.sn[r][k] = 0.f;
         }
         if (j < n) {
             cnt += tp.natoms[type[j]];
@@ -146,7 +142,7 @@ __device__ __forceinline__ void a2c_tile_scan(const Topology<T> &tp, const T (*a
         }
     }
     renorm_if(agg, renorm);
-    Frame<T> inc = warp_scan_frames(agg, lane);
+    Frame<float> inc = warp_scan_frames(agg, lane);
     ts.exc = shfl_up_frame(inc, 1);
     if (lane == 0) frame_identity(ts.exc);
     int ci = cnt;
@@ -165,14 +161,14 @@ __device__ __forceinline__ void a2c_tile_scan(const Topology<T> &tp, const T (*a
 
 // Thread 0: warp prefixes with the tile carry folded in (rotation only: positions
 // are relative to the tile origin), the tile aggregate and the tile atom count.
-template <typename T, int NW>
-__device__ __forceinline__ void a2c_tile_prefix(const Frame<T> &carry, const Frame<T> *s_wtot, const int *s_wcnt,
-                                                bool renorm, Frame<T> *s_wpre, int *s_wcpre, Frame<T> &tile_agg,
+template <int NW>
+__device__ __forceinline__ void a2c_tile_prefix(const Frame<float> &carry, const Frame<float> *s_wtot, const int *s_wcnt,
+                                                bool renorm, Frame<float> *s_wpre, int *s_wcpre, Frame<float> &tile_agg,
                                                 int &tile_cnt) {
-    Frame<T> run;
+    Frame<float> run;
     frame_identity(run);
-    Frame<T> c0 = carry;
-    c0.p[0] = c0.p[1] = c0.p[2] = T(0);
+    Frame<float> c0 = carry;
+    c0.p[0] = c0.p[1] = c0.p[2] = 0.f;
     int cr = 0;
     for (int w = 0; w < NW; w++) {
         s_wpre[w] = compose(c0, run);
@@ -188,43 +184,43 @@ __device__ __forceinline__ void a2c_tile_prefix(const Frame<T> &carry, const Fra
 // All atoms of residue j (type ty) from the frame P at its N atom.  chi_angle(q)
 // returns the residue's chi_(q+1); emit(slot, xyz) receives positions in P's
 // coordinates; returns the frame at the next N.
-template <typename T, typename Chi, typename Emit>
-__device__ __forceinline__ void residue_atoms(const Topology<T> &tp, int ty, Frame<T> &P, const T cs[3],
-                                              const T sn[3], Chi chi_angle, Emit emit) {
+template <typename Chi, typename Emit>
+__device__ __forceinline__ void residue_atoms(const Topology<float> &tp, int ty, Frame<float> &P, const float cs[3],
+                                              const float sn[3], Chi chi_angle, Emit emit) {
     emit(0, P.p);
-    Frame<T> F = P;
+    Frame<float> F = P;
     apply_joint(F, tp.bb_cb[0], tp.bb_sb[0], tp.bb_d[0], cs[0], sn[0]);
     emit(1, F.p);
     const int na = tp.natoms[ty];
     if (tp.pro[ty]) {
         for (int a = 0; a < 3; a++) {
-            T x[3];
+            float x[3];
             frame_point(F, tp.pro_local[a][0], tp.pro_local[a][1], tp.pro_local[a][2], x);
             emit(2 + a, x);
         }
     }
     const int nj = tp.njoints[ty];
     if (nj > 0) {
-        Frame<T> S = F;
+        Frame<float> S = F;
         apply_rx(S, tp.dummy_c, tp.dummy_s);
         for (int k = 0; k < nj; k++) {
             const int chi = tp.jchi[ty][k];
-            T c = T(1), s = T(0);
+            float c = 1.f, s = 0.f;
             if (chi >= 0) sc(chi_angle(chi), &s, &c);
             apply_joint(S, tp.jcb[ty][k], tp.jsb[ty][k], tp.jd[ty][k], c, s);
             const int f0 = tp.jfirst[ty][k];
             for (int a = 0; a < tp.jna[ty][k]; a++) {
-                T x[3];
+                float x[3];
                 frame_point(S, tp.sc[ty][f0 + a][0], tp.sc[ty][f0 + a][1], tp.sc[ty][f0 + a][2], x);
                 emit(2 + f0 + a, x);
             }
         }
     }
-    Frame<T> C = F;
+    Frame<float> C = F;
     apply_joint(C, tp.bb_cb[1], tp.bb_sb[1], tp.bb_d[1], cs[1], sn[1]);
     emit(na - 2, C.p);
     {
-        T x[3];
+        float x[3];
         frame_point(C, tp.o_local[0], tp.o_local[1], tp.o_local[2], x);
         emit(na - 1, x);
     }
@@ -353,28 +349,28 @@ __device__ __forceinline__ void residue_atoms_pair(const RingTopology &tp, uint3
 }
 
 // Copy n staged values (world coordinates, xyz interleaved) to dst, coalesced.
-template <typename T, int NT>
-__device__ __forceinline__ void store_tile_atoms(T *dst, const T *src, int n) {
+template <int NT>
+__device__ __forceinline__ void store_tile_atoms(float *dst, const float *src, int n) {
     for (int i = threadIdx.x; i < n; i += NT) dst[i] = src[i];
 }
 
-template <typename T, int R, int NT>
-__global__ void __launch_bounds__(NT) a2c_fwd_kernel(A2cArgs<T> a, int renorm) {
+template <int R, int NT>
+__global__ void __launch_bounds__(NT) a2c_fwd_kernel(A2cArgs<float> a, int renorm) {
     constexpr int TILE = R * NT, NW = NT / 32;
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    A2cSmemFwd<T, TILE> &smf = *reinterpret_cast<A2cSmemFwd<T, TILE> *>(smem_raw);
-    A2cSmem<T, TILE> &sm = smf.f;
-    __shared__ Frame<T> s_wtot[NW], s_wpre[NW];
+    A2cSmemFwd<TILE> &smf = *reinterpret_cast<A2cSmemFwd<TILE> *>(smem_raw);
+    A2cSmem<TILE> &sm = smf.f;
+    __shared__ Frame<float> s_wtot[NW], s_wpre[NW];
     __shared__ int s_wcnt[NW], s_wcpre[NW];
-    __shared__ Frame<T> s_carry;
-    __shared__ T s_org[3];
+    __shared__ Frame<float> s_carry;
+    __shared__ float s_org[3];
     __shared__ int s_len, s_bad, s_abase, s_tcnt;
 
     const int b = blockIdx.x, tid = threadIdx.x, w = tid >> 5, lane = tid & 31;
-    load_topology<T, NT>(sm.topo, sm.lut);
+    load_topology<NT>(sm.topo, sm.lut);
     const unsigned char *row = a.seq + (size_t)b * a.seq_stride;
     int len = chain_length<NT>(row, a.seq_stride, sm.lut, &s_len, &s_bad);
-    T *out = a.coords + (size_t)b * 3 * a.maxA;
+    float *out = a.coords + (size_t)b * 3 * a.maxA;
     uint32_t *rn = a.res_names ? a.res_names + (size_t)b * a.maxA : nullptr;
     uint32_t *an = a.atom_names ? a.atom_names + (size_t)b * a.maxA : nullptr;
     bool ok = true;
@@ -391,7 +387,7 @@ __global__ void __launch_bounds__(NT) a2c_fwd_kernel(A2cArgs<T> a, int renorm) {
         s_abase = 0;
     }
     __syncthreads();
-    const T *ang_b = a.angles + (size_t)b * 8 * a.L;
+    const float *ang_b = a.angles + (size_t)b * 8 * a.L;
     for (int s0 = 0; ok && s0 < len; s0 += TILE) {
         const int n = min(TILE, len - s0);
         for (int k = 0; k < 8; k++)
@@ -399,35 +395,35 @@ __global__ void __launch_bounds__(NT) a2c_fwd_kernel(A2cArgs<T> a, int renorm) {
         for (int i = tid; i < n; i += NT) sm.type[i] = sm.lut[row[s0 + i]];
         __syncthreads();
         const bool chain_end = (s0 + n == len);
-        TileScan<T, R, NT> ts;
-        a2c_tile_scan<T, R, NT>(sm.topo, sm.ang, sm.type, n, chain_end, renorm, ts, s_wtot, s_wcnt);
+        TileScan<R, NT> ts;
+        a2c_tile_scan<R, NT>(sm.topo, sm.ang, sm.type, n, chain_end, renorm, ts, s_wtot, s_wcnt);
         __syncthreads();
         if (tid == 0) {
-            Frame<T> agg;
+            Frame<float> agg;
             int tcnt;
-            a2c_tile_prefix<T, NW>(s_carry, s_wtot, s_wcnt, renorm, s_wpre, s_wcpre, agg, tcnt);
+            a2c_tile_prefix<NW>(s_carry, s_wtot, s_wcnt, renorm, s_wpre, s_wcpre, agg, tcnt);
             s_org[0] = s_carry.p[0]; s_org[1] = s_carry.p[1]; s_org[2] = s_carry.p[2];
             s_tcnt = tcnt;
-            Frame<T> nc = compose(s_carry, agg);
+            Frame<float> nc = compose(s_carry, agg);
             renorm_if(nc, renorm);
             s_carry = nc;
         }
         __syncthreads();
-        Frame<T> P = compose(s_wpre[w], ts.exc);
+        Frame<float> P = compose(s_wpre[w], ts.exc);
         renorm_if(P, renorm);
         int aoff = s_wcpre[w] + ts.cnt_exc;  // first atom of this thread inside the tile
         const int abase = s_abase;
         // positions are built relative to the tile origin and moved to it as they are
         // staged (the same FP32 addition as at store time, without a per-value modulo)
-        const T org[3] = {s_org[0], s_org[1], s_org[2]};
+        const float org[3] = {s_org[0], s_org[1], s_org[2]};
 #pragma unroll
         for (int r = 0; r < R; r++) {
             const int j = tid * R + r;
             if (j < n) {
                 const int ty = sm.type[j];
-                T *dst = sm.xyz + 3 * aoff;
-                residue_atoms<T>(sm.topo, ty, P, ts.cs[r], ts.sn[r], [&](int q) { return sm.ang[3 + q][j]; },
-                                 [&](int slot, const T *x) {
+                float *dst = sm.xyz + 3 * aoff;
+                residue_atoms(sm.topo, ty, P, ts.cs[r], ts.sn[r], [&](int q) { return sm.ang[3 + q][j]; },
+                                 [&](int slot, const float *x) {
                                      dst[3 * slot] = x[0] + org[0];
                                      dst[3 * slot + 1] = x[1] + org[1];
                                      dst[3 * slot + 2] = x[2] + org[2];
@@ -445,7 +441,7 @@ __global__ void __launch_bounds__(NT) a2c_fwd_kernel(A2cArgs<T> a, int renorm) {
         __syncthreads();
         const int tcnt = s_tcnt;
         const int nstore = max(0, min(tcnt, a.maxA - abase));
-        store_tile_atoms<T, NT>(out + (size_t)3 * abase, sm.xyz, 3 * nstore);
+        store_tile_atoms<NT>(out + (size_t)3 * abase, sm.xyz, 3 * nstore);
         if (rn && an)
             for (int i = tid; i < nstore; i += NT) {
                 rn[abase + i] = smf.res_name[i];
@@ -460,7 +456,7 @@ __global__ void __launch_bounds__(NT) a2c_fwd_kernel(A2cArgs<T> a, int renorm) {
         if (tid == 0) a2c_error(a.hdr, TPL_ERR_ATOMS);
         total = a.maxA;
     }
-    for (int i = 3 * total + tid; i < 3 * a.maxA; i += NT) out[i] = T(0);
+    for (int i = 3 * total + tid; i < 3 * a.maxA; i += NT) out[i] = 0.f;
     if (rn && an)
         for (int i = total + tid; i < a.maxA; i += NT) rn[i] = an[i] = 0u;
     (void)lane;
@@ -711,27 +707,27 @@ __global__ void __launch_bounds__(32 * NW, NW == 4 ? 6 : 3) a2c_fwd_ring_kernel(
 }
 
 // ------------------------------------------------------------------ backward
-template <typename T, int R, int NT>
-__global__ void __launch_bounds__(NT) a2c_bwd_kernel(A2cArgs<T> a, int renorm, int max_tiles) {
+template <int R, int NT>
+__global__ void __launch_bounds__(NT) a2c_bwd_kernel(A2cArgs<float> a, int renorm, int max_tiles) {
     constexpr int TILE = R * NT, NW = NT / 32;
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    A2cSmemBwd<T, TILE> &sm = *reinterpret_cast<A2cSmemBwd<T, TILE> *>(smem_raw);
-    Frame<T> *s_carries = reinterpret_cast<Frame<T> *>(smem_raw + sizeof(A2cSmemBwd<T, TILE>));
+    A2cSmemBwd<TILE> &sm = *reinterpret_cast<A2cSmemBwd<TILE> *>(smem_raw);
+    Frame<float> *s_carries = reinterpret_cast<Frame<float> *>(smem_raw + sizeof(A2cSmemBwd<TILE>));
     int *s_tbase = reinterpret_cast<int *>(s_carries + max_tiles);
-    __shared__ Frame<T> s_wtot[NW], s_wpre[NW];
+    __shared__ Frame<float> s_wtot[NW], s_wpre[NW];
     __shared__ int s_wcnt[NW], s_wcpre[NW];
-    __shared__ T s_wsum[NW][6], s_wsuf[NW][6];
+    __shared__ float s_wsum[NW][6], s_wsuf[NW][6];
     __shared__ double s_tail[6];
     __shared__ int s_len, s_bad;
 
     const int b = blockIdx.x, tid = threadIdx.x, w = tid >> 5, lane = tid & 31;
-    load_topology<T, NT>(sm.f.topo, sm.f.lut);
-    const Topology<T> &tp = sm.f.topo;
+    load_topology<NT>(sm.f.topo, sm.f.lut);
+    const Topology<float> &tp = sm.f.topo;
     const unsigned char *row = a.seq + (size_t)b * a.seq_stride;
     int len = chain_length<NT>(row, a.seq_stride, sm.f.lut, &s_len, &s_bad);
-    T *gout = a.grad_angles + (size_t)b * 8 * a.L;
-    const T *gin = a.grad_coords + (size_t)b * 3 * a.maxA;
-    const T *ang_b = a.angles + (size_t)b * 8 * a.L;
+    float *gout = a.grad_angles + (size_t)b * 8 * a.L;
+    const float *gin = a.grad_coords + (size_t)b * 3 * a.maxA;
+    const float *ang_b = a.angles + (size_t)b * 8 * a.L;
     bool ok = !s_bad && len <= a.L;
     if (tid == 0) {
         if (s_bad) a2c_error(a.hdr, TPL_ERR_SEQUENCE);
@@ -754,15 +750,15 @@ __global__ void __launch_bounds__(NT) a2c_bwd_kernel(A2cArgs<T> a, int renorm, i
             for (int i = tid; i < n; i += NT) sm.f.ang[k][i] = ang_b[(size_t)k * a.L + s0 + i];
         for (int i = tid; i < n; i += NT) sm.f.type[i] = sm.f.lut[row[s0 + i]];
         __syncthreads();
-        TileScan<T, R, NT> ts;
-        a2c_tile_scan<T, R, NT>(tp, sm.f.ang, sm.f.type, n, s0 + n == len, renorm, ts, s_wtot, s_wcnt);
+        TileScan<R, NT> ts;
+        a2c_tile_scan<R, NT>(tp, sm.f.ang, sm.f.type, n, s0 + n == len, renorm, ts, s_wtot, s_wcnt);
         __syncthreads();
         if (tid == 0) {
-            Frame<T> agg;
+            Frame<float> agg;
             int tcnt;
-            a2c_tile_prefix<T, NW>(s_carries[t], s_wtot, s_wcnt, renorm, s_wpre, s_wcpre, agg, tcnt);
+            a2c_tile_prefix<NW>(s_carries[t], s_wtot, s_wcnt, renorm, s_wpre, s_wcpre, agg, tcnt);
             if (t + 1 < max_tiles) {
-                Frame<T> nc = compose(s_carries[t], agg);
+                Frame<float> nc = compose(s_carries[t], agg);
                 renorm_if(nc, renorm);
                 s_carries[t + 1] = nc;
                 s_tbase[t + 1] = s_tbase[t] + tcnt;
@@ -781,26 +777,26 @@ __global__ void __launch_bounds__(NT) a2c_bwd_kernel(A2cArgs<T> a, int renorm, i
             for (int i = tid; i < n; i += NT) sm.f.ang[k][i] = ang_b[(size_t)k * a.L + s0 + i];
         for (int i = tid; i < n; i += NT) sm.f.type[i] = sm.f.lut[row[s0 + i]];
         __syncthreads();
-        TileScan<T, R, NT> ts;
-        a2c_tile_scan<T, R, NT>(tp, sm.f.ang, sm.f.type, n, s0 + n == len, renorm, ts, s_wtot, s_wcnt);
+        TileScan<R, NT> ts;
+        a2c_tile_scan<R, NT>(tp, sm.f.ang, sm.f.type, n, s0 + n == len, renorm, ts, s_wtot, s_wcnt);
         __syncthreads();
         if (tid == 0) {
-            Frame<T> agg;
+            Frame<float> agg;
             int tcnt;
-            a2c_tile_prefix<T, NW>(s_carries[t], s_wtot, s_wcnt, renorm, s_wpre, s_wcpre, agg, tcnt);
+            a2c_tile_prefix<NW>(s_carries[t], s_wtot, s_wcnt, renorm, s_wpre, s_wcpre, agg, tcnt);
             s_wcnt[0] = tcnt;  // reuse: tile atom count
         }
         __syncthreads();
         const int tcnt = s_wcnt[0];
         const int nload = max(0, min(tcnt, a.maxA - abase));
-        for (int i = tid; i < 3 * tcnt; i += NT) sm.g[i] = i < 3 * nload ? gin[(size_t)3 * abase + i] : T(0);
-        Frame<T> P = compose(s_wpre[w], ts.exc);
+        for (int i = tid; i < 3 * tcnt; i += NT) sm.g[i] = i < 3 * nload ? gin[(size_t)3 * abase + i] : 0.f;
+        Frame<float> P = compose(s_wpre[w], ts.exc);
         renorm_if(P, renorm);
-        Frame<T> start[R];
+        Frame<float> start[R];
         int roff[R];
         int aoff = s_wcpre[w] + ts.cnt_exc;
         __syncthreads();  // sm.g complete
-        T G[3] = {0, 0, 0}, S[3] = {0, 0, 0};
+        float G[3] = {0, 0, 0}, S[3] = {0, 0, 0};
 #pragma unroll
         for (int r = 0; r < R; r++) {
             const int j = tid * R + r;
@@ -808,14 +804,14 @@ __global__ void __launch_bounds__(NT) a2c_bwd_kernel(A2cArgs<T> a, int renorm, i
             roff[r] = aoff;
             if (j < n) {
                 const int ty = sm.f.type[j];
-                T *dst = sm.f.xyz + 3 * aoff;
-                const T *gg = sm.g + 3 * aoff;
-                residue_atoms<T>(tp, ty, P, ts.cs[r], ts.sn[r], [&](int q) { return sm.f.ang[3 + q][j]; },
-                                 [&](int slot, const T *x) {
+                float *dst = sm.f.xyz + 3 * aoff;
+                const float *gg = sm.g + 3 * aoff;
+                residue_atoms(tp, ty, P, ts.cs[r], ts.sn[r], [&](int q) { return sm.f.ang[3 + q][j]; },
+                                 [&](int slot, const float *x) {
                     dst[3 * slot] = x[0];
                     dst[3 * slot + 1] = x[1];
                     dst[3 * slot + 2] = x[2];
-                    T xg[3];
+                    float xg[3];
                     cross3(x, gg + 3 * slot, xg);
                     for (int c = 0; c < 3; c++) {
                         G[c] += gg[3 * slot + c];
@@ -826,15 +822,15 @@ __global__ void __launch_bounds__(NT) a2c_bwd_kernel(A2cArgs<T> a, int renorm, i
             }
         }
         // block-exclusive suffix over threads, plus the carry from later tiles
-        T suf[6];
-        const T v[6] = {G[0], G[1], G[2], S[0], S[1], S[2]};
+        float suf[6];
+        const float v[6] = {G[0], G[1], G[2], S[0], S[1], S[2]};
         for (int i = 0; i < 6; i++) {
-            T inc = v[i];
+            float inc = v[i];
             for (int off = 1; off < 32; off <<= 1) {
-                T o = __shfl_down_sync(0xffffffffu, inc, off);
+                float o = __shfl_down_sync(0xffffffffu, inc, off);
                 if (lane + off < 32) inc += o;
             }
-            T tot = __shfl_sync(0xffffffffu, inc, 0);
+            float tot = __shfl_sync(0xffffffffu, inc, 0);
             suf[i] = inc - v[i];
             if (lane == 0) s_wsum[w][i] = tot;
         }
@@ -853,7 +849,7 @@ __global__ void __launch_bounds__(NT) a2c_bwd_kernel(A2cArgs<T> a, int renorm, i
             double tot[6] = {0, 0, 0, 0, 0, 0};
             for (int ww = NW - 1; ww >= 0; ww--)
                 for (int i = 0; i < 6; i++) {
-                    s_wsuf[ww][i] = (T)run[i];
+                    s_wsuf[ww][i] = (float)run[i];
                     run[i] += (double)s_wsum[ww][i];
                     tot[i] += (double)s_wsum[ww][i];
                 }
@@ -865,25 +861,25 @@ __global__ void __launch_bounds__(NT) a2c_bwd_kernel(A2cArgs<T> a, int renorm, i
             }
         }
         __syncthreads();
-        T Gn[3], Sn[3];
+        float Gn[3], Sn[3];
         for (int c = 0; c < 3; c++) {
             Gn[c] = suf[c] + s_wsuf[w][c];
             Sn[c] = suf[3 + c] + s_wsuf[w][3 + c];
         }
-        T(*s_gr)[TILE] = sm.f.ang;  // angles of this tile stay in registers (ts) / are re-read below
+        float(*s_gr)[TILE] = sm.f.ang;  // angles of this tile stay in registers (ts) / are re-read below
 #pragma unroll
         for (int r = R - 1; r >= 0; r--) {
             const int j = tid * R + r;
             if (j >= n) continue;
             const int ty = sm.f.type[j];
             const int na = tp.natoms[ty], nj = tp.njoints[ty];
-            const T *X = sm.f.xyz + 3 * roff[r];
-            const T *Gg = sm.g + 3 * roff[r];
+            const float *X = sm.f.xyz + 3 * roff[r];
+            const float *Gg = sm.g + 3 * roff[r];
             // per-group sums of this residue
-            auto acc = [&](int lo, int hi, T *gs, T *ss) {
-                for (int c = 0; c < 3; c++) gs[c] = ss[c] = T(0);
+            auto acc = [&](int lo, int hi, float *gs, float *ss) {
+                for (int c = 0; c < 3; c++) gs[c] = ss[c] = 0.f;
                 for (int q = lo; q < hi; q++) {
-                    T xg[3];
+                    float xg[3];
                     cross3(X + 3 * q, Gg + 3 * q, xg);
                     for (int c = 0; c < 3; c++) {
                         gs[c] += Gg[3 * q + c];
@@ -891,51 +887,51 @@ __global__ void __launch_bounds__(NT) a2c_bwd_kernel(A2cArgs<T> a, int renorm, i
                     }
                 }
             };
-            T Gco[3], Sco[3], Gmid[3], Smid[3], Gn0[3], Sn0[3];
+            float Gco[3], Sco[3], Gmid[3], Smid[3], Gn0[3], Sn0[3];
             acc(na - 2, na, Gco, Sco);
             acc(1, na - 2, Gmid, Smid);   // CA, Pro ring / side chain
             acc(0, 1, Gn0, Sn0);          // N
             // frames of the residue
-            Frame<T> F = start[r];
+            Frame<float> F = start[r];
             apply_joint(F, tp.bb_cb[0], tp.bb_sb[0], tp.bb_d[0], ts.cs[r][0], ts.sn[r][0]);
-            Frame<T> C = F;
+            Frame<float> C = F;
             apply_joint(C, tp.bb_cb[1], tp.bb_sb[1], tp.bb_d[1], ts.cs[r][1], ts.sn[r][1]);
-            Frame<T> Nn = C;
+            Frame<float> Nn = C;
             apply_joint(Nn, tp.bb_cb[2], tp.bb_sb[2], tp.bb_d[2], ts.cs[r][2], ts.sn[r][2]);
-            T tmp[3], cr[3];
-            auto gradient = [&](const Frame<T> &J, const T *Gs, const T *Ss) {
+            float tmp[3], cr[3];
+            auto gradient = [&](const Frame<float> &J, const float *Gs, const float *Ss) {
                 cross3(J.p, Gs, cr);
                 for (int c = 0; c < 3; c++) tmp[c] = Ss[c] - cr[c];
                 return J.r[0] * tmp[0] + J.r[3] * tmp[1] + J.r[6] * tmp[2];
             };
             const bool last = (s0 + j == len - 1);
-            const T g_om = last ? T(0) : gradient(Nn, Gn, Sn);
-            T Gc[3], Sc[3];
+            const float g_om = last ? 0.f : gradient(Nn, Gn, Sn);
+            float Gc[3], Sc[3];
             for (int c = 0; c < 3; c++) {
                 Gc[c] = Gn[c] + Gco[c];
                 Sc[c] = Sn[c] + Sco[c];
             }
-            const T g_ps = gradient(C, Gc, Sc);
+            const float g_ps = gradient(C, Gc, Sc);
             for (int c = 0; c < 3; c++) {
                 Gc[c] += Gmid[c];
                 Sc[c] += Smid[c];
             }
-            const T g_ph = gradient(F, Gc, Sc);
+            const float g_ph = gradient(F, Gc, Sc);
             // side-chain joints: subtree of joint k = its group and all later groups
-            T g_chi[5] = {0, 0, 0, 0, 0};
+            float g_chi[5] = {0, 0, 0, 0, 0};
             if (nj > 0) {
-                T Gsc[3], Ssc[3];
+                float Gsc[3], Ssc[3];
                 acc(2, na - 2, Gsc, Ssc);
-                Frame<T> Sf = F;
+                Frame<float> Sf = F;
                 apply_rx(Sf, tp.dummy_c, tp.dummy_s);
                 for (int k = 0; k < nj; k++) {
                     const int chi = tp.jchi[ty][k];
-                    T c = T(1), s = T(0);
+                    float c = 1.f, s = 0.f;
                     if (chi >= 0) sc(sm.f.ang[3 + chi][j], &s, &c);
                     apply_joint(Sf, tp.jcb[ty][k], tp.jsb[ty][k], tp.jd[ty][k], c, s);
                     if (chi >= 0) g_chi[chi] = gradient(Sf, Gsc, Ssc);
                     const int f0 = 2 + tp.jfirst[ty][k];
-                    T Gk[3], Sk[3];
+                    float Gk[3], Sk[3];
                     acc(f0, f0 + tp.jna[ty][k], Gk, Sk);
                     for (int q = 0; q < 3; q++) {
                         Gsc[q] -= Gk[q];
@@ -968,7 +964,7 @@ __global__ void __launch_bounds__(NT) a2c_bwd_kernel(A2cArgs<T> a, int renorm, i
     // zeros past the chain (and everywhere when the chain was rejected)
     const int from = ok ? len : 0;
     for (int k = 0; k < 8; k++)
-        for (int i = from + tid; i < a.L; i += NT) gout[(size_t)k * a.L + i] = T(0);
+        for (int i = from + tid; i < a.L; i += NT) gout[(size_t)k * a.L + i] = 0.f;
 }
 
 // ------------------------------------------------- backward from the coordinates
@@ -1292,27 +1288,27 @@ __global__ void __launch_bounds__(32 * NW) a2c_bwd_coords_ring_kernel(A2cArgs<fl
 }
 
 // ------------------------------------------------------------------ host side
-template <typename T, int R, int NT>
-static int launch_a2c_fwd(const A2cArgs<T> &a, int B, int renorm, cudaStream_t st) {
+template <int R, int NT>
+static int launch_a2c_fwd(const A2cArgs<float> &a, int B, int renorm, cudaStream_t st) {
     constexpr int TILE = R * NT;
-    const size_t smem = sizeof(A2cSmemFwd<T, TILE>);
-    auto k = a2c_fwd_kernel<T, R, NT>;
+    const size_t smem = sizeof(A2cSmemFwd<TILE>);
+    auto k = a2c_fwd_kernel<R, NT>;
     if (!set_max_dynamic_smem(reinterpret_cast<const void *>(k), (int)smem))
         return TPL_ERR_LAUNCH;
     k<<<B, NT, smem, st>>>(a, renorm);
     return cudaGetLastError() == cudaSuccess ? TPL_OK : TPL_ERR_LAUNCH;
 }
 
-template <typename T, int R, int NT>
-static int launch_a2c_bwd(const A2cArgs<T> &a, int B, int renorm, cudaStream_t st) {
+template <int R, int NT>
+static int launch_a2c_bwd(const A2cArgs<float> &a, int B, int renorm, cudaStream_t st) {
     constexpr int TILE = R * NT;
     const int max_tiles = (a.L + TILE - 1) / TILE + 1;
-    const size_t smem = sizeof(A2cSmemBwd<T, TILE>) + (sizeof(Frame<T>) + sizeof(int)) * max_tiles;
+    const size_t smem = sizeof(A2cSmemBwd<TILE>) + (sizeof(Frame<float>) + sizeof(int)) * max_tiles;
     int dev = 0, optin = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
     if ((int)smem > optin) return TPL_ERR_UNSUPPORTED;
-    auto k = a2c_bwd_kernel<T, R, NT>;
+    auto k = a2c_bwd_kernel<R, NT>;
     if (!set_max_dynamic_smem(reinterpret_cast<const void *>(k), (int)smem))
         return TPL_ERR_LAUNCH;
     k<<<B, NT, smem, st>>>(a, renorm, max_tiles);
@@ -1384,9 +1380,9 @@ int a2c_forward(bool f64, const unsigned char *seq, int seq_stride, const void *
     switch (opt.threads_per_cta) {
         case 4: return launch_a2c_fwd_ring<4>(a, B, renorm, st);
         case 8: return launch_a2c_fwd_ring<8>(a, B, renorm, st);
-        case 128: return launch_a2c_fwd<float, 2, 128>(a, B, renorm, st);
-        case 256: return launch_a2c_fwd<float, 1, 256>(a, B, renorm, st);
-        case 512: return launch_a2c_fwd<float, 1, 512>(a, B, renorm, st);
+        case 128: return launch_a2c_fwd<2, 128>(a, B, renorm, st);
+        case 256: return launch_a2c_fwd<1, 256>(a, B, renorm, st);
+        case 512: return launch_a2c_fwd<1, 512>(a, B, renorm, st);
     }
     return a2c_ring_warps(B, 8) == 8 ? launch_a2c_fwd_ring<8>(a, B, renorm, st)
                                                                     : launch_a2c_fwd_ring<4>(a, B, renorm, st);
@@ -1404,10 +1400,10 @@ int a2c_backward(bool f64, void *grad_angles, const void *grad_coords, const uns
     A2cArgs<float> a{seq, seq_stride, (const float *)angles, nullptr, nullptr, nullptr, (float *)grad_angles,
                      (const float *)grad_coords, (WsHeader *)ws, L, maxA};
     switch (opt.threads_per_cta) {
-        case 128: return launch_a2c_bwd<float, 2, 128>(a, B, renorm, st);
-        case 512: return launch_a2c_bwd<float, 1, 512>(a, B, renorm, st);
+        case 128: return launch_a2c_bwd<2, 128>(a, B, renorm, st);
+        case 512: return launch_a2c_bwd<1, 512>(a, B, renorm, st);
     }
-    return launch_a2c_bwd<float, 1, 256>(a, B, renorm, st);
+    return launch_a2c_bwd<1, 256>(a, B, renorm, st);
 }
 
 int a2c_backward_coords(float *grad_angles, const float *grad_coords, const float *coords, const unsigned char *seq,

@@ -157,9 +157,6 @@ __device__ __forceinline__ void frame_load(Frame<T> &f, const S *src) {
     for (int i = 0; i < 3; i++) f.p[i] = T(src[9 + i]);
 }
 
-__device__ __forceinline__ void sincos_t(float a, float *s, float *c) { sincosf(a, s, c); }
-__device__ __forceinline__ void sincos_t(double a, double *s, double *c) { sincos(a, s, c); }
-
 __device__ __forceinline__ void cross3(const float *a, const float *b, float *o) {
     o[0] = fmaf(a[1], b[2], -a[2] * b[1]);
     o[1] = fmaf(a[2], b[0], -a[0] * b[2]);

@@ -49,13 +49,10 @@ struct RmsdArgs {
 
 constexpr int kRmsdWarps = kRmsdThreads / 32;
 
-// Block sums of NV per-thread values: in the coordinate type within each warp, then
-// in FP64 across the warps on one lane per value, so that the FP64 work is NV x
-// warps additions rather than a shuffle tree per value on every thread (GB300's
-// FP64 rate is a small fraction of its FP32 rate).  Every thread returns with the
-// sums in s_out.
-template <typename T, int NV>
-__device__ __forceinline__ void block_sums(T (&v)[NV], double *s_red, double *s_out) {
+// Block sums of NV per-thread values (the float64 forward): a shuffle tree within each warp,
+// then across the warps on one lane per value.  Every thread returns with the sums in s_out.
+template <int NV>
+__device__ __forceinline__ void block_sums(double (&v)[NV], double *s_red, double *s_out) {
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
 #pragma unroll
     for (int off = 16; off > 0; off >>= 1)
@@ -63,7 +60,7 @@ __device__ __forceinline__ void block_sums(T (&v)[NV], double *s_red, double *s_
         for (int k = 0; k < NV; k++) v[k] += __shfl_xor_sync(0xffffffffu, v[k], off);
     if (lane == 0)
 #pragma unroll
-        for (int k = 0; k < NV; k++) s_red[w * NV + k] = (double)v[k];
+        for (int k = 0; k < NV; k++) s_red[w * NV + k] = v[k];
     __syncthreads();
     if (threadIdx.x < NV) {
         double r = 0.0;
@@ -576,7 +573,7 @@ __global__ void __launch_bounds__(kRmsdThreads) rmsd_fwd_f64_kernel(RmsdArgs<dou
                 sx[k] += x[3 * i + k];
                 sx[3 + k] += y[3 * i + k];
             }
-        block_sums<double, 6>(sx, s_red, s_out);
+        block_sums<6>(sx, s_red, s_out);
         if (tid < 6) s_c[tid] = n > 0 ? s_out[tid] / n : 0.0;
     } else if (tid < 6) {
         s_c[tid] = 0.0;
@@ -596,7 +593,7 @@ __global__ void __launch_bounds__(kRmsdThreads) rmsd_fwd_f64_kernel(RmsdArgs<dou
             for (int q = 0; q < 3; q++) acc[3 * p + q] = fma(xi[p], yi[q], acc[3 * p + q]);
         acc[9] += xi[0] * xi[0] + xi[1] * xi[1] + xi[2] * xi[2] + yi[0] * yi[0] + yi[1] * yi[1] + yi[2] * yi[2];
     }
-    block_sums<double, 10>(acc, s_red, s_out);
+    block_sums<10>(acc, s_red, s_out);
     if (tid >= 32) return;
     const double r2 = s_out[9];
     double scale, inv;
