@@ -983,3 +983,29 @@ def test_rows_off_16_byte_boundaries_take_four_residues_a_lane(rm, B, L, off):
         if off:
             (rpt, cta), _ = autotune.options_for(view.device, B, L)
             assert torch.equal(Angles2Backbone()(view.clone(), lens), forward(view.clone(), rpt, cta))
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float64])
+@pytest.mark.parametrize("B,L", [(5, 70), (40, 1000), (700, 40), (3, 2500)])
+@pytest.mark.parametrize("value", [float("nan"), float("inf")])
+def test_undefined_angles_that_move_no_atom(rm, dtype, B, L, value):
+    """psi and omega of a chain's last residue move no atom, and what lies past the chain is
+    padding: NaN or infinite there (dihedrals that do not exist), the layer's coordinates and
+    gradients equal those with zeros there, bit for bit.  Chains that end on either residue of
+    a lane, and on the first and last lane of a chunk."""
+    from torchproteinlibrary_gb300.ReducedModel import Angles2Backbone
+    g = torch.Generator("cuda").manual_seed(L)
+    a = (torch.rand(B, 3, L, dtype=dtype, device="cuda", generator=g) * 2 - 1) * 3.1
+    n = torch.randint(1, L + 1, (B,), device="cuda", generator=g, dtype=torch.int32)
+    n[:5] = torch.tensor([1, 32, 33, min(L, 64), L], device="cuda", dtype=torch.int32)[:B]
+    at = torch.arange(L, device="cuda")
+    past = at[None, None] >= n[:, None, None] - torch.tensor([0, 1, 1], device="cuda")[None, :, None]
+    up = torch.randn(B, 9 * L, dtype=dtype, device="cuda", generator=g)
+    results = []
+    for fill in (0.0, value):
+        x = torch.where(past, torch.full_like(a, fill), a).requires_grad_()
+        coords = Angles2Backbone()(x, n)
+        grad, = torch.autograd.grad(coords, x, up)
+        results.append([coords.detach(), grad])
+    for zero, filled in zip(*results):
+        assert torch.equal(zero, filled) and torch.isfinite(zero).all()

@@ -487,7 +487,9 @@ __global__ void __launch_bounds__(32 * NW, 4) a2b_bwd_f64_kernel(BackboneArgs a)
                         for (int i = 0; i < 3; i++) pos[r][3 * k + i] = y[i];
                         add_moment(y, g, v6, v6 + 3);
                     }
-            move_origin(P, v6, v6 + 3);  // about the pass start
+            // about the pass start; a lane past the chain has nothing, and its P may be NaN (psi
+            // of the last residue moves no atom, but the frame after it)
+            if (j0 < len) move_origin(P, v6, v6 + 3);
             suffix_excl(v6, ch.lane, suf, tot);
         }
         ch.publish_sums(tot);
