@@ -664,3 +664,41 @@ def test_float64_nan_side_chain_angle(fm, chi):
             assert np.isfinite(gi[b, :, 3:]).all()
         else:
             assert np.isfinite(gi[b]).all()
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float64])
+def test_angles_without_a_joint_get_zero_beside_nan(built, dtype):
+    """Chi angles that a residue does not have, Ala's fixed one and omega of the last residue get a
+    zero gradient also where the chain's positions or dL/dx are NaN: a NaN in one atom's dL/dx,
+    and a NaN phi, which makes every later position NaN."""
+    from torchproteinlibrary_gb300.FullAtomModel import Angles2Coords
+    seqs = [AA * 3, "GKASPWGRLV" * 5]
+    rng = np.random.default_rng(3)
+    ang = torch.tensor(rng.uniform(-3, 3, (2, 8, 60)), dtype=dtype, device="cuda")
+    layer = Angles2Coords()
+    up = torch.ones_like(layer(ang, seqs)[0])
+
+    def gradient(x, u):
+        x = x.clone().requires_grad_()
+        return torch.autograd.grad(layer(x, seqs)[0], x, u)[0]
+
+    absent = torch.ones(2, 8, 60, dtype=torch.bool)
+    for b, seq in enumerate(seqs):
+        absent[b, :3, :len(seq)] = False
+        absent[b, 2, len(seq) - 1] = True
+    for letter in AA:  # a joint shows in the oracle's coordinates when its angle is NaN
+        for chi in range(3, 8):
+            one = np.zeros((1, 8, 1))
+            one[0, chi] = np.nan
+            if np.isnan(oracle.a2c_forward(one, [letter])[0]).any():
+                for b, seq in enumerate(seqs):
+                    absent[b, chi, [j for j, c in enumerate(seq) if c == letter]] = False
+    absent = absent.cuda()
+    assert (gradient(ang, up)[absent] == 0).all()
+    bad_up, bad_ang = up.clone(), ang.clone()
+    bad_up[:, 3 * 200] = float("nan")
+    bad_ang[:, 0, 21] = float("nan")
+    for x, u in ((ang, bad_up), (bad_ang, up)):
+        g = gradient(x, u)
+        assert torch.isnan(g[:, 0, :20]).all()
+        assert (g[absent] == 0).all()

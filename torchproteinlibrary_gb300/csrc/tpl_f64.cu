@@ -821,12 +821,14 @@ __global__ void __launch_bounds__(32 * NW) a2c_bwd_f64_kernel(A2cArgs<double> a,
             apply_rx(S, g_topo.dummy_c, g_topo.dummy_s);
             const int nj = g_topo.njoints[ty];
             double ju[5][3], jm[5][3];
+            int turning = 0;  // joints that a chi angle turns: the first ones, or none
 #pragma unroll
             for (int k = 0; k < kMaxScJoints; k++) {
 #pragma unroll
                 for (int i = 0; i < 3; i++) ju[k][i] = jm[k][i] = 0.0;
                 if (k >= nj) continue;
                 const bool fixed = g_topo.jchi[ty][k] < 0;
+                if (!fixed) turning = k + 1;
                 apply_joint(S, g_topo.jcb[ty][k], g_topo.jsb[ty][k], g_topo.jd[ty][k], fixed ? 1.0 : q.cs[3 + k],
                             fixed ? 0.0 : q.sn[3 + k]);
                 if (!fixed) {
@@ -848,8 +850,9 @@ __global__ void __launch_bounds__(32 * NW) a2c_bwd_f64_kernel(A2cArgs<double> a,
             }
 #pragma unroll
             for (int k = 0; k < kMaxScJoints; k++)  // u . (S - o x G) = u . S - (u x o) . G
+                if (k < turning)                    // an angle without a joint gets 0, whatever the sums
 #pragma unroll
-                for (int i = 0; i < 3; i++) chi[k] += fma(ju[k][i], Ssc[i], -jm[k][i] * Gsc[i]);
+                    for (int i = 0; i < 3; i++) chi[k] += fma(ju[k][i], Ssc[i], -jm[k][i] * Gsc[i]);
             backbone_joint<1>(X, q.cs[1], q.sn[1]);
             joint(X, 1);
             take(na - 2, X.p, Gco, Sco);
@@ -866,7 +869,7 @@ __global__ void __launch_bounds__(32 * NW) a2c_bwd_f64_kernel(A2cArgs<double> a,
         }
         double suf[6] = {0, 0, 0, 0, 0, 0}, tot[6] = {0, 0, 0, 0, 0, 0}, after, whole;
         if (c0 < len) {
-            move_origin(P, v6, v6 + 3);  // about the pass start
+            if (j < len) move_origin(P, v6, v6 + 3);  // about the pass start
             suffix_excl(v6, ch.lane, suf, tot);
         }
         ch.publish_sums(tot);
