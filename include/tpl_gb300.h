@@ -177,9 +177,8 @@ size_t tpl_a2c_workspace_bytes(int batch, int max_len, int max_atoms, const tpl_
  * reported through the workspace status; such chains are zeroed.  One CTA walks a
  * chain (float32): opt->threads_per_cta 4 or 8 = four or eight warps on chunks of 32
  * residues, one per lane; 256 or 512 threads with one residue each; 128 threads with
- * two residues each; 0 (the default) = eight warps below 8 x (number of SMs) chains
- * (4 x with names), four from there.  float64 always uses 128 threads with one
- * residue each. */
+ * two residues each; 0 (the default) = eight warps up to 8 x (number of SMs) chains,
+ * four past that.  float64 always takes one thread-block cluster per chain. */
 int tpl_a2c_forward_f32(const uint8_t *sequences, int seq_stride, const float *angles, float *coords,
                         uint8_t *res_names, uint8_t *atom_names, void *workspace, size_t workspace_bytes, int batch,
                         int max_len, int max_atoms, const tpl_options *opt, void *stream);

@@ -6,7 +6,8 @@ the scan scheme (warp tiles, CTA tiles, one warp or one CTA per chain), the leng
 which inter-tile carries are composed in FP64, and the residues per lane of the
 backward from coordinates.  For a shape
 (batch, max_len) the tuner times forward+backward of every candidate on
-synthetic chains of that shape with CUDA events and keeps the fastest whose
+synthetic chains of that shape with CUDA events, the calls queued behind a wait on the
+device, and keeps the fastest whose
 coordinates stay within the accuracy bound of the FP64 form.  Results are
 cached per GPU name and shape bucket in a JSON file
 ($TPL_TUNE_CACHE, default ~/.cache/torchproteinlibrary_gb300/tune.json).

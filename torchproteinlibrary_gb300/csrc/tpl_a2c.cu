@@ -1375,8 +1375,8 @@ int a2c_forward(bool f64, const unsigned char *seq, int seq_stride, const void *
     }
     A2cArgs<float> a{seq, seq_stride, (const float *)angles, (float *)coords, res_names, atom_names,
                      nullptr, nullptr, (WsHeader *)ws, L, maxA};
-    // threads_per_cta: 128 = 128 threads x 2 residues; 0 / 256 (default) or 512 = one
-    // residue per thread
+    // threads_per_cta: 4 or 8 = that many warps on chunks of 32 residues (0: by the batch);
+    // 128 = 128 threads x 2 residues; 256 or 512 = one residue per thread
     switch (opt.threads_per_cta) {
         case 4: return launch_a2c_fwd_ring<4>(a, B, renorm, st);
         case 8: return launch_a2c_fwd_ring<8>(a, B, renorm, st);
@@ -1385,7 +1385,7 @@ int a2c_forward(bool f64, const unsigned char *seq, int seq_stride, const void *
         case 512: return launch_a2c_fwd<1, 512>(a, B, renorm, st);
     }
     return a2c_ring_warps(B, 8) == 8 ? launch_a2c_fwd_ring<8>(a, B, renorm, st)
-                                                                    : launch_a2c_fwd_ring<4>(a, B, renorm, st);
+                                     : launch_a2c_fwd_ring<4>(a, B, renorm, st);
 }
 
 int a2c_backward(bool f64, void *grad_angles, const void *grad_coords, const unsigned char *seq, int seq_stride,

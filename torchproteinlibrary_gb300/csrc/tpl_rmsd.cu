@@ -6,8 +6,9 @@
 // Python loop of .item() calls (TorchProteinLibrary/RMSD/Coords2RMSD/Coords2RMSD.py:40-62).
 //
 // Here one CTA per chain does everything in one launch: optional centring, the
-// correlation R_ab = sum x_a y_b and R2 = sum |x|^2 + |y|^2 (sums in the coordinate
-// type per thread and per warp, in FP64 across the warps), the 4x4 matrix T (same
+// correlation R_ab = sum x_a y_b and R2 = sum |x|^2 + |y|^2 (float32: FP32 per thread and
+// over four or eight lanes, two-float sums from there, FP64 from the moments on; float64:
+// FP64 throughout), the 4x4 matrix T (same
 // layout as the reference), its largest eigenpair by the characteristic-polynomial
 // method on one warp (key_eigen_halves), U from the unit quaternion, UT = U^T and
 // rmsd = sqrt((R2 - 2 |lambda_max| + 1e-10) / N).  The backward is one launch with

@@ -61,6 +61,8 @@ struct ShiftArgs {
     int scale_by_count;
 };
 
+// Whether the addend is divided by the count is a template parameter in float64 alone, where the
+// division's instructions cost the calls without one; float32 has one kernel for both.
 template <typename T, bool VEC, bool SCALE>
 __global__ void __launch_bounds__(256) shift_kernel(ShiftArgs a) {
     constexpr int N = VEC ? Vec16<T>::n : 1;
@@ -109,10 +111,10 @@ __global__ void __launch_bounds__(256) shift_kernel(ShiftArgs a) {
     }
 }
 
-// Eight blocks per SM in float32: short rows leave most of a block idle (16000 rows of 20
-// atoms, 38 registers: 17 -> 20 us).
 // The same for rows that start anywhere: vectors between the row's first and last 16-byte
 // boundary where `in` and `out` have the same phase, the elements outside them by themselves.
+// Eight blocks per SM in float32: short rows leave most of a block idle (16000 rows of 20
+// atoms: 17 us, at 38 registers 20).
 template <typename T, bool SCALE>
 __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 8 : 6) shift_rows_kernel(ShiftArgs a) {
     constexpr int N = Vec16<T>::n;
@@ -217,8 +219,8 @@ __global__ void __launch_bounds__(256) rotate_kernel(const T *in, T *out, const 
 // its arithmetic, 4096 of 3471 226 / 236).
 // Grid: y over rows (strided), x over pieces of 512 aligned groups of N atoms
 // (tpl_rows.cuh), two tiles of 32 groups per warp whose loads are in flight together (one
-// tile: 54 us; the launch is then bound by the latency of its many short blocks).  A warp loads and stores its tile as 96 vectors in
-// memory order and turns it to one group per lane and back through shared memory: with a
+// tile: 54 us; the launch is then bound by the latency of its many short blocks).  A warp
+// loads and stores its tile as 96 vectors in memory order and turns it to one group per lane and back through shared memory: with a
 // group per lane straight from memory every 32-byte sector is written in two pieces
 // (strides of 48 bytes), with an atom per lane in three.  48-byte lane strides are free of
 // bank conflicts.  Atoms outside the groups, and rows whose input and output differ in
