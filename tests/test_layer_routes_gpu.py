@@ -138,3 +138,14 @@ def test_captured_backbone_step_fills_only_what_is_read(built, monkeypatch, B, L
                 assert (t.detach() - w).abs().max() <= 1e-4 * w.abs().max()
             else:
                 assert torch.equal(t.detach(), w)
+
+
+def test_backbone_names_functorch_in_its_refusal(built):
+    """float32 Angles2Backbone does not run under functorch transforms, and says so."""
+    from torchproteinlibrary_gb300.ReducedModel import Angles2Backbone
+    layer, n = Angles2Backbone(), torch.tensor([8, 5], dtype=torch.int32, device="cuda")
+    angles = torch.randn(2, 3, 8, device="cuda")
+    with pytest.raises(RuntimeError, match="functorch"):
+        torch.func.grad(lambda a: layer(a, n).sum())(angles)
+    with pytest.raises(RuntimeError, match="functorch"):
+        torch.func.vmap(lambda a: layer(a, n))(torch.stack([angles, angles]))

@@ -156,9 +156,11 @@ class Angles2Backbone(Module):
         # frame in the backward
         batch_size, _, max_len = input.shape
         dev = input.device
-        # (angles that are not contiguous are copied to an allocation of their own)
+        # (angles that are not contiguous are copied to an allocation of their own; a functorch
+        # transform's have no address, and are refused below)
         tuned = autotune.options_for(dev, batch_size, max_len,
-                                     not input.is_contiguous() or input.data_ptr() % 16 == 0)
+                                     not input.is_contiguous() or torch._C._are_functorch_transforms_active()
+                                     or input.data_ptr() % 16 == 0)
         fwd_opts, bwd_opts = tuned if tuned is not None else ((-1, -1), (-1, -1, -1))
         ws = _shared_workspace(batch_size, max_len, dev, fwd_opts, private=True)
         return _ReducedModel.angles2backbone_autograd(input, angles_length, ws, list(fwd_opts), list(bwd_opts))
